@@ -272,7 +272,13 @@ static int threshold_frames_mixed(const T *const *d_images, size_t n, const size
     return SF_OK;
   }
   unsigned char *ws = static_cast<unsigned char *>(d_ws);
-  if (streamed) {
+  const bool dispersion = dispersion_path(P, (int)sizeof(T));
+  // The dispersion path keeps results between its passes where the workspace
+  // has every frame's; a workspace for one frame is enough for it without.
+  const WorkspaceLayout Ln =
+      dispersion ? layout(h, w, capacity, n) : L;
+  const bool all = ws_bytes >= Ln.total;
+  if (streamed || dispersion) {
     FramePtrs F;
     for (size_t j = 0; j < n; j++) {
       F.image[j] = reinterpret_cast<const uint32_t *>(d_images[j]);
@@ -286,11 +292,11 @@ static int threshold_frames_mixed(const T *const *d_images, size_t n, const size
     b.amb = reinterpret_cast<uint32_t *>(ws + L.amb);
     b.prefix = d_word_prefix;
     b.cand = reinterpret_cast<uint32_t *>(ws + L.cand);
-    b.res = reinterpret_cast<uint2 *>(ws + L.res);
-    b.cand_cap = (uint32_t)L.cand_cap;
+    b.res = reinterpret_cast<uint2 *>(ws + (all ? Ln.res : L.res));
+    b.cand_cap = all ? (uint32_t)L.cand_cap : 0u;
     b.counters = reinterpret_cast<uint32_t *>(ws + L.counters);
     b.wide = reinterpret_cast<uint4 *>(ws + L.wide);
-    b.block_sums = reinterpret_cast<uint32_t *>(ws + L.block_sums);
+    b.block_sums = reinterpret_cast<uint32_t *>(ws + (all ? Ln.block_sums : L.block_sums));
     b.capacity = (uint32_t)capacity;
     b.out = d_out;
     b.out_stride = capacity;
@@ -298,7 +304,8 @@ static int threshold_frames_mixed(const T *const *d_images, size_t n, const size
     const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
     t_marks.staged = true;
     cudaError_t e =
-        streamed16 ? launch_stream16(F, (int)n, (int)h, (int)w, P, b, run_rows, stream, marks)
+        dispersion ? launch_dispersion(F, (int)n, (int)sizeof(T), P, b, run_rows, stream, marks)
+        : streamed16 ? launch_stream16(F, (int)n, (int)h, (int)w, P, b, run_rows, stream, marks)
                    : launch_stream(F, (int)n, (int)h, (int)w, P, b, run_rows, stream, marks);
     if (e != cudaSuccess)
       return fail(e, "launching the threshold");

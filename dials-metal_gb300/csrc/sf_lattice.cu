@@ -49,6 +49,7 @@
 
 #include "sf_common.cuh"
 #include "sf_stream.cuh"
+#include "sf_strips.cuh"
 #include "sf_tma.cuh"
 
 namespace sf {
@@ -68,60 +69,10 @@ constexpr int kDec = 8;                     // fixed-point bits of clo / chi
 
 static_assert(kLatOut % 24 == 0, "lane pairs write whole bytes");
 
-// Division of 32-bit numerators by a divisor fixed for a launch (tile
-// counts), by one multiply-high and shifts: the round-up method of
-// Granlund & Montgomery, "Division by invariant integers using
-// multiplication" (PLDI 1994), with its add-and-shift step for multipliers of
-// 33 bits. Exact for every numerator and divisor below 2^32.
-struct FastDiv {
-  uint32_t d, m, s1, s2;
-};
-
 // Marks a tile of stage 2's list whose candidates all failed the exact check.
 constexpr uint32_t kNoTile = 0xFFFFFFFFu;
 
-FastDiv make_fastdiv(uint32_t d) {
-  int l = 0;
-  while ((1ull << l) < d)
-    l++;
-  FastDiv f;
-  f.d = d;
-  f.m = (uint32_t)(((((unsigned long long)1 << l) - d) << 32) / d + 1);
-  f.s1 = l < 1 ? (uint32_t)l : 1u;
-  f.s2 = l > 1 ? (uint32_t)(l - 1) : 0u;
-  return f;
-}
-
-__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv &f) {
-  const uint32_t t = __umulhi(n, f.m);
-  return (t + ((n - t) >> f.s1)) >> f.s2;
-}
-
-
 static_assert(kLatN0 * kLatCap < (1u << kLatPS), "saturated sums stay below the count field");
-
-// Where each frame's share of a launch's warps (lat_stage01: strips x runs)
-// or tile groups (lat_tiles: tile rows x groups of 32 tiles) starts, and how
-// many make one of its rows: every frame of a batch, mixed shapes or not,
-// gets exactly its own.
-struct FrameSpans {
-  int start[kMaxBatch + 1];
-  FastDiv by_row[kMaxBatch];
-};
-
-// The frame whose span holds item g (start[f] <= g < start[f + 1]); g below
-// start[nframes].
-__device__ __forceinline__ int span_frame(const FrameSpans &S, int nframes, int g) {
-  int lo = 0, hi = nframes;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (S.start[mid] <= g)
-      lo = mid;
-    else
-      hi = mid;
-  }
-  return lo;
-}
 
 // The 12 bound bits of a lane from the lattice bits b0-b4 at its columns
 // -1, 2, 5, 8 and 11 (b0 is the lane before's column 11): column c keeps the
@@ -207,38 +158,6 @@ __device__ __forceinline__ void lat_row(const uint32_t v[kLatCols], int lane, ui
   for (int c = 0; c < kLatCols; c++)
     m += k16 ? (ns[c] >> kLatPS) << c : ns[c] >> (kLatPS - c);
   *m12 = m;
-}
-
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-// One piece of 4 pixels: 16 bytes of a 32-bit frame, 8 of a 16-bit one.
-template <typename Pix> __device__ __forceinline__ void cp_async_piece(void *dst, const void *src) {
-  if (sizeof(Pix) == 4)
-    cp_async16(dst, src);
-  else
-    cp_async8(dst, src);
-}
-template <typename Pix> __device__ __forceinline__ void fill_piece_masked(void *dst) {
-  if (sizeof(Pix) == 4)
-    *reinterpret_cast<uint4 *>(dst) = make_uint4(~0u, ~0u, ~0u, ~0u);
-  else
-    *reinterpret_cast<uint2 *>(dst) = make_uint2(~0u, ~0u);
-}
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 // The ring variant (kRing: 4 | width and 16-byte aligned frames) stages each

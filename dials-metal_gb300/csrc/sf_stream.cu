@@ -30,6 +30,7 @@
 #include <mutex>
 
 #include "sf_common.cuh"
+#include "sf_order.cuh"
 #include "sf_scan.cuh"
 #include "sf_stream.cuh"
 
@@ -570,45 +571,6 @@ amb_fix(const __grid_constant__ FramePtrs F, int height, int width,
 // the first pass wrote it), ascending, from two scans over the mask words.
 // Every kernel below runs on a (block, frame) grid.
 // ---------------------------------------------------------------------------
-constexpr int kScanT = 256;                    // threads of a scan block
-constexpr int kScanPer = 8;                    // consecutive items per thread
-constexpr int kScanChunk = kScanT * kScanPer;  // items per block pass
-
-// This block's share [lo, hi) of a frame's n items, in whole passes.
-__device__ __forceinline__ void chunk_of(size_t n, size_t *lo, size_t *hi) {
-  size_t chunk = (n + gridDim.x - 1) / gridDim.x;
-  chunk = (chunk + kScanChunk - 1) / kScanChunk * kScanChunk;
-  *lo = min(n, (size_t)blockIdx.x * chunk);
-  *hi = min(n, *lo + chunk);
-}
-
-// Sum of the block's predecessors' counts in its frame, and the frame's
-// total.
-__device__ __forceinline__ uint32_t block_base(const uint32_t *__restrict__ block_sums,
-                                               uint32_t *total) {
-  __shared__ uint32_t s_base, s_total;
-  if (threadIdx.x < 32) {
-    const uint32_t *bs = block_sums + (size_t)blockIdx.y * gridDim.x;
-    uint32_t b = 0, t = 0;
-    for (uint32_t i = threadIdx.x; i < gridDim.x; i += 32) {
-      const uint32_t v = bs[i];
-      b += i < blockIdx.x ? v : 0u;
-      t += v;
-    }
-    for (int o = 16; o; o >>= 1) {
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-      t += __shfl_xor_sync(0xffffffffu, t, o);
-    }
-    if (threadIdx.x == 0) {
-      s_base = b;
-      s_total = t;
-    }
-  }
-  __syncthreads();
-  *total = s_total;
-  return s_base;
-}
-
 // Every item of [lo, hi) with its count's exclusive prefix (offset by
 // carry): emit(i, item, position) for items that count.
 template <typename V, class Load, class Count, class Emit>
@@ -1051,7 +1013,7 @@ int device_sms() {
 // block walks its share in two passes), at least one, never more than
 // kOrderMaxBlocks over the batch.
 constexpr int kOrderMaxBlocks = 8192;
-static int order_bpf(int nframes, size_t words) {
+int order_blocks(int nframes, size_t words) {
   const long long want = (long long)((words + 2047) / 2048);
   return (int)std::max(1ll, std::min(want, (long long)(kOrderMaxBlocks / nframes)));
 }
@@ -1160,7 +1122,7 @@ static cudaError_t launch_stream_k(const FramePtrs &F, int nframes, int h, int w
   }
   if (marks)
     cudaEventRecord(marks->stage01, stream);
-  const dim3 og((unsigned)order_bpf(nframes, b.words), (unsigned)nframes);
+  const dim3 og((unsigned)order_blocks(nframes, b.words), (unsigned)nframes);
   mask_sums<<<og, kScanT, 0, stream>>>(F, b.bits, b.words, b.block_sums);
   if (K == 3) {
     // Stage 2 on the exact check's tiles, into the list positions.
@@ -1212,7 +1174,7 @@ cudaError_t launch_stream16(const FramePtrs &F, int nframes, int h, int w, const
     return e;
   if (marks)
     cudaEventRecord(marks->stage01, stream);
-  const dim3 og((unsigned)order_bpf(nframes, b.words), (unsigned)nframes);
+  const dim3 og((unsigned)order_blocks(nframes, b.words), (unsigned)nframes);
   mask_sums<<<og, kScanT, 0, stream>>>(F, b.bits, b.words, b.block_sums);
   mask_prefix<<<og, kScanT, 0, stream>>>(F, b.bits, b.words, b.block_sums, b.amb, b.counters);
   if ((e = launch_lattice_stage2(F, nframes, h, w, 1, 2, P, b, stream)) != cudaSuccess)

@@ -96,8 +96,10 @@ struct StreamBuffers {
 
 // Wide-list entries a batch may need (every run hands over at most once).
 size_t stream_wide_entries(int h, int w, int nframes);
-// Blocks of the ordering kernel (the size of block_sums).
+// Blocks of the ordering kernel (the size of block_sums), and the blocks a
+// frame that a launch takes of them.
 int stream_order_blocks();
+int order_blocks(int nframes, size_t words);
 
 void make_stream_tables(const LaunchParams &P, StreamTables *T);
 
@@ -140,6 +142,16 @@ cudaError_t launch_lattice(const FramePtrs &frames, int nframes, int h, int w, i
 cudaError_t launch_stream16(const FramePtrs &frames, int nframes, int h, int w,
                             const LaunchParams &P, const StreamBuffers &b, int run_rows,
                             cudaStream_t stream, const StreamMarks *marks = nullptr);
+
+// The plain dispersion algorithm (sf_dispersion.cu): frames of either pixel
+// type, mixed shapes too, any kernel size. Whether the parameters are ones it
+// takes (32-bit frames: no negative gain or sigma; the tile path has those),
+// and its launch, which uses b.bits, b.words, b.block_sums, the outputs and,
+// unless b.cand_cap is 0, b.res.
+bool dispersion_path(const LaunchParams &P, int pixel_bytes);
+cudaError_t launch_dispersion(const FramePtrs &frames, int nframes, int pixel_bytes,
+                              const LaunchParams &P, const StreamBuffers &b, int run_rows,
+                              cudaStream_t stream, const StreamMarks *marks = nullptr);
 
 // run_rows 0: the default geometry. marks may be null.
 cudaError_t launch_stream(const FramePtrs &frames, int nframes, int h, int w,
