@@ -122,7 +122,8 @@ __device__ __forceinline__ bool disp_maybe0(uint32_t n, uint32_t S, uint32_t Q, 
                                             uint32_t clo, const LaunchParams &P) {
   if constexpr (sizeof(Pix) == 2)
     return stage0_u16(n, S, Q, P);  // the reference's float test itself
-  return Q >= DispG<K>::Big || Q * nk > S * ((S << 4) + clo);
+  // (Bitwise: branches around the halves took the kernel from 344 to 437 us.)
+  return (Q >= DispG<K>::Big) | (Q * nk > S * ((S << 4) + clo));
 }
 template <int K, typename Pix>
 __device__ __forceinline__ bool disp_maybe2(uint32_t p, uint32_t n, uint32_t S, uint32_t kk,
@@ -138,7 +139,7 @@ __device__ __forceinline__ bool disp_maybe2(uint32_t p, uint32_t n, uint32_t S, 
   // unit in d), and d beyond 65535 passes whatever S is.
   const int d = (int)(n * p) - (int)S;
   const uint32_t e = (uint32_t)min(d, 65535);
-  return p >= DispG<K>::Cap || (d > 0 && e * e + e >= S * kk);
+  return (p >= DispG<K>::Cap) | ((d > 0) & (e * e + e >= S * kk));
 }
 
 // One warp walks down a strip of 360 output columns for a run of rows. Lane l
@@ -148,10 +149,10 @@ __device__ __forceinline__ bool disp_maybe2(uint32_t p, uint32_t n, uint32_t S, 
 // window: the lane adds the row to its 12 column sums as it enters, subtracts
 // it as it leaves, and reads it once more as the centre row. A window is 2K +
 // 1 column sums; the K beyond either end of a lane's columns come by shuffles.
-// Bound by issue: 55 instructions a pixel at 60% of the issue rate. 16 frames of
+// Bound by issue: 50 instructions a pixel at 70% of the issue rate. 16 frames of
 // 3262 x 3108 took 4.57 ms as 32 x 32 tiles (each pixel's window summed in
-// 64 bits from shared memory, the halo staged 2.6 times over), and take 0.54 ms
-// here: 437 us in this kernel, 70 and 30 in the two below.
+// 64 bits from shared memory, the halo staged 2.6 times over), and take 0.44 ms
+// here: 344 us in this kernel, 70 and 30 in the two below.
 template <int K, typename Pix>
 __global__ void __launch_bounds__(kDispWarps * 32, DispG<K>::Occ)
 disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,
@@ -320,7 +321,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
             W &= kDispMask;
             valid = v[c] < (1u << kDispPS);
           }
-          out2 |= valid && disp_maybe2<K, Pix>(v[c], n, W, kk, P) ? 1u << c : 0u;
+          out2 |= valid & disp_maybe2<K, Pix>(v[c], n, W, kk, P) ? 1u << c : 0u;
         }
         out &= out2;
       }
