@@ -17,7 +17,7 @@
 #include "sf_common.cuh"
 #include "sf_decompress.cuh"
 #include "sf_frames.cuh"
-#include "sf_scan.cuh"
+#include "sf_lattice.cuh"
 #include "sf_stream.cuh"
 #include "sf_threshold.cuh"
 
@@ -130,11 +130,11 @@ int make_launch_params(const sf_threshold_params *in, LaunchParams *P) {
   return SF_OK;
 }
 
-// One workspace serves both threshold paths: the streaming path (32-bit
-// frames, dispersion_extended, gain 1 and integral sigmas; one frame or a
-// batch) and the tile path (everything else, one frame at a time).
+// One workspace serves every threshold path: strips and the lattice (one frame
+// or a batch) and the tile path (one frame at a time).
 struct WorkspaceLayout {
-  size_t staging, cand, res, scr1, amb, wide, counters, block_sums, tile_base, row_total, total;
+  size_t staging, res, cand, tiles, cand_sums, counters, block_sums, tile_base,
+      row_total, total;
   size_t cand_cap, words;
 };
 
@@ -151,13 +151,15 @@ static WorkspaceLayout layout(size_t h, size_t w, size_t capacity, size_t nframe
     return at;
   };
   L.staging = take(capacity * sizeof(sf_signal_pixel));  // the tile path's, one frame
-  L.cand = take(nframes * L.cand_cap * sizeof(uint32_t));
-  L.res = take(nframes * L.cand_cap * sizeof(uint2));
-  L.scr1 = take(nframes * L.words * sizeof(uint32_t));
-  L.amb = take(nframes * (L.words + 2 * lattice_tiles((int)h, (int)w)) * sizeof(uint32_t));
-  L.wide = take(stream_wide_entries((int)h, (int)w, (int)nframes) * 2 * sizeof(uint4));
-  L.counters = take(counter_words((int)nframes) * sizeof(uint32_t));
-  L.block_sums = take((size_t)std::max(kScanBlocks, stream_order_blocks()) * sizeof(uint32_t));
+  L.res = take(nframes * L.cand_cap * sizeof(uint32_t));  // 3/2 cand_cap results a frame
+  take(nframes * L.cand_cap * sizeof(uint2));
+  L.cand = take(nframes * L.words * sizeof(uint32_t));
+  // (These two are larger than their lists: every workspace keeps its size,
+  // and the no-allocation entry point's fixed scratch the frames it takes.)
+  L.tiles = take(nframes * (L.words + 2 * lattice_tiles((int)h, (int)w)) * sizeof(uint32_t));
+  L.cand_sums = take(nframes * ((w + 239) / 240) * ((h + 15) / 16) * 2 * sizeof(uint4));
+  L.counters = take((4 + 4 * nframes) * sizeof(uint32_t));
+  L.block_sums = take((size_t)kCountBlocks * sizeof(uint32_t));
   L.tile_base = take((size_t)tiles_x((int)w) * tiles_y((int)h) * sizeof(uint32_t));
   L.row_total = take((size_t)tiles_y((int)h) * sizeof(uint32_t));
   L.total = off;
@@ -169,17 +171,18 @@ static bool shape_ok(size_t h, size_t w) {
   return h > 0 && w > 0 && h <= 0x7fffffffu / w;
 }
 
-static bool stream_path(size_t elem, const LaunchParams &P) {
-  return elem == 4 && P.algorithm == SF_DISPERSION_EXTENDED && P.int_ok;
-}
-
-// 16-bit frames take the lattice path for kernel 3,3 (any gain and sigmas:
-// their tests are the reference's float ones) when whole 8-byte pieces of 4
-// pixels tile every row: 4 | width and 8-byte aligned frames.
+// Calls that have always needed a workspace for every frame of the batch, and
+// have refused frames of more candidates than it has places for: 32-bit
+// dispersion_extended at gain 1 with integral sigmas, and 16-bit at kernel 3,3
+// where 4 | width and the frames are 8-byte aligned.
 template <typename T>
-static bool stream16_path(const T *const *d_images, size_t n, const size_t *widths,
-                          const LaunchParams &P) {
-  if (sizeof(T) != 2 || P.algorithm != SF_DISPERSION_EXTENDED || P.half != 3)
+static bool batch_workspace(const T *const *d_images, size_t n, const size_t *widths,
+                            const LaunchParams &P) {
+  if (P.algorithm != SF_DISPERSION_EXTENDED)
+    return false;
+  if (sizeof(T) == 4)
+    return P.int_ok != 0;
+  if (P.half != 3)
     return false;
   for (size_t j = 0; j < n; j++)
     if (widths[j] % 4 != 0 || reinterpret_cast<uintptr_t>(d_images[j]) % 8 != 0)
@@ -224,12 +227,52 @@ static int threshold_frames(const T *const *d_images, size_t n, size_t h, size_t
                                    d_counts, d_word_prefix, d_ws, ws_bytes, run_rows, stream);
 }
 
+// The streaming path's launches for frames whose buffers L lays out in d_ws.
+template <typename T>
+static int threshold_streamed(const T *const *d_images, size_t n, const size_t *heights,
+                              const size_t *widths, size_t h, size_t w, const LaunchParams &P,
+                              const WorkspaceLayout &L, sf_signal_pixel *d_out, size_t capacity,
+                              uint32_t *d_bits, uint32_t *d_counts, uint32_t *d_word_prefix,
+                              void *d_ws, bool limited, int run_rows, cudaStream_t stream) {
+  unsigned char *ws = static_cast<unsigned char *>(d_ws);
+  FramePtrs F;
+  for (size_t j = 0; j < n; j++) {
+    F.image[j] = reinterpret_cast<const uint32_t *>(d_images[j]);
+    F.h[j] = (int)heights[j];
+    F.w[j] = (int)widths[j];
+  }
+  StreamBuffers b;
+  b.bits = d_bits;
+  b.cand = reinterpret_cast<uint32_t *>(ws + L.cand);
+  b.words = L.words;
+  b.prefix = d_word_prefix;
+  b.res = reinterpret_cast<uint2 *>(ws + L.res);
+  b.res_stride = (uint32_t)(L.cand_cap + L.cand_cap / 2);
+  b.tiles = reinterpret_cast<uint32_t *>(ws + L.tiles);
+  b.counters = reinterpret_cast<uint32_t *>(ws + L.counters);
+  b.block_sums = reinterpret_cast<uint32_t *>(ws + L.block_sums);
+  b.cand_sums = reinterpret_cast<uint32_t *>(ws + L.cand_sums);
+  b.cand_limit = limited ? (uint32_t)L.cand_cap : 0xFFFFFFFFu;
+  b.capacity = (uint32_t)capacity;
+  b.out = d_out;
+  b.out_stride = capacity;
+  b.count_out = d_counts;
+  const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
+  t_marks.staged = true;
+  const cudaError_t e =
+      P.algorithm == SF_DISPERSION
+          ? launch_dispersion(F, (int)n, (int)h, (int)w, (int)sizeof(T), P, b, run_rows, stream,
+                              marks)
+          : launch_extended(F, (int)n, (int)h, (int)w, (int)sizeof(T), P, b, run_rows, stream,
+                            marks);
+  return e == cudaSuccess ? SF_OK : fail(e, "launching the threshold");
+}
+
 // Frames d_images[0 .. n) of shapes heights[j] x widths[j], laid out for the
 // envelope H x W (the tallest and the widest): lists at d_out + j * capacity,
 // frame j's mask at d_bits + j * ceil(W / 32) * H in its own rows of
-// ceil(widths[j] / 32) words, counts at d_counts[j]. The kernel-3,3 lattice
-// path takes the mixed frames in one launch sequence; other settings run
-// frames of another shape one launch sequence each.
+// ceil(widths[j] / 32) words, counts at d_counts[j]. The streaming path takes
+// them all in one launch sequence.
 template <typename T>
 static int threshold_frames_mixed(const T *const *d_images, size_t n, const size_t *heights,
                                   const size_t *widths, const sf_threshold_params *params,
@@ -241,76 +284,38 @@ static int threshold_frames_mixed(const T *const *d_images, size_t n, const size
       !d_bits || !d_counts || !d_ws || capacity > 0xffffffffu ||
       !envelope(n, heights, widths, &h, &w))
     return SF_EBADARG;
-  bool mixed = false;
-  for (size_t j = 0; j < n; j++) {
+  for (size_t j = 0; j < n; j++)
     if (!d_images[j])
       return SF_EBADARG;
-    mixed |= heights[j] != h || widths[j] != w;
-  }
   LaunchParams P;
   int rc = make_launch_params(params, &P);
   if (rc != SF_OK)
     return rc;
-  const bool streamed16 = stream16_path(d_images, n, widths, P);
-  const bool streamed = stream_path(sizeof(T), P) || streamed16;
-  const WorkspaceLayout L = layout(h, w, capacity, streamed ? n : 1);
-  if (ws_bytes < L.total)
+  const bool batch = batch_workspace(d_images, n, widths, P);
+  const bool streamed = streaming_path(P, (int)sizeof(T));
+  const WorkspaceLayout Ln = layout(h, w, capacity, n);
+  const bool all = ws_bytes >= Ln.total;
+  const WorkspaceLayout L = all ? Ln : layout(h, w, capacity);
+  if (batch ? !all : ws_bytes < L.total)
     return SF_EBADARG;
-  if (mixed && streamed && P.half != 3) {
-    // The strip path of kernel sizes 2 and 4 takes one shape a launch: each
-    // frame alone, into its slots (its workspace fits in the batch's).
+  if (streamed && !all && n > 1) {
+    // A workspace for one frame: the frames one after another, each into its
+    // slots of the envelope's layout.
     for (size_t j = 0; j < n; j++) {
       const T *one[1] = {d_images[j]};
-      rc = threshold_frames_mixed<T>(one, 1, heights + j, widths + j, params,
-                                     d_out + j * capacity, capacity, d_bits + j * L.words,
-                                     d_counts + j,
-                                     d_word_prefix ? d_word_prefix + j * L.words : nullptr, d_ws,
-                                     ws_bytes, run_rows, stream);
+      rc = threshold_streamed<T>(one, 1, heights + j, widths + j, h, w, P, L, d_out + j * capacity,
+                                 capacity, d_bits + j * L.words, d_counts + j,
+                                 d_word_prefix ? d_word_prefix + j * L.words : nullptr, d_ws,
+                                 batch, run_rows, stream);
       if (rc != SF_OK)
         return rc;
     }
     return SF_OK;
   }
+  if (streamed)
+    return threshold_streamed<T>(d_images, n, heights, widths, h, w, P, L, d_out, capacity, d_bits,
+                                 d_counts, d_word_prefix, d_ws, batch, run_rows, stream);
   unsigned char *ws = static_cast<unsigned char *>(d_ws);
-  const bool dispersion = dispersion_path(P, (int)sizeof(T));
-  // The dispersion path keeps results between its passes where the workspace
-  // has every frame's; a workspace for one frame is enough for it without.
-  const WorkspaceLayout Ln =
-      dispersion ? layout(h, w, capacity, n) : L;
-  const bool all = ws_bytes >= Ln.total;
-  if (streamed || dispersion) {
-    FramePtrs F;
-    for (size_t j = 0; j < n; j++) {
-      F.image[j] = reinterpret_cast<const uint32_t *>(d_images[j]);
-      F.h[j] = (int)heights[j];
-      F.w[j] = (int)widths[j];
-    }
-    StreamBuffers b;
-    b.bits = d_bits;
-    b.words = L.words;
-    b.scr1 = reinterpret_cast<uint32_t *>(ws + L.scr1);
-    b.amb = reinterpret_cast<uint32_t *>(ws + L.amb);
-    b.prefix = d_word_prefix;
-    b.cand = reinterpret_cast<uint32_t *>(ws + L.cand);
-    b.res = reinterpret_cast<uint2 *>(ws + (all ? Ln.res : L.res));
-    b.cand_cap = all ? (uint32_t)L.cand_cap : 0u;
-    b.counters = reinterpret_cast<uint32_t *>(ws + L.counters);
-    b.wide = reinterpret_cast<uint4 *>(ws + L.wide);
-    b.block_sums = reinterpret_cast<uint32_t *>(ws + (all ? Ln.block_sums : L.block_sums));
-    b.capacity = (uint32_t)capacity;
-    b.out = d_out;
-    b.out_stride = capacity;
-    b.count_out = d_counts;
-    const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
-    t_marks.staged = true;
-    cudaError_t e =
-        dispersion ? launch_dispersion(F, (int)n, (int)sizeof(T), P, b, run_rows, stream, marks)
-        : streamed16 ? launch_stream16(F, (int)n, (int)h, (int)w, P, b, run_rows, stream, marks)
-                   : launch_stream(F, (int)n, (int)h, (int)w, P, b, run_rows, stream, marks);
-    if (e != cudaSuccess)
-      return fail(e, "launching the threshold");
-    return SF_OK;
-  }
   const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
   t_marks.staged = false;
   if (marks)
@@ -1151,6 +1156,7 @@ extern "C" int sf_threshold_u32_device_noalloc(
 namespace sf {
 
 constexpr size_t kPlanMaxGraphs = 16;
+constexpr int kTuneMinRows = 16;  // shortest run length the tuner tries
 
 struct Plan {
   size_t h = 0, w = 0, max_frames = 0, capacity = 0, words = 0;
@@ -1340,7 +1346,7 @@ int sf_plan_tune(sf_plan *plan, const uint32_t *const *d_images, size_t n_frames
     cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
     p.per_launch = q == n_frames ? 0 : q;
     for (int rr : cands) {
-      if (rr < kMinRunRows || rr > (int)p.h)
+      if (rr < kTuneMinRows || rr > (int)p.h)
         continue;
       p.run_rows = rr;
       float ms[3];

@@ -128,6 +128,27 @@ static __device__ __noinline__ bool stage2_double(uint32_t p, uint32_t n, unsign
   return (double)p >= t;
 }
 
+// The decision where |E| is too small for stage2_u32's constant bound, from
+// the bound at this mean (out of line: few candidates reach it).
+static __device__ __noinline__ bool stage2_near(uint32_t p, uint32_t n, uint32_t S, float Ef,
+                                                const LaunchParams &P, float *bg) {
+  // |p - t| beyond the double sequence's error err <= 2^-50 t means
+  // |E| > n^2 err (err + 2 sigma_s sqrt(mean)); bound that from above in
+  // float with generous slack (mean < 2^24 here).
+  const float mu = __fdiv_ru((float)S, (float)n);
+  const float rt = __fsqrt_ru(mu) * 1.001f + 1.0f;
+  const float ss = (float)P.sigma_s;
+  const float t = mu + ss * rt + 1.0f;
+  const float err = t * 0x1p-49f;
+  const float nn = (float)n * (float)n;
+  const float bound = nn * err * (err + 2.0f * ss * rt) * 2.0f + 1.0f;
+  if (Ef > bound)
+    return true;
+  if (Ef < -bound)
+    return false;
+  return stage2_double(p, n, S, P, bg);
+}
+
 __device__ __forceinline__ bool stage2_u32(uint32_t p, uint32_t n,
                                            unsigned long long S,
                                            const LaunchParams &P, float *bg) {
@@ -146,21 +167,11 @@ __device__ __forceinline__ bool stage2_u32(uint32_t p, uint32_t n,
       return true; // p - mean > 2^23.6 > sigma_s sqrt(mean) + any rounding
     const long long E =
         d * d - (long long)P.sigma_s2_int * (long long)S * (long long)n;
-    // |p - t| beyond the double sequence's error err <= 2^-50 t means
-    // |E| > n^2 err (err + 2 sigma_s sqrt(mean)); bound that from above in
-    // float with generous slack (mean < 2^24 here).
-    const float mu = __fdiv_ru((float)(uint32_t)S, (float)n);
-    const float rt = __fsqrt_ru(mu) * 1.001f + 1.0f;
-    const float ss = (float)P.sigma_s;
-    const float t = mu + ss * rt + 1.0f;
-    const float err = t * 0x1p-49f;
-    const float nn = (float)n * (float)n;
-    const float bound = nn * err * (err + 2.0f * ss * rt) * 2.0f + 1.0f;
-    const float Ef = (float)E;
-    if (Ef > bound)
-      return true;
-    if (Ef < -bound)
-      return false;
+    // stage2_near's bound is below 2^13 for sigma_s up to 2^8: n <= 169, t <
+    // 2^24 + 2^20.1, sqrt(mean) <= 2^12 give at most 3,840.
+    if (P.sigma_s2_int <= 65536u && (E > 8192 || E < -8192))
+      return E > 0;
+    return stage2_near(p, n, (uint32_t)S, (float)E, P, bg);
   }
   return stage2_double(p, n, S, P, bg);
 }

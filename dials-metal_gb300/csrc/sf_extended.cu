@@ -1,0 +1,782 @@
+// The dispersion_extended threshold (the reference's algorithm,
+// src/spots/dext.cc:53-222), for one frame or a batch of frames per launch
+// sequence, of either pixel type, any kernel size, aligned or not:
+//
+//   ext_strip       stage 0 (the dispersion test) of every pixel and the
+//                   erosion, one warp per strip and run of rows: the candidate
+//                   mask, whose pixels with the masked ones are the reference's
+//                   eroded mask
+//   ext_decide      stage 2 (the Poisson test over the background) at each
+//                   candidate: the strong-pixel mask, the passing pixels'
+//                   results and the blocks' counts
+//   scatter_pixels  the records, ascending (sf_groups.cuh)
+//
+// Each frame is thresholded alone: no sum, mask or list crosses frames, and no
+// list of candidates is kept, so none can overflow.
+//
+// The stage-0 decision of 32-bit frames from exact window sums. The
+// reference's test (dext.cc:99-109) is A > X in double, A = nQ - S^2 - g S (n -
+// 1) and X = g S sigma_b r_n (r_n its double sqrt(2 (n - 1))). Writing c = g (n
+// - 1 + sigma_b r_n), it is n Q > S (S + c). Per window count n the host gives
+// integers clo <= 2^8 c <= chi and nk = 2^8 n (0 when n cannot be tested):
+//   2^8 n Q <= S (2^8 S + clo)           =>  not signal
+//   2^8 n Q >= S (2^8 S + chi) + 2^9     =>  signal
+// both exact in 64-bit integers. With gain 1 and an integral sigma_b, A is
+// exact in double and A >= X + 2 > RN(X) in the second case; with others clo
+// and chi are a unit further out, S / 2^8 of margin against the reference's
+// rounding of sums below 2^38 (under 2^-13). What lies between goes to the
+// reference's own sequence (sf_common.cuh). 16-bit frames are decided by their
+// float sequence everywhere.
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <type_traits>
+
+#include "sf_common.cuh"
+#include "sf_groups.cuh"
+#include "sf_lattice.cuh"
+#include "sf_stream.cuh"
+#include "sf_strips.cuh"
+
+namespace sf {
+namespace {
+
+// By window count n: nk, clo, chi above in 2^-8 units, and clo and chi rounded
+// outwards to 2^-4 units; `big` is the sum of squares from which the 2^-4
+// tests' products may leave 32 bits.
+struct ExtTables {
+  uint32_t nk[kMaxN0 + 1], clo[kMaxN0 + 1], chi[kMaxN0 + 1];
+  uint32_t clo16[kMaxN0 + 1], chi16[kMaxN0 + 1];
+  uint32_t big;
+};
+
+// The largest 2^8 c the 64-bit tests take: with S below 2^20 (sums of pixels
+// below Cap), (S << 8) + chi stays in 32 bits.
+constexpr double kMaxC8 = 2147483648.0;
+
+// The reference's decision for one window of exact sums, out of line: reached
+// only between the two bounds.
+__device__ __noinline__ bool ext_exact(uint32_t n, unsigned long long S, unsigned long long Q,
+                                         const LaunchParams &P) {
+  return stage0_u32(n, S, Q, P, P.root_lo, P.root_hi);
+}
+
+// The stage-0 bits (signal or masked; off the frame counts as set) of the 12
+// windows centred on row y, columns cx ..: from 64-bit sums of the frame's
+// pixels, for rows whose windows may hold a pixel too large for the strip's
+// sums. A column's sums of 2K + 1 rows enter as the windows move right and
+// leave again; a window off the frame is clipped as the reference's is.
+template <int K>
+__device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image, int height,
+                                              int width, int y, int cx, const LaunchParams &P) {
+  constexpr int W0 = 2 * K + 1;
+  if (y < 0 || y >= height)
+    return 0xFFFu;  // off the frame: set
+  uint32_t cn[W0];
+  unsigned long long cS[W0], cQ[W0];
+  uint32_t n = 0, bits = 0;
+  unsigned long long S = 0, Q = 0;
+#pragma unroll
+  for (int j = 0; j < kCols + 2 * K; j++) {
+    const int x = cx - K + j;
+    uint32_t an = 0;
+    unsigned long long aS = 0, aQ = 0;
+    if (x >= 0 && x < width) {
+#pragma unroll
+      for (int d = -K; d <= K; d++) {
+        const uint32_t v = y + d >= 0 && y + d < height
+                               ? __ldg(image + (size_t)(y + d) * width + x)
+                               : 0xFFFFFFFFu;
+        const bool ok = v < 0xFFFFFFFEu;
+        const uint32_t u = ok ? v : 0u;
+        an += ok ? 1u : 0u;
+        aS += u;
+        aQ += (unsigned long long)u * u;
+      }
+    }
+    if (j >= W0) {
+      n -= cn[j % W0];
+      S -= cS[j % W0];
+      Q -= cQ[j % W0];
+    }
+    cn[j % W0] = an;
+    cS[j % W0] = aS;
+    cQ[j % W0] = aQ;
+    n += an;
+    S += aS;
+    Q += aQ;
+    if (j >= 2 * K) {
+      const int xc = x - K;  // the window's centre
+      bool set = true;
+      if (xc >= 0 && xc < width && __ldg(image + (size_t)y * width + xc) < 0xFFFFFFFEu)
+        set = ext_exact(n, S, Q, P);
+      bits |= set ? 1u << (j - 2 * K) : 0u;
+    }
+  }
+  return bits;
+}
+
+// The float sequence of stage0_u16 (sf_common.cuh) with its factors given.
+__device__ __forceinline__ bool ext_float(float m, float root, uint32_t S, uint32_t Q, float g,
+                                          float sb) {
+  const float s = __uint2float_rn(S), s2 = __uint2float_rn(Q);
+  const float gs = __fmul_rn(g, s);
+  return __fsub_rn(__fsub_rn(__fmul_rn(m, s2), __fmul_rn(s, s)),
+                   __fmul_rn(gs, __fsub_rn(m, 1.0f))) > __fmul_rn(__fmul_rn(gs, sb), root);
+}
+
+// A window's constants by its masked count m (n = N0 - m): the 2^-4 tests' {nk,
+// clo, chi - clo} and n, and the 2^-8 tests' {nk, clo, chi}; for 16-bit frames
+// {n, rootf} as floats (rootf NaN, no test passes, below min_local).
+struct ExtRow {
+  uint4 a, b;
+};
+
+// The walk of sf_strips.cuh for stage 0, then the erosion (dext.cc:117-142):
+// the rows' 12 decision bits are kept for 2E + 1 rows and ANDed down the
+// column, then across the lane's and its neighbours' columns. A warp row goes
+// only as far as it must: the lower 2^-4 bound alone where no window of the
+// row may be signal; both 2^-4 bounds; both 2^-8 bounds where a window lies
+// between those or is too big for them; the reference's sequence between
+// those; and 64-bit sums where a window may hold a saturated pixel. Bound by
+// issue (69% of its rate, 57 instructions a pixel): 16 frames of 3262 x 3108 at
+// kernel 4 take 425 us, 556 as 240-column strips with the windows' row sums
+// carried in shared memory, the 64-bit rows and the ambiguous windows
+// in passes of their own.
+template <int K, typename Pix>
+__global__ void __launch_bounds__(kStripWarps * 32, StripG<K>::Occ)
+ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,
+          int run_rows, const __grid_constant__ ExtTables T,
+          const __grid_constant__ LaunchParams P, uint8_t *__restrict__ cand_all,
+          size_t mask_bytes) {
+  using G = StripG<K>;
+  constexpr bool k16 = sizeof(Pix) == 2;
+  constexpr int E = K - 1;
+  extern __shared__ __align__(16) unsigned char ext_raw[];
+  __shared__ ExtRow tab[G::N0 + 1];
+  for (int m = threadIdx.x; m <= G::N0; m += blockDim.x) {
+    const int n = G::N0 - m;
+    if constexpr (k16) {
+      const float root = (uint32_t)n < P.min_local ? __uint_as_float(0x7FFFFFFFu) : P.rootf[n];
+      tab[m].a = make_uint4(__float_as_uint((float)n), __float_as_uint(root), 0u, 0u);
+      tab[m].b = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      tab[m].a = make_uint4(T.nk[n] >> 4, T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
+      tab[m].b = make_uint4(T.nk[n], T.clo[n], T.chi[n], 0u);
+    }
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  StripRun r;
+  if (!strip_run(F, nframes, S, run_rows, r))
+    return;  // whole warp
+  const Pix *image = reinterpret_cast<const Pix *>(F.image[r.frame]);
+  const int rows = r.rb - r.ra + 2 * (K + E);
+  Pix *ring = reinterpret_cast<Pix *>(ext_raw) + (size_t)warp * G::Slots * kStripStride;
+  RowReader<Pix> reader(image, r, r.ra - E - K, rows);
+  auto after = [&](int s) { return s + 1 == G::Slots ? 0 : s + 1; };
+#pragma unroll
+  for (int i = 0; i < G::Ahead; i++) {
+    reader.fetch(ring + i * kStripStride);
+    cp_async_commit();
+  }
+  uint32_t Vn[kCols], Vq[kCols];
+#pragma unroll
+  for (int c = 0; c < kCols; c++)
+    Vn[c] = Vq[c] = 0u;
+  const float gain = (float)P.gain, sigma_b = (float)P.sigma_b;
+  uint8_t *out_row = cand_all + (size_t)r.frame * mask_bytes + (size_t)r.ra * r.bytes_per_row +
+                     r.pair_byte;
+  const int bytes_left = r.bytes_per_row - r.pair_byte;
+  // The last 2E + 1 rows' decision bits and the last E + 1 rows' masked bits,
+  // 12 bits a row in 16-bit halves, the newest lowest.
+  uint32_t dec[4] = {0u, 0u, 0u, 0u}, msk[2] = {0u, 0u};
+  // Slots of the row in flight, the current, the centre and the leaving row.
+  int s_in = G::Ahead, s_cur = 0, s_mid = G::Slots - K, s_old = G::Slots - G::W0;
+  for (int i = 0; i < rows; i++) {
+    __syncwarp();  // every lane is done with the slot that is filled next
+    reader.fetch(ring + s_in * kStripStride);
+    cp_async_commit();
+    cp_async_wait<G::Ahead>();
+    __syncwarp();
+    {
+      uint32_t v[kCols], o[kCols];
+      read_row<K, Pix, true>(ring + s_cur * kStripStride, lane, v);
+      if (i >= G::W0) {  // warp-uniform
+        read_row<K, Pix, false>(ring + s_old * kStripStride, lane, o);
+      } else {
+#pragma unroll
+        for (int c = 0; c < kCols; c++)
+          o[c] = 0u;
+      }
+#pragma unroll
+      for (int c = 0; c < kCols; c++) {
+        Vn[c] += v[c] - o[c];
+        Vq[c] += v[c] * v[c] - o[c] * o[c];
+      }
+    }
+    if (i >= 2 * K) {  // warp-uniform: the windows are whole
+      uint32_t hn[kCols], hq[kCols];
+      window_sums<K>(Vn, hn);
+      window_sums<K>(Vq, hq);
+      uint32_t any_masked = 0;
+#pragma unroll
+      for (int c = 0; c < kCols; c++)
+        any_masked |= hn[c];
+      // Warp rows whose windows hold no masked pixel (most) take the whole
+      // window's constants; the others look each window's count up.
+      const bool uniform = !__any_sync(0xffffffffu, any_masked >> kCountShift);
+      uint32_t sig = 0, masked12 = 0;
+      if (!uniform) {
+        uint32_t v[kCols];
+        read_row<K, Pix, false>(ring + s_mid * kStripStride, lane, v);
+#pragma unroll
+        for (int c = 0; c < kCols; c++)
+          masked12 |= v[c] >> kCountShift << c;
+      }
+      if constexpr (k16) {
+        if (uniform) {
+          const uint4 t = tab[0].a;
+          const float m = __uint_as_float(t.x), root = __uint_as_float(t.y);
+#pragma unroll
+          for (int c = 0; c < kCols; c++)
+            sig |= ext_float(m, root, hn[c], hq[c], gain, sigma_b) ? 1u << c : 0u;
+        } else {
+#pragma unroll
+          for (int c = 0; c < kCols; c++) {
+            const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].a;
+            sig |= ext_float(__uint_as_float(t.x), __uint_as_float(t.y), hn[c] & kSumMask, hq[c],
+                             gain, sigma_b)
+                       ? 1u << c
+                       : 0u;
+          }
+        }
+      } else {
+        // The lower 2^-4 bound; a big window may be signal. (Bitwise
+        // throughout: a branch around half a test costs more than the half.)
+        uint32_t maybe = 0;
+        const uint4 t0 = tab[0].a;
+        if (uniform) {
+#pragma unroll
+          for (int c = 0; c < kCols; c++)
+            maybe |= (hq[c] >= T.big) | (hq[c] * t0.x > hn[c] * ((hn[c] << 4) + t0.y)) ? 1u << c
+                                                                                        : 0u;
+        } else {
+#pragma unroll
+          for (int c = 0; c < kCols; c++) {
+            const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].a;
+            const uint32_t s = hn[c] & kSumMask;
+            maybe |= (hq[c] >= T.big) | (hq[c] * t.x > s * ((s << 4) + t.y)) ? 1u << c : 0u;
+          }
+        }
+        sig = maybe;
+        if (__any_sync(0xffffffffu, maybe != 0u)) {
+          uint32_t sure = 0, most = 0;
+#pragma unroll
+          for (int c = 0; c < kCols; c++) {
+            uint4 t = t0;
+            uint32_t s = hn[c];
+            if (!uniform) {
+              t = tab[min(s >> kCountShift, (uint32_t)G::N0)].a;
+              s &= kSumMask;
+            }
+            sure |= (hq[c] < T.big) & (hq[c] * t.x >= s * ((s << 4) + t.y) + s * t.z + 32u)
+                        ? 1u << c
+                        : 0u;
+            most = max(most, hq[c]);
+          }
+          sig = sure;
+          if (__any_sync(0xffffffffu, (maybe & ~sure) != 0u)) {
+            if (__any_sync(0xffffffffu, most >= G::Cap * G::Cap)) {
+              // A window may hold a saturated pixel: this row in 64 bits.
+              sig = ext_wide_row<K>(reinterpret_cast<const uint32_t *>(image), r.height, r.width,
+                                    r.ra - E + i - 2 * K, r.cx, P);
+            } else {
+              uint32_t between = 0;
+              sig = 0;
+#pragma unroll
+              for (int c = 0; c < kCols; c++) {
+                const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].b;
+                const uint32_t s = hn[c] & kSumMask;
+                const unsigned long long L = (unsigned long long)hq[c] * t.x;
+                const bool above = L > (unsigned long long)s * ((s << 8) + t.y);
+                const bool over = L >= (unsigned long long)s * ((s << 8) + t.z) + (2ull << 8);
+                sig |= over ? 1u << c : 0u;
+                between |= above & !over ? 1u << c : 0u;
+              }
+              if (__any_sync(0xffffffffu, between != 0u)) {
+#pragma unroll
+                for (int c = 0; c < kCols; c++) {
+                  if ((between >> c) & 1u) {
+                    const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
+                    if (ext_exact(G::N0 - m, hn[c] & kSumMask, hq[c], P))
+                      sig |= 1u << c;
+                  }
+                }
+              }
+            }
+          }
+        }
+      }
+      // Row d = ra - E + i - 2K: signal or masked; then the erosion of row d - E.
+#pragma unroll
+      for (int k = 3; k > 0; k--)
+        dec[k] = __funnelshift_l(dec[k - 1], dec[k], 16);
+      dec[0] = dec[0] << 16 | sig | masked12;
+      msk[1] = __funnelshift_l(msk[0], msk[1], 16);
+      msk[0] = msk[0] << 16 | masked12;
+      if (i >= 2 * K + 2 * E) {  // warp-uniform
+        uint32_t col = dec[0];
+#pragma unroll
+        for (int k = 1; k <= 2 * E; k++)
+          col &= k & 1 ? dec[k >> 1] >> 16 : dec[k >> 1];
+        col &= 0xFFFu;
+        const uint32_t left = __shfl_up_sync(0xffffffffu, col, 1);
+        const uint32_t right = __shfl_down_sync(0xffffffffu, col, 1);
+        const uint32_t all = left >> (kCols - E) | col << E | right << (kCols + E);
+        uint32_t kept = all;
+#pragma unroll
+        for (int k = 1; k <= 2 * E; k++)
+          kept &= all >> k;
+        const uint32_t mrow = E & 1 ? msk[E >> 1] >> 16 : msk[E >> 1];
+        write_bits(r, out_row, bytes_left, kept & ~mrow & r.inside12);
+        out_row += r.bytes_per_row;
+      }
+    }
+    s_in = after(s_in);
+    s_cur = after(s_cur);
+    s_mid = after(s_mid);
+    s_old = after(s_old);
+  }
+  cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
+// Stage 2 (dext.cc:151-222): a candidate's background is the valid pixels
+// outside the eroded mask (the candidates and the masked pixels) in its clipped
+// (2K + 5)-square window.
+// ---------------------------------------------------------------------------
+
+// One warp's chunk: the background's {count, sum} over the window's rows by
+// output row and column, the pixels of the output rows, and the run's strong
+// words and counts so far.
+struct ExtWarp {
+  uint2 col[kBandRows][32];
+  uint32_t px[kBandRows][32];
+  uint32_t strong[kBandRows * kRunWords];
+  uint32_t passed[kBandRows];
+};
+
+// A window's background one pixel after another, in 64 bits, for chunks that
+// hold a pixel of 2^24 or more.
+template <typename Pix>
+__device__ __noinline__ void ext_wide_window(const Pix *image, const uint32_t *cand, int height,
+                                             int width, int half, int y, int x, uint32_t *n_out,
+                                             unsigned long long *S_out) {
+  const uint32_t wpr = ((uint32_t)width + 31u) >> 5;
+  uint32_t n = 0;
+  unsigned long long S = 0;
+  for (int yy = max(0, y - half); yy <= min(height - 1, y + half); yy++)
+    for (int xx = max(0, x - half); xx <= min(width - 1, x + half); xx++) {
+      const uint32_t v = __ldg(image + (size_t)yy * width + xx);
+      if (v < Traits<Pix>::kMasked &&
+          (__ldg(cand + (size_t)yy * wpr + (xx >> 5)) >> (xx & 31) & 1u) == 0u) {
+        n++;
+        S += v;
+      }
+    }
+  *n_out = n;
+  *S_out = S;
+}
+
+// A warp takes a run of a band at a time (128 columns x 8 rows, a word a lane)
+// and its candidates in chunks: from the leftmost column with one left, the NC
+// columns whose windows 32 columns cover, for all 8 rows (a spot's candidates
+// are about 7 x 7). The chunk's pixels are read once, a lane a column, added up
+// over the window's rows into shared memory; then its candidates are spread
+// over the lanes, each adding up its window's columns for the test. The warps
+// of a block take the runs of its bands in turn from a counter, so that those
+// with many candidates even out. Bound by issue: 32 frames of 4362 x 4148 (174
+// thousand candidates each) take 292 us. A window a candidate, four lanes each,
+// took 568 us, chunks of one row 427, and tests row by row, only the row's
+// candidates' lanes busy, 553.
+template <int K, typename Pix>
+__global__ void __launch_bounds__(kScanT, 4)
+ext_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchParams P,
+           const uint32_t *__restrict__ cand_all, uint32_t *__restrict__ bits_all, size_t words,
+           Kept kept, uint32_t *__restrict__ block_sums, uint32_t *__restrict__ cand_sums) {
+  constexpr int K2 = K + 2, W2 = 2 * K2 + 1, NC = 32 - 2 * K2, ROWS = kBandRows + 2 * K2;
+  __shared__ ExtWarp s_warps[kScanT / 32];
+  __shared__ uint32_t s_count[2], s_next;
+  ExtWarp &sm = s_warps[threadIdx.x >> 5];
+  const int f = blockIdx.y, lane = threadIdx.x & 31;
+  const Pix *image = reinterpret_cast<const Pix *>(F.image[f]);
+  const int height = F.h[f], width = F.w[f];
+  const uint32_t wpr = ((uint32_t)width + 31u) >> 5, rpr = (uint32_t)runs_per_row(width);
+  const uint32_t lane_bit = 1u << lane;
+  const uint32_t *cand = cand_all + (size_t)f * words;
+  uint32_t *bits = bits_all + (size_t)f * words;
+  uint2 *res = kept.res + (size_t)f * kept.stride;
+  if (threadIdx.x < 2)
+    s_count[threadIdx.x] = 0u;
+  if (threadIdx.x == 0)
+    s_next = 0u;
+  __syncthreads();
+  int row_lo, row_hi;
+  band_share(height, &row_lo, &row_hi);
+  const uint32_t items = (uint32_t)((row_hi - row_lo + kBandRows - 1) / kBandRows) * rpr;
+  const int lr = lane / kRunWords, lc = lane % kRunWords;  // this lane's row and word of a run
+  uint32_t count = 0, total = 0;
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0)
+      item = atomicAdd(&s_next, 1u);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= items)
+      break;  // whole warp
+    const uint32_t band = item / rpr, run = item - band * rpr;
+    const int y0 = row_lo + (int)band * kBandRows, xr = (int)run * kRunWords * 32;
+    const bool in = y0 + lr < row_hi && run * kRunWords + lc < wpr;
+    const size_t wi = (size_t)(y0 + lr) * wpr + run * kRunWords + lc;
+    uint32_t left = in ? __ldg(cand + wi) : 0u;  // this lane's candidates not yet decided
+    if (!__any_sync(0xffffffffu, left != 0u)) {
+      if (in)
+        bits[wi] = 0u;
+      continue;
+    }
+    total += (uint32_t)__popc(left);
+    sm.strong[lane] = 0u;
+    if (lane < kBandRows)
+      sm.passed[lane] = 0u;
+    for (;;) {
+      // The leftmost column with a candidate left.
+      uint32_t any = left;
+      any |= __shfl_xor_sync(0xffffffffu, any, 4);
+      any |= __shfl_xor_sync(0xffffffffu, any, 8);
+      any |= __shfl_xor_sync(0xffffffffu, any, 16);
+      const unsigned live = __ballot_sync(0xffffffffu, any != 0u) & 0xFu;
+      if (!live)
+        break;  // whole warp
+      const int c0 = __ffs(live) - 1, s = __ffs(__shfl_sync(0xffffffffu, any, c0)) - 1;
+      const int x0 = xr + 32 * c0 + s;
+      const unsigned long long span = (unsigned long long)((1u << NC) - 1u) << s;
+      left &= lc == c0 ? ~(uint32_t)span : lc == c0 + 1 ? ~(uint32_t)(span >> 32) : ~0u;
+      // The chunk's pixels start at (xl, yt); lane d holds the 32 mask bits over row d.
+      const int xl = x0 - K2, yt = y0 - K2;
+      uint32_t er_row = 0, v[ROWS];
+      if (xl >= 0 && xl + 32 <= width && yt >= 0 && yt + ROWS <= height) {  // warp-uniform
+        if (lane < ROWS) {
+          const uint32_t *cw = cand + (uint32_t)(yt + lane) * wpr + (uint32_t)(xl >> 5);
+          er_row = __funnelshift_r(__ldg(cw), __ldg(cw + ((xl & 31) != 0 ? 1 : 0)), xl & 31);
+        }
+        const Pix *at = image + (size_t)yt * width + (xl + lane);
+#pragma unroll
+        for (int d = 0; d < ROWS; d++) {
+          v[d] = (uint32_t)__ldg(at);
+          at += width;
+        }
+      } else {
+        if (lane < ROWS && yt + lane >= 0 && yt + lane < height) {
+          const uint32_t *row = cand + (size_t)(yt + lane) * wpr;
+          const int w0 = xl >> 5;  // (-1 left of the frame)
+          const uint32_t a = w0 >= 0 ? __ldg(row + w0) : 0u;
+          const uint32_t b = w0 + 1 < (int)wpr ? __ldg(row + w0 + 1) : 0u;
+          er_row = __funnelshift_r(a, b, xl & 31);
+        }
+        const int x = xl + lane;
+#pragma unroll
+        for (int d = 0; d < ROWS; d++) {
+          const bool inside = x >= 0 && x < width && yt + d >= 0 && yt + d < height;
+          v[d] = inside ? (uint32_t)__ldg(image + (size_t)(yt + d) * width + x)
+                        : Traits<Pix>::kMasked;
+        }
+      }
+      // Row r's candidates of the chunk, in lane r (columns past the run are
+      // the next one's), and the candidates before them.
+      uint32_t mine = __shfl_sync(0xffffffffu, er_row, (lane + K2) & 31) >> K2;
+      mine &= lane < kBandRows ? (1u << NC) - 1u : 0u;
+      if (x0 + NC > xr + 32 * kRunWords)
+        mine &= (1u << (xr + 32 * kRunWords - x0)) - 1u;
+      const uint32_t incl = warp_inclusive((uint32_t)__popc(mine), lane);
+      const uint32_t ncand = __shfl_sync(0xffffffffu, incl, 31);
+      // The background over the window's rows, by column.
+      uint32_t most = 0;
+      {
+        uint32_t n = 0, sum = 0;
+#pragma unroll
+        for (int d = 0; d < ROWS; d++) {
+          const bool ok = (v[d] < Traits<Pix>::kMasked) &
+                          ((__shfl_sync(0xffffffffu, er_row, d) & lane_bit) == 0u);
+          if (d >= K2 && d < K2 + kBandRows)
+            sm.px[d - K2][lane] = v[d];
+          v[d] = ok ? v[d] : Traits<Pix>::kMasked;  // background or not, from here on
+          n += ok ? 1u : 0u;
+          sum += ok ? v[d] : 0u;
+          most |= ok ? v[d] : 0u;
+          if (d >= W2 - 1) {
+            sm.col[d - (W2 - 1)][lane] = make_uint2(n, sum);
+            const bool was = v[d - (W2 - 1)] < Traits<Pix>::kMasked;
+            n -= was ? 1u : 0u;
+            sum -= was ? v[d - (W2 - 1)] : 0u;
+          }
+        }
+      }
+      const bool wide = sizeof(Pix) == 4 && __any_sync(0xffffffffu, most >= 1u << 24);
+      __syncwarp();
+      for (uint32_t q0 = 0; q0 < ncand; q0 += 32) {  // warp-uniform
+        const uint32_t q = q0 + lane;
+        int r = 0;
+#pragma unroll
+        for (int k = 4; k; k >>= 1)
+          r += __shfl_sync(0xffffffffu, incl, r + k - 1) <= q ? k : 0;
+        r &= 7;
+        const uint32_t row_bits = __shfl_sync(0xffffffffu, mine, r);
+        const uint32_t first = __shfl_sync(0xffffffffu, incl, r) - (uint32_t)__popc(row_bits);
+        bool ok = q < ncand;
+        const int j = ok ? select_bit(row_bits, q - first) : 0;
+        uint32_t n = 0, s32 = 0;
+#pragma unroll
+        for (int k = 0; k < W2; k++) {
+          const uint2 c = sm.col[r][j + k];
+          n += c.x;
+          s32 += c.y;
+        }
+        unsigned long long S = s32;
+        if (sizeof(Pix) == 4 && wide && ok)
+          ext_wide_window(image, cand, height, width, K2, y0 + r, x0 + j, &n, &S);
+        float mean = 0.0f;
+        if (ok) {
+          const uint32_t p = sm.px[r][j + K2];
+          // dext.cc:205: only pixels above the global threshold are tested.
+          ok = (uint64_t)p >= P.p_min;
+          if (ok) {
+            if constexpr (sizeof(Pix) == 2)
+              ok = stage2_u16(p, n, (uint32_t)S, P, &mean);
+            else
+              ok = stage2_u32(p, n, S, P, &mean);
+          }
+        }
+        // This row's passing candidates in these lanes, and before them.
+        const unsigned pass = __ballot_sync(0xffffffffu, ok);
+        const int from = max((int)first - (int)q0, 0);
+        const uint32_t before = sm.passed[r];
+        const uint32_t at = before + (uint32_t)__popc(pass & (lane_bit - 1u) & (~0u << from));
+        if (ok) {
+          if (at < kept.keep)
+            res[((size_t)(y0 + r) * rpr + run) * kept.keep + at] =
+                make_uint2(__float_as_uint(mean), n);
+          const int b = x0 + j - xr;
+          atomicOr(&sm.strong[r * kRunWords + (b >> 5)], 1u << (b & 31));
+        }
+        __syncwarp();
+        if (ok)
+          atomicMax(&sm.passed[r], at + 1u);
+        count += ok ? 1u : 0u;
+        __syncwarp();
+      }
+      __syncwarp();  // the next chunk rewrites the shared sums
+    }
+    if (in)
+      bits[wi] = sm.strong[lane];
+    __syncwarp();
+  }
+  count = __reduce_add_sync(0xffffffffu, count);
+  total = __reduce_add_sync(0xffffffffu, total);
+  if (lane == 0) {
+    atomicAdd(&s_count[0], count);
+    atomicAdd(&s_count[1], total);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    block_sums[(size_t)f * gridDim.x + blockIdx.x] = s_count[0];
+    cand_sums[(size_t)f * gridDim.x + blockIdx.x] = s_count[1];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Host side.
+// ---------------------------------------------------------------------------
+
+bool testable(const LaunchParams &P, int n, int n0) {
+  return n >= 1 && (uint32_t)n >= P.min_local && n <= n0;
+}
+
+// c = g (n - 1 + sigma_b r_n) as integers in 2^-8 units below and above it.
+// With gain 1 and an integral sigma_b from r_n's 2^-20 brackets, exactly; else
+// from the double product, a unit outwards.
+void bracket_c(const LaunchParams &P, int n, double *lo, double *hi) {
+  if (P.int_ok) {
+    const int shift = kRootShift - 8;
+    const uint64_t sb = P.sigma_b_int, base = (uint64_t)(n - 1) << 8;
+    *lo = (double)(base + ((sb * P.root_lo[n]) >> shift));
+    *hi = (double)(base + ((sb * P.root_hi[n] + ((1ull << shift) - 1)) >> shift));
+  } else {
+    const double c = 256.0 * P.gain * (n - 1 + P.sigma_b * P.root[n]);
+    *lo = std::max(0.0, std::floor(c) - 1.0);
+    *hi = std::ceil(c) + 1.0;
+  }
+}
+
+ExtTables make_ext_tables(const LaunchParams &P) {
+  ExtTables T;
+  const int n0 = (2 * P.half + 1) * (2 * P.half + 1);
+  T.big = P.half == 2 ? StripG<2>::Big : P.half == 3 ? StripG<3>::Big : StripG<4>::Big;
+  for (int n = 0; n <= kMaxN0; n++) {
+    double lo = 0.0, hi = 0.0;
+    if (testable(P, n, n0))
+      bracket_c(P, n, &lo, &hi);
+    T.clo[n] = (uint32_t)lo;
+    T.chi[n] = (uint32_t)hi;
+    T.clo16[n] = T.clo[n] >> 4;
+    T.chi16[n] = (T.chi[n] + 15u) >> 4;
+    // nk 0 makes every such window "surely not" (0 <= S (2^8 S + clo)).
+    T.nk[n] = testable(P, n, n0) ? (uint32_t)n << 8 : 0u;
+    if (T.chi16[n] >= kMaxC16)
+      T.big = 0;  // constants too large for the 32-bit tests: every window is big
+  }
+  return T;
+}
+
+// Whether stage 0 and the erosion take the lattice (sf_lattice.cu): kernel 3,3,
+// 32-bit frames at gain 1 with integral sigmas, or 16-bit ones where 4 | width
+// and they are 8-byte aligned. Spots cover a few percent of such frames, and
+// the lattice decides a ninth of the windows and the tiles that hold a
+// candidate: 32 frames of 4362 x 4148 take 0.95 ms so and 1.38 ms on strips.
+bool lattice_path(const FramePtrs &F, int nframes, int pixel_bytes, const LaunchParams &P) {
+  if (P.half != 3 || P.algorithm != SF_DISPERSION_EXTENDED)
+    return false;
+  if (pixel_bytes == 4)
+    return P.int_ok != 0;
+  for (int f = 0; f < nframes; f++)
+    if (F.w[f] % 4 != 0 || reinterpret_cast<uintptr_t>(F.image[f]) % 8 != 0)
+      return false;
+  return true;
+}
+
+template <int K, typename Pix> cudaError_t ext_slots(int *slots_out) {
+  using G = StripG<K>;
+  constexpr size_t smem = strip_smem<K, Pix>();
+  static_assert(sizeof(Pix) == 2 ||
+                    (smem + sizeof(ExtRow) * (G::N0 + 1) + 1024) * G::Occ <= 228 * 1024,
+                "the blocks an SM that the kernel is built for");
+  static std::once_flag configured;
+  static cudaError_t config_error = cudaSuccess;
+  static int slots = 0;
+  std::call_once(configured, [] {
+    config_error = cudaFuncSetAttribute(ext_strip<K, Pix>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per = 0;
+    if (config_error == cudaSuccess)
+      config_error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ext_strip<K, Pix>,
+                                                                   kStripWarps * 32, smem);
+    slots = std::max(1, per) * kStripWarps * device_sms();
+  });
+  *slots_out = slots;
+  return config_error;
+}
+
+template <int K, typename Pix>
+cudaError_t launch_ext(const FramePtrs &F, int nframes, int h, int w, const LaunchParams &P,
+                       const StreamBuffers &b, int run_rows, cudaStream_t stream,
+                       const StreamMarks *marks) {
+  const bool lattice = lattice_path(F, nframes, (int)sizeof(Pix), P);
+  cudaError_t e;
+  if (lattice) {
+    e = launch_lattice(F, nframes, h, w, (int)sizeof(Pix), P, b, run_rows, stream);
+    if (e != cudaSuccess)
+      return e;
+  } else {
+    int slots = 0;
+    if ((e = ext_slots<K, Pix>(&slots)) != cudaSuccess)
+      return e;
+    FrameSpans S;
+    run_rows = strip_spans(F, nframes, slots, run_rows, &S);
+    const unsigned blocks = (unsigned)((S.start[nframes] + kStripWarps - 1) / kStripWarps);
+    ext_strip<K, Pix><<<blocks, kStripWarps * 32, strip_smem<K, Pix>(), stream>>>(
+        F, nframes, S, run_rows, make_ext_tables(P), P, reinterpret_cast<uint8_t *>(b.cand),
+        b.words * sizeof(uint32_t));
+  }
+  if (marks)
+    cudaEventRecord(marks->stage01, stream);
+  const dim3 grid = band_grid(nframes, h);
+  const Kept kept = make_kept(b, h, w);
+  ext_decide<K, Pix><<<grid, kScanT, 0, stream>>>(F, P, b.cand, b.bits, b.words, kept,
+                                                  b.block_sums, b.cand_sums);
+  if (marks)
+    cudaEventRecord(marks->stage2, stream);
+  scatter_pixels<Pix, true><<<grid, kScanT, 0, stream>>>(
+      F, b.bits, b.words, b.cand, K + 2, kept, P.min_local, b.block_sums, b.cand_sums,
+      b.cand_limit, lattice ? b.counters + kCtrFault : nullptr, b.out, b.out_stride, b.capacity,
+      b.count_out, b.prefix);
+  if (marks)
+    cudaEventRecord(marks->order, stream);
+  return cudaGetLastError();
+}
+
+} // namespace
+
+int device_sms() {
+  static int cached = 0;
+  if (cached)
+    return cached;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      sms <= 0)
+    return 152;  // not cached: asked again once a device answers
+  cached = sms;
+  return cached;
+}
+
+bool streaming_path(const LaunchParams &P, int pixel_bytes) {
+  if (pixel_bytes == 2)
+    return true;
+  if (!(P.gain >= 0.0 && P.sigma_b >= 0.0 && P.sigma_s >= 0.0))
+    return false;
+  double lo, hi;
+  bracket_c(P, kMaxN0, &lo, &hi);
+  return hi < kMaxC8;
+}
+
+cudaError_t launch_extended(const FramePtrs &F, int nframes, int h, int w, int pixel_bytes,
+                            const LaunchParams &P, const StreamBuffers &b, int run_rows,
+                            cudaStream_t stream, const StreamMarks *marks) {
+  if (nframes < 1 || nframes > kMaxBatch || P.algorithm != SF_DISPERSION_EXTENDED ||
+      !streaming_path(P, pixel_bytes))
+    return cudaErrorInvalidValue;
+  if (marks)
+    cudaEventRecord(marks->start, stream);
+  auto launch = [&](auto k) {
+    constexpr int K = decltype(k)::value;
+    return pixel_bytes == 2 ? launch_ext<K, uint16_t>(F, nframes, h, w, P, b, run_rows, stream, marks)
+                            : launch_ext<K, uint32_t>(F, nframes, h, w, P, b, run_rows, stream, marks);
+  };
+  switch (P.half) {
+  case 2:
+    return launch(std::integral_constant<int, 2>());
+  case 3:
+    return launch(std::integral_constant<int, 3>());
+  case 4:
+    return launch(std::integral_constant<int, 4>());
+  default:
+    return cudaErrorInvalidValue;
+  }
+}
+
+int stream_default_run_rows(const LaunchParams &P, int h, int w, int nframes) {
+  if (P.half == 3 && P.int_ok)
+    return lattice_geometry(h, w, nframes, 0).run_rows;
+  int slots = 0;
+  const cudaError_t e = P.half == 2   ? ext_slots<2, uint32_t>(&slots)
+                        : P.half == 3 ? ext_slots<3, uint32_t>(&slots)
+                                      : ext_slots<4, uint32_t>(&slots);
+  if (e != cudaSuccess)
+    cudaGetLastError();
+  return strip_run_rows(h, (long long)nframes * strips_of(w), slots, 0);
+}
+
+} // namespace sf

@@ -1,0 +1,314 @@
+// What the kernels that decide a mask's pixels and write them out in order
+// share (sf_extended.cu, sf_dispersion.cu). A mask row is cut into runs of 4
+// words (128 pixels), numbered along the rows; a block takes whole bands of 8
+// rows, so that its runs, and the pixels it counts, are consecutive.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+#include "sf_common.cuh"
+#include "sf_scan.cuh"
+#include "sf_stream.cuh"
+
+namespace sf {
+
+constexpr int kScanT = 256;   // threads of a block
+constexpr int kRunWords = 4;  // words of a run
+constexpr int kBandRows = 8;  // rows of a band
+
+__host__ __device__ inline int runs_per_row(int width) {
+  return (((width + 31) >> 5) + kRunWords - 1) / kRunWords;
+}
+
+// This block's rows [lo, hi) of a frame, whole bands.
+__device__ __forceinline__ void band_share(int height, int *lo, int *hi) {
+  const int bands = (height + kBandRows - 1) / kBandRows;
+  const int share = (bands + (int)gridDim.x - 1) / (int)gridDim.x * kBandRows;
+  *lo = min(height, (int)blockIdx.x * share);
+  *hi = min(height, *lo + share);
+}
+
+// The grid: blocks a frame (a band each while kCountBlocks over the batch
+// allows), and the frames.
+inline dim3 band_grid(int nframes, int height) {
+  const int bands = (height + kBandRows - 1) / kBandRows, most = kCountBlocks / nframes;
+  return dim3((unsigned)(bands < most ? bands : most), (unsigned)nframes);
+}
+
+// Sum of the block's predecessors' counts in its frame, and the frame's
+// total.
+__device__ __forceinline__ uint32_t block_base(const uint32_t *__restrict__ block_sums,
+                                               uint32_t *total) {
+  __shared__ uint32_t s_base, s_total;
+  if (threadIdx.x < 32) {
+    const uint32_t *bs = block_sums + (size_t)blockIdx.y * gridDim.x;
+    uint32_t b = 0, t = 0;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += 32) {
+      const uint32_t v = bs[i];
+      b += i < blockIdx.x ? v : 0u;
+      t += v;
+    }
+    for (int o = 16; o; o >>= 1) {
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+      t += __shfl_xor_sync(0xffffffffu, t, o);
+    }
+    if (threadIdx.x == 0) {
+      s_base = b;
+      s_total = t;
+    }
+  }
+  __syncthreads();
+  *total = s_total;
+  return s_base;
+}
+
+// The k-th set bit (from 0) of a word that has more than k.
+__device__ __forceinline__ int select_bit(uint32_t w, uint32_t k) {
+  int at = 0;
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const uint32_t c = __popc(w & ((1u << s) - 1u));
+    if (k >= c) {
+      k -= c;
+      w >>= s;
+      at += s;
+    }
+  }
+  return at;
+}
+
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o)
+      v += t;
+  }
+  return v;
+}
+
+// Results kept between the two kernels, the passing pixels' backgrounds and
+// populations: `keep` places a run. What did not fit is summed again.
+struct Kept {
+  uint2 *res;
+  uint32_t stride, keep;  // places a frame, and a run
+};
+inline Kept make_kept(const StreamBuffers &b, int h, int w) {
+  return {b.res, b.res_stride,
+          (uint32_t)(b.res_stride / ((size_t)h * (size_t)runs_per_row(w)))};
+}
+
+// The window's mean as the records hold it: float(RN_double(S / n)) is
+// RN_float(S / n) for S below 2^24 (sf_common.cuh), and 16-bit frames divide in
+// float. A window short of valid pixels has the mean 0 (dext.cc:204).
+template <typename Pix>
+__device__ __forceinline__ float window_mean(uint32_t n, unsigned long long S,
+                                             uint32_t min_local) {
+  if (n < min_local)
+    return 0.0f;
+  return sizeof(Pix) == 2 || S < (1ull << 24)
+             ? __fdiv_rn(__uint2float_rn((uint32_t)S), __uint2float_rn(n))
+             : __double2float_rn(__ddiv_rn(__ull2double_rn(S), (double)n));
+}
+
+// A lane's run: its row, first word and words (zeros past the row's end).
+struct LaneRun {
+  int y, word;
+  uint32_t w[kRunWords];
+};
+__device__ __forceinline__ LaneRun load_run(const uint32_t *bits, uint32_t run, uint32_t end,
+                                            uint32_t rpr, uint32_t wpr) {
+  LaneRun r;
+  const uint32_t y = run / rpr, first = (run - y * rpr) * kRunWords;
+  r.y = (int)y;
+  r.word = (int)first;
+#pragma unroll
+  for (int k = 0; k < kRunWords; k++)
+    r.w[k] = run < end && first + k < wpr ? bits[(size_t)y * wpr + first + k] : 0u;
+  return r;
+}
+__device__ __forceinline__ uint32_t run_pixels(const LaneRun &r) {
+  uint32_t c = 0;
+#pragma unroll
+  for (int k = 0; k < kRunWords; k++)
+    c += (uint32_t)__popc(r.w[k]);
+  return c;
+}
+
+// The set pixels of a warp's 32 consecutive runs (a lane each; incl the
+// inclusive prefix of their counts), in order, 32 / kLanes at a time with
+// kLanes lanes each: visit(live, q, rank, owner, k, bit, y, x), q the pixel's
+// place among them, rank its place in its run, owner the lane that holds the
+// run, k its word there. The whole warp calls it.
+template <int kLanes, class Visit>
+__device__ __forceinline__ void visit_pixels(const LaneRun &r, uint32_t incl, int lane,
+                                             Visit visit) {
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+  const uint32_t excl = incl - run_pixels(r);
+  for (uint32_t q0 = 0; q0 < total; q0 += 32 / kLanes) {  // warp-uniform
+    const uint32_t q = q0 + lane / kLanes;
+    const bool live = q < total;
+    int owner = 0;
+#pragma unroll
+    for (int s = 16; s; s >>= 1)
+      owner += __shfl_sync(0xffffffffu, incl, owner + s - 1) <= q ? s : 0;
+    owner &= 31;
+    const uint32_t rank = q - __shfl_sync(0xffffffffu, excl, owner);
+    uint32_t left = rank, word = 0;
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < kRunWords; i++) {
+      const uint32_t x = __shfl_sync(0xffffffffu, r.w[i], owner), c = (uint32_t)__popc(x);
+      word = k == i ? x : word;
+      if (k == i && i + 1 < kRunWords && left >= c) {
+        left -= c;
+        k = i + 1;
+      }
+    }
+    const int bit = live ? select_bit(word, left) : 0;
+    const int y = __shfl_sync(0xffffffffu, r.y, owner);
+    const int x = (__shfl_sync(0xffffffffu, r.word, owner) + k) * 32 + bit;
+    visit(live, q, rank, owner, k, bit, y, x);
+  }
+}
+
+// The count and sum of a clipped window's pixels, by the whole warp: valid
+// ones, and outside the mask `out` where one is given.
+template <typename Pix>
+__device__ __noinline__ void sum_window(const Pix *image, const uint32_t *out, int height,
+                                        int width, int half, int y, int x, uint32_t *n_out,
+                                        unsigned long long *S_out) {
+  const int side = 2 * half + 1;
+  const uint32_t wpr = ((uint32_t)width + 31u) >> 5;
+  uint32_t n = 0;
+  unsigned long long S = 0;
+  for (int i = threadIdx.x & 31; i < side * side; i += 32) {
+    const int yy = y - half + i / side, xx = x - half + i % side;
+    if (yy < 0 || yy >= height || xx < 0 || xx >= width)
+      continue;
+    const uint32_t v = __ldg(image + (size_t)yy * width + xx);
+    const uint32_t o = out ? __ldg(out + (size_t)yy * wpr + (xx >> 5)) >> (xx & 31) & 1u : 0u;
+    if (v < Traits<Pix>::kMasked && o == 0u) {
+      n++;
+      S += v;
+    }
+  }
+  __syncwarp();
+  *n_out = __reduce_add_sync(0xffffffffu, n);
+#pragma unroll
+  for (int s = 16; s; s >>= 1)
+    S += __shfl_xor_sync(0xffffffffu, S, s);
+  *S_out = S;
+}
+
+// The mask's pixels as records, ascending by index (src/spots/dext.cc:212-220
+// emits in scan order), each at its place from the blocks' counts, and, when
+// asked for, each word's place. Their results come from their run's places
+// (kByRun), or from those of the warp's 32 runs together; a pixel beyond them
+// has its window summed again (half its half-width, `excluded` the mask that
+// its pixels are outside of, if any). With cand_sums (the blocks' counts of
+// candidates) a frame of more than cand_limit of them reports an overflowing
+// count; with a fault recorded (a device wait that ran out) every count says so.
+template <typename Pix, bool kByRun>
+__global__ void __launch_bounds__(kScanT, 6)
+scatter_pixels(const __grid_constant__ FramePtrs F, const uint32_t *__restrict__ bits_all,
+               size_t words, const uint32_t *__restrict__ excluded_all, int half, Kept kept,
+               uint32_t min_local, const uint32_t *__restrict__ block_sums,
+               const uint32_t *__restrict__ cand_sums, uint32_t cand_limit,
+               const uint32_t *__restrict__ fault, sf_signal_pixel *__restrict__ out_all,
+               size_t out_stride, uint32_t capacity, uint32_t *__restrict__ count_out,
+               uint32_t *__restrict__ prefix_all) {
+  const int f = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Pix *image = reinterpret_cast<const Pix *>(F.image[f]);
+  const int height = F.h[f], width = F.w[f];
+  const uint32_t wpr = ((uint32_t)width + 31u) >> 5, rpr = (uint32_t)runs_per_row(width);
+  const uint32_t *bits = bits_all + (size_t)f * words;
+  const uint32_t *excluded = excluded_all ? excluded_all + (size_t)f * words : nullptr;
+  const uint2 *res = kept.res + (size_t)f * kept.stride;
+  sf_signal_pixel *out = out_all + (size_t)f * out_stride;
+  uint32_t total;
+  uint32_t pos = block_base(block_sums, &total);
+  if (blockIdx.x == 0 && warp == 0) {
+    uint32_t cand = 0;
+    if (cand_sums)
+      for (uint32_t i = lane; i < gridDim.x; i += 32)
+        cand += cand_sums[(size_t)f * gridDim.x + i];
+    cand = __reduce_add_sync(0xffffffffu, cand);
+    if (lane == 0)
+      count_out[f] = fault && *fault ? kCountFault : cand > cand_limit ? 0xFFFFFFFFu : total;
+  }
+  // Each warp's share of the block's runs, in order, and its pixels' first
+  // place: counted first, then written (a block scan for each 256 runs
+  // instead cost two barriers each).
+  __shared__ uint32_t s_warp[kScanT / 32];
+  int row_lo, row_hi;
+  band_share(height, &row_lo, &row_hi);
+  const uint32_t run_lo = (uint32_t)row_lo * rpr, run_hi = (uint32_t)row_hi * rpr;
+  const uint32_t share = ((run_hi - run_lo + kScanT - 1) / kScanT) * 32u;
+  const uint32_t lo = min(run_hi, run_lo + (uint32_t)warp * share), end = min(run_hi, lo + share);
+  uint32_t mine = 0;
+  for (uint32_t run0 = lo; run0 < end; run0 += 32)
+    mine += run_pixels(load_run(bits, run0 + lane, end, rpr, wpr));
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0)
+    s_warp[warp] = mine;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kScanT / 32; k++)
+    pos += k < warp ? s_warp[k] : 0u;
+  if (!prefix_all && mine == 0)
+    return;  // whole warp
+  for (uint32_t run0 = lo; run0 < end; run0 += 32) {
+    const LaneRun r = load_run(bits, run0 + lane, end, rpr, wpr);
+    const uint32_t incl = warp_inclusive(run_pixels(r), lane);
+    if (prefix_all) {
+      uint32_t at = pos + incl - run_pixels(r);
+#pragma unroll
+      for (int k = 0; k < kRunWords; k++) {
+        if (run0 + lane < end && (uint32_t)r.word + k < wpr)
+          prefix_all[(size_t)f * words + (size_t)r.y * wpr + r.word + k] = at;
+        at += (uint32_t)__popc(r.w[k]);
+      }
+    }
+    visit_pixels<1>(r, incl, lane,
+                    [&](bool live, uint32_t q, uint32_t rank, int owner, int, int, int y, int x) {
+                      const uint32_t index = (uint32_t)y * (uint32_t)width + (uint32_t)x;
+                      const uint32_t held = kByRun ? kept.keep : 32u * kept.keep;
+                      const uint32_t place = kByRun ? rank : q;
+                      const size_t at =
+                          (size_t)(run0 + (kByRun ? (uint32_t)owner : 0u)) * kept.keep + place;
+                      uint2 b = make_uint2(0u, 0u);
+                      uint32_t value = 0;
+                      if (live) {
+                        value = (uint32_t)__ldg(image + index);
+                        if (place < held)
+                          b = __ldg(res + at);
+                      }
+                      for (unsigned more = __ballot_sync(0xffffffffu, live && place >= held); more;
+                           more &= more - 1u) {
+                        const int k = __ffs(more) - 1;
+                        uint32_t n;
+                        unsigned long long S;
+                        sum_window(image, excluded, height, width, half,
+                                   __shfl_sync(0xffffffffu, y, k), __shfl_sync(0xffffffffu, x, k),
+                                   &n, &S);
+                        if (lane == k)
+                          b = make_uint2(__float_as_uint(window_mean<Pix>(n, S, min_local)), n);
+                      }
+                      if (live && pos + q < capacity) {
+                        sf_signal_pixel rec;
+                        rec.index = index;
+                        rec.value = value;
+                        rec.background = __uint_as_float(b.x);
+                        rec.population = (uint16_t)b.y;
+                        rec.reserved = 0;
+                        out[pos + q] = rec;
+                      }
+                    });
+    pos += __shfl_sync(0xffffffffu, incl, 31);
+  }
+}
+
+} // namespace sf

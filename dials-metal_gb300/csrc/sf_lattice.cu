@@ -8,11 +8,6 @@
 //                a candidate of the bound; the candidates that fail leave the
 //                mask, which is then the reference's candidate mask
 //
-// The reference's eroded mask (stage 1's signal after the erosion, which
-// stage 2 keeps out of each background) is the candidate mask with the
-// masked pixels added, and stage 2 reads it so: the candidate mask's bits
-// and its staged pixels' masked values. No separate eroded mask is written.
-//
 // Why the bound holds. The erosion (src/spots/dext.cc:117-142) keeps a valid
 // pixel only if every in-frame pixel of its 5 x 5 neighbourhood is signal or
 // masked after stage 0. ANDing over only the lattice pixels of the
@@ -23,7 +18,7 @@
 // and around spots.
 //
 // The lattice decisions are an upper bound too: a window counts as signal
-// when the lower of the two integer bounds of sf_stream.cuh says it may be,
+// when the lower of the two integer bounds of sf_lattice.cuh says it may be,
 // and when its sums may not be exact. Valid pixels are summed saturated at
 // kLatCap (2^15 - 1), so every packed sum is exact for the saturated values;
 // a window whose saturated sum S is below kLatCap - 1 holds no saturated
@@ -33,22 +28,20 @@
 //
 // The tile check decides only the stage-0 windows within 2 of a candidate
 // (the only ones whose decision can clear one), about a fifth of a tile's,
-// spread over the warp's lanes. Its 18 x 38 pixels cover the stage-2 window
-// (11 x 11) of every candidate of the tile, so it is also where a frame is
-// marked for the 64-bit stage 2: a tile holding a valid pixel at or above
-// narrow_max marks its frame.
+// spread over the warp's lanes.
 
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
 #include <cudaTypedefs.h>
 
 #include "sf_common.cuh"
-#include "sf_stream.cuh"
+#include "sf_lattice.cuh"
 #include "sf_strips.cuh"
 #include "sf_tma.cuh"
 
@@ -65,12 +58,8 @@ constexpr int kLatOcc = 5;                  // blocks an SM the kernel is built 
 constexpr uint32_t kLatPS = 26;             // masked count above a 26-bit sum
 constexpr uint32_t kLatMask = (1u << kLatPS) - 1u;
 constexpr uint32_t kLatCap = 32767;         // valid pixels saturate here
-constexpr int kDec = 8;                     // fixed-point bits of clo / chi
 
 static_assert(kLatOut % 24 == 0, "lane pairs write whole bytes");
-
-// Marks a tile of stage 2's list whose candidates all failed the exact check.
-constexpr uint32_t kNoTile = 0xFFFFFFFFu;
 
 static_assert(kLatN0 * kLatCap < (1u << kLatPS), "saturated sums stay below the count field");
 
@@ -170,7 +159,6 @@ __device__ __forceinline__ void lat_row(const uint32_t v[kLatCols], int lane, ui
 // rows, with 4 | width, start 8-byte aligned). Both fetch 96 pieces from
 // column X - 12, and lane l reads its 12 pixels from column 12 l of the slot.
 constexpr int kRingSlots = 4;
-constexpr int kRingPieces = 96;   // pieces fetched a row: 3 a lane
 constexpr int kRingStride = 384;  // pixels a slot
 template <typename Pix>
 constexpr size_t ring_bytes() {
@@ -343,7 +331,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
         mprev[k] = mcur[k];
       continue;  // warp-uniform: the windows are not yet whole
     }
-    // Lattice row p0 - 1: four decisions by the lower bound (sf_stream.cuh),
+    // Lattice row p0 - 1: four decisions by the lower bound (sf_lattice.cuh),
     // windows whose sums may be inexact taken as signal, masked centres set.
     uint32_t b4 = cmprev;
 #pragma unroll
@@ -415,12 +403,10 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
 // loads' latency is hidden behind the arithmetic. Column sums of 7 rows go to
 // shared memory; then only the stage-0 windows within 2 of a candidate (the
 // only ones that can clear one, about a fifth of the tile's) are decided,
-// spread over the lanes: the two bounds of sf_stream.cuh, and the reference's
+// spread over the lanes: the two bounds of sf_lattice.cuh, and the reference's
 // sequence between them (sf_common.cuh). Tiles share mask words, so the
 // clearing is an atomic AND; each candidate belongs to one tile, so the order
-// does not matter. A tile's 18 x 38 pixels cover the stage-2 window (11 x 11)
-// of each of its candidates, so a tile holding a valid pixel at or above
-// narrow_max marks its frame for the 64-bit stage 2.
+// does not matter.
 // ---------------------------------------------------------------------------
 constexpr int kVerRows = 8;                  // output rows of a tile
 constexpr int kVerTW = 28;                   // output columns of a tile
@@ -430,7 +416,6 @@ constexpr int kVerPC = 38;                   // pixel columns
 constexpr int kVerPW = 44;                   // staged columns: 11 16-byte pieces
 constexpr int kVerWarps = 4;
 constexpr int kVerOcc = 6;                   // exact-check blocks an SM (a pixel buffer a warp)
-constexpr int kS2Occ = 5;                    // stage-2 blocks an SM (two pixel buffers a warp)
 
 __host__ __device__ inline int ver_ntx(int w) { return (w + kVerTW - 1) / kVerTW; }
 __host__ __device__ inline int ver_nty(int h) { return (h + kVerRows - 1) / kVerRows; }
@@ -719,8 +704,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
            int env_h, int env_w, int vec, const __grid_constant__ LaunchParams P,
            const __grid_constant__ StreamTables T, uint32_t *__restrict__ final_all, size_t words,
            const uint32_t *__restrict__ list,
-           uint32_t *__restrict__ counters, FastDiv by_ntiles, FastDiv by_ntx,
-           uint32_t *__restrict__ list2) {
+           uint32_t *__restrict__ counters, FastDiv by_ntiles, FastDiv by_ntx) {
   extern __shared__ __align__(128) unsigned char ver_smem_raw[];
   // The launch gives 128 bytes more than the layout needs: the tile buffers
   // start on a 128-byte boundary whatever the base's alignment.
@@ -844,8 +828,6 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     const bool wide = !k16 && __any_sync(0xffffffffu, mx >= narrow2);
     if (!wide)
       stage_next();  // the windows come from the column sums, not the pixels
-    if (wide && lane == 0)
-      counters[kCtrBatch + (size_t)f * kCtrCount + kCtrWideFrame] = 1u;
     // The stage-0 positions within 2 of a candidate: lane d first forms row
     // d's (row r0 - 2 + d, bit = column c0 - 2 + bit), then every lane takes
     // its own column's rows of them, less those whose centre is masked (set
@@ -922,9 +904,8 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
       D[d] = __ballot_sync(0xffffffffu, (keep >> d) & 1u);
     __syncwarp();  // the next tile rewrites the shared rows
     // The exact erosion of the tile's rows; the candidates that fail leave
-    // the mask, and a tile with a candidate left goes on stage 2's list.
+    // the mask.
     uint32_t *fin = final_all + (size_t)f * words;
-    uint32_t left = 0;
 #pragma unroll
     for (int o = 0; o < kVerRows; o++) {
       uint32_t V = 0xFFFFFFFFu;
@@ -935,7 +916,6 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
 #pragma unroll
       for (int u = 1; u < 5; u++)
         H &= V >> u;
-      left |= cj[o] & H;
       const uint32_t clear = cj[o] & ~H;
       if (clear && lane < 2) {
         const unsigned long long c64 = (unsigned long long)clear << sh;
@@ -946,8 +926,6 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
         }
       }
     }
-    if (lane == 0)
-      list2[k] = left ? e : kNoTile;  // same place as in the tile list: no atomics
   }
   // After a fault: the load still in flight (bounded) before the buffer goes.
   if (tma && inflight)
@@ -955,287 +933,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
   cp_async_wait<0>();
 }
 
-// ---------------------------------------------------------------------------
-// Stage 2 (src/spots/dext.cc:151-222) on the listed tiles, after the exact
-// check: a candidate's background is the valid pixels of its clipped 11 x 11
-// window outside the eroded mask, and the tile's 18 x 38 pixels hold every
-// window of its candidates. A warp stages them with the candidate-mask words
-// over them (cp.async, the next tile's while it works on this one; a pixel is
-// in the eroded mask when its bit is set or it is masked), takes
-// column sums of 11 rows once per tile, then per candidate adds 11 of them
-// and runs the reference's test (sf_common.cuh). The result goes to the
-// candidate's place in the ascending candidate list, from the per-word list
-// positions of the candidate mask (mask_prefix); the mask itself is left as
-// it is until every position is taken (pass_sums clears the failures).
-// ---------------------------------------------------------------------------
-template <typename Pix> struct alignas(128) S2Warp {
-  TileBuf<Pix> pix[2];              // staged pixels, two tiles
-  uint64_t bar[2];                  // their TMA mbarriers
-  uint32_t ew[2][kVerPR][3];        // candidate-mask words over the staged columns
-  uint32_t cw[2][kVerRows][2];      // candidate-mask words of the tile's rows
-  uint32_t pw[2][kVerRows][2];      // their list positions
-  uint2 cs[kVerRows][kVerPC + 2];   // {count, sum} of 11 rows of background
-};
-
-template <typename Pix>
-__device__ __forceinline__ void s2_stage(S2Warp<Pix> &sm, int s, uint32_t e, const FramePtrs &F,
-                                         const TileMaps &M, int tma, int vec, uint32_t ntiles,
-                                         int ntx, const FastDiv &by_ntiles,
-                                         const FastDiv &by_ntx,
-                                         const uint32_t *__restrict__ final_all,
-                                         const uint32_t *__restrict__ prefix_all, size_t words,
-                                         int lane) {
-  const TileAt a = tile_at(e, ntiles, ntx, by_ntiles, by_ntx);
-  const int f = a.f, r0 = a.r0, c0 = a.c0;
-  const int height = F.h[f], width = F.w[f];
-  const int xs = tile_xs<Pix>(c0);
-  if (tma)
-    tma_stage<Pix>(sm.pix[s], &sm.bar[s], M, f, r0, xs, lane);
-  else
-    stage_pixels<Pix>(sm.pix[s].px, reinterpret_cast<const Pix *>(F.image[f]), height, width,
-                      vec, r0, xs, lane);
-  const int wpr = (width + 31) >> 5;
-  const uint32_t *fin = final_all + (size_t)f * words;
-  for (int k = lane; k < kVerPR * 3; k += 32) {
-    const int r = k / 3, j = k - 3 * r;
-    const int y = r0 - 5 + r, wd = (xs >> 5) + j;
-    uint32_t *dst = &sm.ew[s][r][j];
-    if (y >= 0 && y < height && wd >= 0 && wd < wpr)
-      cp_async4(dst, fin + (size_t)y * wpr + wd);
-    else
-      *dst = 0u;
-  }
-  if (lane < 2 * kVerRows) {
-    const int o = lane >> 1, wdx = (c0 >> 5) + (lane & 1);
-    const bool in = r0 + o < height && wdx < wpr;
-    const size_t at = (size_t)f * words + (size_t)(r0 + o) * wpr + wdx;
-    if (in) {
-      cp_async4(&sm.cw[s][o][lane & 1], final_all + at);
-      cp_async4(&sm.pw[s][o][lane & 1], prefix_all + at);
-    } else {
-      sm.cw[s][o][lane & 1] = 0u;
-      sm.pw[s][o][lane & 1] = 0u;
-    }
-  }
-}
-
-template <int kOcc, typename Pix>
-__global__ void __launch_bounds__(kVerWarps * 32, kOcc)
-lat_stage2(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps M, int tma,
-           int env_h, int env_w, int vec, const __grid_constant__ LaunchParams P,
-           const uint32_t *__restrict__ final_all, const uint32_t *__restrict__ prefix_all,
-           size_t words,
-           const uint32_t *__restrict__ list, uint32_t *__restrict__ counters,
-           uint32_t *__restrict__ cand_all, uint2 *__restrict__ res_all, uint32_t cand_cap,
-           FastDiv by_ntiles, FastDiv by_ntx) {
-  extern __shared__ __align__(128) unsigned char s2_smem_raw[];
-  // 128 bytes more than the layout: the tile buffers start on a 128-byte
-  // boundary whatever the base's alignment.
-  unsigned char *s2_smem = s2_smem_raw + ((128u - (smem_addr(s2_smem_raw) & 127u)) & 127u);
-  constexpr bool k16 = sizeof(Pix) == 2;
-  // A fault in the exact check leaves its tile list partly unwritten: nothing
-  // to do (the launch's counts report the fault).
-  if (counters[kCtrFault])
-    return;
-  S2Warp<Pix> &sm = reinterpret_cast<S2Warp<Pix> *>(s2_smem)[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  if (tma && lane == 0) {
-    mbar_init(&sm.bar[0], 1);
-    mbar_init(&sm.bar[1], 1);
-    mbar_init_fence();
-  }
-  __syncwarp();
-  uint32_t parity = 0;  // bit b: the phase the next wait on bar[b] waits for
-  // Tile numbers are laid out over the batch's largest frame.
-  const int ntx = ver_ntx(env_w);
-  const uint32_t ntiles = (uint32_t)ntx * (uint32_t)ver_nty(env_h);
-  // The exact check's tile list with the tiles left without a candidate
-  // marked kNoTile; a warp takes every nw-th entry and stages the next one it
-  // will check while it checks the current one.
-  const uint32_t count = counters[kCtrTiles];
-  const uint32_t nw = gridDim.x * kVerWarps;
-  auto next_live = [&](uint32_t from, uint32_t *at) {
-    uint32_t x = kNoTile;
-    for (; from < count; from += nw) {
-      x = list[from];
-      if (x != kNoTile)
-        break;
-    }
-    *at = from;
-    return from < count ? x : kNoTile;
-  };
-  uint32_t k, k1;
-  uint32_t e = next_live(blockIdx.x * kVerWarps + (threadIdx.x >> 5), &k);
-  uint32_t e1 = next_live(k + nw, &k1);
-  if (k < count)
-    s2_stage<Pix>(sm, 0, e, F, M, tma, vec, ntiles, ntx, by_ntiles, by_ntx, final_all,
-                  prefix_all, words, lane);
-  cp_async_commit();
-  uint32_t inflight = k < count ? 1u : 0u;  // bit b: a TMA load into buffer b not waited for
-  for (int s = 0; k < count; s ^= 1) {
-    if (k1 < count) {
-      s2_stage<Pix>(sm, s ^ 1, e1, F, M, tma, vec, ntiles, ntx, by_ntiles, by_ntx, final_all,
-                    prefix_all, words, lane);
-      inflight |= 2u >> s;
-    }
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncwarp();
-    const TileAt a = tile_at(e, ntiles, ntx, by_ntiles, by_ntx);
-    const int f = a.f, r0 = a.r0, c0 = a.c0;
-    const int height = F.h[f], width = F.w[f];
-    const int xs = tile_xs<Pix>(c0), off = (c0 - 5) - xs;
-    if (tma) {
-      inflight &= ~(1u << s);
-      if (!tma_landed<Pix>(sm.pix[s], &sm.bar[s], (parity >> s) & 1u, height, width, r0, xs,
-                           lane)) {
-        if (lane == 0)
-          atomicOr(counters + kCtrFault, 1u);
-        break;  // whole warp
-      }
-      parity ^= 1u << s;
-    }
-    const int w0 = c0 >> 5, sh = c0 & 31;
-    uint32_t cj[kVerRows], late = 0;
-    int incl = 0;
-#pragma unroll
-    for (int o = 0; o < kVerRows; o++) {
-      const unsigned long long x =
-          (unsigned long long)sm.cw[s][o][0] | (unsigned long long)sm.cw[s][o][1] << 32;
-      cj[o] = (uint32_t)(x >> sh) & ((1u << kVerTW) - 1u);
-      late |= cj[o] >> 22;
-      incl += __popc(cj[o]);
-    }
-    const int total = incl;  // the tile's candidates (the same in every lane)
-    if (total == 0) {
-      __syncwarp();
-      k = k1;
-      e = e1;
-      e1 = next_live(k1 + nw, &k1);
-      continue;
-    }
-    // Background by column: A = staged column off + lane, B = off + 32 + lane
-    // (needed only for candidates in the tile's last 6 columns). Valid
-    // pixels below 2^24 keep the sums of 121 of them within 32 bits; a tile
-    // holding a larger one sums each window in 64 bits instead.
-    uint32_t mx = 0;
-    const int npass = late ? 2 : 1;
-#pragma unroll
-    for (int pass = 0; pass < 2; pass++) {
-      if (pass == npass)
-        break;
-      if (pass == 1 && lane >= kVerPC - 32)
-        break;
-      const int j = off + 32 * pass + lane;
-      const int x = xs + j, wi = (x >> 5) - (xs >> 5), b = x & 31;
-      uint32_t bn[kVerPR], bs[kVerPR];
-#pragma unroll
-      for (int r = 0; r < kVerPR; r++) {
-        const uint32_t v = sm.pix[s].px[r][j];
-        const bool eroded = (sm.ew[s][r][wi] >> b) & 1u;
-        const bool bg = !is_masked_px<Pix>(v) && !eroded;
-        if (!k16)
-          mx = max(mx, v + 2u);
-        bn[r] = bg ? 1u : 0u;
-        bs[r] = bg ? v : 0u;
-      }
-      uint32_t cn = 0, cs = 0;
-#pragma unroll
-      for (int r = 0; r < 10; r++) {
-        cn += bn[r];
-        cs += bs[r];
-      }
-#pragma unroll
-      for (int o = 0; o < kVerRows; o++) {
-        cn += bn[o + 10];
-        cs += bs[o + 10];
-        sm.cs[o][32 * pass + lane] = make_uint2(cn, cs);
-        cn -= bn[o];
-        cs -= bs[o];
-      }
-    }
-    // 121 16-bit pixels sum below 2^23: 16-bit frames are never wide.
-    const bool wide = !k16 && __any_sync(0xffffffffu, mx >= (1u << 24) + 2u);
-    __syncwarp();
-    // The tile's candidates, spread over the lanes in order.
-    int pre[kVerRows];
-    {
-      int run = 0;
-#pragma unroll
-      for (int o = 0; o < kVerRows; o++) {
-        pre[o] = run;
-        run += __popc(cj[o]);
-      }
-    }
-    uint32_t *cand = cand_all + (size_t)f * cand_cap;
-    uint2 *res = res_all + (size_t)f * cand_cap;
-    for (int q = lane; q < total; q += 32) {
-      int o = 0;
-#pragma unroll
-      for (int e2 = 1; e2 < kVerRows; e2++)
-        o += q >= pre[e2] ? 1 : 0;
-      uint32_t bits = 0;
-#pragma unroll
-      for (int e2 = 0; e2 < kVerRows; e2++)
-        bits = e2 == o ? cj[e2] : bits;
-      const int tcol = (int)__fns(bits, 0u, q - pre[o] + 1);
-      uint32_t n = 0;
-      unsigned long long S = 0;
-      if (!wide) {
-        uint32_t s32 = 0;
-#pragma unroll
-        for (int u = 0; u < 11; u++) {
-          const uint2 c = sm.cs[o][tcol + u];
-          n += c.x;
-          s32 += c.y;
-        }
-        S = s32;
-      } else {
-        for (int r = o; r < o + 11; r++)
-          for (int u = 0; u < 11; u++) {
-            const int j = off + tcol + u, x = xs + j;
-            const uint32_t v = sm.pix[s].px[r][j];
-            const bool eroded = (sm.ew[s][r][(x >> 5) - (xs >> 5)] >> (x & 31)) & 1u;
-            if (!is_masked_px<Pix>(v) && !eroded) {
-              n++;
-              S += v;
-            }
-          }
-      }
-      const uint32_t p = sm.pix[s].px[o + 5][off + tcol + 5];
-      float bg = 0.0f;
-      // dext.cc:205: only pixels above the global threshold are tested.
-      bool sig = (uint64_t)p >= P.p_min;
-      if (sig) {
-        if constexpr (k16)
-          sig = stage2_u16(p, n, (uint32_t)S, P, &bg);  // the reference's float test
-        else
-          sig = stage2_u32(p, n, S, P, &bg);
-      }
-      const int x = c0 + tcol, jw = (x >> 5) - w0, bit = x & 31;
-      const uint32_t i = sm.pw[s][o][jw] + (uint32_t)__popc(sm.cw[s][o][jw] & ((1u << bit) - 1u));
-      if (i < cand_cap) {
-        cand[i] = (uint32_t)(r0 + o) * (uint32_t)width + (uint32_t)x;
-        res[i] = make_uint2(__float_as_uint(bg), n | (sig ? 1u << 16 : 0u));
-      }
-    }
-    __syncwarp();  // the next tile rewrites the shared sums
-    k = k1;
-    e = e1;
-    e1 = next_live(k1 + nw, &k1);
-  }
-  // After a fault: the load still in flight (bounded) before the buffers go.
-  for (int b = 0; b < 2; b++)
-    if (tma && ((inflight >> b) & 1u))
-      (void)mbar_wait(&sm.bar[b], (parity >> b) & 1u);
-  cp_async_wait<0>();
-}
-
-// Both add 128 bytes for aligning the tile buffers (see the kernels).
-template <typename Pix> constexpr size_t s2_smem_bytes() {
-  return sizeof(S2Warp<Pix>) * kVerWarps + 128;
-}
-
+// Adds 128 bytes for aligning the tile buffers (see the kernel).
 template <typename Pix> constexpr size_t ver_smem_bytes() {
   return sizeof(uint4) * 64 + sizeof(VerWarp<Pix>) * kVerWarps + 128;
 }
@@ -1278,31 +976,6 @@ template <typename Pix> int make_tile_maps(const FramePtrs &F, int nframes, int 
   return 1;
 }
 
-template <typename Pix>
-cudaError_t lattice_stage2(const FramePtrs &F, int nframes, int h, int w, int vec,
-                           const LaunchParams &P, const StreamBuffers &b, cudaStream_t stream) {
-  static std::once_flag configured;
-  static cudaError_t config_error = cudaSuccess;
-  static int blocks = 0;
-  std::call_once(configured, [] {
-    config_error = persistent_blocks(lat_stage2<kS2Occ, Pix>, s2_smem_bytes<Pix>(), &blocks);
-  });
-  if (config_error != cudaSuccess)
-    return config_error;
-  // The tiles the exact check left a candidate in (its second list).
-  const uint32_t *prefix = b.amb;
-  const size_t tiles = (size_t)ver_ntx(w) * (size_t)ver_nty(h);
-  const uint32_t *list = b.amb + (size_t)nframes * (b.words + tiles);
-  TileMaps M;
-  const int tma = make_tile_maps<Pix>(F, nframes, h, w, &M);
-  lat_stage2<kS2Occ, Pix><<<blocks * device_sms(), kVerWarps * 32, s2_smem_bytes<Pix>(),
-                             stream>>>(F, M, tma, h, w, vec, P, b.bits, prefix, b.words,
-                                       list, b.counters, b.cand, b.res, b.cand_cap,
-                                       make_fastdiv((uint32_t)tiles),
-                                       make_fastdiv((uint32_t)ver_ntx(w)));
-  return cudaGetLastError();
-}
-
 // Strips of a frame w wide (whole mask rows: the last strip reaches the end
 // of the row's last word).
 int lat_strips(int w) { return ((w + 31) / 32 * 32 + kLatOut - 1) / kLatOut; }
@@ -1321,7 +994,7 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, int vec, cons
   }
   const size_t mask_bytes = b.words * sizeof(uint32_t);
   const unsigned lb = (unsigned)((S.start[nframes] + kLatWarps - 1) / kLatWarps);
-  uint8_t *fin = reinterpret_cast<uint8_t *>(b.bits);
+  uint8_t *fin = reinterpret_cast<uint8_t *>(b.cand);
   if (sizeof(Pix) == 2 || vec)
     lat_stage01<kLatOcc, true, Pix><<<lb, kLatWarps * 32, ring_bytes<Pix>(), stream>>>(
         F, nframes, vec, S, run_rows, T, P, fin, mask_bytes);
@@ -1337,9 +1010,6 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, int vec, cons
   });
   if (config_error != cudaSuccess)
     return config_error;
-  // The ambiguous-mask buffer of the other streaming path holds, here, the
-  // candidate mask's per-word list positions (stage 2), the tile list and the
-  // list of tiles the exact check leaves a candidate in.
   // Tile groups: each frame's tile rows x groups of 32 tiles.
   FrameSpans G;
   G.start[0] = 0;
@@ -1356,17 +1026,16 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, int vec, cons
   const long long twarps = (tgroups + trun - 1) / trun;
   const unsigned tb = (unsigned)((twarps + 7) / 8);
   const size_t tiles = (size_t)ver_ntx(w) * (size_t)ver_nty(h);
-  uint32_t *list = b.amb + (size_t)nframes * b.words;
+  uint32_t *list = b.tiles;
   const FastDiv by_ntiles = make_fastdiv((uint32_t)tiles);
   const FastDiv by_ntx = make_fastdiv((uint32_t)ver_ntx(w));
-  lat_tiles<<<tb, 256, 0, stream>>>(F, nframes, h, w, b.bits, b.words, list, b.counters, G,
+  lat_tiles<<<tb, 256, 0, stream>>>(F, nframes, h, w, b.cand, b.words, list, b.counters, G,
                                     trun);
   TileMaps M;
   const int tma = make_tile_maps<Pix>(F, nframes, h, w, &M);
   lat_verify<kVerOcc, Pix><<<ver_blocks * device_sms(), kVerWarps * 32, ver_smem_bytes<Pix>(),
-                             stream>>>(F, M, tma, h, w, vec, P, T, b.bits, b.words, list,
-                                       b.counters, by_ntiles, by_ntx,
-                                       list + (size_t)nframes * tiles);
+                             stream>>>(F, M, tma, h, w, vec, P, T, b.cand, b.words, list,
+                                       b.counters, by_ntiles, by_ntx);
   return cudaGetLastError();
 }
 
@@ -1405,23 +1074,16 @@ bool encode_frame_map(CUtensorMap *map, const void *base, int h, int w, int byte
 
 size_t lattice_tiles(int h, int w) { return (size_t)ver_ntx(w) * (size_t)ver_nty(h); }
 
-cudaError_t launch_lattice_stage2(const FramePtrs &F, int nframes, int h, int w, int vec,
-                                  int pixel_bytes, const LaunchParams &P, const StreamBuffers &b,
-                                  cudaStream_t stream) {
-  return pixel_bytes == 2 ? lattice_stage2<uint16_t>(F, nframes, h, w, vec, P, b, stream)
-                          : lattice_stage2<uint32_t>(F, nframes, h, w, vec, P, b, stream);
-}
-
 // The run length for a launch whose tallest frame has h rows and whose
 // frames have `strips` strips in all: the resident warps filled once (no
 // tail wave) by the tallest frame's runs, unless run_rows is given; at least
-// kMinRunRows, in whole triples of rows.
+// kLatMinRunRows, in whole triples of rows.
 static int lat_run_rows(int h, long long strips, int run_rows) {
   if (run_rows <= 0) {
     const long long nruns = std::max(1ll, (long long)lat_slots() / std::max(1ll, strips));
     run_rows = (int)((h + nruns - 1) / nruns);
   }
-  run_rows = std::max(run_rows, kMinRunRows);
+  run_rows = std::max(run_rows, kLatMinRunRows);
   return (run_rows + 2) / 3 * 3;
 }
 
@@ -1433,14 +1095,52 @@ LatticeGeometry lattice_geometry(int h, int w, int nframes, int run_rows) {
   return g;
 }
 
-cudaError_t launch_lattice(const FramePtrs &F, int nframes, int h, int w, int vec,
-                           int pixel_bytes, const LaunchParams &P, const StreamTables &T,
-                           const StreamBuffers &b, int run_rows, cudaStream_t stream) {
+// The lattice pass's and the tile check's constants (sf_lattice.cu): a window
+// of 49 pixels, its masked count above a 26-bit sum.
+static void make_stream_tables(const LaunchParams &P, StreamTables *T) {
+  constexpr int n0 = 49;
+  // Exact 32-bit sums: the count and sum packed below 2^32, and the window's
+  // sum of p^2 below 2^32 (p < sqrt(2^32 / n0) = 9362).
+  const uint32_t by_pack = ((1u << 26) - 1u) / (uint32_t)n0;
+  uint32_t by_sq = (uint32_t)std::floor(std::sqrt(4294967295.0 / n0));
+  while ((uint64_t)by_sq * by_sq * (uint64_t)n0 > 0xFFFFFFFFull)
+    by_sq--;
+  T->narrow_max = std::min(by_pack, by_sq + 1);
+  for (int n = 0; n <= kMaxN0; n++) {
+    const bool testable = n >= 1 && (uint32_t)n >= P.min_local && n <= n0;
+    // 2^8 (n - 1 + sigma_b r_n) bracketed from r_n's 2^-20 floor and ceiling.
+    const uint64_t sb = P.sigma_b_int;
+    const uint64_t lo = testable ? (sb * P.root_lo[n]) >> (kRootShift - kDec) : 0;
+    const uint64_t hi =
+        testable ? (sb * P.root_hi[n] + ((1ull << (kRootShift - kDec)) - 1)) >>
+                       (kRootShift - kDec)
+                 : 0;
+    const uint64_t base = testable ? (uint64_t)(n - 1) << kDec : 0;
+    T->clo[n] = (uint32_t)(base + lo);
+    T->chi[n] = (uint32_t)(base + hi);
+    // nk 0 makes every such window "surely not" (0 <= S (2^8 S + clo)).
+    T->nk[n] = testable ? (uint32_t)n << kDec : 0u;
+  }
+}
+
+cudaError_t launch_lattice(const FramePtrs &F, int nframes, int h, int w, int pixel_bytes,
+                           const LaunchParams &P, const StreamBuffers &b, int run_rows,
+                           cudaStream_t stream) {
   if (P.half != kLatK)
     return cudaErrorInvalidValue;
+  const cudaError_t e =
+      cudaMemsetAsync(b.counters, 0, kCounterWords * sizeof(uint32_t), stream);
+  if (e != cudaSuccess)
+    return e;
+  StreamTables T;
+  make_stream_tables(P, &T);
+  int vec = 1;
   long long strips = 0;
-  for (int f = 0; f < nframes; f++)
+  for (int f = 0; f < nframes; f++) {
     strips += lat_strips(F.w[f]);
+    if (F.w[f] % 4 != 0 || reinterpret_cast<uintptr_t>(F.image[f]) % (4 * pixel_bytes) != 0)
+      vec = 0;
+  }
   const int rr = lat_run_rows(h, strips, run_rows);
   return pixel_bytes == 2 ? lattice<uint16_t>(F, nframes, h, w, vec, P, T, b, rr, stream)
                           : lattice<uint32_t>(F, nframes, h, w, vec, P, T, b, rr, stream);

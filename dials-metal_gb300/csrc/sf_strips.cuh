@@ -1,10 +1,16 @@
-// What the kernels that walk strips of a frame share (sf_lattice.cu,
-// sf_dispersion.cu): a batch's division into each frame's own strips x runs,
-// and the asynchronous copies that stage pixel rows in shared memory.
+// What the kernels that walk strips of a frame share (sf_extended.cu,
+// sf_dispersion.cu). A warp walks down a strip of 360 output columns for a run
+// of rows. Lane l owns 12 columns; lanes 1-30 write, and lanes 0 and 31 hold the
+// columns on either side of the strip that the others' windows reach into.
+// Each pixel row is staged in shared memory by cp.async a row or two ahead and
+// stays there until it leaves the window.
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "sf_stream.cuh"
 
@@ -36,10 +42,9 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv &f) {
   return (t + ((n - t) >> f.s1)) >> f.s2;
 }
 
-// Where each frame's share of a launch's warps (lat_stage01: strips x runs)
-// or tile groups (lat_tiles: tile rows x groups of 32 tiles) starts, and how
-// many make one of its rows: every frame of a batch, mixed shapes or not,
-// gets exactly its own.
+// Where each frame's share of a launch's warps (strips x runs) starts, and its
+// strips a run: every frame of a batch, mixed shapes or not, gets exactly its
+// own.
 struct FrameSpans {
   int start[kMaxBatch + 1];
   FastDiv by_row[kMaxBatch];
@@ -89,6 +94,246 @@ __device__ __forceinline__ void cp_async_commit() {
 }
 template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+
+constexpr int kCols = 12;              // columns a lane owns
+constexpr int kStripOut = kCols * 30;  // output columns a warp
+constexpr int kStripStride = kCols * 32;  // pixels a staged row
+constexpr int kStripWarps = 2;         // warps a block
+// A window's masked count above its sum: 81 << 25 and 81 x 65533 both fit.
+constexpr uint32_t kCountShift = 25;
+constexpr uint32_t kSumMask = (1u << kCountShift) - 1u;
+
+// Windows of 2K + 1 pixels square, with E rows of decisions either side of an
+// output row (0: none).
+template <int K> struct StripG {
+  static constexpr int W0 = 2 * K + 1;
+  static constexpr int N0 = W0 * W0;
+  // Rows in flight ahead of the current one, the staged rows (from the one
+  // leaving the window to the last in flight) and the blocks an SM that those
+  // of 32-bit frames leave room for. One row's arithmetic takes longer than a
+  // load, so few rows ahead and more warps.
+  static constexpr int Ahead = K == 4 ? 1 : 2;
+  static constexpr int Slots = W0 + Ahead + 1;
+  static constexpr int Occ = K == 2 ? 8 : K == 3 ? 7 : 6;
+  // Valid 32-bit pixels saturate at Cap, so that a window's sum of squares
+  // stays below 2^32. Below Big a window's sum is at most sqrt(N0 Big) =
+  // 2^13.5, and the products of the 32-bit tests stay below 2^32.
+  static constexpr uint32_t Cap = K == 2 ? 13107 : K == 3 ? 9362 : 7281;
+  static constexpr uint32_t Big = (1u << 27) / N0;
+  static_assert((unsigned long long)Cap * Cap * N0 < (1ull << 32) && Cap * Cap >= Big,
+                "exact squares, and a saturated pixel makes its window big");
+};
+constexpr uint32_t kMaxC16 = 1u << 17;  // keeps 16 S^2 + S c below 2^32 for S <= 2^13.5
+
+template <int K, typename Pix> constexpr size_t strip_smem() {
+  return (size_t)kStripWarps * StripG<K>::Slots * kStripStride * sizeof(Pix);
+}
+
+// A valid pixel's value, or a lone count bit for a masked one (whose square
+// wraps to 0).
+template <int K, typename Pix> __device__ __forceinline__ uint32_t pack_pixel(uint32_t v) {
+  if (sizeof(Pix) == 2)
+    return v >= 0xFFFEu ? 1u << kCountShift : v;
+  return v >= 0xFFFFFFFEu ? 1u << kCountShift : min(v, StripG<K>::Cap);
+}
+
+// A lane's 12 staged pixels, packed. 32-bit rows are packed in place when
+// they arrive (kRaw reads them first), 16-bit rows whenever they are read.
+template <int K, typename Pix, bool kRaw>
+__device__ __forceinline__ void read_row(Pix *slot, int lane, uint32_t v[kCols]) {
+  if constexpr (sizeof(Pix) == 2) {
+    const uint2 *src = reinterpret_cast<const uint2 *>(slot + kCols * lane);
+#pragma unroll
+    for (int i = 0; i < kCols / 4; i++) {
+      const uint2 x = src[i];
+      v[4 * i] = pack_pixel<K, Pix>(x.x & 0xFFFFu), v[4 * i + 1] = pack_pixel<K, Pix>(x.x >> 16);
+      v[4 * i + 2] = pack_pixel<K, Pix>(x.y & 0xFFFFu);
+      v[4 * i + 3] = pack_pixel<K, Pix>(x.y >> 16);
+    }
+  } else {
+    uint4 *src = reinterpret_cast<uint4 *>(slot + kCols * lane);
+#pragma unroll
+    for (int i = 0; i < kCols / 4; i++) {
+      uint4 x = src[i];
+      if (kRaw) {
+        x.x = pack_pixel<K, Pix>(x.x), x.y = pack_pixel<K, Pix>(x.y);
+        x.z = pack_pixel<K, Pix>(x.z), x.w = pack_pixel<K, Pix>(x.w);
+        src[i] = x;
+      }
+      v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+    }
+  }
+}
+
+// One warp's strip and run: where it reads and writes.
+struct StripRun {
+  int frame, height, width, bytes_per_row;
+  int X, cx;      // the strip's and this lane's first column
+  int ra, rb;     // output rows
+  bool writer, first_of_pair;
+  int pair_byte;  // this lane's first mask byte (lane pairs share three)
+  uint32_t inside12;
+};
+
+// False (for the whole warp) past the last strip.
+__device__ __forceinline__ bool strip_run(const FramePtrs &F, int nframes, const FrameSpans &S,
+                                          int run_rows, StripRun &r) {
+  const int lane = threadIdx.x & 31;
+  const int gw = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
+  if (gw >= S.start[nframes])
+    return false;
+  const int f = span_frame(S, nframes, gw);
+  const uint32_t local = (uint32_t)(gw - S.start[f]);
+  const int ry = (int)fast_div(local, S.by_row[f]);
+  const int sx = (int)(local - (uint32_t)ry * S.by_row[f].d);
+  r.frame = f;
+  r.height = F.h[f];
+  r.width = F.w[f];
+  r.bytes_per_row = ((r.width + 31) >> 5) * 4;
+  r.X = kStripOut * sx;
+  r.cx = r.X + kCols * (lane - 1);
+  r.ra = ry * run_rows;
+  r.rb = min(r.height, r.ra + run_rows);
+  r.writer = lane >= 1 && lane <= 30;
+  r.first_of_pair = (lane & 1) != 0;
+  r.pair_byte = (r.X + 24 * ((lane - 1) >> 1)) >> 3;
+  r.inside12 = (r.cx < 0 || r.cx >= r.width)
+                   ? 0u
+                   : (r.cx + kCols <= r.width ? 0xFFFu : ((1u << (r.width - r.cx)) - 1u));
+  return true;
+}
+
+// The strip's pixel rows [pbeg, pend), fetched in turn into slots of the ring.
+// Where the frame's rows are whole aligned pieces of 4 pixels a lane copies
+// pieces l, l + 32, l + 64 (a warp's copy covers 128 pixels), else pixels a
+// lane apart. Bit u of `inside`: its u-th piece or pixel lies in the frame;
+// what lies off it is staged as masked.
+template <typename Pix> struct RowReader {
+  const Pix *next_row;
+  int next_p, pend, width, lane;
+  uint32_t inside;
+  bool aligned;
+
+  __device__ __forceinline__ RowReader(const Pix *image, const StripRun &r, int pbeg, int rows)
+      : next_p(pbeg), pend(min(r.height, pbeg + rows)), width(r.width),
+        lane(threadIdx.x & 31), inside(0) {
+    aligned = width % 4 == 0 && reinterpret_cast<uintptr_t>(image) % (4 * sizeof(Pix)) == 0;
+    const int x0 = r.X - kCols;  // the staged row's first column
+#pragma unroll
+    for (int u = 0; u < kCols; u++) {
+      const int c = aligned ? x0 + 4 * lane + 128 * u : x0 + lane + 32 * u;
+      const bool in = aligned ? u < 3 && c >= 0 && c + 4 <= width : c >= 0 && c < width;
+      inside |= in ? 1u << u : 0u;
+    }
+    next_row = image + (ptrdiff_t)pbeg * width + x0 + (aligned ? 4 * lane : lane);
+  }
+  __device__ __forceinline__ void fetch(Pix *slot) {
+    const uint32_t in = next_p >= 0 && next_p < pend ? inside : 0u;
+    if (aligned) {
+      Pix *dst = slot + 4 * lane;
+#pragma unroll
+      for (int u = 0; u < 3; u++) {
+        if ((in >> u) & 1u)
+          cp_async_piece<Pix>(dst + 128 * u, next_row + 128 * u);
+        else
+          fill_piece_masked<Pix>(dst + 128 * u);
+      }
+    } else {
+      Pix *dst = slot + lane;
+#pragma unroll
+      for (int u = 0; u < kCols; u++) {
+        if constexpr (sizeof(Pix) == 4) {
+          if ((in >> u) & 1u)
+            cp_async4(dst + 32 * u, next_row + 32 * u);
+          else
+            dst[32 * u] = (Pix)~0u;
+        } else {
+          dst[32 * u] = (in >> u) & 1u ? __ldg(next_row + 32 * u) : (Pix)~0u;
+        }
+      }
+    }
+    next_row += width;
+    next_p++;
+  }
+};
+
+// A lane's 12 mask bits of a row into the mask: lane pairs write three bytes,
+// the first lane (odd) two and the second the third. The whole warp calls it;
+// `row` is the row's pair_byte in a mask row that has `left` bytes from there.
+__device__ __forceinline__ void write_bits(const StripRun &r, uint8_t *row, int left,
+                                           uint32_t bits) {
+  const uint32_t next = __shfl_down_sync(0xffffffffu, bits, 1);
+  if (!r.writer)
+    return;
+  if (r.first_of_pair) {
+    if (left > 0)
+      row[0] = (uint8_t)bits;
+    if (left > 1)
+      row[1] = (uint8_t)((bits >> 8) | (next & 0xFu) << 4);
+  } else if (left > 2) {
+    row[2] = (uint8_t)(bits >> 4);
+  }
+}
+
+// The column sums V of a lane and, by shuffles, of the K columns either side
+// of its own, summed over the 2K + 1 columns around each of the 12.
+template <int K>
+__device__ __forceinline__ void window_sums(const uint32_t V[kCols], uint32_t h[kCols]) {
+  uint32_t e[kCols + 2 * K];
+#pragma unroll
+  for (int c = 0; c < kCols; c++)
+    e[K + c] = V[c];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    e[k] = __shfl_up_sync(0xffffffffu, V[kCols - K + k], 1);
+    e[K + kCols + k] = __shfl_down_sync(0xffffffffu, V[k], 1);
+  }
+  h[0] = 0u;
+#pragma unroll
+  for (int k = 0; k <= 2 * K; k++)
+    h[0] += e[k];
+#pragma unroll
+  for (int c = 1; c < kCols; c++)
+    h[c] = h[c - 1] + e[c + 2 * K] - e[c - 1];
+}
+
+// Host: strips of a frame w wide (whole mask rows), and the run length and
+// spans of a launch. run_rows 0: runs that fill `slots` resident warps
+// kStripWaves times over, so that warps of unequal cost even out (one wave
+// left a third of the warps' time idle), as long as a run keeps kLongRun
+// rows (each run reads some rows more than it writes); else once, down to
+// runs of kMinRunRows.
+constexpr int kMinRunRows = 8;
+constexpr int kLongRun = 64;
+constexpr int kStripWaves = 4;
+
+inline int strips_of(int w) { return ((w + 31) / 32 * 32 + kStripOut - 1) / kStripOut; }
+
+inline int strip_run_rows(int tallest, long long strips, int slots, int run_rows) {
+  if (run_rows <= 0) {
+    const long long runs = std::max(1ll, slots / std::max(1ll, strips));
+    const int once = (int)((tallest + runs - 1) / runs);
+    run_rows = std::min(once, std::max(kLongRun, (once + kStripWaves - 1) / kStripWaves));
+  }
+  return std::max(run_rows, kMinRunRows);
+}
+
+inline int strip_spans(const FramePtrs &F, int nframes, int slots, int run_rows, FrameSpans *S) {
+  long long strips = 0;
+  int tallest = 0;
+  for (int f = 0; f < nframes; f++) {
+    strips += strips_of(F.w[f]);
+    tallest = std::max(tallest, F.h[f]);
+  }
+  run_rows = strip_run_rows(tallest, strips, slots, run_rows);
+  S->start[0] = 0;
+  for (int f = 0; f < nframes; f++) {
+    S->start[f + 1] = S->start[f] + strips_of(F.w[f]) * ((F.h[f] + run_rows - 1) / run_rows);
+    S->by_row[f] = make_fastdiv((uint32_t)strips_of(F.w[f]));
+  }
+  return run_rows;
 }
 
 } // namespace sf

@@ -14,7 +14,7 @@ from concurrent.futures import ThreadPoolExecutor
 
 from . import _paths
 
-CUDA_SOURCES = ["sf_threshold.cu", "sf_stream.cu", "sf_lattice.cu", "sf_dispersion.cu", "sf_api.cu", "sf_label.cu",
+CUDA_SOURCES = ["sf_threshold.cu", "sf_lattice.cu", "sf_extended.cu", "sf_dispersion.cu", "sf_api.cu", "sf_label.cu",
                 "sf_serve.cu", "sf_refl.cu", "sf_decompress.cu", "sf_frames.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",

@@ -1,8 +1,8 @@
-"""The plain dispersion threshold's strips against the oracle, bit for bit:
-widths around a strip's 360 columns and a mask word's 32, rows that are whole
-aligned pieces of 4 pixels and rows that are not, heights around a run's
-rows, values at and beyond the strips' saturation and 2^32, masked bands, and
-parameters that leave the integer decisions."""
+"""Both algorithms' strips against the oracle, bit for bit: widths around a
+strip's 360 columns and a mask word's 32, rows that are whole aligned pieces of
+4 pixels and rows that are not, heights around a run's rows, values at and
+beyond the strips' saturation and 2^32, masked bands, and parameters that leave
+the integer decisions."""
 import numpy as np
 import pytest
 
@@ -23,30 +23,35 @@ def _frames(h, w, seed):
     masked[:, w // 2:w // 2 + 5] = 0xFFFFFFFE
     large = base.copy()
     hit = rng.random((h, w)) < 0.02
-    large[hit] = rng.choice(np.array([32765, 32766, 32767, 32768, 65532, 1 << 24, 0xFFFFFFFD],
-                                     np.uint32), int(hit.sum()))
+    large[hit] = rng.choice(np.array([7280, 7281, 7282, 9361, 9362, 9363, 13107, 13108, 65532,
+                                      (1 << 24) - 1, 1 << 24, 0xFFFFFFFD], np.uint32), int(hit.sum()))
+    spots = base.copy()
+    for _ in range(3):
+        spots[rng.integers(0, h), rng.integers(0, w)] = rng.choice([9362, 40000, 3_000_000_000])
     high = rng.integers(30000, 41000, (h, w)).astype(np.uint32)
     high[rng.random((h, w)) < 0.01] = 0xFFFFFFFF
-    return [base, masked, large, high]
+    return [base, masked, large, spots, high]
 
 
 def _as16(f):
     return np.where(f >= 0xFFFFFFFE, f & 0xFFFF, np.minimum(f, 65533)).astype(np.uint16)
 
 
+@pytest.mark.parametrize("algorithm", [0, 1])
 @pytest.mark.parametrize("bits", [32, 16])
 @pytest.mark.parametrize("kernel", [2, 3, 4])
 @pytest.mark.parametrize("h,w", [(1, 1), (5, 31), (23, 360), (8, 364), (37, 361), (61, 724),
                                  (130, 1030), (257, 392)])
-def test_strips_against_oracle(h, w, kernel, bits):
+def test_strips_against_oracle(h, w, kernel, bits, algorithm):
     import torch
     from sfgb import api
     frames = _frames(h, w, h * 10000 + w)
     if bits == 16:
         frames = [_as16(f) for f in frames]
     for kw in (dict(), dict(gain=1.5, sigma_b=4.25, sigma_s=0.0, min_local=0),
+               dict(sigma_b=1000.0, sigma_s=2.0), dict(sigma_b=2.5, gain=0.7),
                dict(gain=0.0, sigma_s=2.5, min_local=20, global_threshold=5.0)):
-        p = dict(algorithm=1, kernel_x=kernel, kernel_y=kernel, **kw)
+        p = dict(algorithm=algorithm, kernel_x=kernel, kernel_y=kernel, **kw)
         b = api.DeviceBatch(h, w, len(frames), capacity=h * w, params=api.Params(**p),
                             word_prefix=True)
         dt = np.int32 if bits == 32 else np.int16
