@@ -408,7 +408,7 @@ cudaError_t launch_disp(const FramePtrs &F, int nframes, int h, int w, const Lau
       b.words * sizeof(uint32_t));
   if (marks)
     cudaEventRecord(marks->stage01, stream);
-  const dim3 grid = band_grid(nframes, h);
+  const dim3 grid = band_grid(nframes, h, w);
   const Kept kept = make_kept(b, h, w);
   disp_decide<K, Pix><<<grid, kScanT, 0, stream>>>(F, P, b.bits, b.words, kept, b.block_sums);
   if (marks)

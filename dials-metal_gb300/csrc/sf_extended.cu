@@ -702,7 +702,7 @@ cudaError_t launch_ext(const FramePtrs &F, int nframes, int h, int w, const Laun
   }
   if (marks)
     cudaEventRecord(marks->stage01, stream);
-  const dim3 grid = band_grid(nframes, h);
+  const dim3 grid = band_grid(nframes, h, w);
   const Kept kept = make_kept(b, h, w);
   ext_decide<K, Pix><<<grid, kScanT, 0, stream>>>(F, P, b.cand, b.bits, b.words, kept,
                                                   b.block_sums, b.cand_sums);

@@ -8,6 +8,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "sf_common.cuh"
 #include "sf_scan.cuh"
 #include "sf_stream.cuh"
@@ -30,11 +32,16 @@ __device__ __forceinline__ void band_share(int height, int *lo, int *hi) {
   *hi = min(height, *lo + share);
 }
 
-// The grid: blocks a frame (a band each while kCountBlocks over the batch
-// allows), and the frames.
-inline dim3 band_grid(int nframes, int height) {
-  const int bands = (height + kBandRows - 1) / kBandRows, most = kCountBlocks / nframes;
-  return dim3((unsigned)(bands < most ? bands : most), (unsigned)nframes);
+// The grid: blocks a frame, and the frames. A block of 8 warps takes enough
+// bands for 128 runs (four a warp's round in the last pass: blocks of one band
+// left six of its warps idle) while the batch still makes kMinBlocks blocks,
+// else a band; at most kCountBlocks over the batch.
+constexpr int kMinBlocks = 1024;
+inline dim3 band_grid(int nframes, int height, int width) {
+  const int bands = (height + kBandRows - 1) / kBandRows, rpr = runs_per_row(width);
+  const int per = std::max(1, std::min((128 + rpr - 1) / rpr, bands * nframes / kMinBlocks));
+  return dim3((unsigned)std::min((bands + per - 1) / per, kCountBlocks / nframes),
+              (unsigned)nframes);
 }
 
 // Sum of the block's predecessors' counts in its frame, and the frame's

@@ -74,30 +74,6 @@ __host__ __device__ constexpr uint32_t lat_bound12(uint32_t b) {
          b4 << 11;
 }
 
-__device__ __forceinline__ void lat_load(const uint32_t *__restrict__ image, int height, int width,
-                                         bool interior, int cx, int p, uint32_t v[kLatCols]) {
-  if (p < 0 || p >= height) {
-#pragma unroll
-    for (int i = 0; i < kLatCols; i++)
-      v[i] = 0xFFFFFFFFu;
-    return;
-  }
-  const uint32_t *row = image + (size_t)p * width + cx;
-  if (interior) {
-#pragma unroll
-    for (int f = 0; f < kLatCols / 4; f++) {
-      const uint4 t = __ldg(reinterpret_cast<const uint4 *>(row) + f);
-      v[4 * f] = t.x, v[4 * f + 1] = t.y, v[4 * f + 2] = t.z, v[4 * f + 3] = t.w;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kLatCols; i++) {
-      const int gx = cx + i;
-      v[i] = (gx >= 0 && gx < width) ? __ldg(row + i) : 0xFFFFFFFFu;
-    }
-  }
-}
-
 // One pixel row of a lane: its 12 pixels packed (masked as a lone count bit
 // whose square wraps to 0, valid saturated at kLatCap), the row sums of 7
 // columns at the lattice columns 2, 5, 8, 11, and the masked bits of the 12
@@ -149,31 +125,23 @@ __device__ __forceinline__ void lat_row(const uint32_t v[kLatCols], int lane, ui
   *m12 = m;
 }
 
-// The ring variant (kRing: 4 | width and 16-byte aligned frames) stages each
-// warp's pixel rows in shared memory by cp.async, kRingSlots - 1 rows ahead:
-// a row is the 96 16-byte pieces from column X - 12 (X the strip's first
-// output column) that the lanes read, 12 columns a lane. The other variant
-// loads each lane's 12 columns straight from the frame, a row ahead.
-//
-// A piece is 4 pixels: 16 bytes of a 32-bit frame, 8 of a 16-bit one (whose
-// rows, with 4 | width, start 8-byte aligned). Both fetch 96 pieces from
-// column X - 12, and lane l reads its 12 pixels from column 12 l of the slot.
+// Each warp's pixel rows are staged in shared memory by cp.async (RowReader,
+// sf_strips.cuh), kRingSlots - 1 rows ahead, 12 columns a lane from column X - 12
+// (X the strip's first output column).
 constexpr int kRingSlots = 4;
-constexpr int kRingStride = 384;  // pixels a slot
 template <typename Pix>
 constexpr size_t ring_bytes() {
-  return (size_t)kLatWarps * kRingSlots * kRingStride * sizeof(Pix);
+  return (size_t)kLatWarps * kRingSlots * kStripStride * sizeof(Pix);
 }
 
-template <int kOcc, bool kRing, typename Pix>
+template <int kOcc, typename Pix>
 __global__ void __launch_bounds__(kLatWarps * 32, kOcc)
-lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
+lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
             const __grid_constant__ FrameSpans S, int run_rows,
             const __grid_constant__ StreamTables T,
             const __grid_constant__ LaunchParams P, uint8_t *__restrict__ final_bytes,
             size_t mask_bytes) {
   constexpr bool k16 = sizeof(Pix) == 2;
-  static_assert(!k16 || kRing, "16-bit frames take the ring variant only");
   extern __shared__ __align__(16) unsigned char lat_ring_raw[];
   Pix *lat_ring = reinterpret_cast<Pix *>(lat_ring_raw);
   // Lower-bound constants by masked count m (window count 49 - m).
@@ -200,7 +168,6 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
   // Lane l holds columns X + 12 (l - 1) .. + 11: lanes 1-30 the strip's
   // 360, lane 0 the 12 before it, lane 31 the 12 after it.
   const int cx = kLatOut * sx + kLatCols * (lane - 1);
-  const bool interior = vec && cx >= 0 && cx + kLatCols <= width;
   // This lane's first mask byte (lane pairs 1-2, 3-4, .. share three
   // bytes), and the bits of its columns inside the frame.
   const int pair_byte = (kLatOut * sx + 24 * ((lane - 1) >> 1)) >> 3;
@@ -224,82 +191,52 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
 
   // Pixel rows [pbeg, pend) of the run.
   const int pbeg = 3 * (ja - 2), pend = 3 * (ja + ntrip + 1);
-  Pix *ring = lat_ring + (size_t)warp * kRingSlots * kRingStride;
-  // The ring's pieces of this lane: l, l + 32, l + 64 (a warp's copy
-  // instruction covers 128 contiguous pixels), and whether each lies in the
-  // frame.
-  const int X = kLatOut * sx;
-  const int x0 = X - kLatCols + 4 * lane;
-  bool pin[3];
+  Pix *ring = lat_ring + (size_t)warp * kRingSlots * kStripStride;
+  StripRun r;
+  r.X = kLatOut * sx;
+  r.height = height;
+  r.width = width;
+  RowReader<Pix> reader(image, r, pbeg, pend - pbeg);
 #pragma unroll
-  for (int i = 0; i < 3; i++)
-    pin[i] = x0 + 128 * i >= 0 && x0 + 128 * i + 4 <= width;
-  auto fetch = [&](int p) {
-    Pix *dst = ring + ((p - pbeg) % kRingSlots) * kRingStride + 4 * lane;
-    const bool rowin = p >= 0 && p < height && p < pend;
-    const Pix *src = image + (size_t)(rowin ? p : 0) * width + x0;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      if (rowin && pin[i])
-        cp_async_piece<Pix>(dst + 128 * i, src + 128 * i);
-      else
-        fill_piece_masked<Pix>(dst + 128 * i);
-    }
-  };
-  if (kRing) {
-#pragma unroll
-    for (int i = 0; i < kRingSlots - 1; i++) {
-      fetch(pbeg + i);
-      cp_async_commit();
-    }
+  for (int i = 0; i < kRingSlots - 1; i++) {
+    reader.fetch(ring + i * kStripStride);
+    cp_async_commit();
   }
 
   uint32_t v[kLatCols];
-  if constexpr (!kRing)
-    lat_load(reinterpret_cast<const uint32_t *>(image), height, width, interior, cx, pbeg, v);
+  int slot_in = kRingSlots - 1, slot_now = 0;
   for (int t = 0; t < ntrip + 3; t++) {
     const int p0 = 3 * (ja - 2 + t);
     uint32_t Tn[4], Tq[4], mcur[3], cm = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const int p = p0 + k;
-      uint32_t nxt[kLatCols];
-      if (kRing) {
-        // Row p + kRingSlots - 1 goes out; row p has landed.
-        __syncwarp();
-        fetch(p + kRingSlots - 1);
-        cp_async_commit();
-        cp_async_wait<kRingSlots - 1>();
-        __syncwarp();
-        const Pix *slot = ring + ((p - pbeg) % kRingSlots) * kRingStride;
-        if constexpr (k16) {
-          const uint2 *src = reinterpret_cast<const uint2 *>(slot + kLatCols * lane);
+      // Row p0 + k + kRingSlots - 1 goes out; row p0 + k has landed.
+      __syncwarp();
+      reader.fetch(ring + slot_in * kStripStride);
+      cp_async_commit();
+      cp_async_wait<kRingSlots - 1>();
+      __syncwarp();
+      const Pix *slot = ring + slot_now * kStripStride;
+      slot_in = (slot_in + 1) % kRingSlots;
+      slot_now = (slot_now + 1) % kRingSlots;
+      if constexpr (k16) {
+        const uint2 *src = reinterpret_cast<const uint2 *>(slot + kLatCols * lane);
 #pragma unroll
-          for (int i = 0; i < kLatCols / 4; i++) {
-            const uint2 x = src[i];
-            v[4 * i] = x.x & 0xFFFFu, v[4 * i + 1] = x.x >> 16;
-            v[4 * i + 2] = x.y & 0xFFFFu, v[4 * i + 3] = x.y >> 16;
-          }
-        } else {
-          const uint4 *src = reinterpret_cast<const uint4 *>(slot) + 3 * lane;
-#pragma unroll
-          for (int i = 0; i < kLatCols / 4; i++) {
-            const uint4 x = src[i];
-            v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
-          }
+        for (int i = 0; i < kLatCols / 4; i++) {
+          const uint2 x = src[i];
+          v[4 * i] = x.x & 0xFFFFu, v[4 * i + 1] = x.x >> 16;
+          v[4 * i + 2] = x.y & 0xFFFFu, v[4 * i + 3] = x.y >> 16;
         }
-      } else if (k < 2 || t + 1 < ntrip + 3) {
-        // The next row's loads go out before this row's arithmetic.
-        lat_load(reinterpret_cast<const uint32_t *>(image), height, width, interior, cx,
-                 p + 1, nxt);
+      } else {
+        const uint4 *src = reinterpret_cast<const uint4 *>(slot) + 3 * lane;
+#pragma unroll
+        for (int i = 0; i < kLatCols / 4; i++) {
+          const uint4 x = src[i];
+          v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+        }
       }
       uint32_t hn[4], hq[4];
       lat_row<Pix>(v, lane, hn, hq, &mcur[k]);
-      if (!kRing) {
-#pragma unroll
-        for (int i = 0; i < kLatCols; i++)
-          v[i] = nxt[i];
-      }
 #pragma unroll
       for (int a = 0; a < 4; a++) {
         Tn[a] = k == 0 ? hn[a] : Tn[a] + hn[a];
@@ -347,7 +284,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
         const uint2 c = tab[m];
         const unsigned long long L = (unsigned long long)Tq[a] * c.x;
         const unsigned long long Rr = (unsigned long long)S * ((S << kDec) + c.y);
-        sig = L > Rr || S >= kLatCap - 1u;
+        sig = (L > Rr) | (S >= kLatCap - 1u);  // (no branch)
       }
       b4 |= sig ? 1u << a : 0u;
     }
@@ -385,8 +322,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes, int vec,
     for (int k = 0; k < 3; k++)
       mprev[k] = mcur[k];
   }
-  if (kRing)
-    cp_async_wait<0>();
+  cp_async_wait<0>();
 }
 
 // ---------------------------------------------------------------------------
@@ -451,6 +387,8 @@ template <typename Pix> struct alignas(128) VerWarp {
 // TMA staging of the exact check and stage 2.
 struct TileMaps {
   CUtensorMap map[kMaxBatch];
+  unsigned long long mapped;  // bit f: frame f has a map (else its tiles are staged per lane)
+  __device__ __forceinline__ bool has(int f) const { return (mapped >> f) & 1ull; }
 };
 
 template <typename Pix> __device__ __forceinline__ bool is_masked_px(uint32_t v) {
@@ -571,10 +509,10 @@ lat_tiles(const __grid_constant__ FramePtrs F, int nframes, int env_h, int env_w
 // come here only when 4 | width and they are 8-byte aligned.
 template <typename Pix>
 __device__ __forceinline__ void stage_pixels(Pix (*pix)[VerPix<Pix>::kPW], const Pix *image,
-                                             int height, int width, int vec, int r0, int xs,
+                                             int height, int width, int r0, int xs,
                                              int lane) {
   constexpr int kPW = VerPix<Pix>::kPW, kPieces = kPW / 4;
-  if (sizeof(Pix) == 2 || vec) {
+  if (width % 4 == 0 && reinterpret_cast<uintptr_t>(image) % (4 * sizeof(Pix)) == 0) {
     // Pieces of 4 pixels, each wholly inside the frame or wholly outside it.
     for (int k = lane; k < kVerPR * kPieces; k += 32) {
       const int r = k / kPieces, ch = k - r * kPieces;
@@ -654,7 +592,7 @@ template <typename Pix> __device__ __forceinline__ int tile_xs(int c0) {
 
 template <typename Pix>
 __device__ __forceinline__ void ver_stage(VerWarp<Pix> &sm, int s, uint32_t e, const FramePtrs &F,
-                                          const TileMaps &M, int tma, int vec, uint32_t ntiles,
+                                          const TileMaps &M, uint32_t ntiles,
                                           int ntx, const FastDiv &by_ntiles,
                                           const FastDiv &by_ntx,
                                           const uint32_t *__restrict__ final_all,
@@ -664,11 +602,11 @@ __device__ __forceinline__ void ver_stage(VerWarp<Pix> &sm, int s, uint32_t e, c
   const int height = F.h[f], width = F.w[f];
   const int xs = tile_xs<Pix>(c0);
   __syncwarp();  // every lane is done with the pixel buffer
-  if (tma)
+  if (M.has(f))
     tma_stage<Pix>(sm.pix[0], &sm.bar[0], M, f, r0, xs, lane);
   else
-    stage_pixels<Pix>(sm.pix[0].px, reinterpret_cast<const Pix *>(F.image[f]), height, width,
-                      vec, r0, xs, lane);
+    stage_pixels<Pix>(sm.pix[0].px, reinterpret_cast<const Pix *>(F.image[f]), height, width, r0,
+                      xs, lane);
   if (lane < 2 * kVerRows) {
     const int o = lane >> 1, wdx = (c0 >> 5) + (lane & 1);
     const int wpr = (width + 31) >> 5;
@@ -700,8 +638,8 @@ __device__ __forceinline__ void ver_window(const VerWarp<Pix> &sm, int d, int co
 
 template <int kOcc, typename Pix>
 __global__ void __launch_bounds__(kVerWarps * 32, kOcc)
-lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps M, int tma,
-           int env_h, int env_w, int vec, const __grid_constant__ LaunchParams P,
+lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps M, int env_h,
+           int env_w, const __grid_constant__ LaunchParams P,
            const __grid_constant__ StreamTables T, uint32_t *__restrict__ final_all, size_t words,
            const uint32_t *__restrict__ list,
            uint32_t *__restrict__ counters, FastDiv by_ntiles, FastDiv by_ntx) {
@@ -716,7 +654,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     tab[m] = make_uint4(T.nk[kLatN0 - m], T.clo[kLatN0 - m], T.chi[kLatN0 - m], 0u);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   VerWarp<Pix> &sm = warps[warp];
-  if (tma && lane == 0) {
+  if (lane == 0) {
     mbar_init(&sm.bar[0], 1);
     mbar_init_fence();
   }
@@ -737,11 +675,13 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
   uint32_t e = k < count ? list[k] : 0u;
   uint32_t e1 = k + nw < count ? list[k + nw] : 0u;
   if (k < count)
-    ver_stage<Pix>(sm, 0, e, F, M, tma, vec, ntiles, ntx, by_ntiles, by_ntx, final_all, words,
+    ver_stage<Pix>(sm, 0, e, F, M, ntiles, ntx, by_ntiles, by_ntx, final_all, words,
                    lane);
   cp_async_commit();
   uint32_t e2 = 0u;
-  uint32_t inflight = k < count ? 1u : 0u;  // a TMA load not waited for
+  // A TMA load not waited for.
+  auto mapped = [&](uint32_t x) { return M.has((int)fast_div(x, by_ntiles)); };
+  bool inflight = k < count && mapped(e);
   for (int s = 0; k < count; k += nw, s ^= 1, e = e1, e1 = e2) {
     e2 = k + 2 * nw < count ? list[k + 2 * nw] : 0u;
     cp_async_wait<0>();  // this tile's pieces have landed
@@ -749,8 +689,8 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     const TileAt a = tile_at(e, ntiles, ntx, by_ntiles, by_ntx);
     const int f = a.f, r0 = a.r0, c0 = a.c0;
     const int height = F.h[f], width = F.w[f], wpr = (width + 31) >> 5;
-    if (tma) {
-      inflight = 0u;
+    if (inflight) {
+      inflight = false;
       if (!tma_landed<Pix>(sm.pix[0], &sm.bar[0], parity & 1u, height, width, r0,
                            tile_xs<Pix>(c0), lane)) {
         if (lane == 0)
@@ -762,9 +702,9 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     // The next tile's load, once this tile's pixels have been read.
     auto stage_next = [&]() {
       if (k + nw < count) {
-        ver_stage<Pix>(sm, s ^ 1, e1, F, M, tma, vec, ntiles, ntx, by_ntiles, by_ntx,
+        ver_stage<Pix>(sm, s ^ 1, e1, F, M, ntiles, ntx, by_ntiles, by_ntx,
                        final_all, words, lane);
-        inflight = 1u;
+        inflight = mapped(e1);
       }
       cp_async_commit();
     };
@@ -884,7 +824,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
         const bool maybe = L > (unsigned long long)S * ((S << kDec) + c.y);
         const bool sure = L >= (unsigned long long)S * ((S << kDec) + c.z) + (2ull << kDec);
         keep &= maybe ? ~0u : ~(1u << d);
-        amb |= (maybe && !sure) ? 1u << d : 0u;
+        amb |= (maybe & !sure) ? 1u << d : 0u;
       }
       while (amb) {
         const int d = __ffs(amb) - 1;
@@ -928,7 +868,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     }
   }
   // After a fault: the load still in flight (bounded) before the buffer goes.
-  if (tma && inflight)
+  if (inflight)
     (void)mbar_wait(&sm.bar[0], parity & 1u);
   cp_async_wait<0>();
 }
@@ -945,7 +885,7 @@ int lat_slots() {
   static int slots = 0;
   if (!slots) {
     int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lat_stage01<kLatOcc, true, uint32_t>,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lat_stage01<kLatOcc, uint32_t>,
                                                   kLatWarps * 32, ring_bytes<uint32_t>());
     slots = std::max(1, per) * kLatWarps * device_sms();
   }
@@ -963,17 +903,15 @@ template <class Kernel> cudaError_t persistent_blocks(Kernel k, size_t bytes, in
   return e;
 }
 
-// The launch's frames mapped for the TMA staging of tiles (1), or not
-// mappable (0: a frame not 16-byte aligned, a row pitch that is not a
-// multiple of 16 bytes, no driver entry point), the per-lane staging then.
-template <typename Pix> int make_tile_maps(const FramePtrs &F, int nframes, int h, int w,
-                                           TileMaps *M) {
+// The launch's frames mapped for the TMA staging of tiles; a frame that cannot
+// be (not 16-byte aligned, a row pitch that is not a multiple of 16 bytes, no
+// driver entry point) has its tiles staged per lane.
+template <typename Pix> void make_tile_maps(const FramePtrs &F, int nframes, TileMaps *M) {
   std::memset(M, 0, sizeof(*M));
   for (int f = 0; f < nframes; f++)
-    if (!encode_frame_map(&M->map[f], F.image[f], F.h[f], F.w[f], (int)sizeof(Pix),
-                          VerPix<Pix>::kPW, kVerPR))
-      return 0;
-  return 1;
+    if (encode_frame_map(&M->map[f], F.image[f], F.h[f], F.w[f], (int)sizeof(Pix),
+                         VerPix<Pix>::kPW, kVerPR))
+      M->mapped |= 1ull << f;
 }
 
 // Strips of a frame w wide (whole mask rows: the last strip reaches the end
@@ -981,7 +919,7 @@ template <typename Pix> int make_tile_maps(const FramePtrs &F, int nframes, int 
 int lat_strips(int w) { return ((w + 31) / 32 * 32 + kLatOut - 1) / kLatOut; }
 
 template <typename Pix>
-cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, int vec, const LaunchParams &P,
+cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, const LaunchParams &P,
                     const StreamTables &T, const StreamBuffers &b, int run_rows,
                     cudaStream_t stream) {
   // Each frame's strips x runs of run_rows rows, frame after frame.
@@ -995,12 +933,8 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, int vec, cons
   const size_t mask_bytes = b.words * sizeof(uint32_t);
   const unsigned lb = (unsigned)((S.start[nframes] + kLatWarps - 1) / kLatWarps);
   uint8_t *fin = reinterpret_cast<uint8_t *>(b.cand);
-  if (sizeof(Pix) == 2 || vec)
-    lat_stage01<kLatOcc, true, Pix><<<lb, kLatWarps * 32, ring_bytes<Pix>(), stream>>>(
-        F, nframes, vec, S, run_rows, T, P, fin, mask_bytes);
-  else
-    lat_stage01<kLatOcc, false, uint32_t><<<lb, kLatWarps * 32, 0, stream>>>(
-        F, nframes, vec, S, run_rows, T, P, fin, mask_bytes);
+  lat_stage01<kLatOcc, Pix><<<lb, kLatWarps * 32, ring_bytes<Pix>(), stream>>>(
+      F, nframes, S, run_rows, T, P, fin, mask_bytes);
   static std::once_flag configured;
   static cudaError_t config_error = cudaSuccess;
   static int ver_blocks = 0;
@@ -1032,9 +966,9 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, int vec, cons
   lat_tiles<<<tb, 256, 0, stream>>>(F, nframes, h, w, b.cand, b.words, list, b.counters, G,
                                     trun);
   TileMaps M;
-  const int tma = make_tile_maps<Pix>(F, nframes, h, w, &M);
+  make_tile_maps<Pix>(F, nframes, &M);
   lat_verify<kVerOcc, Pix><<<ver_blocks * device_sms(), kVerWarps * 32, ver_smem_bytes<Pix>(),
-                             stream>>>(F, M, tma, h, w, vec, P, T, b.cand, b.words, list,
+                             stream>>>(F, M, h, w, P, T, b.cand, b.words, list,
                                        b.counters, by_ntiles, by_ntx);
   return cudaGetLastError();
 }
@@ -1074,14 +1008,16 @@ bool encode_frame_map(CUtensorMap *map, const void *base, int h, int w, int byte
 
 size_t lattice_tiles(int h, int w) { return (size_t)ver_ntx(w) * (size_t)ver_nty(h); }
 
-// The run length for a launch whose tallest frame has h rows and whose
-// frames have `strips` strips in all: the resident warps filled once (no
-// tail wave) by the tallest frame's runs, unless run_rows is given; at least
-// kLatMinRunRows, in whole triples of rows.
+// The run length for a launch whose tallest frame has h rows and whose frames
+// have `strips` strips in all, unless run_rows is given, in whole triples of
+// rows: the resident warps filled kLatWaves times over by runs of at least
+// kLatLongRun rows (each reads 9 rows more than it writes), so that warps of
+// unequal speed even out; else once, down to runs of kLatMinRunRows.
 static int lat_run_rows(int h, long long strips, int run_rows) {
   if (run_rows <= 0) {
     const long long nruns = std::max(1ll, (long long)lat_slots() / std::max(1ll, strips));
-    run_rows = (int)((h + nruns - 1) / nruns);
+    const int once = (int)((h + nruns - 1) / nruns);
+    run_rows = std::min(once, std::max(kLatLongRun, (once + kLatWaves - 1) / kLatWaves));
   }
   run_rows = std::max(run_rows, kLatMinRunRows);
   return (run_rows + 2) / 3 * 3;
@@ -1134,16 +1070,12 @@ cudaError_t launch_lattice(const FramePtrs &F, int nframes, int h, int w, int pi
     return e;
   StreamTables T;
   make_stream_tables(P, &T);
-  int vec = 1;
   long long strips = 0;
-  for (int f = 0; f < nframes; f++) {
+  for (int f = 0; f < nframes; f++)
     strips += lat_strips(F.w[f]);
-    if (F.w[f] % 4 != 0 || reinterpret_cast<uintptr_t>(F.image[f]) % (4 * pixel_bytes) != 0)
-      vec = 0;
-  }
   const int rr = lat_run_rows(h, strips, run_rows);
-  return pixel_bytes == 2 ? lattice<uint16_t>(F, nframes, h, w, vec, P, T, b, rr, stream)
-                          : lattice<uint32_t>(F, nframes, h, w, vec, P, T, b, rr, stream);
+  return pixel_bytes == 2 ? lattice<uint16_t>(F, nframes, h, w, P, T, b, rr, stream)
+                          : lattice<uint32_t>(F, nframes, h, w, P, T, b, rr, stream);
 }
 
 } // namespace sf

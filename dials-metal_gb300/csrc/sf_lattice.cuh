@@ -40,11 +40,11 @@ struct StreamTables {
 
 // The lattice pass for kernel 3,3 (sf_lattice.cu): strips of 360 output
 // columns (one warp each) by runs of run_rows rows, a multiple of 3.
-constexpr int kLatMinRunRows = 16;
+constexpr int kLatMinRunRows = 9, kLatLongRun = 144, kLatWaves = 3;
 struct LatticeGeometry {
   int nstrips, nruns, run_rows;
 };
-// run_rows 0 picks runs that fill the resident warps once.
+// run_rows 0: the default geometry.
 LatticeGeometry lattice_geometry(int h, int w, int nframes, int run_rows);
 // Stage 0 and the erosion for kernel 3,3: the lattice bound, then the exact
 // check of its candidates; writes the candidate masks b.cand (the reference's
