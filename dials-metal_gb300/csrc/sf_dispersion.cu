@@ -79,6 +79,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
            int run_rows, const __grid_constant__ DispTables T,
            const __grid_constant__ LaunchParams P, uint8_t *__restrict__ mask_all,
            size_t mask_bytes) {
+  previous_done();
   using G = StripG<K>;
   extern __shared__ __align__(16) unsigned char disp_raw[];
   __shared__ uint4 tab[G::N0 + 1];  // by masked count m: nk, clo, kk of n = N0 - m
@@ -298,6 +299,7 @@ __global__ void __launch_bounds__(kScanT)
 disp_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchParams P,
             uint32_t *__restrict__ bits_all, size_t words, Kept kept,
             uint32_t *__restrict__ block_sums) {
+  previous_done();
   __shared__ uint32_t s_clear[kScanT / 32][32 * kRunWords];
   const int f = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Pix *image = reinterpret_cast<const Pix *>(F.image[f]);
@@ -410,12 +412,13 @@ cudaError_t launch_disp(const FramePtrs &F, int nframes, int h, int w, const Lau
     cudaEventRecord(marks->stage01, stream);
   const dim3 grid = band_grid(nframes, h, w);
   const Kept kept = make_kept(b, h, w);
-  disp_decide<K, Pix><<<grid, kScanT, 0, stream>>>(F, P, b.bits, b.words, kept, b.block_sums);
+  launch_after(disp_decide<K, Pix>, grid, kScanT, 0, stream, F, P, b.bits, b.words, kept,
+               b.block_sums);
   if (marks)
     cudaEventRecord(marks->stage2, stream);
-  scatter_pixels<Pix, false><<<grid, kScanT, 0, stream>>>(
-      F, b.bits, b.words, nullptr, K, kept, P.min_local, b.block_sums, nullptr, 0u, nullptr, b.out,
-      b.out_stride, b.capacity, b.count_out, b.prefix);
+  launch_after(scatter_pixels<Pix, false>, grid, kScanT, 0, stream, F, b.bits, b.words, nullptr, K,
+               kept, P.min_local, b.block_sums, nullptr, 0u, nullptr, b.out, b.out_stride,
+               b.capacity, b.count_out, b.prefix);
   if (marks)
     cudaEventRecord(marks->order, stream);
   return cudaGetLastError();

@@ -153,6 +153,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           int run_rows, const __grid_constant__ ExtTables T,
           const __grid_constant__ LaunchParams P, uint8_t *__restrict__ cand_all,
           size_t mask_bytes) {
+  previous_done();
   using G = StripG<K>;
   constexpr bool k16 = sizeof(Pix) == 2;
   constexpr int E = K - 1;
@@ -384,7 +385,7 @@ __device__ __noinline__ void ext_wide_window(const Pix *image, const uint32_t *c
     for (int xx = max(0, x - half); xx <= min(width - 1, x + half); xx++) {
       const uint32_t v = __ldg(image + (size_t)yy * width + xx);
       if (v < Traits<Pix>::kMasked &&
-          (__ldg(cand + (size_t)yy * wpr + (xx >> 5)) >> (xx & 31) & 1u) == 0u) {
+          (cand[(size_t)yy * wpr + (xx >> 5)] >> (xx & 31) & 1u) == 0u) {
         n++;
         S += v;
       }
@@ -409,6 +410,7 @@ __global__ void __launch_bounds__(kScanT, 4)
 ext_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchParams P,
            const uint32_t *__restrict__ cand_all, uint32_t *__restrict__ bits_all, size_t words,
            Kept kept, uint32_t *__restrict__ block_sums, uint32_t *__restrict__ cand_sums) {
+  previous_done();
   constexpr int K2 = K + 2, W2 = 2 * K2 + 1, NC = 32 - 2 * K2, ROWS = kBandRows + 2 * K2;
   __shared__ ExtWarp s_warps[kScanT / 32];
   __shared__ uint32_t s_count[2], s_next;
@@ -704,14 +706,14 @@ cudaError_t launch_ext(const FramePtrs &F, int nframes, int h, int w, const Laun
     cudaEventRecord(marks->stage01, stream);
   const dim3 grid = band_grid(nframes, h, w);
   const Kept kept = make_kept(b, h, w);
-  ext_decide<K, Pix><<<grid, kScanT, 0, stream>>>(F, P, b.cand, b.bits, b.words, kept,
-                                                  b.block_sums, b.cand_sums);
+  launch_after(ext_decide<K, Pix>, grid, kScanT, 0, stream, F, P, b.cand, b.bits, b.words, kept,
+               b.block_sums, b.cand_sums);
   if (marks)
     cudaEventRecord(marks->stage2, stream);
-  scatter_pixels<Pix, true><<<grid, kScanT, 0, stream>>>(
-      F, b.bits, b.words, b.cand, K + 2, kept, P.min_local, b.block_sums, b.cand_sums,
-      b.cand_limit, lattice ? b.counters + kCtrFault : nullptr, b.out, b.out_stride, b.capacity,
-      b.count_out, b.prefix);
+  launch_after(scatter_pixels<Pix, true>, grid, kScanT, 0, stream, F, b.bits, b.words, b.cand,
+               K + 2, kept, P.min_local, b.block_sums, b.cand_sums, b.cand_limit,
+               lattice ? b.counters + kCtrFault : nullptr, b.out, b.out_stride, b.capacity,
+               b.count_out, b.prefix);
   if (marks)
     cudaEventRecord(marks->order, stream);
   return cudaGetLastError();

@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "sf_common.cuh"
+#include "sf_launch.cuh"
 #include "sf_scan.cuh"
 #include "sf_stream.cuh"
 
@@ -35,8 +36,10 @@ __device__ __forceinline__ void band_share(int height, int *lo, int *hi) {
 // The grid: blocks a frame, and the frames. A block of 8 warps takes enough
 // bands for 128 runs (four a warp's round in the last pass: blocks of one band
 // left six of its warps idle) while the batch still makes kMinBlocks blocks,
-// else a band; at most kCountBlocks over the batch.
-constexpr int kMinBlocks = 1024;
+// else a band; at most kCountBlocks over the batch. (16 blocks an SM: 32 frames of
+// 2162 x 2068 at kernel 2 take 490 us, 513 with 1024 blocks; 16 of 3262 x 3108 at
+// kernel 4 647 and 700.)
+constexpr int kMinBlocks = 16 * 152;
 inline dim3 band_grid(int nframes, int height, int width) {
   const int bands = (height + kBandRows - 1) / kBandRows, rpr = runs_per_row(width);
   const int per = std::max(1, std::min((128 + rpr - 1) / rpr, bands * nframes / kMinBlocks));
@@ -46,7 +49,7 @@ inline dim3 band_grid(int nframes, int height, int width) {
 
 // Sum of the block's predecessors' counts in its frame, and the frame's
 // total.
-__device__ __forceinline__ uint32_t block_base(const uint32_t *__restrict__ block_sums,
+__device__ __forceinline__ uint32_t block_base(const uint32_t *block_sums,
                                                uint32_t *total) {
   __shared__ uint32_t s_base, s_total;
   if (threadIdx.x < 32) {
@@ -196,7 +199,7 @@ __device__ __noinline__ void sum_window(const Pix *image, const uint32_t *out, i
     if (yy < 0 || yy >= height || xx < 0 || xx >= width)
       continue;
     const uint32_t v = __ldg(image + (size_t)yy * width + xx);
-    const uint32_t o = out ? __ldg(out + (size_t)yy * wpr + (xx >> 5)) >> (xx & 31) & 1u : 0u;
+    const uint32_t o = out ? out[(size_t)yy * wpr + (xx >> 5)] >> (xx & 31) & 1u : 0u;
     if (v < Traits<Pix>::kMasked && o == 0u) {
       n++;
       S += v;
@@ -220,13 +223,13 @@ __device__ __noinline__ void sum_window(const Pix *image, const uint32_t *out, i
 // count; with a fault recorded (a device wait that ran out) every count says so.
 template <typename Pix, bool kByRun>
 __global__ void __launch_bounds__(kScanT, 6)
-scatter_pixels(const __grid_constant__ FramePtrs F, const uint32_t *__restrict__ bits_all,
-               size_t words, const uint32_t *__restrict__ excluded_all, int half, Kept kept,
-               uint32_t min_local, const uint32_t *__restrict__ block_sums,
-               const uint32_t *__restrict__ cand_sums, uint32_t cand_limit,
-               const uint32_t *__restrict__ fault, sf_signal_pixel *__restrict__ out_all,
+scatter_pixels(const __grid_constant__ FramePtrs F, const uint32_t *bits_all, size_t words,
+               const uint32_t *excluded_all, int half, Kept kept, uint32_t min_local,
+               const uint32_t *block_sums, const uint32_t *cand_sums, uint32_t cand_limit,
+               const uint32_t *fault, sf_signal_pixel *__restrict__ out_all,
                size_t out_stride, uint32_t capacity, uint32_t *__restrict__ count_out,
                uint32_t *__restrict__ prefix_all) {
+  previous_done();
   const int f = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const Pix *image = reinterpret_cast<const Pix *>(F.image[f]);
   const int height = F.h[f], width = F.w[f];
@@ -291,7 +294,7 @@ scatter_pixels(const __grid_constant__ FramePtrs F, const uint32_t *__restrict__
                       if (live) {
                         value = (uint32_t)__ldg(image + index);
                         if (place < held)
-                          b = __ldg(res + at);
+                          b = res[at];
                       }
                       for (unsigned more = __ballot_sync(0xffffffffu, live && place >= held); more;
                            more &= more - 1u) {

@@ -159,6 +159,7 @@ __device__ __forceinline__ uint32_t lower_bound_warp(const uint32_t *__restrict_
 static_assert(kLabelMaxBatch <= 64, "two frames a lane");
 __global__ void k_offsets(LabelStatus *st, const BatchArgs *__restrict__ ap,
                           uint32_t capacity) {
+  previous_done();
   if (st->error)
     return;
   const BatchArgs &a = *ap;
@@ -207,6 +208,7 @@ __global__ void k_offsets(LabelStatus *st, const BatchArgs *__restrict__ ap,
 // k_link's left-neighbour union.
 __global__ void k_append(LabelStatus *st, const BatchArgs *__restrict__ ap, int32_t *frame,
                          uint32_t *index, uint32_t *value, uint32_t *parent) {
+  previous_done();
   if (st->error)
     return;
   const BatchArgs &a = *ap;
@@ -250,6 +252,7 @@ __global__ void k_append(LabelStatus *st, const BatchArgs *__restrict__ ap, int3
 __global__ void k_rows(LabelStatus *st, const BatchArgs *__restrict__ ap,
                        const uint32_t *__restrict__ index, uint32_t *__restrict__ rows,
                        uint32_t height) {
+  previous_done();
   if (st->error)
     return;
   const BatchArgs &a = *ap;
@@ -337,6 +340,7 @@ __global__ void k_link(LabelStatus *st, const BatchArgs *__restrict__ ap,
                        const uint32_t *__restrict__ index, uint32_t *parent,
                        const uint32_t *__restrict__ rows, uint32_t height, uint2 *edges,
                        uint32_t edge_cap) {
+  previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
@@ -390,6 +394,7 @@ __global__ void k_link(LabelStatus *st, const BatchArgs *__restrict__ ap,
 // The listed edges joined, a thread each.
 __global__ void k_unite(LabelStatus *st, const uint2 *__restrict__ edges, uint32_t edge_cap,
                         uint32_t *parent) {
+  previous_done();
   if (st->error)
     return;
   const uint32_t n = min(st->n_edges, edge_cap);
@@ -402,6 +407,7 @@ __global__ void k_unite(LabelStatus *st, const uint2 *__restrict__ edges, uint32
 
 __global__ void k_flatten(LabelStatus *st, uint32_t *parent, uint32_t *root, int32_t *zlast,
                           uint32_t *csize, uint32_t *candid) {
+  previous_done();
   if (st->error)
     return;
   const uint32_t n = st->n_total;
@@ -420,6 +426,7 @@ __global__ void k_flatten(LabelStatus *st, uint32_t *parent, uint32_t *root, int
 __global__ void k_comp_stats(LabelStatus *st, const uint32_t *__restrict__ root,
                              const int32_t *__restrict__ frame, int32_t *zlast,
                              uint32_t *csize) {
+  previous_done();
   if (st->error)
     return;
   const uint32_t n = st->n_total;
@@ -469,6 +476,7 @@ enum : uint32_t { kClosingRoot = 1u, kOpenPixel = 2u };
 __global__ void k_closing_flags(LabelStatus *st, const BatchArgs *__restrict__ ap,
                                 const uint32_t *__restrict__ root,
                                 const int32_t *__restrict__ zlast, uint32_t *flag) {
+  previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
@@ -525,6 +533,7 @@ constexpr int kBucketBlocks = 152;  // the partition's chunks
 
 __global__ void __launch_bounds__(kThreads)
 k_bucket_hist(LabelStatus *st, const uint32_t *__restrict__ cbucket, uint32_t *hist) {
+  previous_done();
   if (st->error)
     return;
   __shared__ uint32_t h[kBuckets];
@@ -544,6 +553,7 @@ k_bucket_hist(LabelStatus *st, const uint32_t *__restrict__ cbucket, uint32_t *h
 // bucket's counts in place (each lane a run of blocks); the buckets' own
 // offsets follow the counts, and the scatter adds them.
 __global__ void __launch_bounds__(1024) k_bucket_offsets(LabelStatus *st, uint32_t *hist) {
+  previous_done();
   if (st->error)
     return;
   __shared__ uint32_t btotal[kBuckets];
@@ -605,6 +615,7 @@ __global__ void __launch_bounds__(kThreads)
 k_bucket_scatter(LabelStatus *st, const uint32_t *__restrict__ clist,
                  const uint32_t *__restrict__ cbucket, const uint32_t *__restrict__ hist,
                  uint32_t *order) {
+  previous_done();
   if (st->error)
     return;
   constexpr int W = kThreads / 32;
@@ -725,6 +736,7 @@ __global__ void k_gather(LabelStatus *st, const uint32_t *__restrict__ root,
                          const uint32_t *__restrict__ candid,
                          const uint32_t *__restrict__ cand_off, uint32_t *cursor,
                          uint32_t *members) {
+  previous_done();
   if (st->error)
     return;
   const uint32_t n = st->n_total;
@@ -1033,6 +1045,7 @@ k_sort(LabelStatus *st, const uint32_t *__restrict__ cand_n,
        const uint32_t *__restrict__ cand_off, uint32_t *members,
        const int32_t *__restrict__ frame, const uint32_t *__restrict__ index,
        const uint32_t *__restrict__ value, sf_pixel *mpix, uint32_t *mcand, uint32_t *big) {
+  previous_done();
   if (st->error)
     return;
   extern __shared__ __align__(16) uint32_t s_sort[];
@@ -1153,6 +1166,7 @@ k_sort(LabelStatus *st, const uint32_t *__restrict__ cand_n,
 // One block: the bins' exclusive offsets (into the cursors, hist +
 // kSizeBins), and the counts cleared for the next call.
 __global__ void __launch_bounds__(kSizeBins) k_perm_offsets(LabelStatus *st, uint32_t *hist) {
+  previous_done();
   if (st->error)
     return;
   uint32_t total;
@@ -1164,6 +1178,7 @@ __global__ void __launch_bounds__(kSizeBins) k_perm_offsets(LabelStatus *st, uin
 
 __global__ void k_perm_scatter(LabelStatus *st, const uint32_t *__restrict__ cand_n,
                                uint32_t *hist, uint32_t *perm) {
+  previous_done();
   if (st->error)
     return;
   const uint32_t ncand = st->n_cand;
@@ -1190,6 +1205,7 @@ __global__ void __launch_bounds__(kThreads)
 k_first(LabelStatus *st, const BatchArgs *__restrict__ ap, const uint32_t *__restrict__ cand_n,
         const uint32_t *__restrict__ cand_off, const sf_pixel *__restrict__ mpix, CandSpot *cs,
         uint32_t *acc_n) {
+  previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
@@ -1267,6 +1283,7 @@ __global__ void k_terms(LabelStatus *st, const BatchArgs *__restrict__ ap,
                         const sf_pixel *__restrict__ mpix, const uint32_t *__restrict__ mcand,
                         const uint32_t *__restrict__ acc_n, const CandSpot *__restrict__ cs,
                         double *__restrict__ terms, size_t terms_stride) {
+  previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
@@ -1295,6 +1312,7 @@ __global__ void k_pix(LabelStatus *st, const sf_pixel *__restrict__ mpix,
                       const uint32_t *__restrict__ mcand, const uint32_t *__restrict__ cand_off,
                       const uint32_t *__restrict__ acc_n, const uint32_t *__restrict__ acc_off,
                       sf_pixel *pixels, size_t pixels_cap) {
+  previous_done();
   if (st->error)
     return;
   const uint32_t n = st->n_cand_pixels;
@@ -1340,6 +1358,7 @@ __global__ void k_var(LabelStatus *st, const BatchArgs *__restrict__ ap,
                       const uint32_t *__restrict__ acc_off, const CandSpot *__restrict__ cs,
                       const sf_pixel *__restrict__ mpix, const double *__restrict__ terms,
                       size_t terms_stride, sf_spot *spots, size_t spots_cap) {
+  previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
@@ -1450,6 +1469,7 @@ __global__ void k_compact(LabelStatus *st, const BatchArgs *__restrict__ ap,
                           const uint32_t *__restrict__ index, const uint32_t *__restrict__ value,
                           int32_t *frame2, uint32_t *index2, uint32_t *value2,
                           uint32_t *parent2) {
+  previous_done();
   if (st->error)
     return;
   const BatchArgs &a = *ap;
@@ -1764,44 +1784,46 @@ struct Labeller {
     const dim3 g2(kGrid / 4 > 0 ? kGrid / 4 : 1, nb);
     cudaError_t e;
     k_offsets<<<1, 32, 0, s>>>(st, ap, (uint32_t)capacity);
-    k_append<<<g2, kThreads, 0, s>>>(st, ap, frame[c], index[c], value[c], parent[c]);
+    launch_after(k_append, g2, kThreads, 0, s, st, ap, frame[c], index[c], value[c], parent[c]);
     if (rows)
-      k_rows<<<dim3(kGrid / 4 > 0 ? kGrid / 4 : 1, nb + 1), kThreads, 0, s>>>(
-          st, ap, index[c], rows, (uint32_t)height);
-    k_link<<<g2, kThreads, 0, s>>>(st, ap, index[c], parent[c], rows, (uint32_t)height, edges,
-                                   (uint32_t)capacity);
-    k_unite<<<kPassGrid, kThreads, 0, s>>>(st, edges, (uint32_t)capacity, parent[c]);
-    k_flatten<<<kPassGrid, kThreads, 0, s>>>(st, parent[c], root, zlast, csize, candid);
-    k_comp_stats<<<kPassGrid, kThreads, 0, s>>>(st, root, frame[c], zlast, csize);
-    k_closing_flags<<<kPassGrid, kThreads, 0, s>>>(st, ap, root, zlast, flag);
+      launch_after(k_rows, dim3(kGrid / 4 > 0 ? kGrid / 4 : 1, nb + 1), kThreads, 0, s, st, ap,
+                   index[c], rows, (uint32_t)height);
+    launch_after(k_link, g2, kThreads, 0, s, st, ap, index[c], parent[c], rows, (uint32_t)height,
+                 edges, (uint32_t)capacity);
+    launch_after(k_unite, kPassGrid, kThreads, 0, s, st, edges, (uint32_t)capacity, parent[c]);
+    launch_after(k_flatten, kPassGrid, kThreads, 0, s, st, parent[c], root, zlast, csize, candid);
+    launch_after(k_comp_stats, kPassGrid, kThreads, 0, s, st, root, frame[c], zlast, csize);
+    launch_after(k_closing_flags, kPassGrid, kThreads, 0, s, st, ap, root, zlast, flag);
     if ((e = scan_pairs(ClosingScan{st, ap, flag, zlast, clist, cbucket, newpos}, scan_sums64,
                         s)) != cudaSuccess)
       return e;
-    k_bucket_hist<<<kBucketBlocks, kThreads, 0, s>>>(st, cbucket, hist);
-    k_bucket_offsets<<<1, 1024, 0, s>>>(st, hist);
-    k_bucket_scatter<<<kBucketBlocks, kThreads, 0, s>>>(st, clist, cbucket, hist, order);
+    launch_after(k_bucket_hist, kBucketBlocks, kThreads, 0, s, st, cbucket, hist);
+    launch_after(k_bucket_offsets, 1, 1024, 0, s, st, hist);
+    launch_after(k_bucket_scatter, kBucketBlocks, kThreads, 0, s, st, clist, cbucket, hist, order);
     if ((e = scan_pairs(CandidateScan{st, ap, order, csize, cand_n, cand_off, candid, cursor,
                                       phist, 0u, 0u, 0u},
                         scan_sums64, s)) != cudaSuccess)
       return e;
-    k_gather<<<kPassGrid, kThreads, 0, s>>>(st, root, candid, cand_off, cursor, members);
-    k_sort<false><<<kSortGrid, kThreads,
-                    (kThreads / 32) * (kWarpSortMax + 2 * kWarpSegMax) * 4, s>>>(
-        st, cand_n, cand_off, members, frame[c], index[c], value[c], mpix, mcand, big);
-    k_sort<true><<<kGrid / 2, kThreads, kBlockSortMax * 4, s>>>(
-        st, cand_n, cand_off, members, frame[c], index[c], value[c], mpix, mcand, big);
-    k_perm_offsets<<<1, kSizeBins, 0, s>>>(st, phist);
-    k_perm_scatter<<<kPassGrid, kThreads, 0, s>>>(st, cand_n, phist, perm);
-    k_first<<<kPassGrid, kThreads, 0, s>>>(st, ap, cand_n, cand_off, mpix, cspots, acc_n);
+    launch_after(k_gather, kPassGrid, kThreads, 0, s, st, root, candid, cand_off, cursor, members);
+    launch_after(k_sort<false>, kSortGrid, kThreads,
+                 (kThreads / 32) * (kWarpSortMax + 2 * kWarpSegMax) * 4, s, st, cand_n, cand_off,
+                 members, frame[c], index[c], value[c], mpix, mcand, big);
+    launch_after(k_sort<true>, kGrid / 2, kThreads, kBlockSortMax * 4, s, st, cand_n, cand_off,
+                 members, frame[c], index[c], value[c], mpix, mcand, big);
+    launch_after(k_perm_offsets, 1, kSizeBins, 0, s, st, phist);
+    launch_after(k_perm_scatter, kPassGrid, kThreads, 0, s, st, cand_n, phist, perm);
+    launch_after(k_first, kPassGrid, kThreads, 0, s, st, ap, cand_n, cand_off, mpix, cspots,
+                 acc_n);
     if ((e = scan_pairs(AcceptScan{st, acc_n, acc_idx, acc_off}, scan_sums64, s)) != cudaSuccess)
       return e;
-    k_pix<<<kPassGrid, kThreads, 0, s>>>(st, mpix, mcand, cand_off, acc_n, acc_off, d_pixels,
-                                         capacity);
-    k_terms<<<kPassGrid, kThreads, 0, s>>>(st, ap, mpix, mcand, acc_n, cspots, terms, capacity);
-    k_var<<<kPassGrid, kThreads, 0, s>>>(st, ap, perm, cand_off, acc_n, acc_idx, acc_off, cspots,
-                                         mpix, terms, capacity, d_spots, spots_cap);
-    k_compact<<<kPassGrid, kThreads, 0, s>>>(st, ap, flag, newpos, root, frame[c], index[c],
-                                             value[c], frame[o], index[o], value[o], parent[o]);
+    launch_after(k_pix, kPassGrid, kThreads, 0, s, st, mpix, mcand, cand_off, acc_n, acc_off,
+                 d_pixels, capacity);
+    launch_after(k_terms, kPassGrid, kThreads, 0, s, st, ap, mpix, mcand, acc_n, cspots, terms,
+                 capacity);
+    launch_after(k_var, kPassGrid, kThreads, 0, s, st, ap, perm, cand_off, acc_n, acc_idx, acc_off,
+                 cspots, mpix, terms, capacity, d_spots, spots_cap);
+    launch_after(k_compact, kPassGrid, kThreads, 0, s, st, ap, flag, newpos, root, frame[c],
+                 index[c], value[c], frame[o], index[o], value[o], parent[o]);
     return cudaGetLastError();
   }
 

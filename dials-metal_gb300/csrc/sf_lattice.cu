@@ -140,7 +140,10 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
             const __grid_constant__ FrameSpans S, int run_rows,
             const __grid_constant__ StreamTables T,
             const __grid_constant__ LaunchParams P, uint8_t *__restrict__ final_bytes,
-            size_t mask_bytes) {
+            size_t mask_bytes, uint32_t *__restrict__ counters) {
+  previous_done();
+  if (blockIdx.x == 0 && threadIdx.x < kCounterWords)
+    counters[threadIdx.x] = 0u;  // for the next two kernels
   constexpr bool k16 = sizeof(Pix) == 2;
   extern __shared__ __align__(16) unsigned char lat_ring_raw[];
   Pix *lat_ring = reinterpret_cast<Pix *>(lat_ring_raw);
@@ -441,8 +444,9 @@ constexpr int kTileRun = 8;
 
 __global__ void __launch_bounds__(256)
 lat_tiles(const __grid_constant__ FramePtrs F, int nframes, int env_h, int env_w,
-          const uint32_t *__restrict__ final_all, size_t words, uint32_t *__restrict__ list,
+          const uint32_t *final_all, size_t words, uint32_t *__restrict__ list,
           uint32_t *__restrict__ counters, const __grid_constant__ FrameSpans S, int run) {
+  previous_done();
   const int lane = threadIdx.x & 31;
   // Tile numbers are laid out over the batch's largest frame; each frame has
   // its own tile groups (S) and its own shape bounds its tiles.
@@ -641,8 +645,8 @@ __global__ void __launch_bounds__(kVerWarps * 32, kOcc)
 lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps M, int env_h,
            int env_w, const __grid_constant__ LaunchParams P,
            const __grid_constant__ StreamTables T, uint32_t *__restrict__ final_all, size_t words,
-           const uint32_t *__restrict__ list,
-           uint32_t *__restrict__ counters, FastDiv by_ntiles, FastDiv by_ntx) {
+           const uint32_t *list, uint32_t *__restrict__ counters, FastDiv by_ntiles, FastDiv by_ntx) {
+  previous_done();
   extern __shared__ __align__(128) unsigned char ver_smem_raw[];
   // The launch gives 128 bytes more than the layout needs: the tile buffers
   // start on a 128-byte boundary whatever the base's alignment.
@@ -934,7 +938,7 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, const LaunchP
   const unsigned lb = (unsigned)((S.start[nframes] + kLatWarps - 1) / kLatWarps);
   uint8_t *fin = reinterpret_cast<uint8_t *>(b.cand);
   lat_stage01<kLatOcc, Pix><<<lb, kLatWarps * 32, ring_bytes<Pix>(), stream>>>(
-      F, nframes, S, run_rows, T, P, fin, mask_bytes);
+      F, nframes, S, run_rows, T, P, fin, mask_bytes, b.counters);
   static std::once_flag configured;
   static cudaError_t config_error = cudaSuccess;
   static int ver_blocks = 0;
@@ -963,13 +967,13 @@ cudaError_t lattice(const FramePtrs &F, int nframes, int h, int w, const LaunchP
   uint32_t *list = b.tiles;
   const FastDiv by_ntiles = make_fastdiv((uint32_t)tiles);
   const FastDiv by_ntx = make_fastdiv((uint32_t)ver_ntx(w));
-  lat_tiles<<<tb, 256, 0, stream>>>(F, nframes, h, w, b.cand, b.words, list, b.counters, G,
-                                    trun);
+  launch_after(lat_tiles, tb, 256, 0, stream, F, nframes, h, w, b.cand, b.words, list, b.counters,
+               G, trun);
   TileMaps M;
   make_tile_maps<Pix>(F, nframes, &M);
-  lat_verify<kVerOcc, Pix><<<ver_blocks * device_sms(), kVerWarps * 32, ver_smem_bytes<Pix>(),
-                             stream>>>(F, M, h, w, P, T, b.cand, b.words, list,
-                                       b.counters, by_ntiles, by_ntx);
+  launch_after(lat_verify<kVerOcc, Pix>, ver_blocks * device_sms(), kVerWarps * 32,
+               ver_smem_bytes<Pix>(), stream, F, M, h, w, P, T, b.cand, b.words, list, b.counters,
+               by_ntiles, by_ntx);
   return cudaGetLastError();
 }
 
@@ -1064,10 +1068,6 @@ cudaError_t launch_lattice(const FramePtrs &F, int nframes, int h, int w, int pi
                            cudaStream_t stream) {
   if (P.half != kLatK)
     return cudaErrorInvalidValue;
-  const cudaError_t e =
-      cudaMemsetAsync(b.counters, 0, kCounterWords * sizeof(uint32_t), stream);
-  if (e != cudaSuccess)
-    return e;
   StreamTables T;
   make_stream_tables(P, &T);
   long long strips = 0;

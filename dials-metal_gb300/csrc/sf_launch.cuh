@@ -1,0 +1,42 @@
+// Launches that overlap their start with the end of the kernel before them on
+// the stream (programmatic dependent launch). A kernel launched by launch_after
+// calls previous_done() before it reads or writes anything that an earlier
+// kernel may: its blocks may start once the blocks of the kernel before have
+// left, and wait there until that kernel has completed and its writes are
+// visible, so that the order of the stream's work is as without. Every thread
+// of every block calls it, first of all: a block that left without would let
+// its kernel complete before the one it follows. A sequence's first kernel is
+// launched the ordinary way, after whatever the stream held. One frame of 4362
+// x 4148 takes 76 us with and 84 without, 4 frames of 1649 x 1752 60 and 70.
+// (Letting the next kernel's blocks in
+// while this one's still run, as soon as the last has started, took batches
+// from 1.30 to 1.40 ms.)
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace sf {
+
+__device__ __forceinline__ void previous_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... Params, class... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t stream, Args &&...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, Params(std::forward<Args>(args))...);
+}
+
+} // namespace sf

@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sf_launch.cuh"
+
 namespace sf {
 
 constexpr int kScanBlocks = 512;
@@ -112,6 +114,7 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan64(unsigned lo
 template <class Scan>
 static __global__ void __launch_bounds__(kScanThreads)
 scan_pair_sums(Scan scan, unsigned long long *__restrict__ block_sums) {
+  previous_done();
   if (scan.skip())
     return;
   uint32_t lo, hi;
@@ -129,6 +132,7 @@ scan_pair_sums(Scan scan, unsigned long long *__restrict__ block_sums) {
 template <class Scan>
 static __global__ void __launch_bounds__(kScanThreads)
 scan_pair_apply(Scan scan, const unsigned long long *__restrict__ block_sums) {
+  previous_done();
   if (scan.skip())
     return;
   // This block's offset: the chunk sums of the blocks before it.
@@ -168,8 +172,8 @@ scan_pair_apply(Scan scan, const unsigned long long *__restrict__ block_sums) {
 // block_sums holds kScanBlocks values.
 template <class Scan>
 cudaError_t scan_pairs(const Scan &scan, unsigned long long *block_sums, cudaStream_t stream) {
-  scan_pair_sums<<<kScanBlocks, kScanThreads, 0, stream>>>(scan, block_sums);
-  scan_pair_apply<<<kScanBlocks, kScanThreads, 0, stream>>>(scan, block_sums);
+  launch_after(scan_pair_sums<Scan>, kScanBlocks, kScanThreads, 0, stream, scan, block_sums);
+  launch_after(scan_pair_apply<Scan>, kScanBlocks, kScanThreads, 0, stream, scan, block_sums);
   return cudaGetLastError();
 }
 

@@ -12,6 +12,7 @@
 
 #include <algorithm>
 
+#include "sf_launch.cuh"
 #include "sf_stream.cuh"
 
 namespace sf {
