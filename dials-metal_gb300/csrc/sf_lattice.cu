@@ -384,6 +384,8 @@ template <typename Pix> struct alignas(128) VerWarp {
   uint32_t cw[2][kVerRows][2];           // the tile's candidate words, two tiles (s)
   uint2 vs[kVerDR][kVerPC + 2];          // column sums of 7 rows
   uint32_t msk[kVerPC + 2];              // masked pixels by row, a word a column
+  // The sums of squares' high words (32-bit frames, tiles with large counts).
+  uint16_t vh[sizeof(Pix) == 4 ? kVerDR : 1][kVerPC + 2];
 };
 
 // The frames' 2-D tensor maps, boxes of one tile (kPW x 18 pixels), for the
@@ -640,6 +642,80 @@ __device__ __forceinline__ void ver_window(const VerWarp<Pix> &sm, int d, int co
   *Wq = q;
 }
 
+// A tile that holds a valid pixel too large for the 32-bit sums but below
+// kWidePixel: its column sums again, the masked count above a 28-bit sum and the
+// sum of squares in 48 bits, so that a window still costs 7 columns' loads. (A
+// launch of 4 dense frames of 4362 x 4148, whose tiles nearly all hold an
+// overload, checks its tiles in 967 us so and took 2136 summing each window's
+// 49 pixels.)
+constexpr uint32_t kWidePixel = 1u << 22;
+constexpr int kWideCount = 28;
+static_assert((2 * kLatK + 1) * (kWidePixel - 1) < (1u << kWideCount) &&
+                  (2ull * kLatK + 1) * (kWidePixel - 1) * (kWidePixel - 1) < (1ull << 48),
+              "a column's sums fit their fields");
+// 2^8 n Q and S (2^8 S + c), c < 2^26, stay below 2^64.
+static_assert(49ull * 49ull * (kWidePixel >> 11) * (kWidePixel >> 11) < (1ull << 34),
+              "a window's products fit 64 bits");
+
+__device__ __noinline__ void ver_wide_columns(VerWarp<uint32_t> &sm, int off, int npass,
+                                              int lane) {
+  for (int pass = 0; pass < npass; pass++) {
+    const int i = 32 * pass + lane;
+    if (i >= kVerPC)
+      break;
+    uint32_t cs = 0;  // count and sum
+    unsigned long long cq = 0;
+#pragma unroll
+    for (int r = 0; r < kVerPR; r++) {
+      const uint32_t v = sm.pix[0].px[r][off + i];
+      const uint32_t u = is_masked_px<uint32_t>(v) ? 0u : v;
+      cs += is_masked_px<uint32_t>(v) ? 1u << kWideCount : v;
+      cq += (unsigned long long)u * u;
+      if (r >= 2 * kLatK) {
+        const int d = r - 2 * kLatK;
+        sm.vs[d][i] = make_uint2(cs, (uint32_t)cq);
+        sm.vh[d][i] = (uint16_t)(cq >> 32);
+        const uint32_t o = sm.pix[0].px[d][off + i];
+        const uint32_t w = is_masked_px<uint32_t>(o) ? 0u : o;
+        cs -= is_masked_px<uint32_t>(o) ? 1u << kWideCount : o;
+        cq -= (unsigned long long)w * w;
+      }
+    }
+  }
+}
+
+// The needed windows (`rows`) of a lane's column from those sums: bit d clears
+// when row d's window is not signal. The same two bounds in 64 bits (S < 2^28,
+// Q < 2^50), then the reference's sequence.
+__device__ __noinline__ uint32_t ver_wide_rows(const VerWarp<uint32_t> &sm, uint32_t rows,
+                                               int lane, const uint4 *tab,
+                                               const LaunchParams &P) {
+  uint32_t keep = 0xFFFFFFFFu;
+  while (rows) {
+    const int d = __ffs(rows) - 1;
+    rows &= rows - 1u;
+    uint32_t m = 0, S = 0, hi = 0;
+    unsigned long long Q = 0;
+#pragma unroll
+    for (int u = 0; u <= 2 * kLatK; u++) {
+      const uint2 x = sm.vs[d][lane + u];
+      m += x.x >> kWideCount;
+      S += x.x & ((1u << kWideCount) - 1u);
+      hi += sm.vh[d][lane + u];
+      Q += x.y;
+    }
+    Q += (unsigned long long)hi << 32;
+    m = min(m, (uint32_t)kLatN0);
+    const uint4 c = tab[m];
+    const unsigned long long L = Q * c.x, S8 = (unsigned long long)S << kDec;
+    bool sig = L >= S * (S8 + c.z) + (2ull << kDec);
+    if (!sig && L > S * (S8 + c.y))
+      sig = stage0_u32((uint32_t)kLatN0 - m, S, Q, P, P.root_lo, P.root_hi);
+    keep &= sig ? ~0u : ~(1u << d);
+  }
+  return keep;
+}
+
 template <int kOcc, typename Pix>
 __global__ void __launch_bounds__(kVerWarps * 32, kOcc)
 lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps M, int env_h,
@@ -770,7 +846,14 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     __syncwarp();
     // 16-bit frames sum in 32 bits as the reference does: never wide.
     const bool wide = !k16 && __any_sync(0xffffffffu, mx >= narrow2);
-    if (!wide)
+    const bool huge = !k16 && wide && __any_sync(0xffffffffu, mx >= kWidePixel + 2u);
+    if constexpr (!k16) {
+      if (wide && !huge) {
+        ver_wide_columns(sm, off, npass, lane);
+        __syncwarp();
+      }
+    }
+    if (!huge)
       stage_next();  // the windows come from the column sums, not the pixels
     // The stage-0 positions within 2 of a candidate: lane d first forms row
     // d's (row r0 - 2 + d, bit = column c0 - 2 + bit), then every lane takes
@@ -804,7 +887,9 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
         if (!stage0_u16((uint32_t)kLatN0 - m, Wn & kLatMask, Wq, P))
           keep &= ~(1u << d);
       }
-    } else if (wide) {
+    } else if (wide && !huge) {
+      keep = ver_wide_rows(sm, rows, lane, tab, P);
+    } else if (huge) {
       // 64-bit sums from the staged tile (frames with very large counts).
       while (rows) {
         const int d = __ffs(rows) - 1;
@@ -840,7 +925,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
           keep &= ~(1u << d);
       }
     }
-    if (wide)
+    if (huge)
       stage_next();
     uint32_t D[kVerDR];
 #pragma unroll
