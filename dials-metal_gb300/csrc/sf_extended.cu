@@ -647,9 +647,16 @@ ExtTables make_ext_tables(const LaunchParams &P) {
 // 32-bit frames at gain 1 with integral sigmas, or 16-bit ones where 4 | width
 // and they are 8-byte aligned. Spots cover a few percent of such frames, and
 // the lattice decides a ninth of the windows and the tiles that hold a
-// candidate: 32 frames of 4362 x 4148 take 0.95 ms so and 1.38 ms on strips.
+// candidate: 32 frames of 4362 x 4148 take 0.95 ms so and 1.38 ms on strips. One
+// frame alone takes strips up to kStripAlone pixels, where the call is bound by
+// its launches (lattice and strips, called directly: 512 x 512 53 and 43 us, 1065
+// x 1030 52 and 43, 2162 x 2068 53-58 and 46-60, 3262 x 3108 60 and 66; in a
+// captured graph: 32 and 33, 37 and 38, 41 and 45, 59 and 66).
+constexpr long long kStripAlone = 3000000;
 bool lattice_path(const FramePtrs &F, int nframes, int pixel_bytes, const LaunchParams &P) {
   if (P.half != 3 || P.algorithm != SF_DISPERSION_EXTENDED)
+    return false;
+  if (nframes == 1 && (long long)F.h[0] * F.w[0] <= kStripAlone)
     return false;
   if (pixel_bytes == 4)
     return P.int_ok != 0;
