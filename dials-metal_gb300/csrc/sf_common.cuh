@@ -180,19 +180,20 @@ __device__ __forceinline__ bool stage2_u32(uint32_t p, uint32_t n,
 // 16-bit frames: the tests are float (src/spots/dext.hh:31-33) and cheap, so
 // they run as the reference's sequence of IEEE float operations.
 // ---------------------------------------------------------------------------
+// Stage 0 with its factors m = n and root = sqrt(2 (n - 1)) given.
+__device__ __forceinline__ bool stage0_float(float m, float root, uint32_t S, uint32_t Q, float g,
+                                             float sb) {
+  const float s = __uint2float_rn(S), s2 = __uint2float_rn(Q);
+  const float gs = __fmul_rn(g, s);
+  return __fsub_rn(__fsub_rn(__fmul_rn(m, s2), __fmul_rn(s, s)),
+                   __fmul_rn(gs, __fsub_rn(m, 1.0f))) > __fmul_rn(__fmul_rn(gs, sb), root);
+}
+
 __device__ __forceinline__ bool stage0_u16(uint32_t n, uint32_t S, uint32_t Q,
                                            const LaunchParams &P) {
   if (n < P.min_local)
     return false;
-  const float g = (float)P.gain, sb = (float)P.sigma_b;
-  const float m = __uint2float_rn(n);
-  const float s = __uint2float_rn(S);
-  const float s2 = __uint2float_rn(Q);
-  const float gs = __fmul_rn(g, s);
-  const float lhs = __fsub_rn(__fsub_rn(__fmul_rn(m, s2), __fmul_rn(s, s)),
-                              __fmul_rn(gs, __fsub_rn(m, 1.0f)));
-  const float rhs = __fmul_rn(__fmul_rn(gs, sb), P.rootf[n]);
-  return lhs > rhs;
+  return stage0_float(__uint2float_rn(n), P.rootf[n], S, Q, (float)P.gain, (float)P.sigma_b);
 }
 
 __device__ __forceinline__ bool stage2_u16(uint32_t p, uint32_t n, uint32_t S,

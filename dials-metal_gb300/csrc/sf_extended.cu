@@ -120,15 +120,6 @@ __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image
   return bits;
 }
 
-// The float sequence of stage0_u16 (sf_common.cuh) with its factors given.
-__device__ __forceinline__ bool ext_float(float m, float root, uint32_t S, uint32_t Q, float g,
-                                          float sb) {
-  const float s = __uint2float_rn(S), s2 = __uint2float_rn(Q);
-  const float gs = __fmul_rn(g, s);
-  return __fsub_rn(__fsub_rn(__fmul_rn(m, s2), __fmul_rn(s, s)),
-                   __fmul_rn(gs, __fsub_rn(m, 1.0f))) > __fmul_rn(__fmul_rn(gs, sb), root);
-}
-
 // A window's constants by its masked count m (n = N0 - m): the 2^-4 tests' {nk,
 // clo, chi - clo} and n, and the 2^-8 tests' {nk, clo, chi}; for 16-bit frames
 // {n, rootf} as floats (rootf NaN, no test passes, below min_local).
@@ -245,12 +236,12 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           const float m = __uint_as_float(t.x), root = __uint_as_float(t.y);
 #pragma unroll
           for (int c = 0; c < kCols; c++)
-            sig |= ext_float(m, root, hn[c], hq[c], gain, sigma_b) ? 1u << c : 0u;
+            sig |= stage0_float(m, root, hn[c], hq[c], gain, sigma_b) ? 1u << c : 0u;
         } else {
 #pragma unroll
           for (int c = 0; c < kCols; c++) {
             const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].a;
-            sig |= ext_float(__uint_as_float(t.x), __uint_as_float(t.y), hn[c] & kSumMask, hq[c],
+            sig |= stage0_float(__uint_as_float(t.x), __uint_as_float(t.y), hn[c] & kSumMask, hq[c],
                              gain, sigma_b)
                        ? 1u << c
                        : 0u;

@@ -26,9 +26,8 @@
 // of the reference. A window with a larger S is taken as signal, and the tile
 // check decides it exactly.
 //
-// The tile check decides only the stage-0 windows within 2 of a candidate
-// (the only ones whose decision can clear one), about a fifth of a tile's,
-// spread over the warp's lanes.
+// The tile check decides the stage-0 windows of the rows within 2 of a candidate
+// (the only ones whose decision can clear one), four next to one another a lane.
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -333,19 +332,24 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
 //
 //   lat_tiles   lists the tiles that hold a candidate (any order)
 //   lat_verify  one warp per listed tile, persistent: the tile's 12 x 32
-//               stage-0 windows (rows r0 - 2 .., columns c0 - 2 .., lane =
-//               column) from its 18 x 38 pixels, the erosion of its 8 x 28
-//               pixels, and the candidates that fail cleared from both masks
+//               stage-0 windows (rows r0 - 2 .., columns c0 - 2 ..) from its
+//               18 x 38 pixels, the erosion of its 8 x 28 pixels, and the
+//               candidates that fail cleared from the mask
 //
-// A warp copies the next tile's pixels into shared memory (cp.async, 16-byte
-// pieces where the frame allows) while it checks the current one, so the
-// loads' latency is hidden behind the arithmetic. Column sums of 7 rows go to
-// shared memory; then only the stage-0 windows within 2 of a candidate (the
-// only ones that can clear one, about a fifth of the tile's) are decided,
-// spread over the lanes: the two bounds of sf_lattice.cuh, and the reference's
-// sequence between them (sf_common.cuh). Tiles share mask words, so the
-// clearing is an atomic AND; each candidate belongs to one tile, so the order
-// does not matter.
+// A warp copies the next tile's pixels into shared memory (a TMA box where the
+// frame allows) while it checks the current one, so the loads' latency is
+// hidden behind the arithmetic. A lane a column, the column sums of 7 rows go
+// to shared memory; then four rows of windows at a time, eight lanes a row, each
+// lane decides four windows next to one another from ten column sums: the two
+// bounds of sf_lattice.cuh, and the reference's sequence between them
+// (sf_common.cuh). Rows without a window within 2 of a candidate are left out.
+// The candidates, the decisions and the erosion are a row a lane. Tiles share
+// mask words, so the clearing is an atomic AND; each candidate belongs to one
+// tile, so the order does not matter. Bound by issue (64% of its rate, 820
+// instructions a tile): 32 frames of 4362 x 4148 take 297 us, 148 of 16 bits, 4
+// dense ones 783; with a lane a column for the windows too, each lane taking its
+// column's needed ones in turn (11 rounds a tile, 12 lanes in them), and the
+// erosion a row after another in every lane, 449, 250 and 967 us.
 // ---------------------------------------------------------------------------
 constexpr int kVerRows = 8;                  // output rows of a tile
 constexpr int kVerTW = 28;                   // output columns of a tile
@@ -382,10 +386,12 @@ template <typename Pix> struct alignas(128) VerWarp {
                                          // once the current one's are read)
   uint64_t bar[1];                       // its TMA mbarrier
   uint32_t cw[2][kVerRows][2];           // the tile's candidate words, two tiles (s)
-  uint2 vs[kVerDR][kVerPC + 2];          // column sums of 7 rows
-  uint32_t msk[kVerPC + 2];              // masked pixels by row, a word a column
+  alignas(16) uint2 vs[kVerDR][kVerPC + 2];  // column sums of 7 rows
+  // Masked centres, a word a column (column i's at i + 1, so that a lane's four
+  // are one load), bit d for stage-0 row d.
+  alignas(16) uint32_t msk[kVerPC + 2];
   // The sums of squares' high words (32-bit frames, tiles with large counts).
-  uint16_t vh[sizeof(Pix) == 4 ? kVerDR : 1][kVerPC + 2];
+  alignas(8) uint16_t vh[sizeof(Pix) == 4 ? kVerDR : 1][kVerPC + 2];
 };
 
 // The frames' 2-D tensor maps, boxes of one tile (kPW x 18 pixels), for the
@@ -624,30 +630,88 @@ __device__ __forceinline__ void ver_stage(VerWarp<Pix> &sm, int s, uint32_t e, c
   }
 }
 
-// The packed sums of the stage-0 window of row d, column `col` of a tile
-// (seven column sums of seven rows; a window holds 49 pixels, so its masked
-// count m <= 49 -- callers clamp it anyway, which keeps the per-count tables
-// in bounds whatever the sums).
-template <typename Pix>
-__device__ __forceinline__ void ver_window(const VerWarp<Pix> &sm, int d, int col, uint32_t *Wn,
-                                           uint32_t *Wq) {
-  uint32_t n = 0, q = 0;
+// A lane decides four windows next to one another: stage-0 row d, columns 4j ..
+// 4j + 3, of which only those of `need` matter. Their sums share the ten column
+// sums they read; the result has bit c set where window c is signal. A window's
+// masked count is clamped to its 49 pixels, which keeps the per-count tables in
+// bounds whatever the sums.
+constexpr int kVerGroup = 4;
+static_assert(kVerDR * 32 / kVerGroup % 32 == 0, "whole rounds of groups over the lanes");
+
+template <class Decide>
+__device__ __forceinline__ void ver_windows(const uint2 *vs, Decide decide) {
+  uint32_t n[kVerGroup + 6], q[kVerGroup + 6];
 #pragma unroll
-  for (int u = 0; u <= 2 * kLatK; u++) {
-    const uint2 x = sm.vs[d][col + u];
-    n += x.x;
-    q += x.y;
+  for (int c = 0; c < (kVerGroup + 6) / 2; c++) {
+    const uint4 x = reinterpret_cast<const uint4 *>(vs)[c];
+    n[2 * c] = x.x, q[2 * c] = x.y, n[2 * c + 1] = x.z, q[2 * c + 1] = x.w;
   }
-  *Wn = n;
-  *Wq = q;
+  uint32_t Wn = 0, Wq = 0;
+#pragma unroll
+  for (int c = 0; c < 7; c++) {
+    Wn += n[c];
+    Wq += q[c];
+  }
+#pragma unroll
+  for (int c = 0; c < kVerGroup; c++) {
+    if (c) {
+      Wn = Wn - n[c - 1] + n[c + 6];
+      Wq = Wq - q[c - 1] + q[c + 6];
+    }
+    decide(c, Wn, Wq);
+  }
+}
+
+// 32-bit frames: the two bounds first; the needed windows between them (rare)
+// by the reference's sequence. kClean: the tile holds no masked pixel.
+template <bool kClean>
+__device__ __forceinline__ uint32_t ver_group(const VerWarp<uint32_t> &sm, int d, int j,
+                                              uint32_t need, const uint4 *tab,
+                                              const LaunchParams &P) {
+  uint32_t sig = 0, amb = 0;
+  const uint4 t0 = tab[0];
+  ver_windows(&sm.vs[d][kVerGroup * j], [&](int c, uint32_t Wn, uint32_t Wq) {
+    const uint32_t S = kClean ? Wn : Wn & kLatMask;
+    const uint4 t = kClean ? t0 : tab[min(Wn >> kLatPS, (uint32_t)kLatN0)];
+    const unsigned long long L = (unsigned long long)Wq * t.x;
+    const bool maybe = L > (unsigned long long)S * ((S << kDec) + t.y);
+    const bool sure = L >= (unsigned long long)S * ((S << kDec) + t.z) + (2ull << kDec);
+    sig |= sure ? 1u << c : 0u;
+    amb |= (maybe & !sure) ? 1u << c : 0u;
+  });
+  amb &= need;
+  if (amb) {
+    ver_windows(&sm.vs[d][kVerGroup * j], [&](int c, uint32_t Wn, uint32_t Wq) {
+      const uint32_t m = min(Wn >> kLatPS, (uint32_t)kLatN0);
+      if ((amb >> c & 1u) && lat_exact((uint32_t)kLatN0 - m, Wn & kLatMask, Wq, P))
+        sig |= 1u << c;
+    });
+  }
+  return sig;
+}
+
+// 16-bit frames: the reference's float test, exactly, its factors {n, root} from
+// the table.
+template <bool kClean>
+__device__ __forceinline__ uint32_t ver_group(const VerWarp<uint16_t> &sm, int d, int j, uint32_t,
+                                              const uint4 *tab, const LaunchParams &P) {
+  uint32_t sig = 0;
+  const float gain = (float)P.gain, sigma_b = (float)P.sigma_b;
+  const uint4 t0 = tab[0];
+  ver_windows(&sm.vs[d][kVerGroup * j], [&](int c, uint32_t Wn, uint32_t Wq) {
+    const uint32_t S = kClean ? Wn : Wn & kLatMask;
+    const uint4 t = kClean ? t0 : tab[min(Wn >> kLatPS, (uint32_t)kLatN0)];
+    sig |= stage0_float(__uint_as_float(t.x), __uint_as_float(t.y), S, Wq, gain, sigma_b) ? 1u << c
+                                                                                         : 0u;
+  });
+  return sig;
 }
 
 // A tile that holds a valid pixel too large for the 32-bit sums but below
 // kWidePixel: its column sums again, the masked count above a 28-bit sum and the
-// sum of squares in 48 bits, so that a window still costs 7 columns' loads. (A
-// launch of 4 dense frames of 4362 x 4148, whose tiles nearly all hold an
-// overload, checks its tiles in 967 us so and took 2136 summing each window's
-// 49 pixels.)
+// sum of squares in 48 bits. (A launch of 4 dense frames of 4362 x 4148, whose
+// tiles nearly all hold an overload, takes less than half of what summing each
+// window's 49 pixels took: 2136 us.)
 constexpr uint32_t kWidePixel = 1u << 22;
 constexpr int kWideCount = 28;
 static_assert((2 * kLatK + 1) * (kWidePixel - 1) < (1u << kWideCount) &&
@@ -665,12 +729,15 @@ __device__ __noinline__ void ver_wide_columns(VerWarp<uint32_t> &sm, int off, in
       break;
     uint32_t cs = 0;  // count and sum
     unsigned long long cq = 0;
+    uint32_t mk = 0;
 #pragma unroll
     for (int r = 0; r < kVerPR; r++) {
       const uint32_t v = sm.pix[0].px[r][off + i];
       const uint32_t u = is_masked_px<uint32_t>(v) ? 0u : v;
       cs += is_masked_px<uint32_t>(v) ? 1u << kWideCount : v;
       cq += (unsigned long long)u * u;
+      if (r >= kLatK && r < kLatK + kVerDR)
+        mk |= is_masked_px<uint32_t>(v) ? 1u << (r - kLatK) : 0u;
       if (r >= 2 * kLatK) {
         const int d = r - 2 * kLatK;
         sm.vs[d][i] = make_uint2(cs, (uint32_t)cq);
@@ -681,39 +748,45 @@ __device__ __noinline__ void ver_wide_columns(VerWarp<uint32_t> &sm, int off, in
         cq -= (unsigned long long)w * w;
       }
     }
+    sm.msk[i + 1] = mk;
   }
 }
 
-// The needed windows (`rows`) of a lane's column from those sums: bit d clears
-// when row d's window is not signal. The same two bounds in 64 bits (S < 2^28,
-// Q < 2^50), then the reference's sequence.
-__device__ __noinline__ uint32_t ver_wide_rows(const VerWarp<uint32_t> &sm, uint32_t rows,
-                                               int lane, const uint4 *tab,
-                                               const LaunchParams &P) {
-  uint32_t keep = 0xFFFFFFFFu;
-  while (rows) {
-    const int d = __ffs(rows) - 1;
-    rows &= rows - 1u;
-    uint32_t m = 0, S = 0, hi = 0;
-    unsigned long long Q = 0;
+// ver_group from those sums: the same two bounds in 64 bits (S < 2^28, Q <
+// 2^50), then the reference's sequence.
+__device__ __noinline__ uint32_t ver_wide_group(const VerWarp<uint32_t> &sm, int d, int j,
+                                                uint32_t need, const uint4 *tab,
+                                                const LaunchParams &P) {
+  constexpr int kN = kVerGroup + 6;
+  uint32_t n[kN], lo[kN], hi[kN];
 #pragma unroll
-    for (int u = 0; u <= 2 * kLatK; u++) {
-      const uint2 x = sm.vs[d][lane + u];
-      m += x.x >> kWideCount;
-      S += x.x & ((1u << kWideCount) - 1u);
-      hi += sm.vh[d][lane + u];
-      Q += x.y;
-    }
-    Q += (unsigned long long)hi << 32;
-    m = min(m, (uint32_t)kLatN0);
-    const uint4 c = tab[m];
-    const unsigned long long L = Q * c.x, S8 = (unsigned long long)S << kDec;
-    bool sig = L >= S * (S8 + c.z) + (2ull << kDec);
-    if (!sig && L > S * (S8 + c.y))
-      sig = stage0_u32((uint32_t)kLatN0 - m, S, Q, P, P.root_lo, P.root_hi);
-    keep &= sig ? ~0u : ~(1u << d);
+  for (int c = 0; c < kN / 2; c++) {
+    const uint4 x = reinterpret_cast<const uint4 *>(&sm.vs[d][kVerGroup * j])[c];
+    const uint32_t h = reinterpret_cast<const uint32_t *>(&sm.vh[d][kVerGroup * j])[c];
+    n[2 * c] = x.x, lo[2 * c] = x.y, hi[2 * c] = h & 0xFFFFu;
+    n[2 * c + 1] = x.z, lo[2 * c + 1] = x.w, hi[2 * c + 1] = h >> 16;
   }
-  return keep;
+  uint32_t m = 0, S = 0, sig = 0;
+  unsigned long long Q = 0;
+#pragma unroll
+  for (int c = 0; c < kN; c++) {
+    m += n[c] >> kWideCount;
+    S += n[c] & ((1u << kWideCount) - 1u);
+    Q += (unsigned long long)hi[c] << 32 | lo[c];
+    if (c >= 6) {
+      const uint32_t mc = min(m, (uint32_t)kLatN0);
+      const uint4 t = tab[mc];
+      const unsigned long long L = Q * t.x, S8 = (unsigned long long)S << kDec;
+      bool is = L >= S * (S8 + t.z) + (2ull << kDec);
+      if (!is && (need >> (c - 6) & 1u) && L > S * (S8 + t.y))
+        is = stage0_u32((uint32_t)kLatN0 - mc, S, Q, P, P.root_lo, P.root_hi);
+      sig |= is ? 1u << (c - 6) : 0u;
+      m -= n[c - 6] >> kWideCount;
+      S -= n[c - 6] & ((1u << kWideCount) - 1u);
+      Q -= (unsigned long long)hi[c - 6] << 32 | lo[c - 6];
+    }
+  }
+  return sig;
 }
 
 template <int kOcc, typename Pix>
@@ -731,7 +804,14 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
   constexpr bool k16 = sizeof(Pix) == 2;
   VerWarp<Pix> *warps = reinterpret_cast<VerWarp<Pix> *>(ver_smem + sizeof(uint4) * 64);
   for (int m = threadIdx.x; m <= kLatN0; m += blockDim.x)
-    tab[m] = make_uint4(T.nk[kLatN0 - m], T.clo[kLatN0 - m], T.chi[kLatN0 - m], 0u);
+    if constexpr (k16) {
+      const int n = kLatN0 - m;  // (a NaN root: no test passes)
+      tab[m] = make_uint4(__float_as_uint((float)n),
+                          (uint32_t)n < P.min_local ? 0x7FFFFFFFu : __float_as_uint(P.rootf[n]),
+                          0u, 0u);
+    } else {
+      tab[m] = make_uint4(T.nk[kLatN0 - m], T.clo[kLatN0 - m], T.chi[kLatN0 - m], 0u);
+    }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   VerWarp<Pix> &sm = warps[warp];
   if (lane == 0) {
@@ -790,25 +870,21 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     };
     const int off = (c0 - 5) - tile_xs<Pix>(c0);
     const int w0 = c0 >> 5, sh = c0 & 31;
-    uint32_t cj[kVerRows];
-#pragma unroll
-    for (int o = 0; o < kVerRows; o++) {
-      const unsigned long long x =
-          (unsigned long long)sm.cw[s][o][0] | (unsigned long long)sm.cw[s][o][1] << 32;
-      cj[o] = (uint32_t)(x >> sh) & ((1u << kVerTW) - 1u);
-    }
+    // The tile's candidates, a row a lane (lanes 0-7).
+    uint32_t cj = 0;
+    if (lane < kVerRows)
+      cj = (uint32_t)(((unsigned long long)sm.cw[s][lane][0] |
+                       (unsigned long long)sm.cw[s][lane][1] << 32) >> sh) &
+           ((1u << kVerTW) - 1u);
     // Columns B (pixel columns 32-37, stage-0 columns 26-31) matter only
     // when a candidate lies in the tile's last 6 columns.
-    uint32_t late = 0;
-#pragma unroll
-    for (int o = 0; o < kVerRows; o++)
-      late |= cj[o] >> 22;
+    const bool late = __any_sync(0xffffffffu, (cj >> 22) != 0u);
     const int npass = late ? 2 : 1;
     // Pixel columns off + lane (A) and off + 32 + lane (B, lanes 0-5): the
-    // masked pixels by row, the largest valid one, and the column sums of 7
+    // masked centres, the largest valid pixel, and the column sums of 7
     // rows for the 12 stage-0 rows (exact in 32 bits unless the tile holds a
     // valid pixel at or above narrow_max, which the check below catches).
-    uint32_t mx = 0;
+    uint32_t mx = 0, masked = 0;
 #pragma unroll
     for (int pass = 0; pass < 2; pass++) {
       if (pass == npass)
@@ -820,14 +896,17 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
 #pragma unroll
       for (int r = 0; r < kVerPR; r++) {
         const uint32_t v = sm.pix[0].px[r][col];
-        const bool masked = is_masked_px<Pix>(v);
         if (!k16)
           mx = max(mx, v + 2u);
-        mk |= (masked ? 1u : 0u) << r;
-        ns[r] = masked ? (1u << kLatPS) : v;
+        ns[r] = is_masked_px<Pix>(v) ? (1u << kLatPS) : v;
         q[r] = ns[r] * ns[r];
       }
-      sm.msk[32 * pass + lane] = mk;
+      // A valid pixel below narrow_max (2^14) leaves nothing of itself when
+      // its count bit is shifted down; a 16-bit one may.
+#pragma unroll
+      for (int d = 0; d < kVerDR; d++)
+        mk += k16 ? (ns[d + kLatK] >> kLatPS) << d : ns[d + kLatK] >> (kLatPS - d);
+      sm.msk[32 * pass + lane + 1] = mk;
       uint32_t cn = 0, cq = 0;
 #pragma unroll
       for (int r = 0; r < 2 * kLatK; r++) {
@@ -839,6 +918,8 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
         cn += ns[d + 2 * kLatK];
         cq += q[d + 2 * kLatK];
         sm.vs[d][32 * pass + lane] = make_uint2(cn, cq);
+        if (d == 0 || d == 7 || d == kVerDR - 1)
+          masked |= cn;  // (these three cover the column)
         cn -= ns[d];
         cq -= q[d];
       }
@@ -855,105 +936,68 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     }
     if (!huge)
       stage_next();  // the windows come from the column sums, not the pixels
-    // The stage-0 positions within 2 of a candidate: lane d first forms row
-    // d's (row r0 - 2 + d, bit = column c0 - 2 + bit), then every lane takes
-    // its own column's rows of them, less those whose centre is masked (set
-    // whatever the window).
-    uint32_t need = 0;
-#pragma unroll
-    for (int o = 0; o < kVerRows; o++)
-      need |= (o >= lane - 4 && o <= lane) ? cj[o] : 0u;
-    {
-      const uint32_t x2 = need | need << 1;
-      need = lane < kVerDR ? (x2 | x2 << 2 | need << 4) : 0u;
-    }
-    uint32_t rows = 0;
-#pragma unroll
-    for (int d = 0; d < kVerDR; d++)
-      rows |= ((__shfl_sync(0xffffffffu, need, d) >> lane) & 1u) << d;
-    rows &= ~(sm.msk[lane + kLatK] >> kLatK);
-    // Each lane decides its column's needed windows (lane = column, so no
-    // two lanes share a result bit): a row's bit clears when its window is
-    // not signal.
-    uint32_t keep = 0xFFFFFFFFu;  // bit d: row d's window here is signal (or not needed)
-    if constexpr (k16) {
-      // The reference's float test of every needed window, exactly.
-      while (rows) {
-        const int d = __ffs(rows) - 1;
-        rows &= rows - 1u;
-        uint32_t Wn, Wq;
-        ver_window(sm, d, lane, &Wn, &Wq);
-        const uint32_t m = min(Wn >> kLatPS, (uint32_t)kLatN0);
-        if (!stage0_u16((uint32_t)kLatN0 - m, Wn & kLatMask, Wq, P))
-          keep &= ~(1u << d);
+    // The stage-0 positions within 2 of a candidate, lane d row d's (row r0 - 2
+    // + d, bit = column c0 - 2 + bit): the rows' candidates d - 4 .. d (a lane
+    // without a row so far up ORs itself again).
+    uint32_t need = cj | __shfl_up_sync(0xffffffffu, cj, 1);
+    need |= __shfl_up_sync(0xffffffffu, need, 2);
+    need |= __shfl_up_sync(0xffffffffu, cj, 4);
+    need = (need | need << 1) | (need | need << 1) << 2 | need << 4;
+    const unsigned live = __ballot_sync(0xffffffffu, need != 0u);
+    const bool clean = !wide && !__any_sync(0xffffffffu, (masked >> kLatPS) != 0u);
+    // Rounds of four rows, a group of four windows a lane. A row's bit is set
+    // where its window is signal, its centre masked, or neither needed.
+    uint32_t D = 0xFFFFFFFFu;  // lane d: row d
+#pragma unroll 1
+    for (int d0 = 0; d0 < kVerDR; d0 += kVerGroup) {
+      if (!(live >> d0 & ((1u << kVerGroup) - 1u)))
+        continue;  // warp-uniform
+      const int d = d0 + (lane >> 3), j = lane & 7;
+      uint32_t nd = __shfl_sync(0xffffffffu, need, d) >> (kVerGroup * j) & 15u, sig;
+      if (huge) {
+        // 64-bit sums of each window's pixels (frames with very large counts).
+        sig = 0;
+        if constexpr (!k16)
+          for (int c = 0; c < kVerGroup; c++)
+            if (nd >> c & 1u)
+              sig |= lat_wide(sm.pix[0].px, d, off + kVerGroup * j + c, P) ? 1u << c : 0u;
+      } else if (clean) {
+        sig = ver_group<true>(sm, d, j, nd, tab, P);
+      } else {
+        const uint4 m = *reinterpret_cast<const uint4 *>(&sm.msk[kVerGroup * j + kLatK + 1]);
+        nd &= ~((m.x >> d & 1u) | (m.y >> d & 1u) << 1 | (m.z >> d & 1u) << 2 |
+                (m.w >> d & 1u) << 3);
+        if (!wide)
+          sig = ver_group<false>(sm, d, j, nd, tab, P);
+        else if constexpr (!k16)
+          sig = ver_wide_group(sm, d, j, nd, tab, P);
       }
-    } else if (wide && !huge) {
-      keep = ver_wide_rows(sm, rows, lane, tab, P);
-    } else if (huge) {
-      // 64-bit sums from the staged tile (frames with very large counts).
-      while (rows) {
-        const int d = __ffs(rows) - 1;
-        rows &= rows - 1u;
-        if (!lat_wide(reinterpret_cast<const uint32_t (*)[kVerPW]>(sm.pix[0].px), d,
-                      off + lane, P))
-          keep &= ~(1u << d);
-      }
-    } else {
-      // The two bounds first; the windows between them (rare) are decided by
-      // the reference's sequence afterwards, out of the loop.
-      uint32_t amb = 0;
-      while (rows) {
-        const int d = __ffs(rows) - 1;
-        rows &= rows - 1u;
-        uint32_t Wn, Wq;
-        ver_window(sm, d, lane, &Wn, &Wq);
-        const uint32_t m = min(Wn >> kLatPS, (uint32_t)kLatN0), S = Wn & kLatMask;
-        const uint4 c = tab[m];
-        const unsigned long long L = (unsigned long long)Wq * c.x;
-        const bool maybe = L > (unsigned long long)S * ((S << kDec) + c.y);
-        const bool sure = L >= (unsigned long long)S * ((S << kDec) + c.z) + (2ull << kDec);
-        keep &= maybe ? ~0u : ~(1u << d);
-        amb |= (maybe & !sure) ? 1u << d : 0u;
-      }
-      while (amb) {
-        const int d = __ffs(amb) - 1;
-        amb &= amb - 1u;
-        uint32_t Wn, Wq;
-        ver_window(sm, d, lane, &Wn, &Wq);
-        const uint32_t m = min(Wn >> kLatPS, (uint32_t)kLatN0);
-        if (!lat_exact((uint32_t)kLatN0 - m, Wn & kLatMask, Wq, P))
-          keep &= ~(1u << d);
-      }
+      uint32_t row = ((~nd | sig) & 15u) << (kVerGroup * j);
+      row |= __shfl_xor_sync(0xffffffffu, row, 1);
+      row |= __shfl_xor_sync(0xffffffffu, row, 2);
+      row |= __shfl_xor_sync(0xffffffffu, row, 4);
+      row = __shfl_sync(0xffffffffu, row, (8 * (lane - d0)) & 31);
+      if (lane >= d0 && lane < d0 + kVerGroup)
+        D = row;
     }
     if (huge)
       stage_next();
-    uint32_t D[kVerDR];
-#pragma unroll
-    for (int d = 0; d < kVerDR; d++)
-      D[d] = __ballot_sync(0xffffffffu, (keep >> d) & 1u);
     __syncwarp();  // the next tile rewrites the shared rows
-    // The exact erosion of the tile's rows; the candidates that fail leave
-    // the mask.
-    uint32_t *fin = final_all + (size_t)f * words;
-#pragma unroll
-    for (int o = 0; o < kVerRows; o++) {
-      uint32_t V = 0xFFFFFFFFu;
-#pragma unroll
-      for (int u = 0; u < 5; u++)
-        V &= D[o + u];
-      uint32_t H = V;
-#pragma unroll
-      for (int u = 1; u < 5; u++)
-        H &= V >> u;
-      const uint32_t clear = cj[o] & ~H;
-      if (clear && lane < 2) {
-        const unsigned long long c64 = (unsigned long long)clear << sh;
-        const uint32_t part = (uint32_t)(c64 >> (32 * lane));
-        if (part && w0 + lane < wpr) {
-          const size_t at = (size_t)(r0 + o) * wpr + w0 + lane;
-          atomicAnd(fin + at, ~part);
-        }
-      }
+    // The exact erosion, lane o row o's; the candidates that fail leave the mask.
+    uint32_t V = D & __shfl_down_sync(0xffffffffu, D, 1);
+    V &= __shfl_down_sync(0xffffffffu, V, 2);
+    V &= __shfl_down_sync(0xffffffffu, D, 4);
+    uint32_t H = V & V >> 1;
+    H &= H >> 2;
+    H &= V >> 4;
+    const uint32_t clear = cj & ~H;  // (cj is 0 in lanes without a row)
+    if (clear) {
+      const unsigned long long c64 = (unsigned long long)clear << sh;
+      uint32_t *at = final_all + (size_t)f * words + (size_t)(r0 + lane) * wpr + w0;
+      if ((uint32_t)c64)
+        atomicAnd(at, ~(uint32_t)c64);
+      if ((uint32_t)(c64 >> 32) && w0 + 1 < wpr)
+        atomicAnd(at + 1, ~(uint32_t)(c64 >> 32));
     }
   }
   // After a fault: the load still in flight (bounded) before the buffer goes.

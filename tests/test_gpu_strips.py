@@ -67,3 +67,34 @@ def test_strips_against_oracle(h, w, kernel, bits, algorithm):
             per = words.reshape(-1, 32).sum(axis=1)
             got = b.word_prefix[j].cpu().numpy()
             assert np.array_equal(got, np.cumsum(per) - per), (j, p)
+
+
+@pytest.mark.parametrize("top", [9361, 9362, (1 << 22) - 1, 1 << 22])
+@pytest.mark.parametrize("h,w", [(24, 84), (37, 361), (90, 412)])
+def test_tiles_of_large_counts_against_oracle(h, w, top):
+    """Frames whose largest pixel is just below or at the counts where a tile's
+    check changes its sums: spots and flat fields of that count, with and without
+    masked pixels beside them."""
+    import torch
+    from sfgb import api
+    rng = np.random.default_rng(h + top)
+    sparse = rng.poisson(3.0, (h, w)).astype(np.uint32)
+    for _ in range(max(3, h * w // 400)):
+        y, x = rng.integers(0, h), rng.integers(0, w)
+        sparse[max(0, y - 1):y + 2, max(0, x - 2):x + 2] = top
+    dense = rng.poisson(20.0, (h, w)).astype(np.uint32)
+    dense[rng.random((h, w)) < 0.02] = top
+    flat = rng.integers(top - 40, top + 1, (h, w)).astype(np.uint32)
+    flat[h // 2:h // 2 + 3, w // 3:w // 3 + 3] = 5
+    frames = [sparse, dense, flat]
+    for f in frames[:]:
+        g = f.copy()
+        g[rng.random((h, w)) < 0.03] = 0xFFFFFFFF
+        g[:, w // 2:w // 2 + 4] = 0xFFFFFFFE
+        frames.append(g)
+    for kw in (dict(), dict(sigma_b=2.0, sigma_s=1.0, min_local=5), dict(sigma_b=0.0, sigma_s=0.0)):
+        p = dict(algorithm=1, kernel_x=3, kernel_y=3, **kw)
+        b = api.DeviceBatch(h, w, len(frames), capacity=h * w, params=api.Params(**p))
+        b([torch.from_numpy(f.view(np.int32)).cuda() for f in frames])
+        for j, f in enumerate(frames):
+            assert b.result(j).tobytes() == O.dext(f, O.Params(**p)).tobytes(), (j, p)
