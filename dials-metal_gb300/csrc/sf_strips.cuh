@@ -305,8 +305,11 @@ __device__ __forceinline__ void window_sums(const uint32_t V[kCols], uint32_t h[
 // kStripWaves times over, so that warps of unequal cost even out (one wave
 // left a third of the warps' time idle), as long as a run keeps kLongRun
 // rows (each run reads some rows more than it writes); else once, down to
-// runs of kMinRunRows.
-constexpr int kMinRunRows = 8;
+// runs of kMinRunRows: a launch that cannot fill the device is a warp's walk
+// long. (One frame of 1065 x 1030: the strips take 21 us with 2 to 4 rows, 26
+// with 8; one of 430 x 393 whose windows need 64-bit sums is 92 us in all with 2,
+// 110 with 4, 145 with 8.)
+constexpr int kMinRunRows = 2;
 constexpr int kLongRun = 64;
 constexpr int kStripWaves = 4;
 
