@@ -385,15 +385,21 @@ __device__ __noinline__ void ext_wide_window(const Pix *image, const uint32_t *c
   *S_out = S;
 }
 
+constexpr int kListItems = 256;  // runs listed at a time
+constexpr int kListAhead = 4;    // their words read together
+constexpr uint32_t kHeavyRun = 48;  // candidates of a run that is taken early
+
 // A warp takes a run of a band at a time (128 columns x 8 rows, a word a lane)
 // and its candidates in chunks: from the leftmost column with one left, the NC
 // columns whose windows 32 columns cover, for all 8 rows (a spot's candidates
 // are about 7 x 7). The chunk's pixels are read once, a lane a column, added up
 // over the window's rows into shared memory; then its candidates are spread
-// over the lanes, each adding up its window's columns for the test. The warps
-// of a block take the runs of its bands in turn from a counter, so that those
-// with many candidates even out. Bound by issue: 32 frames of 4362 x 4148 (174
-// thousand candidates each) take 292 us. A window a candidate, four lanes each,
+// over the lanes, each adding up its window's columns for the test. A
+// block first lists the runs of its bands that hold a candidate, four a warp on
+// their way at once; its warps then take them in turn, those with many candidates
+// first, so that they even out. Bound by issue: 32 frames of 4362 x 4148 (174
+// thousand candidates each) take 266 us, 290 with the runs taken in order, the
+// empty ones among them, each read when its turn came (one frame 19 and 22). A window a candidate, four lanes each,
 // took 568 us, chunks of one row 427, and tests row by row, only the row's
 // candidates' lanes busy, 553.
 template <int K, typename Pix>
@@ -404,7 +410,8 @@ ext_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchPa
   previous_done();
   constexpr int K2 = K + 2, W2 = 2 * K2 + 1, NC = 32 - 2 * K2, ROWS = kBandRows + 2 * K2;
   __shared__ ExtWarp s_warps[kScanT / 32];
-  __shared__ uint32_t s_count[2], s_next;
+  __shared__ uint32_t s_count[2], s_heavy, s_light, s_next;
+  __shared__ uint16_t s_items[kListItems];
   ExtWarp &sm = s_warps[threadIdx.x >> 5];
   const int f = blockIdx.y, lane = threadIdx.x & 31;
   const Pix *image = reinterpret_cast<const Pix *>(F.image[f]);
@@ -416,169 +423,197 @@ ext_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchPa
   uint2 *res = kept.res + (size_t)f * kept.stride;
   if (threadIdx.x < 2)
     s_count[threadIdx.x] = 0u;
-  if (threadIdx.x == 0)
-    s_next = 0u;
-  __syncthreads();
   int row_lo, row_hi;
   band_share(height, &row_lo, &row_hi);
   const uint32_t items = (uint32_t)((row_hi - row_lo + kBandRows - 1) / kBandRows) * rpr;
   const int lr = lane / kRunWords, lc = lane % kRunWords;  // this lane's row and word of a run
   uint32_t count = 0, total = 0;
-  for (;;) {
-    uint32_t item = 0;
-    if (lane == 0)
-      item = atomicAdd(&s_next, 1u);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= items)
-      break;  // whole warp
-    const uint32_t band = item / rpr, run = item - band * rpr;
-    const int y0 = row_lo + (int)band * kBandRows, xr = (int)run * kRunWords * 32;
-    const bool in = y0 + lr < row_hi && run * kRunWords + lc < wpr;
-    const size_t wi = (size_t)(y0 + lr) * wpr + run * kRunWords + lc;
-    uint32_t left = in ? __ldg(cand + wi) : 0u;  // this lane's candidates not yet decided
-    if (!__any_sync(0xffffffffu, left != 0u)) {
-      if (in)
-        bits[wi] = 0u;
-      continue;
+  for (uint32_t base = 0; base < items; base += kListItems) {
+    // The runs that hold a candidate, those with many from the list's front and
+    // the others from its back; the rest have no strong pixel.
+    const uint32_t chunk = min(items - base, (uint32_t)kListItems);
+    if (threadIdx.x == 0)
+      s_heavy = s_light = s_next = 0u;
+    __syncthreads();
+    for (uint32_t i0 = threadIdx.x >> 5; i0 < chunk; i0 += kListAhead * (kScanT / 32)) {
+      uint32_t w[kListAhead];
+      size_t at[kListAhead];
+#pragma unroll
+      for (int u = 0; u < kListAhead; u++) {
+        const uint32_t i = i0 + u * (kScanT / 32), band = (base + i) / rpr,
+                       run = base + i - band * rpr;
+        const int y = row_lo + (int)band * kBandRows + lr;
+        const bool in = i < chunk && y < row_hi && run * kRunWords + lc < wpr;
+        at[u] = in ? (size_t)y * wpr + run * kRunWords + lc : ~(size_t)0;
+        w[u] = in ? __ldg(cand + at[u]) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < kListAhead; u++) {
+        const uint32_t n = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(w[u]));
+        total += n;  // (the same in every lane)
+        if (n == 0u) {
+          if (at[u] != ~(size_t)0)
+            bits[at[u]] = 0u;
+        } else if (lane == 0) {
+          const uint32_t place = n >= kHeavyRun ? atomicAdd(&s_heavy, 1u)
+                                                : kListItems - 1u - atomicAdd(&s_light, 1u);
+          s_items[place] = (uint16_t)(i0 + u * (kScanT / 32));
+        }
+      }
     }
-    total += (uint32_t)__popc(left);
-    sm.strong[lane] = 0u;
-    if (lane < kBandRows)
-      sm.passed[lane] = 0u;
+    __syncthreads();
+    const uint32_t heavy = s_heavy, listed = heavy + s_light;
     for (;;) {
-      // The leftmost column with a candidate left.
-      uint32_t any = left;
-      any |= __shfl_xor_sync(0xffffffffu, any, 4);
-      any |= __shfl_xor_sync(0xffffffffu, any, 8);
-      any |= __shfl_xor_sync(0xffffffffu, any, 16);
-      const unsigned live = __ballot_sync(0xffffffffu, any != 0u) & 0xFu;
-      if (!live)
+      uint32_t item = 0;
+      if (lane == 0)
+        item = atomicAdd(&s_next, 1u);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item >= listed)
         break;  // whole warp
-      const int c0 = __ffs(live) - 1, s = __ffs(__shfl_sync(0xffffffffu, any, c0)) - 1;
-      const int x0 = xr + 32 * c0 + s;
-      const unsigned long long span = (unsigned long long)((1u << NC) - 1u) << s;
-      left &= lc == c0 ? ~(uint32_t)span : lc == c0 + 1 ? ~(uint32_t)(span >> 32) : ~0u;
-      // The chunk's pixels start at (xl, yt); lane d holds the 32 mask bits over row d.
-      const int xl = x0 - K2, yt = y0 - K2;
-      uint32_t er_row = 0, v[ROWS];
-      if (xl >= 0 && xl + 32 <= width && yt >= 0 && yt + ROWS <= height) {  // warp-uniform
-        if (lane < ROWS) {
-          const uint32_t *cw = cand + (uint32_t)(yt + lane) * wpr + (uint32_t)(xl >> 5);
-          er_row = __funnelshift_r(__ldg(cw), __ldg(cw + ((xl & 31) != 0 ? 1 : 0)), xl & 31);
-        }
-        const Pix *at = image + (size_t)yt * width + (xl + lane);
+      item = base + s_items[item < heavy ? item : kListItems - 1u - (item - heavy)];
+      const uint32_t band = item / rpr, run = item - band * rpr;
+      const int y0 = row_lo + (int)band * kBandRows, xr = (int)run * kRunWords * 32;
+      const bool in = y0 + lr < row_hi && run * kRunWords + lc < wpr;
+      const size_t wi = (size_t)(y0 + lr) * wpr + run * kRunWords + lc;
+      uint32_t left = in ? __ldg(cand + wi) : 0u;  // this lane's candidates not yet decided
+      sm.strong[lane] = 0u;
+      if (lane < kBandRows)
+        sm.passed[lane] = 0u;
+      for (;;) {
+        // The leftmost column with a candidate left.
+        uint32_t any = left;
+        any |= __shfl_xor_sync(0xffffffffu, any, 4);
+        any |= __shfl_xor_sync(0xffffffffu, any, 8);
+        any |= __shfl_xor_sync(0xffffffffu, any, 16);
+        const unsigned live = __ballot_sync(0xffffffffu, any != 0u) & 0xFu;
+        if (!live)
+          break;  // whole warp
+        const int c0 = __ffs(live) - 1, s = __ffs(__shfl_sync(0xffffffffu, any, c0)) - 1;
+        const int x0 = xr + 32 * c0 + s;
+        const unsigned long long span = (unsigned long long)((1u << NC) - 1u) << s;
+        left &= lc == c0 ? ~(uint32_t)span : lc == c0 + 1 ? ~(uint32_t)(span >> 32) : ~0u;
+        // The chunk's pixels start at (xl, yt); lane d holds the 32 mask bits over row d.
+        const int xl = x0 - K2, yt = y0 - K2;
+        uint32_t er_row = 0, v[ROWS];
+        if (xl >= 0 && xl + 32 <= width && yt >= 0 && yt + ROWS <= height) {  // warp-uniform
+          if (lane < ROWS) {
+            const uint32_t *cw = cand + (uint32_t)(yt + lane) * wpr + (uint32_t)(xl >> 5);
+            er_row = __funnelshift_r(__ldg(cw), __ldg(cw + ((xl & 31) != 0 ? 1 : 0)), xl & 31);
+          }
+          const Pix *at = image + (size_t)yt * width + (xl + lane);
 #pragma unroll
-        for (int d = 0; d < ROWS; d++) {
-          v[d] = (uint32_t)__ldg(at);
-          at += width;
-        }
-      } else {
-        if (lane < ROWS && yt + lane >= 0 && yt + lane < height) {
-          const uint32_t *row = cand + (size_t)(yt + lane) * wpr;
-          const int w0 = xl >> 5;  // (-1 left of the frame)
-          const uint32_t a = w0 >= 0 ? __ldg(row + w0) : 0u;
-          const uint32_t b = w0 + 1 < (int)wpr ? __ldg(row + w0 + 1) : 0u;
-          er_row = __funnelshift_r(a, b, xl & 31);
-        }
-        const int x = xl + lane;
+          for (int d = 0; d < ROWS; d++) {
+            v[d] = (uint32_t)__ldg(at);
+            at += width;
+          }
+        } else {
+          if (lane < ROWS && yt + lane >= 0 && yt + lane < height) {
+            const uint32_t *row = cand + (size_t)(yt + lane) * wpr;
+            const int w0 = xl >> 5;  // (-1 left of the frame)
+            const uint32_t a = w0 >= 0 ? __ldg(row + w0) : 0u;
+            const uint32_t b = w0 + 1 < (int)wpr ? __ldg(row + w0 + 1) : 0u;
+            er_row = __funnelshift_r(a, b, xl & 31);
+          }
+          const int x = xl + lane;
 #pragma unroll
-        for (int d = 0; d < ROWS; d++) {
-          const bool inside = x >= 0 && x < width && yt + d >= 0 && yt + d < height;
-          v[d] = inside ? (uint32_t)__ldg(image + (size_t)(yt + d) * width + x)
-                        : Traits<Pix>::kMasked;
-        }
-      }
-      // Row r's candidates of the chunk, in lane r (columns past the run are
-      // the next one's), and the candidates before them.
-      uint32_t mine = __shfl_sync(0xffffffffu, er_row, (lane + K2) & 31) >> K2;
-      mine &= lane < kBandRows ? (1u << NC) - 1u : 0u;
-      if (x0 + NC > xr + 32 * kRunWords)
-        mine &= (1u << (xr + 32 * kRunWords - x0)) - 1u;
-      const uint32_t incl = warp_inclusive((uint32_t)__popc(mine), lane);
-      const uint32_t ncand = __shfl_sync(0xffffffffu, incl, 31);
-      // The background over the window's rows, by column.
-      uint32_t most = 0;
-      {
-        uint32_t n = 0, sum = 0;
-#pragma unroll
-        for (int d = 0; d < ROWS; d++) {
-          const bool ok = (v[d] < Traits<Pix>::kMasked) &
-                          ((__shfl_sync(0xffffffffu, er_row, d) & lane_bit) == 0u);
-          if (d >= K2 && d < K2 + kBandRows)
-            sm.px[d - K2][lane] = v[d];
-          v[d] = ok ? v[d] : Traits<Pix>::kMasked;  // background or not, from here on
-          n += ok ? 1u : 0u;
-          sum += ok ? v[d] : 0u;
-          most |= ok ? v[d] : 0u;
-          if (d >= W2 - 1) {
-            sm.col[d - (W2 - 1)][lane] = make_uint2(n, sum);
-            const bool was = v[d - (W2 - 1)] < Traits<Pix>::kMasked;
-            n -= was ? 1u : 0u;
-            sum -= was ? v[d - (W2 - 1)] : 0u;
+          for (int d = 0; d < ROWS; d++) {
+            const bool inside = x >= 0 && x < width && yt + d >= 0 && yt + d < height;
+            v[d] = inside ? (uint32_t)__ldg(image + (size_t)(yt + d) * width + x)
+                          : Traits<Pix>::kMasked;
           }
         }
-      }
-      const bool wide = sizeof(Pix) == 4 && __any_sync(0xffffffffu, most >= 1u << 24);
-      __syncwarp();
-      for (uint32_t q0 = 0; q0 < ncand; q0 += 32) {  // warp-uniform
-        const uint32_t q = q0 + lane;
-        int r = 0;
+        // Row r's candidates of the chunk, in lane r (columns past the run are
+        // the next one's), and the candidates before them.
+        uint32_t mine = __shfl_sync(0xffffffffu, er_row, (lane + K2) & 31) >> K2;
+        mine &= lane < kBandRows ? (1u << NC) - 1u : 0u;
+        if (x0 + NC > xr + 32 * kRunWords)
+          mine &= (1u << (xr + 32 * kRunWords - x0)) - 1u;
+        const uint32_t incl = warp_inclusive((uint32_t)__popc(mine), lane);
+        const uint32_t ncand = __shfl_sync(0xffffffffu, incl, 31);
+        // The background over the window's rows, by column.
+        uint32_t most = 0;
+        {
+          uint32_t n = 0, sum = 0;
 #pragma unroll
-        for (int k = 4; k; k >>= 1)
-          r += __shfl_sync(0xffffffffu, incl, r + k - 1) <= q ? k : 0;
-        r &= 7;
-        const uint32_t row_bits = __shfl_sync(0xffffffffu, mine, r);
-        const uint32_t first = __shfl_sync(0xffffffffu, incl, r) - (uint32_t)__popc(row_bits);
-        bool ok = q < ncand;
-        const int j = ok ? select_bit(row_bits, q - first) : 0;
-        uint32_t n = 0, s32 = 0;
-#pragma unroll
-        for (int k = 0; k < W2; k++) {
-          const uint2 c = sm.col[r][j + k];
-          n += c.x;
-          s32 += c.y;
+          for (int d = 0; d < ROWS; d++) {
+            const bool ok = (v[d] < Traits<Pix>::kMasked) &
+                            ((__shfl_sync(0xffffffffu, er_row, d) & lane_bit) == 0u);
+            if (d >= K2 && d < K2 + kBandRows)
+              sm.px[d - K2][lane] = v[d];
+            v[d] = ok ? v[d] : Traits<Pix>::kMasked;  // background or not, from here on
+            n += ok ? 1u : 0u;
+            sum += ok ? v[d] : 0u;
+            most |= ok ? v[d] : 0u;
+            if (d >= W2 - 1) {
+              sm.col[d - (W2 - 1)][lane] = make_uint2(n, sum);
+              const bool was = v[d - (W2 - 1)] < Traits<Pix>::kMasked;
+              n -= was ? 1u : 0u;
+              sum -= was ? v[d - (W2 - 1)] : 0u;
+            }
+          }
         }
-        unsigned long long S = s32;
-        if (sizeof(Pix) == 4 && wide && ok)
-          ext_wide_window(image, cand, height, width, K2, y0 + r, x0 + j, &n, &S);
-        float mean = 0.0f;
-        if (ok) {
-          const uint32_t p = sm.px[r][j + K2];
-          // dext.cc:205: only pixels above the global threshold are tested.
-          ok = (uint64_t)p >= P.p_min;
+        const bool wide = sizeof(Pix) == 4 && __any_sync(0xffffffffu, most >= 1u << 24);
+        __syncwarp();
+        for (uint32_t q0 = 0; q0 < ncand; q0 += 32) {  // warp-uniform
+          const uint32_t q = q0 + lane;
+          int r = 0;
+#pragma unroll
+          for (int k = 4; k; k >>= 1)
+            r += __shfl_sync(0xffffffffu, incl, r + k - 1) <= q ? k : 0;
+          r &= 7;
+          const uint32_t row_bits = __shfl_sync(0xffffffffu, mine, r);
+          const uint32_t first = __shfl_sync(0xffffffffu, incl, r) - (uint32_t)__popc(row_bits);
+          bool ok = q < ncand;
+          const int j = ok ? select_bit(row_bits, q - first) : 0;
+          uint32_t n = 0, s32 = 0;
+#pragma unroll
+          for (int k = 0; k < W2; k++) {
+            const uint2 c = sm.col[r][j + k];
+            n += c.x;
+            s32 += c.y;
+          }
+          unsigned long long S = s32;
+          if (sizeof(Pix) == 4 && wide && ok)
+            ext_wide_window(image, cand, height, width, K2, y0 + r, x0 + j, &n, &S);
+          float mean = 0.0f;
           if (ok) {
-            if constexpr (sizeof(Pix) == 2)
-              ok = stage2_u16(p, n, (uint32_t)S, P, &mean);
-            else
-              ok = stage2_u32(p, n, S, P, &mean);
+            const uint32_t p = sm.px[r][j + K2];
+            // dext.cc:205: only pixels above the global threshold are tested.
+            ok = (uint64_t)p >= P.p_min;
+            if (ok) {
+              if constexpr (sizeof(Pix) == 2)
+                ok = stage2_u16(p, n, (uint32_t)S, P, &mean);
+              else
+                ok = stage2_u32(p, n, S, P, &mean);
+            }
           }
+          // This row's passing candidates in these lanes, and before them.
+          const unsigned pass = __ballot_sync(0xffffffffu, ok);
+          const int from = max((int)first - (int)q0, 0);
+          const uint32_t before = sm.passed[r];
+          const uint32_t at = before + (uint32_t)__popc(pass & (lane_bit - 1u) & (~0u << from));
+          if (ok) {
+            if (at < kept.keep)
+              res[((size_t)(y0 + r) * rpr + run) * kept.keep + at] =
+                  make_uint2(__float_as_uint(mean), n);
+            const int b = x0 + j - xr;
+            atomicOr(&sm.strong[r * kRunWords + (b >> 5)], 1u << (b & 31));
+          }
+          __syncwarp();
+          if (ok)
+            atomicMax(&sm.passed[r], at + 1u);
+          count += ok ? 1u : 0u;
+          __syncwarp();
         }
-        // This row's passing candidates in these lanes, and before them.
-        const unsigned pass = __ballot_sync(0xffffffffu, ok);
-        const int from = max((int)first - (int)q0, 0);
-        const uint32_t before = sm.passed[r];
-        const uint32_t at = before + (uint32_t)__popc(pass & (lane_bit - 1u) & (~0u << from));
-        if (ok) {
-          if (at < kept.keep)
-            res[((size_t)(y0 + r) * rpr + run) * kept.keep + at] =
-                make_uint2(__float_as_uint(mean), n);
-          const int b = x0 + j - xr;
-          atomicOr(&sm.strong[r * kRunWords + (b >> 5)], 1u << (b & 31));
-        }
-        __syncwarp();
-        if (ok)
-          atomicMax(&sm.passed[r], at + 1u);
-        count += ok ? 1u : 0u;
-        __syncwarp();
+        __syncwarp();  // the next chunk rewrites the shared sums
       }
-      __syncwarp();  // the next chunk rewrites the shared sums
+      if (in)
+        bits[wi] = sm.strong[lane];
+      __syncwarp();
     }
-    if (in)
-      bits[wi] = sm.strong[lane];
-    __syncwarp();
+    __syncthreads();
   }
   count = __reduce_add_sync(0xffffffffu, count);
-  total = __reduce_add_sync(0xffffffffu, total);
   if (lane == 0) {
     atomicAdd(&s_count[0], count);
     atomicAdd(&s_count[1], total);
