@@ -45,6 +45,7 @@ constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
 constexpr int kGrid = 2 * 152;
 constexpr int kPassGrid = 8 * 152;      // grid-stride passes over pixels / candidates
+constexpr int kVarBlocks = 2;           // k_var's blocks an SM (registers)
 constexpr int kSortGrid = 6 * 152;      // warp sorts: 6 blocks an SM (registers)
 constexpr int kWarpSortMax = 512;       // members ordered by one warp
 constexpr int kWarpSegMax = 128;        // runs a warp orders without sorting the members
@@ -154,74 +155,128 @@ __device__ __forceinline__ uint32_t lower_bound_warp(const uint32_t *__restrict_
 // Kernels of one batch, in launch order.
 // ---------------------------------------------------------------------------
 
-// Each frame's offset in the batch, the exclusive prefix of the counts: one
-// warp, frames 2l and 2l + 1 on lane l.
+// The batch's frames within it: their offsets (the exclusive prefix of their
+// counts) from `off`, nb + 1 of them. Every block forms them for itself, its
+// first warp with frames 2l and 2l + 1 on lane l; false where a list is longer
+// than its stride (one that overflowed its threshold's capacity: incomplete, and
+// refused).
 static_assert(kLabelMaxBatch <= 64, "two frames a lane");
-__global__ void k_offsets(LabelStatus *st, const BatchArgs *__restrict__ ap,
-                          uint32_t capacity) {
-  previous_done();
-  if (st->error)
-    return;
-  const BatchArgs &a = *ap;
-  const int lane = threadIdx.x & 31, nb = a.nb;
-  const int j0 = 2 * lane, j1 = j0 + 1;
-  const uint32_t c0 = j0 < nb ? a.counts[j0] : 0u, c1 = j1 < nb ? a.counts[j1] : 0u;
-  // A list whose count exceeds its stride is one that overflowed its
-  // threshold's capacity: it is incomplete, and refused.
-  if (__any_sync(0xffffffffu, c0 > a.stride || c1 > a.stride)) {
-    if (lane == 0)
-      st->error |= kErrListOverflow;
-    return;
-  }
-  uint32_t incl = c0 + c1;
+__device__ __forceinline__ bool frame_offsets(const BatchArgs &a, uint32_t *off) {
+  __shared__ bool s_fits;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, nb = a.nb, j0 = 2 * lane, j1 = j0 + 1;
+    const uint32_t c0 = j0 < nb ? a.counts[j0] : 0u, c1 = j1 < nb ? a.counts[j1] : 0u;
+    const bool fits = !__any_sync(0xffffffffu, c0 > a.stride || c1 > a.stride);
+    uint32_t incl = c0 + c1;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o)
-      incl += t;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o)
+        incl += t;
+    }
+    const uint32_t excl = incl - c0 - c1;
+    if (j0 < nb)
+      off[j0] = excl;
+    if (j1 < nb)
+      off[j1] = excl + c0;
+    if (lane == 31) {
+      off[nb] = incl;
+      s_fits = fits;
+    }
   }
-  const uint32_t excl = incl - c0 - c1;
-  if (j0 < nb)
-    st->frame_off[j0] = excl;
-  if (j1 < nb)
-    st->frame_off[j1] = excl + c0;
-  const uint32_t off = __shfl_sync(0xffffffffu, incl, 31);
-  if (lane != 0)
-    return;
-  st->frame_off[nb] = off;
-  st->n_big = 0;
-  st->n_edges = 0;
-  const unsigned long long total = (unsigned long long)st->n_live + off;
-  if (total > capacity) {
-    st->error |= kErrLiveFull;
-    return;
-  }
-  st->n_total = (uint32_t)total;
-  st->counts[kCntSignal] += off;
+  __syncthreads();
+  return s_fits;
 }
 
-// The batch's lists into the pool. Each warp appends 32 consecutive pixels
-// and points each one straight at the first pixel of its run (consecutive
-// indices of one row) within those 32: the union-find then starts from trees
-// one level deep instead of chains along the rows, whose finds would walk
-// the row at memory latency. Runs crossing a warp's boundary are joined by
-// k_link's left-neighbour union.
-__global__ void k_append(LabelStatus *st, const BatchArgs *__restrict__ ap, int32_t *frame,
-                         uint32_t *index, uint32_t *value, uint32_t *parent) {
-  previous_done();
-  if (st->error)
-    return;
+// Pool position p's rows of a segment's start table (below): those after the
+// row of the pixel before it, up to its own, and beyond where it is the last.
+__device__ __forceinline__ void put_rows(uint32_t *row, uint32_t p, uint32_t first, uint32_t y,
+                                         bool last, uint32_t height) {
+  for (uint32_t r = first; r <= y; r++)
+    row[r] = p;
+  if (last)
+    for (uint32_t r = y + 1; r <= height; r++)
+      row[r] = p + 1u;
+}
+
+// The batch's lists into the pool, a row of blocks a frame (blockIdx.y). Each
+// warp appends 32 consecutive pixels and points each one straight at the first
+// pixel of its run (consecutive indices of one row) within those 32: the
+// union-find then starts from trees one level deep instead of chains along the
+// rows, whose finds would walk the row at memory latency. Runs crossing a
+// warp's boundary are joined by k_link's left-neighbour union. The components'
+// sums start here too (zlast, csize, candid, a word a position). The last row
+// of blocks does that for the live pool, and keeps the call's offsets.
+//
+// Per-row start tables of the frames a batch links (rows non-null): segment 0
+// is the frame before the batch (the live pool's tail, [prev_start, n_live)),
+// segment j + 1 the batch's frame j. rows[s * (height + 1) + y] is the first
+// position of segment s whose index is at or beyond row y; entry `height` is
+// the segment's end. Every entry is written once: by the pixel that starts the
+// row (or the first pixel after a run of empty rows), or by the segment's
+// last pixel for the rows after it.
+//
+// Bound by memory latency and its stores. As three launches (the offsets, the
+// lists, the row tables from the pool's indexes) they took 68 us in the three
+// calls of a 32-frame sweep of 4362 x 4148, together 44.
+__global__ void __launch_bounds__(kThreads)
+k_append(LabelStatus *st, const BatchArgs *__restrict__ ap, uint32_t capacity, int32_t *frame,
+         uint32_t *index, uint32_t *value, uint32_t *parent, uint32_t *rows, uint32_t height,
+         int32_t *zlast, uint32_t *csize, uint32_t *candid) {
+  __shared__ uint32_t off[kLabelMaxBatch + 1];
   const BatchArgs &a = *ap;
-  const sf_signal_pixel *__restrict__ lists = a.lists;
-  const size_t stride = a.stride;
-  const int j = blockIdx.y;
-  const uint32_t n = st->frame_off[j + 1] - st->frame_off[j];
-  const uint32_t base = st->n_live + st->frame_off[j];
+  // The offsets' block alone writes the status, and nothing that is read here
+  // by the others but the error, for which they stop by themselves.
+  const uint32_t error = st->error, live = st->n_live;
+  const bool fits = frame_offsets(a, off);
+  if (error)
+    return;
+  const int j = blockIdx.y, nb = a.nb;
+  const bool room = (unsigned long long)live + off[nb] <= capacity;
+  if (j == nb && blockIdx.x == 0) {
+    if (!fits || !room) {
+      if (threadIdx.x == 0)
+        st->error = fits ? kErrLiveFull : kErrListOverflow;
+      return;
+    }
+    if (threadIdx.x <= nb)
+      st->frame_off[threadIdx.x] = off[threadIdx.x];
+    if (threadIdx.x == 0) {
+      st->n_big = 0;
+      st->n_edges = 0;
+      st->n_total = live + off[nb];
+      st->counts[kCntSignal] += off[nb];
+    }
+  }
+  if (!fits || !room)
+    return;
+  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
   const uint32_t width = a.width;
-  const sf_signal_pixel *list = lists + (size_t)j * stride;
+  uint32_t *row = rows ? rows + (size_t)(j == nb ? 0 : j + 1) * (height + 1) : nullptr;
+  if (j == nb) {
+    for (uint32_t p = t0; p < live; p += nt) {
+      zlast[p] = INT_MIN;
+      csize[p] = 0;
+      candid[p] = kNone;
+    }
+    if (!row || !a.link_prev[0])
+      return;  // the batch's first frame does not link back: no table needed
+    const uint32_t lo = st->prev_start;
+    if (lo == live)
+      for (uint32_t y = t0; y <= height; y += nt)
+        row[y] = lo;
+    for (uint32_t p = lo + t0; p < live; p += nt)
+      put_rows(row, p, p == lo ? 0u : index[p - 1] / width + 1u, index[p] / width, p == live - 1,
+               height);
+    return;
+  }
+  const uint32_t n = off[j + 1] - off[j], base = live + off[j];
+  if (row && n == 0)
+    for (uint32_t y = t0; y <= height; y += nt)
+      row[y] = base;
+  const sf_signal_pixel *__restrict__ list = a.lists + (size_t)j * a.stride;
   const int lane = threadIdx.x & 31;
-  for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < n;
-       i0 += gridDim.x * blockDim.x) {  // warp-uniform
+  for (uint32_t i0 = t0 & ~31u; i0 < n; i0 += nt) {  // warp-uniform
     const uint32_t i = i0 + lane;
     const bool in = i < n;
     sf_signal_pixel s;
@@ -229,8 +284,11 @@ __global__ void k_append(LabelStatus *st, const BatchArgs *__restrict__ ap, int3
     s.value = 0;
     if (in)
       s = list[i];
-    const uint32_t before = __shfl_up_sync(0xffffffffu, s.index, 1);
-    const bool starts = !in || lane == 0 || s.index % width == 0 || before != s.index - 1;
+    uint32_t before = __shfl_up_sync(0xffffffffu, s.index, 1);
+    if (row && lane == 0 && i0 > 0)
+      before = list[i0 - 1].index;
+    const uint32_t y = s.index / width;
+    const bool starts = !in || lane == 0 || s.index == y * width || before != s.index - 1;
     const unsigned mask = __ballot_sync(0xffffffffu, starts) & (0xffffffffu >> (31 - lane));
     if (in) {
       const uint32_t p = base + i;
@@ -238,51 +296,12 @@ __global__ void k_append(LabelStatus *st, const BatchArgs *__restrict__ ap, int3
       index[p] = s.index;
       value[p] = s.value;
       parent[p] = base + i0 + (31 - __clz(mask));
+      zlast[p] = INT_MIN;
+      csize[p] = 0;
+      candid[p] = kNone;
+      if (row)
+        put_rows(row, p, i == 0 ? 0u : before / width + 1u, y, i == n - 1, height);
     }
-  }
-}
-
-// Per-row start tables of the frames a batch links: segment 0 is the frame
-// before the batch (the live pool's tail, [prev_start, n_live)), segment
-// j + 1 the batch's frame j. rows[s * (height + 1) + y] is the first position
-// of segment s whose index is at or beyond row y; entry `height` is the
-// segment's end. Every entry is written once: by the pixel that starts the
-// row (or the first pixel after a run of empty rows), or by the segment's
-// last pixel for the rows after it.
-__global__ void k_rows(LabelStatus *st, const BatchArgs *__restrict__ ap,
-                       const uint32_t *__restrict__ index, uint32_t *__restrict__ rows,
-                       uint32_t height) {
-  previous_done();
-  if (st->error)
-    return;
-  const BatchArgs &a = *ap;
-  const int s = blockIdx.y;
-  uint32_t lo, hi;
-  if (s == 0) {
-    if (!a.link_prev[0])
-      return;  // the batch's first frame does not link back: no table needed
-    lo = st->prev_start;
-    hi = st->n_live;
-  } else {
-    lo = st->n_live + st->frame_off[s - 1];
-    hi = st->n_live + st->frame_off[s];
-  }
-  uint32_t *row = rows + (size_t)s * (height + 1);
-  const uint32_t width = a.width;
-  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-  if (lo == hi) {
-    for (uint32_t y = t0; y <= height; y += nt)
-      row[y] = lo;
-    return;
-  }
-  for (uint32_t p = lo + t0; p < hi; p += nt) {
-    const uint32_t y = index[p] / width;
-    const uint32_t first = p == lo ? 0u : index[p - 1] / width + 1u;
-    for (uint32_t r = first; r <= y; r++)
-      row[r] = p;
-    if (p == hi - 1)
-      for (uint32_t r = y + 1; r <= height; r++)
-        row[r] = hi;
   }
 }
 
@@ -405,27 +424,10 @@ __global__ void k_unite(LabelStatus *st, const uint2 *__restrict__ edges, uint32
   }
 }
 
-__global__ void k_flatten(LabelStatus *st, uint32_t *parent, uint32_t *root, int32_t *zlast,
-                          uint32_t *csize, uint32_t *candid) {
-  previous_done();
-  if (st->error)
-    return;
-  const uint32_t n = st->n_total;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += gridDim.x * blockDim.x) {
-    uint32_t r = p;
-    while (parent[r] != r)
-      r = parent[r];
-    root[p] = r;
-    zlast[p] = INT_MIN;
-    csize[p] = 0;
-    candid[p] = kNone;
-  }
-}
-
-__global__ void k_comp_stats(LabelStatus *st, const uint32_t *__restrict__ root,
-                             const int32_t *__restrict__ frame, int32_t *zlast,
-                             uint32_t *csize) {
+// Every position's root, and the components' sizes and last frames (37 us in the
+// three calls of a 32-frame sweep of 4362 x 4148, 57 as two launches).
+__global__ void k_flatten(LabelStatus *st, const uint32_t *parent, uint32_t *root,
+                          const int32_t *__restrict__ frame, int32_t *zlast, uint32_t *csize) {
   previous_done();
   if (st->error)
     return;
@@ -438,8 +440,14 @@ __global__ void k_comp_stats(LabelStatus *st, const uint32_t *__restrict__ root,
        p0 += gridDim.x * blockDim.x) {
     const uint32_t p = p0 + lane;
     const bool in = p < n;
-    const uint32_t r = in ? root[p] : kNone;
     const int32_t z = in ? frame[p] : INT_MIN;
+    uint32_t r = kNone;
+    if (in) {
+      r = p;
+      for (uint32_t q = parent[r]; q != r; q = parent[r])
+        r = q;
+      root[p] = r;
+    }
     const unsigned same = __match_any_sync(0xffffffffu, r);
     const int32_t zmax = __reduce_max_sync(same, z);
     if (in && lane == __ffs(same) - 1) {
@@ -473,35 +481,28 @@ __device__ __forceinline__ uint32_t bucket_of(const BatchArgs &a, int32_t z) {
 // open one.
 enum : uint32_t { kClosingRoot = 1u, kOpenPixel = 2u };
 
-__global__ void k_closing_flags(LabelStatus *st, const BatchArgs *__restrict__ ap,
-                                const uint32_t *__restrict__ root,
-                                const int32_t *__restrict__ zlast, uint32_t *flag) {
-  previous_done();
-  const BatchArgs &a = *ap;
-  if (st->error)
-    return;
-  const uint32_t n = st->n_total;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += gridDim.x * blockDim.x) {
-    const uint32_t r = root[p];
-    flag[p] = !closes(a, zlast[r]) ? kOpenPixel : r == p ? kClosingRoot : 0u;
-  }
-}
-
-// The scan of those (sf_scan.cuh): a closing root takes the next place of the
-// closing list, with its emission event, an open pixel the next of the pool.
+// Those flags (noted in the first pass) and their scan (sf_scan.cuh): a closing
+// root takes the next place of the closing list, with its emission event, an
+// open pixel the next of the pool.
 struct ClosingScan {
   LabelStatus *st;
   const BatchArgs *ap;
-  const uint32_t *flag;
+  const uint32_t *root;
+  uint32_t *flag;
   const int32_t *zlast;
   uint32_t *clist, *cbucket, *newpos;
   __device__ bool skip() const { return st->error != 0u; }
   __device__ uint32_t size() const { return st->n_total; }
-  __device__ unsigned long long load(uint32_t p) const {
-    const uint32_t f = flag[p];
+  __device__ static unsigned long long pair(uint32_t f) {
     return (unsigned long long)(f & kClosingRoot) << 32 | (f & kOpenPixel) >> 1;
   }
+  __device__ unsigned long long first(uint32_t p) const {
+    const uint32_t r = root[p];
+    const uint32_t f = !closes(*ap, zlast[r]) ? kOpenPixel : r == p ? kClosingRoot : 0u;
+    flag[p] = f;
+    return pair(f);
+  }
+  __device__ unsigned long long load(uint32_t p) const { return pair(flag[p]); }
   __device__ void sums_done() {}
   __device__ void store(uint32_t p, unsigned long long v, unsigned long long before) const {
     if (v >> 32) {
@@ -546,84 +547,58 @@ k_bucket_hist(LabelStatus *st, const uint32_t *__restrict__ cbucket, uint32_t *h
     atomicAdd(&h[cbucket[k]], 1u);
   __syncthreads();
   for (int b = threadIdx.x; b < kBuckets; b += blockDim.x)
-    hist[blockIdx.x * kBuckets + b] = h[b];
+    hist[b * kBucketBlocks + blockIdx.x] = h[b];
 }
 
-// Exclusive scan over (bucket, block) in bucket-major order: a warp scans a
-// bucket's counts in place (each lane a run of blocks); the buckets' own
-// offsets follow the counts, and the scatter adds them.
-__global__ void __launch_bounds__(1024) k_bucket_offsets(LabelStatus *st, uint32_t *hist) {
-  previous_done();
-  if (st->error)
-    return;
-  __shared__ uint32_t btotal[kBuckets];
-  constexpr int kPer = (kBucketBlocks + 31) / 32;  // blocks a lane
-  const int lane = threadIdx.x & 31;
-  const int lo = min(kBucketBlocks, lane * kPer), hi = min(kBucketBlocks, lo + kPer);
-  for (int b = threadIdx.x >> 5; b < kBuckets; b += blockDim.x >> 5) {  // warp-uniform
-    uint32_t v[kPer], sum = 0;
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-      v[k] = lo + k < hi ? hist[(lo + k) * kBuckets + b] : 0u;
-      sum += v[k];
-    }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o)
-        incl += t;
-    }
-    uint32_t run = incl - sum;
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-      if (lo + k < hi)
-        hist[(lo + k) * kBuckets + b] = run;
-      run += v[k];
-    }
-    if (lane == 31)
-      btotal[b] = incl;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // kBuckets is 65: three values a lane.
-    static_assert(kBuckets <= 96, "three buckets a lane");
-    uint32_t v[3], sum = 0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      v[k] = 3 * lane + k < kBuckets ? btotal[3 * lane + k] : 0u;
-      sum += v[k];
-    }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o)
-        incl += t;
-    }
-    uint32_t run = incl - sum;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      if (3 * lane + k < kBuckets)
-        hist[kBucketBlocks * kBuckets + 3 * lane + k] = run;
-      run += v[k];
-    }
-  }
-}
-
+// Each block's places in the buckets: a bucket's start (the buckets before it),
+// and in it the blocks before this one, a warp a bucket over the counts. (With a
+// launch of its own for them, one block, the partition took 60 us in the three
+// calls of a 32-frame sweep of 4362 x 4148; so 36.)
 __global__ void __launch_bounds__(kThreads)
 k_bucket_scatter(LabelStatus *st, const uint32_t *__restrict__ clist,
-                 const uint32_t *__restrict__ cbucket, const uint32_t *__restrict__ hist,
-                 uint32_t *order) {
+                 const uint32_t *__restrict__ cbucket, const uint32_t *hist, uint32_t *order) {
   previous_done();
   if (st->error)
     return;
   constexpr int W = kThreads / 32;
   __shared__ uint32_t wcnt[W][kBuckets];
-  __shared__ uint32_t running[kBuckets];
+  __shared__ uint32_t running[kBuckets], total[kBuckets];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int b = threadIdx.x; b < kBuckets; b += blockDim.x)
-    running[b] = hist[blockIdx.x * kBuckets + b] + hist[kBucketBlocks * kBuckets + b];
+  constexpr int kPer = (kBucketBlocks + 31) / 32;
+#pragma unroll 3
+  for (int b = warp; b < kBuckets; b += W) {
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      const int i = k * 32 + lane;
+      const uint32_t v = i < kBucketBlocks ? hist[b * kBucketBlocks + i] : 0u;
+      all += v;
+      before += i < (int)blockIdx.x ? v : 0u;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if (lane == 0) {
+      running[b] = before;
+      total[b] = all;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t carry = 0;
+    for (int b0 = 0; b0 < kBuckets; b0 += 32) {
+      const uint32_t v = b0 + lane < kBuckets ? total[b0 + lane] : 0u;
+      uint32_t incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+          incl += t;
+      }
+      if (b0 + lane < kBuckets)
+        running[b0 + lane] += carry + incl - v;
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+  }
   uint32_t lo, hi;
   bucket_chunk(st->n_closing, &lo, &hi);
   for (uint32_t base = lo; base < hi; base += blockDim.x) {
@@ -664,7 +639,7 @@ __device__ __forceinline__ uint32_t size_bin(uint32_t n) {
 // The size filters (dials_spots.cc:224-231) over the closing components in
 // emission order, as a scan: each that passes is the next candidate, its
 // members after those of the candidates before it. The sums pass counts the
-// others, and the second pass the candidates by size (k_perm_*).
+// others, and the second pass the candidates by size (perm_offsets).
 struct CandidateScan {
   LabelStatus *st;
   const BatchArgs *ap;
@@ -673,7 +648,7 @@ struct CandidateScan {
   uint32_t small, large, groups;  // this thread's, in the sums pass
   __device__ bool skip() const { return st->error != 0u; }
   __device__ uint32_t size() const { return st->n_closing; }
-  __device__ unsigned long long load(uint32_t e) {
+  __device__ unsigned long long first(uint32_t e) {
     const uint32_t sz = csize[order[e]];
     const bool s = sz < ap->min_size, l = sz > ap->max_size;
     groups++;
@@ -681,6 +656,7 @@ struct CandidateScan {
     large += !s && l;
     return s || l ? 0ull : 1ull << 32 | sz;
   }
+  __device__ unsigned long long load(uint32_t e) { return first(e); }
   __device__ void sums_done() {
     const uint32_t s = __reduce_add_sync(0xffffffffu, small);
     const uint32_t l = __reduce_add_sync(0xffffffffu, large);
@@ -721,6 +697,7 @@ struct AcceptScan {
     const uint32_t n = acc_n[c];
     return n ? 1ull << 32 | n : 0ull;
   }
+  __device__ unsigned long long first(uint32_t c) const { return load(c); }
   __device__ void sums_done() {}
   __device__ void store(uint32_t c, unsigned long long, unsigned long long before) const {
     acc_idx[c] = (uint32_t)(before >> 32);
@@ -732,13 +709,44 @@ struct AcceptScan {
   }
 };
 
-__global__ void k_gather(LabelStatus *st, const uint32_t *__restrict__ root,
-                         const uint32_t *__restrict__ candid,
-                         const uint32_t *__restrict__ cand_off, uint32_t *cursor,
-                         uint32_t *members) {
+// The candidates ordered by size, largest first (a counting sort over
+// kSizeBins bins; sizes of kSizeBins - 1 and more share the first bin, and
+// the order within a bin is arbitrary): perm[i] is the i-th candidate to
+// process. hist holds 2 * kSizeBins words, the counts (CandidateScan) first.
+// One block takes the bins' exclusive offsets (into the cursors, hist +
+// kSizeBins) and clears the counts for the next call (beside k_gather's
+// blocks); threads put the candidates in their places (beside k_first's warps).
+__device__ __forceinline__ void perm_offsets(uint32_t *hist) {
+  constexpr int kPer = kSizeBins / kThreads;
+  static_assert(kPer * kThreads == kSizeBins, "whole bins a thread");
+  uint32_t v[kPer], sum = 0, total;
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    v[k] = hist[threadIdx.x * kPer + k];
+    sum += v[k];
+  }
+  uint32_t at = block_exclusive_scan(sum, &total);
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    hist[kSizeBins + threadIdx.x * kPer + k] = at;
+    hist[threadIdx.x * kPer + k] = 0;
+    at += v[k];
+  }
+}
+
+// The candidates' members, in any order; the launch's last block perm_offsets.
+__global__ void __launch_bounds__(kThreads)
+k_gather(LabelStatus *st, const uint32_t *__restrict__ root, const uint32_t *__restrict__ candid,
+         const uint32_t *__restrict__ cand_off, uint32_t *cursor, uint32_t *members,
+         uint32_t *phist) {
   previous_done();
   if (st->error)
     return;
+  const uint32_t blocks = gridDim.x - 1u;
+  if (blockIdx.x == blocks) {
+    perm_offsets(phist);
+    return;
+  }
   const uint32_t n = st->n_total;
   const int lane = threadIdx.x & 31;
   // The lanes of one candidate take their member slots with one atomic: a
@@ -747,7 +755,7 @@ __global__ void k_gather(LabelStatus *st, const uint32_t *__restrict__ root,
   // (kRunHead: positions are below 2^31, the pool's limit), so that k_sort
   // can order the runs instead of the members.
   for (uint32_t p0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); p0 < n;
-       p0 += gridDim.x * blockDim.x) {
+       p0 += blocks * blockDim.x) {
     const uint32_t p = p0 + lane;
     const uint32_t c = p < n ? candid[root[p]] : kNone;
     const unsigned same = __match_any_sync(0xffffffffu, c);
@@ -886,12 +894,12 @@ __device__ __forceinline__ bool fp_finish(FirstPass &f) {
 //   k_first        a warp per candidate: the first pass as exact integer
 //                  sums across the lanes (redux.sync); its FP64 part (the
 //                  centroid divisions, the peak-separation test) then runs
-//                  for 32 candidates at once, one a lane.
-//   k_pix          a thread per member: the accepted spots' pixels out.
+//                  for 32 candidates at once, one a lane. The candidates in
+//                  order of size (largest first), so that those sharing a
+//                  warp in k_var have similar sizes.
 //   k_terms        a thread per member: its three variance-pass terms
-//                  RN(RN(v d) d), d = (c + 0.5) - centre.
-//   k_perm_*       the candidates ordered by size (largest first), so that
-//                  the candidates sharing a warp in k_var have similar sizes.
+//                  RN(RN(v d) d), d = (c + 0.5) - centre; the accepted
+//                  spots' pixels out.
 //   k_var          four lanes per candidate, in size order: one axis a lane,
 //                  the terms summed with rounding in member order (the one
 //                  part whose order matters), the variances, the spot record.
@@ -1158,35 +1166,6 @@ k_sort(LabelStatus *st, const uint32_t *__restrict__ cand_n,
   }
 }
 
-// The candidates ordered by size, largest first (a counting sort over
-// kSizeBins bins; sizes of kSizeBins - 1 and more share the first bin, and
-// the order within a bin is arbitrary): perm[i] is the i-th candidate to
-// process. hist holds 2 * kSizeBins words, the counts (CandidateScan) first.
-
-// One block: the bins' exclusive offsets (into the cursors, hist +
-// kSizeBins), and the counts cleared for the next call.
-__global__ void __launch_bounds__(kSizeBins) k_perm_offsets(LabelStatus *st, uint32_t *hist) {
-  previous_done();
-  if (st->error)
-    return;
-  uint32_t total;
-  const uint32_t v = hist[threadIdx.x];
-  const uint32_t e = block_exclusive_scan(v, &total);
-  hist[kSizeBins + threadIdx.x] = e;
-  hist[threadIdx.x] = 0;
-}
-
-__global__ void k_perm_scatter(LabelStatus *st, const uint32_t *__restrict__ cand_n,
-                               uint32_t *hist, uint32_t *perm) {
-  previous_done();
-  if (st->error)
-    return;
-  const uint32_t ncand = st->n_cand;
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncand;
-       c += gridDim.x * blockDim.x)
-    perm[atomicAdd(&hist[kSizeBins + size_bin(cand_n[c])], 1u)] = c;
-}
-
 // Warp-wide sum modulo 2^64 of one 64-bit value a lane, by redux.sync on
 // 22-bit limbs (each limb's sum over 32 lanes fits in 32 bits).
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
@@ -1204,13 +1183,18 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 __global__ void __launch_bounds__(kThreads)
 k_first(LabelStatus *st, const BatchArgs *__restrict__ ap, const uint32_t *__restrict__ cand_n,
         const uint32_t *__restrict__ cand_off, const sf_pixel *__restrict__ mpix, CandSpot *cs,
-        uint32_t *acc_n) {
+        uint32_t *acc_n, uint32_t *phist, uint32_t *perm) {
   previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
   const uint32_t ncand = st->n_cand;
   const int lane = threadIdx.x & 31;
+  // The candidates by size (perm_offsets), by the last threads first: the first
+  // warps have candidates of their own.
+  const uint32_t nt = gridDim.x * blockDim.x;
+  for (uint32_t c = nt - 1u - (blockIdx.x * blockDim.x + threadIdx.x); c < ncand; c += nt)
+    perm[atomicAdd(&phist[kSizeBins + size_bin(cand_n[c])], 1u)] = c;
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   // Few warps of several candidates each rather than every warp with one: the
   // FP64 part costs the same for one candidate as for 32.
@@ -1274,15 +1258,20 @@ k_first(LabelStatus *st, const BatchArgs *__restrict__ ap, const uint32_t *__res
     atomicAdd(&st->counts[kCntSeparated], (unsigned long long)separated);
 }
 
-// A thread per member of the batch's candidates whose sums are exact and
-// positive: the member's three variance-pass terms RN(RN(v d) d), d =
-// (c + 0.5) - centre (dials_spots.cc:331-341), every lane busy. c + 0.5 and
+// A thread per member of the batch's accepted candidates, every lane busy: the
+// member out, in member order (dials_spots.cc:355-359), and where the
+// candidate's sums are exact and positive its three variance-pass terms
+// RN(RN(v d) d), d = (c + 0.5) - centre (dials_spots.cc:331-341). c + 0.5 and
 // v are built as doubles from their bits (coordinates below 2^20, values
-// below 2^26 there).
+// below 2^26 there). The three calls of a
+// 32-frame sweep of 4362 x 4148 take 94 us; the two passes as launches of their
+// own, each reading the member and its candidate, 116.
 __global__ void k_terms(LabelStatus *st, const BatchArgs *__restrict__ ap,
                         const sf_pixel *__restrict__ mpix, const uint32_t *__restrict__ mcand,
-                        const uint32_t *__restrict__ acc_n, const CandSpot *__restrict__ cs,
-                        double *__restrict__ terms, size_t terms_stride) {
+                        const uint32_t *__restrict__ cand_off,
+                        const uint32_t *__restrict__ acc_n, const uint32_t *__restrict__ acc_off,
+                        const CandSpot *__restrict__ cs, double *__restrict__ terms,
+                        size_t terms_stride, sf_pixel *__restrict__ pixels, size_t pixels_cap) {
   previous_done();
   const BatchArgs &a = *ap;
   if (st->error)
@@ -1291,9 +1280,16 @@ __global__ void k_terms(LabelStatus *st, const BatchArgs *__restrict__ ap,
   for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n;
        m += gridDim.x * blockDim.x) {
     const uint32_t c = mcand[m];
-    if (!acc_n[c] || (cs[c].mode & (kModeExact | kModeSpread)) != (kModeExact | kModeSpread))
-      continue;
     const sf_pixel px = mpix[m];
+    if (!acc_n[c])
+      continue;
+    const size_t at = (size_t)acc_off[c] + (m - cand_off[c]);
+    if (at < pixels_cap)
+      pixels[at] = px;
+    else
+      atomicOr(&st->error, kErrOutFull);
+    if ((cs[c].mode & (kModeExact | kModeSpread)) != (kModeExact | kModeSpread))
+      continue;
     int32_t coord[3];
     pixel_xyz(px, a, &coord[0], &coord[1], &coord[2]);
     const double centre[3] = {cs[c].pos[0], cs[c].pos[1], cs[c].cz};
@@ -1303,30 +1299,6 @@ __global__ void k_terms(LabelStatus *st, const BatchArgs *__restrict__ ap,
       const double d = __dsub_rn(half_up((uint32_t)coord[ax]), centre[ax]);
       terms[ax * terms_stride + m] = __dmul_rn(__dmul_rn(val, d), d);
     }
-  }
-}
-
-// A thread per member of the batch's candidates: the accepted spots' pixels
-// into the batch output, in member order (dials_spots.cc:355-359).
-__global__ void k_pix(LabelStatus *st, const sf_pixel *__restrict__ mpix,
-                      const uint32_t *__restrict__ mcand, const uint32_t *__restrict__ cand_off,
-                      const uint32_t *__restrict__ acc_n, const uint32_t *__restrict__ acc_off,
-                      sf_pixel *pixels, size_t pixels_cap) {
-  previous_done();
-  if (st->error)
-    return;
-  const uint32_t n = st->n_cand_pixels;
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n;
-       m += gridDim.x * blockDim.x) {
-    const uint32_t c = mcand[m];
-    if (!acc_n[c])
-      continue;
-    const size_t at = (size_t)acc_off[c] + (m - cand_off[c]);
-    if (at >= pixels_cap) {
-      atomicOr(&st->error, kErrOutFull);
-      continue;
-    }
-    pixels[at] = mpix[m];
   }
 }
 
@@ -1346,19 +1318,63 @@ __device__ void variance_sequence(const sf_pixel *mp, uint32_t n, const BatchArg
   }
 }
 
+// The open components' pixels into the next live pool, and (block 0, for the
+// next call) the state carried over. It needs nothing of k_var, whose blocks let
+// it in once they have started (by when all before them is complete): it runs
+// beside k_var's longest chains, and waits for k_var at its end, so that the
+// stream's next work still follows both.
+struct OpenPool {
+  const uint32_t *flag, *newpos, *root;
+  const int32_t *frame;
+  const uint32_t *index, *value;
+  int32_t *frame2;
+  uint32_t *index2, *value2, *parent2;
+};
+__global__ void __launch_bounds__(kThreads)
+k_compact(LabelStatus *st, const BatchArgs *__restrict__ ap, OpenPool o) {
+  const BatchArgs &a = *ap;
+  const uint32_t n = st->error ? 0u : st->n_total;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n;
+       p += gridDim.x * blockDim.x) {
+    if (o.flag[p] & kOpenPixel) {
+      const uint32_t q = o.newpos[p];
+      o.frame2[q] = o.frame[p];
+      o.index2[q] = o.index[p];
+      o.value2[q] = o.value[p];
+      o.parent2[q] = o.newpos[o.root[p]];
+    }
+  }
+  previous_done();
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !st->error) {
+    st->counts[kCntAccepted] += st->n_accept;
+    st->n_live = st->n_open;
+    if (st->n_open == 0) {
+      st->prev_start = 0;
+    } else {
+      // Every pixel of the last frame belongs to a component still open, and
+      // they are the tail of the pool (dials_spots.cc:378-380).
+      const uint32_t last = st->frame_off[a.nb] - st->frame_off[a.nb - 1];
+      st->prev_start = st->n_open - last;
+    }
+  }
+}
+
 // Four lanes per candidate, in size order (so that the candidates sharing a
 // warp have similar sizes): lanes 0-2 each run one axis of the variance pass
 // -- the reference's rounded additions of the member terms, in member order
 // (dials_spots.cc:331-353) -- and the variance formula; lane 0 writes the
 // accepted spot's record. Where the first pass was not exact, lane 0 runs the
-// whole sequence alone.
-__global__ void k_var(LabelStatus *st, const BatchArgs *__restrict__ ap,
+// whole sequence alone. The largest candidates' chains of additions set this
+// kernel's time, on few of the warps: k_compact runs beside it.
+__global__ void __launch_bounds__(kThreads, kVarBlocks)
+k_var(LabelStatus *st, const BatchArgs *__restrict__ ap,
                       const uint32_t *__restrict__ perm, const uint32_t *__restrict__ cand_off,
                       const uint32_t *__restrict__ acc_n, const uint32_t *__restrict__ acc_idx,
                       const uint32_t *__restrict__ acc_off, const CandSpot *__restrict__ cs,
                       const sf_pixel *__restrict__ mpix, const double *__restrict__ terms,
                       size_t terms_stride, sf_spot *spots, size_t spots_cap) {
   previous_done();
+  next_may_start();
   const BatchArgs &a = *ap;
   if (st->error)
     return;
@@ -1460,44 +1476,6 @@ __global__ void k_var(LabelStatus *st, const BatchArgs *__restrict__ ap,
   }
 }
 
-// The open components' pixels into the next live pool, and (block 0, for the
-// next call: nothing here reads them) the state carried over.
-__global__ void k_compact(LabelStatus *st, const BatchArgs *__restrict__ ap,
-                          const uint32_t *__restrict__ flag,
-                          const uint32_t *__restrict__ newpos,
-                          const uint32_t *__restrict__ root, const int32_t *__restrict__ frame,
-                          const uint32_t *__restrict__ index, const uint32_t *__restrict__ value,
-                          int32_t *frame2, uint32_t *index2, uint32_t *value2,
-                          uint32_t *parent2) {
-  previous_done();
-  if (st->error)
-    return;
-  const BatchArgs &a = *ap;
-  const uint32_t n = st->n_total;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += gridDim.x * blockDim.x) {
-    if (flag[p] & kOpenPixel) {
-      const uint32_t q = newpos[p];
-      frame2[q] = frame[p];
-      index2[q] = index[p];
-      value2[q] = value[p];
-      parent2[q] = newpos[root[p]];
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    st->counts[kCntAccepted] += st->n_accept;
-    st->n_live = st->n_open;
-    if (st->n_open == 0) {
-      st->prev_start = 0;
-    } else {
-      // Every pixel of the last frame belongs to a component still open, and
-      // they are the tail of the pool (dials_spots.cc:378-380).
-      const uint32_t last = st->frame_off[a.nb] - st->frame_off[a.nb - 1];
-      st->prev_start = st->n_open - last;
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
@@ -1591,17 +1569,20 @@ template <typename T> struct DeviceStore {
 // they are), by asking for each one's attributes.
 static cudaError_t load_label_kernels() {
   const void *kernels[] = {
-      (const void *)k_offsets,        (const void *)k_append,
-      (const void *)k_rows,           (const void *)k_link,
-      (const void *)k_unite,          (const void *)k_flatten,
-      (const void *)k_comp_stats,     (const void *)k_closing_flags,
-      (const void *)k_bucket_hist,    (const void *)k_bucket_offsets,
-      (const void *)k_bucket_scatter, (const void *)k_gather,
-      (const void *)k_sort<false>,    (const void *)k_sort<true>,
-      (const void *)k_perm_offsets,   (const void *)k_perm_scatter,
-      (const void *)k_first,          (const void *)k_pix,
-      (const void *)k_terms,          (const void *)k_var,
-      (const void *)k_compact,        (const void *)scan_pair_sums<ClosingScan>,
+      (const void *)k_append,
+      (const void *)k_link,
+      (const void *)k_unite,
+      (const void *)k_flatten,
+      (const void *)k_bucket_hist,
+      (const void *)k_bucket_scatter,
+      (const void *)k_gather,
+      (const void *)k_sort<false>,
+      (const void *)k_sort<true>,
+      (const void *)k_first,
+      (const void *)k_terms,
+      (const void *)k_var,
+      (const void *)k_compact,
+      (const void *)scan_pair_sums<ClosingScan>,
       (const void *)scan_pair_apply<ClosingScan>,
       (const void *)scan_pair_sums<CandidateScan>,
       (const void *)scan_pair_apply<CandidateScan>,
@@ -1728,7 +1709,7 @@ struct Labeller {
     acc_n = csize;
     acc_off = reinterpret_cast<uint32_t *>(zlast);
     acc_idx = candid;
-    take(hist, (size_t)(kBucketBlocks + 1) * kBuckets);
+    take(hist, (size_t)kBucketBlocks * kBuckets);
     take(scan_sums64, kScanBlocks);
     if (height <= kRowTableMaxRows)
       take(rows, (size_t)(kLabelMaxBatch + 1) * (height + 1));
@@ -1783,47 +1764,41 @@ struct Labeller {
     const BatchArgs *ap = d_args;
     const dim3 g2(kGrid / 4 > 0 ? kGrid / 4 : 1, nb);
     cudaError_t e;
-    k_offsets<<<1, 32, 0, s>>>(st, ap, (uint32_t)capacity);
-    launch_after(k_append, g2, kThreads, 0, s, st, ap, frame[c], index[c], value[c], parent[c]);
-    if (rows)
-      launch_after(k_rows, dim3(kGrid / 4 > 0 ? kGrid / 4 : 1, nb + 1), kThreads, 0, s, st, ap,
-                   index[c], rows, (uint32_t)height);
+    k_append<<<dim3(g2.x, nb + 1), kThreads, 0, s>>>(st, ap, (uint32_t)capacity, frame[c],
+                                                     index[c], value[c], parent[c], rows,
+                                                     (uint32_t)height, zlast, csize, candid);
     launch_after(k_link, g2, kThreads, 0, s, st, ap, index[c], parent[c], rows, (uint32_t)height,
                  edges, (uint32_t)capacity);
     launch_after(k_unite, kPassGrid, kThreads, 0, s, st, edges, (uint32_t)capacity, parent[c]);
-    launch_after(k_flatten, kPassGrid, kThreads, 0, s, st, parent[c], root, zlast, csize, candid);
-    launch_after(k_comp_stats, kPassGrid, kThreads, 0, s, st, root, frame[c], zlast, csize);
-    launch_after(k_closing_flags, kPassGrid, kThreads, 0, s, st, ap, root, zlast, flag);
-    if ((e = scan_pairs(ClosingScan{st, ap, flag, zlast, clist, cbucket, newpos}, scan_sums64,
-                        s)) != cudaSuccess)
+    launch_after(k_flatten, kPassGrid, kThreads, 0, s, st, parent[c], root, frame[c], zlast,
+                 csize);
+    if ((e = scan_pairs(ClosingScan{st, ap, root, flag, zlast, clist, cbucket, newpos},
+                        scan_sums64, s)) != cudaSuccess)
       return e;
     launch_after(k_bucket_hist, kBucketBlocks, kThreads, 0, s, st, cbucket, hist);
-    launch_after(k_bucket_offsets, 1, 1024, 0, s, st, hist);
     launch_after(k_bucket_scatter, kBucketBlocks, kThreads, 0, s, st, clist, cbucket, hist, order);
     if ((e = scan_pairs(CandidateScan{st, ap, order, csize, cand_n, cand_off, candid, cursor,
                                       phist, 0u, 0u, 0u},
                         scan_sums64, s)) != cudaSuccess)
       return e;
-    launch_after(k_gather, kPassGrid, kThreads, 0, s, st, root, candid, cand_off, cursor, members);
+    launch_after(k_gather, kPassGrid + 1, kThreads, 0, s, st, root, candid, cand_off, cursor,
+                 members, phist);
     launch_after(k_sort<false>, kSortGrid, kThreads,
                  (kThreads / 32) * (kWarpSortMax + 2 * kWarpSegMax) * 4, s, st, cand_n, cand_off,
                  members, frame[c], index[c], value[c], mpix, mcand, big);
     launch_after(k_sort<true>, kGrid / 2, kThreads, kBlockSortMax * 4, s, st, cand_n, cand_off,
                  members, frame[c], index[c], value[c], mpix, mcand, big);
-    launch_after(k_perm_offsets, 1, kSizeBins, 0, s, st, phist);
-    launch_after(k_perm_scatter, kPassGrid, kThreads, 0, s, st, cand_n, phist, perm);
     launch_after(k_first, kPassGrid, kThreads, 0, s, st, ap, cand_n, cand_off, mpix, cspots,
-                 acc_n);
+                 acc_n, phist, perm);
     if ((e = scan_pairs(AcceptScan{st, acc_n, acc_idx, acc_off}, scan_sums64, s)) != cudaSuccess)
       return e;
-    launch_after(k_pix, kPassGrid, kThreads, 0, s, st, mpix, mcand, cand_off, acc_n, acc_off,
-                 d_pixels, capacity);
-    launch_after(k_terms, kPassGrid, kThreads, 0, s, st, ap, mpix, mcand, acc_n, cspots, terms,
-                 capacity);
-    launch_after(k_var, kPassGrid, kThreads, 0, s, st, ap, perm, cand_off, acc_n, acc_idx, acc_off,
-                 cspots, mpix, terms, capacity, d_spots, spots_cap);
-    launch_after(k_compact, kPassGrid, kThreads, 0, s, st, ap, flag, newpos, root, frame[c],
-                 index[c], value[c], frame[o], index[o], value[o], parent[o]);
+    launch_after(k_terms, kPassGrid, kThreads, 0, s, st, ap, mpix, mcand, cand_off, acc_n, acc_off,
+                 cspots, terms, capacity, d_pixels, capacity);
+    launch_after(k_var, kVarBlocks * 152, kThreads, 0, s, st, ap, perm, cand_off, acc_n, acc_idx,
+                 acc_off, cspots, mpix, terms, capacity, d_spots, spots_cap);
+    launch_after(k_compact, kPassGrid, kThreads, 0, s, st, ap,
+                 OpenPool{flag, newpos, root, frame[c], index[c], value[c], frame[o], index[o],
+                          value[o], parent[o]});
     return cudaGetLastError();
   }
 

@@ -23,6 +23,13 @@ __device__ __forceinline__ void previous_done() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Lets the next kernel's blocks in before this one's leave, once all of them
+// have called it or left: for a kernel that leaves most of the device idle before
+// one that needs nothing of it.
+__device__ __forceinline__ void next_may_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <class... Params, class... Args>
 cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
                          cudaStream_t stream, Args &&...args) {

@@ -69,8 +69,9 @@ __device__ __forceinline__ void scan_chunk(uint32_t n, uint32_t *lo, uint32_t *h
 // whose sums stay below 2^32 each) by a Scan object:
 //   skip()             nothing to do (an error earlier in the pipeline)
 //   size()             how many items there are (on the device)
-//   load(i)            item i's pair; called once an item in each pass
-//   sums_done()        after the first pass's loads, by every thread
+//   first(i)           item i's pair, in the first pass
+//   load(i)            the same, in the second
+//   sums_done()        after the first pass's items, by every thread
 //   store(i, v, e)     item i's pair and the sum of those before it
 //   totals(t)          the sum of all, by one thread in the second pass
 // size() may not depend on what totals() or store() writes.
@@ -121,7 +122,7 @@ scan_pair_sums(Scan scan, unsigned long long *__restrict__ block_sums) {
   scan_chunk(scan.size(), &lo, &hi);
   unsigned long long acc = 0;
   for (uint32_t i = lo + threadIdx.x; i < hi; i += kScanThreads)
-    acc += scan.load(i);
+    acc += scan.first(i);
   scan.sums_done();
   unsigned long long total;
   (void)block_exclusive_scan64(acc, &total);
