@@ -8,7 +8,7 @@
 //   disp_decide   each set pixel decided from its window's full sums by the
 //                 reference's sequence; the failures leave the mask, which is
 //                 then the strong-pixel mask, and the blocks count theirs
-//   disp_scatter  the mask's pixels as records, ascending, each at its place
+//   scatter_pixels  the mask's pixels as records, ascending, each at its place
 //                 from the counts (and, when asked for, each word's place)
 //
 // No list of candidates is kept between the passes (the records' sums are
@@ -34,45 +34,32 @@ namespace {
 // The filters' constants for a window of n valid pixels, rounded down: nk =
 // 16 n (0 when n cannot be tested), clo <= 16 c where the dispersion test is n
 // Q - S (S + c) > 0 but for rounding, and kk <= sigma_s^2 gain n.
-constexpr uint32_t kDispMaxKK = 7200;     // keeps S kk below 65535 x 65536 for S <= 81 x 7281
+constexpr uint32_t kDispMaxKK = 3640;  // keeps S kk below 2^31 for S <= 81 x 7281
+constexpr int kDispMaxD = 46340;       // d^2 + d below 2^31, and not below S kk
+static_assert((uint64_t)kDispMaxKK * 81u * 7281u <= (uint64_t)kDispMaxD * (kDispMaxD + 1) - 1u &&
+                  (uint64_t)kDispMaxD * (kDispMaxD + 1) < (1ull << 31),
+              "both sides of the second filter fit, and the largest d passes");
 struct DispTables {
   uint32_t nk[kMaxN0 + 1], clo[kMaxN0 + 1], kk[kMaxN0 + 1];
 };
 
-// The tests of one window of n valid pixels with sum S and sum of squares Q,
-// and of its centre pixel p (packed): false only where the reference's are.
-template <int K, typename Pix>
-__device__ __forceinline__ bool disp_maybe0(uint32_t n, uint32_t S, uint32_t Q, uint32_t nk,
-                                            uint32_t clo, const LaunchParams &P) {
-  if constexpr (sizeof(Pix) == 2)
-    return stage0_u16(n, S, Q, P);  // the reference's float test itself
-  // (Bitwise: branches around the halves took the kernel from 344 to 437 us.)
-  return (Q >= StripG<K>::Big) | (Q * nk > S * ((S << 4) + clo));
-}
-template <int K, typename Pix>
-__device__ __forceinline__ bool disp_maybe2(uint32_t p, uint32_t n, uint32_t S, uint32_t kk,
+// The second test of a window of n valid 16-bit pixels with sum S and of its
+// centre pixel p: the reference's float sequence.
+__device__ __forceinline__ bool disp_float2(uint32_t p, uint32_t n, uint32_t S,
                                             const LaunchParams &P) {
-  if constexpr (sizeof(Pix) == 2) {
-    const float m = __uint2float_rn(n), s = __uint2float_rn(S), v = __uint2float_rn(p);
-    return __fsub_rn(__fmul_rn(m, v), s) >
-           __fmul_rn((float)P.sigma_s, __fsqrt_rn(__fmul_rn(__fmul_rn((float)P.gain, s), m)));
-  }
-  // d = n p - S against sqrt(kk S): d falls and kk S rises with S, so a
-  // saturated sum, at most the true one, passes wherever the true one does.
-  // d^2 + d covers the rounding of the reference's right side (under half a
-  // unit in d), and d beyond 65535 passes whatever S is.
-  const int d = (int)(n * p) - (int)S;
-  const uint32_t e = (uint32_t)min(d, 65535);
-  return (p >= StripG<K>::Cap) | ((d > 0) & (e * e + e >= S * kk));
+  const float m = __uint2float_rn(n), s = __uint2float_rn(S), v = __uint2float_rn(p);
+  return __fsub_rn(__fmul_rn(m, v), s) >
+         __fmul_rn((float)P.sigma_s, __fsqrt_rn(__fmul_rn(__fmul_rn((float)P.gain, s), m)));
 }
 
 // The walk of sf_strips.cuh: a lane adds each row to its 12 column sums as it
 // enters the window, subtracts it as it leaves, and reads it once more as the
 // centre row; a window is 2K + 1 column sums.
-// Bound by issue: 50 instructions a pixel at 70% of the issue rate. 16 frames of
+// Bound by issue: 40 instructions a pixel at 66% of the issue rate. 16 frames of
 // 3262 x 3108 took 4.57 ms as 32 x 32 tiles (each pixel's window summed in
-// 64 bits from shared memory, the halo staged 2.6 times over), and take 0.44 ms
-// here: 344 us in this kernel, 70 and 30 in the two below.
+// 64 bits from shared memory, the halo staged 2.6 times over), and take 0.39 ms
+// here: 282 us in this kernel (344 with both tests compared, selected and ORed,
+// 437 with branches around their halves), 70 and 30 in the two below.
 template <int K, typename Pix>
 __global__ void __launch_bounds__(kStripWarps * 32, StripG<K>::Occ)
 disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,
@@ -82,9 +69,9 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
   previous_done();
   using G = StripG<K>;
   extern __shared__ __align__(16) unsigned char disp_raw[];
-  __shared__ uint4 tab[G::N0 + 1];  // by masked count m: nk, clo, kk of n = N0 - m
+  __shared__ uint4 tab[G::N0 + 1];  // by masked count m: -nk, clo, kk of n = N0 - m
   for (int m = threadIdx.x; m <= G::N0; m += blockDim.x)
-    tab[m] = make_uint4(T.nk[G::N0 - m], T.clo[G::N0 - m], T.kk[G::N0 - m], 0u);
+    tab[m] = make_uint4(0u - T.nk[G::N0 - m], T.clo[G::N0 - m], T.kk[G::N0 - m], 0u);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   StripRun r;
@@ -125,11 +112,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
       for (int c = 0; c < kCols; c++)
         o[c] = 0u;
     }
-#pragma unroll
-    for (int c = 0; c < kCols; c++) {
-      Vn[c] += v[c] - o[c];
-      Vq[c] += v[c] * v[c] - o[c] * o[c];
-    }
+    add_rows(Vn, Vq, v, o);
     if (i >= 2 * K) {  // warp-uniform: the windows are whole
       uint32_t hn[kCols], hq[kCols];
       window_sums<K>(Vn, hn);
@@ -141,37 +124,83 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
       // Warp rows whose windows hold no masked pixel (most) take the whole
       // window's constants; the others look each window's count up.
       const bool uniform = !__any_sync(0xffffffffu, any_masked >> kCountShift);
+      // The lower bound of the dispersion test, by the sign of its difference
+      // (sf_strips.cuh); a window too big for it passes.
       uint32_t out = 0;
-      if (uniform) {
+      if constexpr (sizeof(Pix) == 2) {
+        // (The reference's float test itself.)
+        if (uniform) {
+#pragma unroll
+          for (int c = 0; c < kCols; c++)
+            out |= stage0_u16(G::N0, hn[c], hq[c], P) ? 1u << c : 0u;
+        } else {
+#pragma unroll
+          for (int c = 0; c < kCols; c++) {
+            const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
+            out |= stage0_u16(G::N0 - m, hn[c] & kSumMask, hq[c], P) ? 1u << c : 0u;
+          }
+        }
+      } else {
+        out = uniform ? sign_bits([&](int c) {
+          return hq[c] * whole.x + hn[c] * ((hn[c] << 4) + whole.y);
+        })
+                      : sign_bits([&](int c) {
+                          const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)];
+                          const uint32_t s = hn[c] & kSumMask;
+                          return hq[c] * t.x + s * ((s << 4) + t.y);
+                        });
+        uint32_t most = 0;
 #pragma unroll
         for (int c = 0; c < kCols; c++)
-          out |= disp_maybe0<K, Pix>(G::N0, hn[c], hq[c], whole.x, whole.y, P) ? 1u << c : 0u;
-      } else {
+          most = max(most, hq[c]);
+        if (__any_sync(0xffffffffu, most >= G::Big)) {
 #pragma unroll
-        for (int c = 0; c < kCols; c++) {
-          const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
-          const uint4 t = tab[m];
-          out |= disp_maybe0<K, Pix>(G::N0 - m, hn[c] & kSumMask, hq[c], t.x, t.y, P) ? 1u << c
-                                                                                      : 0u;
+          for (int c = 0; c < kCols; c++)
+            out |= hq[c] >= G::Big ? 1u << c : 0u;
         }
       }
       out &= r.inside12;
       if (__any_sync(0xffffffffu, out != 0u)) {
         read_row<K, Pix, false>(ring + s_mid * kStripStride, lane, v);
-        uint32_t out2 = 0;
+        uint32_t out2 = 0, masked12 = 0;
+        if (!uniform) {
 #pragma unroll
-        for (int c = 0; c < kCols; c++) {
-          uint32_t n = G::N0, kk = whole.z, W = hn[c];
-          bool valid = true;
-          if (!uniform) {
-            const uint32_t m = min(W >> kCountShift, (uint32_t)G::N0);
-            n -= m;
-            kk = tab[m].z;
-            W &= kSumMask;
-            valid = v[c] < (1u << kCountShift);
-          }
-          out2 |= valid & disp_maybe2<K, Pix>(v[c], n, W, kk, P) ? 1u << c : 0u;
+          for (int c = 0; c < kCols; c++)
+            masked12 |= v[c] >> kCountShift << c;
         }
+        if constexpr (sizeof(Pix) == 2) {
+#pragma unroll
+          for (int c = 0; c < kCols; c++) {
+            const uint32_t m = uniform ? 0u : min(hn[c] >> kCountShift, (uint32_t)G::N0);
+            out2 |= disp_float2(v[c], G::N0 - m, hn[c] & kSumMask, P) ? 1u << c : 0u;
+          }
+        } else {
+          // d = n p - S against sqrt(kk S): d falls and kk S rises with S, so a
+          // saturated sum, at most the true one, passes wherever the true one
+          // does. d^2 + d covers the rounding of the reference's right side (under
+          // half a unit in d, and kk is a unit low), and a d of kDispMaxD or more
+          // passes whatever S is.
+          auto below = [&](int c, uint32_t n, uint32_t s, uint32_t kk) {
+            const uint32_t e = (uint32_t)max(min((int)(n * v[c]) - (int)s, kDispMaxD), 0);
+            return s * kk - (e * e + e);
+          };
+          out2 = uniform ? sign_bits([&](int c) { return below(c, G::N0, hn[c], whole.z); })
+                         : sign_bits([&](int c) {
+                             const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
+                             return below(c, G::N0 - m, hn[c] & kSumMask, tab[m].z);
+                           });
+          uint32_t most = 0;
+#pragma unroll
+          for (int c = 0; c < kCols; c++)
+            most = max(most, v[c]);
+          if (__any_sync(0xffffffffu, most >= G::Cap)) {
+            // A saturated pixel's own test is left to the next pass.
+#pragma unroll
+            for (int c = 0; c < kCols; c++)
+              out2 |= v[c] >= G::Cap ? 1u << c : 0u;
+          }
+        }
+        out2 &= ~masked12;
         out &= out2;
       }
       write_bits(r, out_row, bytes_left, out);
@@ -272,7 +301,7 @@ __device__ __forceinline__ bool disp_strong(uint32_t p, uint32_t n, unsigned lon
     return false;
   if constexpr (sizeof(Pix) == 2) {
     return stage0_u16(n, (uint32_t)S, (uint32_t)Q, P) &&
-           disp_maybe2<2, Pix>(p, n, (uint32_t)S, 0u, P);  // the float test itself
+           disp_float2(p, n, (uint32_t)S, P);
   } else {
     if (!stage0_u32(n, S, Q, P, P.root_lo, P.root_hi))
       return false;

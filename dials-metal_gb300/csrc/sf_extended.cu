@@ -134,10 +134,11 @@ struct ExtRow {
 // row may be signal; both 2^-4 bounds; both 2^-8 bounds where a window lies
 // between those or is too big for them; the reference's sequence between
 // those; and 64-bit sums where a window may hold a saturated pixel. Bound by
-// issue (69% of its rate, 57 instructions a pixel): 16 frames of 3262 x 3108 at
-// kernel 4 take 425 us, 556 as 240-column strips with the windows' row sums
-// carried in shared memory, the 64-bit rows and the ambiguous windows
-// in passes of their own.
+// issue and, at 10 to 13 warps an SM (registers), its latency: 48 instructions a
+// pixel at 59% of the issue rate. 16 frames of 3262 x 3108 at kernel 4 take 372
+// us, 425 with the decisions compared, selected and ORed (66 instructions), 556
+// as 240-column strips with the windows' row sums carried in shared memory, the
+// 64-bit rows and the ambiguous windows in passes of their own.
 template <int K, typename Pix>
 __global__ void __launch_bounds__(kStripWarps * 32, StripG<K>::Occ)
 ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,
@@ -157,7 +158,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
       tab[m].a = make_uint4(__float_as_uint((float)n), __float_as_uint(root), 0u, 0u);
       tab[m].b = make_uint4(0u, 0u, 0u, 0u);
     } else {
-      tab[m].a = make_uint4(T.nk[n] >> 4, T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
+      tab[m].a = make_uint4(0u - (T.nk[n] >> 4), T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
       tab[m].b = make_uint4(T.nk[n], T.clo[n], T.chi[n], 0u);
     }
   }
@@ -205,11 +206,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
         for (int c = 0; c < kCols; c++)
           o[c] = 0u;
       }
-#pragma unroll
-      for (int c = 0; c < kCols; c++) {
-        Vn[c] += v[c] - o[c];
-        Vq[c] += v[c] * v[c] - o[c] * o[c];
-      }
+      add_rows(Vn, Vq, v, o);
     }
     if (i >= 2 * K) {  // warp-uniform: the windows are whole
       uint32_t hn[kCols], hq[kCols];
@@ -248,66 +245,60 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           }
         }
       } else {
-        // The lower 2^-4 bound; a big window may be signal. (Bitwise
-        // throughout: a branch around half a test costs more than the half.)
-        uint32_t maybe = 0;
-        const uint4 t0 = tab[0].a;
-        if (uniform) {
+        // A row with a window too big for the 2^-4 bounds takes the 2^-8 ones at
+        // once; else the lower 2^-4 bound, and the upper where it leaves any.
+        // (Signs gathered by shifts: four instructions a window for the lower bound,
+        // seven compared, selected and ORed.)
+        uint32_t most = 0;
 #pragma unroll
-          for (int c = 0; c < kCols; c++)
-            maybe |= (hq[c] >= T.big) | (hq[c] * t0.x > hn[c] * ((hn[c] << 4) + t0.y)) ? 1u << c
-                                                                                        : 0u;
-        } else {
-#pragma unroll
-          for (int c = 0; c < kCols; c++) {
+        for (int c = 0; c < kCols; c++)
+          most = max(most, hq[c]);
+        bool finer = __any_sync(0xffffffffu, most >= T.big);
+        if (!finer) {
+          const uint4 t0 = tab[0].a;
+          // The lower bound's difference (and what the upper adds to it).
+          auto plain = [&](int c) { return hq[c] * t0.x + hn[c] * ((hn[c] << 4) + t0.y); };
+          auto looked_up = [&](int c, bool upper) {
             const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].a;
             const uint32_t s = hn[c] & kSumMask;
-            maybe |= (hq[c] >= T.big) | (hq[c] * t.x > s * ((s << 4) + t.y)) ? 1u << c : 0u;
+            return hq[c] * t.x + s * ((s << 4) + t.y) + (upper ? s * t.z + 31u : 0u);
+          };
+          const uint32_t maybe =
+              uniform ? sign_bits(plain) : sign_bits([&](int c) { return looked_up(c, false); });
+          sig = maybe;
+          if (__any_sync(0xffffffffu, maybe != 0u)) {
+            const uint32_t sure =
+                uniform ? sign_bits([&](int c) { return plain(c) + hn[c] * t0.z + 31u; })
+                        : sign_bits([&](int c) { return looked_up(c, true); });
+            sig = sure;
+            finer = __any_sync(0xffffffffu, (maybe & ~sure) != 0u);
           }
         }
-        sig = maybe;
-        if (__any_sync(0xffffffffu, maybe != 0u)) {
-          uint32_t sure = 0, most = 0;
+        if (finer) {
+          if (__any_sync(0xffffffffu, most >= G::Cap * G::Cap)) {
+            // A window may hold a saturated pixel: this row in 64 bits.
+            sig = ext_wide_row<K>(reinterpret_cast<const uint32_t *>(image), r.height, r.width,
+                                  r.ra - E + i - 2 * K, r.cx, P);
+          } else {
+            uint32_t between = 0;
+            sig = 0;
 #pragma unroll
-          for (int c = 0; c < kCols; c++) {
-            uint4 t = t0;
-            uint32_t s = hn[c];
-            if (!uniform) {
-              t = tab[min(s >> kCountShift, (uint32_t)G::N0)].a;
-              s &= kSumMask;
+            for (int c = 0; c < kCols; c++) {
+              const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].b;
+              const uint32_t s = hn[c] & kSumMask;
+              const unsigned long long L = (unsigned long long)hq[c] * t.x;
+              const bool above = L > (unsigned long long)s * ((s << 8) + t.y);
+              const bool over = L >= (unsigned long long)s * ((s << 8) + t.z) + (2ull << 8);
+              sig |= over ? 1u << c : 0u;
+              between |= above & !over ? 1u << c : 0u;
             }
-            sure |= (hq[c] < T.big) & (hq[c] * t.x >= s * ((s << 4) + t.y) + s * t.z + 32u)
-                        ? 1u << c
-                        : 0u;
-            most = max(most, hq[c]);
-          }
-          sig = sure;
-          if (__any_sync(0xffffffffu, (maybe & ~sure) != 0u)) {
-            if (__any_sync(0xffffffffu, most >= G::Cap * G::Cap)) {
-              // A window may hold a saturated pixel: this row in 64 bits.
-              sig = ext_wide_row<K>(reinterpret_cast<const uint32_t *>(image), r.height, r.width,
-                                    r.ra - E + i - 2 * K, r.cx, P);
-            } else {
-              uint32_t between = 0;
-              sig = 0;
+            if (__any_sync(0xffffffffu, between != 0u)) {
 #pragma unroll
               for (int c = 0; c < kCols; c++) {
-                const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].b;
-                const uint32_t s = hn[c] & kSumMask;
-                const unsigned long long L = (unsigned long long)hq[c] * t.x;
-                const bool above = L > (unsigned long long)s * ((s << 8) + t.y);
-                const bool over = L >= (unsigned long long)s * ((s << 8) + t.z) + (2ull << 8);
-                sig |= over ? 1u << c : 0u;
-                between |= above & !over ? 1u << c : 0u;
-              }
-              if (__any_sync(0xffffffffu, between != 0u)) {
-#pragma unroll
-                for (int c = 0; c < kCols; c++) {
-                  if ((between >> c) & 1u) {
-                    const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
-                    if (ext_exact(G::N0 - m, hn[c] & kSumMask, hq[c], P))
-                      sig |= 1u << c;
-                  }
+                if ((between >> c) & 1u) {
+                  const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
+                  if (ext_exact(G::N0 - m, hn[c] & kSumMask, hq[c], P))
+                    sig |= 1u << c;
                 }
               }
             }

@@ -119,14 +119,37 @@ template <int K> struct StripG {
   static constexpr int Slots = W0 + Ahead + 1;
   static constexpr int Occ = K == 2 ? 8 : K == 3 ? 7 : 6;
   // Valid 32-bit pixels saturate at Cap, so that a window's sum of squares
-  // stays below 2^32. Below Big a window's sum is at most sqrt(N0 Big) =
-  // 2^13.5, and the products of the 32-bit tests stay below 2^32.
+  // stays below 2^32. Below Big a window's sum S is below sqrt(N0 Big) = 2^13,
+  // and both sides of the 32-bit tests (16 n Q; S (16 S + c) + 32, c < kMaxC16)
+  // below 2^31: their difference's sign bit is the decision.
   static constexpr uint32_t Cap = K == 2 ? 13107 : K == 3 ? 9362 : 7281;
-  static constexpr uint32_t Big = (1u << 27) / N0;
+  static constexpr uint32_t Big = (1u << 26) / N0;
   static_assert((unsigned long long)Cap * Cap * N0 < (1ull << 32) && Cap * Cap >= Big,
                 "exact squares, and a saturated pixel makes its window big");
 };
-constexpr uint32_t kMaxC16 = 1u << 17;  // keeps 16 S^2 + S c below 2^32 for S <= 2^13.5
+constexpr uint32_t kMaxC16 = 1u << 17;
+
+// The sign bits of x(c) for the lane's columns c, two chains of shifts.
+template <class X> __device__ __forceinline__ uint32_t sign_bits(X x) {
+  uint32_t lo = 0, hi = 0;
+#pragma unroll
+  for (int c = kCols / 2 - 1; c >= 0; c--) {
+    lo = __funnelshift_l(x(c), lo, 1);
+    hi = __funnelshift_l(x(c + kCols / 2), hi, 1);
+  }
+  return hi << (kCols / 2) | lo;
+}
+
+// A row into and another out of a lane's column sums and sums of squares.
+__device__ __forceinline__ void add_rows(uint32_t Vn[kCols], uint32_t Vq[kCols],
+                                         const uint32_t v[kCols], const uint32_t o[kCols]) {
+#pragma unroll
+  for (int c = 0; c < kCols; c++) {
+    Vn[c] += v[c] - o[c];
+    const uint32_t u = o[c] * o[c] - Vq[c];  // (two multiply-adds)
+    Vq[c] = v[c] * v[c] - u;
+  }
+}
 
 template <int K, typename Pix> constexpr size_t strip_smem() {
   return (size_t)kStripWarps * StripG<K>::Slots * kStripStride * sizeof(Pix);
@@ -215,7 +238,7 @@ template <typename Pix> struct RowReader {
   const Pix *next_row;
   int next_p, pend, width, lane;
   uint32_t inside;
-  bool aligned;
+  bool aligned, whole;  // whole: every lane's pieces lie in the frame's columns
 
   __device__ __forceinline__ RowReader(const Pix *image, const StripRun &r, int pbeg, int rows)
       : next_p(pbeg), pend(min(r.height, pbeg + rows)), width(r.width),
@@ -228,11 +251,16 @@ template <typename Pix> struct RowReader {
       const bool in = aligned ? u < 3 && c >= 0 && c + 4 <= width : c >= 0 && c < width;
       inside |= in ? 1u << u : 0u;
     }
+    whole = __all_sync(0xffffffffu, aligned && inside == 7u);
     next_row = image + (ptrdiff_t)pbeg * width + x0 + (aligned ? 4 * lane : lane);
   }
   __device__ __forceinline__ void fetch(Pix *slot) {
     const uint32_t in = next_p >= 0 && next_p < pend ? inside : 0u;
-    if (aligned) {
+    if (whole && next_p >= 0 && next_p < pend) {
+#pragma unroll
+      for (int u = 0; u < 3; u++)
+        cp_async_piece<Pix>(slot + 4 * lane + 128 * u, next_row + 128 * u);
+    } else if (aligned) {
       Pix *dst = slot + 4 * lane;
 #pragma unroll
       for (int u = 0; u < 3; u++) {
