@@ -69,9 +69,10 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
   previous_done();
   using G = StripG<K>;
   extern __shared__ __align__(16) unsigned char disp_raw[];
-  __shared__ uint4 tab[G::N0 + 1];  // by masked count m: -nk, clo, kk of n = N0 - m
-  for (int m = threadIdx.x; m <= G::N0; m += blockDim.x)
-    tab[m] = make_uint4(0u - T.nk[G::N0 - m], T.clo[G::N0 - m], T.kk[G::N0 - m], 0u);
+  __shared__ uint4 rows_tab[G::N0 + 1];  // by n: -nk, clo, kk
+  const uint4 *tab = rows_tab + G::N0;   // by -m, m masked pixels of the window
+  for (int n = threadIdx.x; n <= G::N0; n += blockDim.x)
+    rows_tab[n] = make_uint4(0u - T.nk[n], T.clo[n], T.kk[n], 0u);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   StripRun r;
@@ -95,18 +96,18 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
   uint8_t *out_row = mask_all + (size_t)r.frame * mask_bytes + (size_t)r.ra * r.bytes_per_row +
                      r.pair_byte;
   const int bytes_left = r.bytes_per_row - r.pair_byte;
-  // Slots of the row in flight, the current, the centre and the leaving row.
-  int s_in = G::Ahead, s_cur = 0, s_mid = G::Slots - K, s_old = G::Slots - G::W0;
+  int s_cur = 0;  // the current row's slot
   for (int i = 0; i < rows; i++) {
     __syncwarp();  // every lane is done with the slot that is filled next
+    const int s_in = s_cur + G::Ahead < G::Slots ? s_cur + G::Ahead : s_cur + G::Ahead - G::Slots;
     reader.fetch(ring + s_in * kStripStride);
     cp_async_commit();
     cp_async_wait<G::Ahead>();
     __syncwarp();
     uint32_t v[kCols], o[kCols];
-    read_row<K, Pix, true>(ring + s_cur * kStripStride, lane, v);
+    read_row<Pix, G::Cap, true>(ring + s_cur * kStripStride, lane, v);
     if (i >= G::W0) {  // warp-uniform
-      read_row<K, Pix, false>(ring + s_old * kStripStride, lane, o);
+      read_row<Pix, G::Cap, false>(ring + after(s_in) * kStripStride, lane, o);
     } else {
 #pragma unroll
       for (int c = 0; c < kCols; c++)
@@ -136,8 +137,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
         } else {
 #pragma unroll
           for (int c = 0; c < kCols; c++) {
-            const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
-            out |= stage0_u16(G::N0 - m, hn[c] & kSumMask, hq[c], P) ? 1u << c : 0u;
+            out |= stage0_u16(G::N0 + masked_of(hn[c]), hn[c] & kSumMask, hq[c], P) ? 1u << c : 0u;
           }
         }
       } else {
@@ -145,7 +145,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
           return hq[c] * whole.x + hn[c] * ((hn[c] << 4) + whole.y);
         })
                       : sign_bits([&](int c) {
-                          const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)];
+                          const uint4 t = tab[masked_of(hn[c])];
                           const uint32_t s = hn[c] & kSumMask;
                           return hq[c] * t.x + s * ((s << 4) + t.y);
                         });
@@ -161,18 +161,16 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
       }
       out &= r.inside12;
       if (__any_sync(0xffffffffu, out != 0u)) {
-        read_row<K, Pix, false>(ring + s_mid * kStripStride, lane, v);
+        const int s_mid = s_cur >= K ? s_cur - K : s_cur + G::Slots - K;
+        read_row<Pix, G::Cap, false>(ring + s_mid * kStripStride, lane, v);
         uint32_t out2 = 0, masked12 = 0;
-        if (!uniform) {
-#pragma unroll
-          for (int c = 0; c < kCols; c++)
-            masked12 |= v[c] >> kCountShift << c;
-        }
+        if (!uniform)
+          masked12 = sign_bits([&](int c) { return v[c]; });
         if constexpr (sizeof(Pix) == 2) {
 #pragma unroll
           for (int c = 0; c < kCols; c++) {
-            const uint32_t m = uniform ? 0u : min(hn[c] >> kCountShift, (uint32_t)G::N0);
-            out2 |= disp_float2(v[c], G::N0 - m, hn[c] & kSumMask, P) ? 1u << c : 0u;
+            const uint32_t n = G::N0 + (uniform ? 0 : masked_of(hn[c]));
+            out2 |= disp_float2(v[c], n, hn[c] & kSumMask, P) ? 1u << c : 0u;
           }
         } else {
           // d = n p - S against sqrt(kk S): d falls and kk S rises with S, so a
@@ -186,18 +184,18 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
           };
           out2 = uniform ? sign_bits([&](int c) { return below(c, G::N0, hn[c], whole.z); })
                          : sign_bits([&](int c) {
-                             const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
-                             return below(c, G::N0 - m, hn[c] & kSumMask, tab[m].z);
+                             const int m = masked_of(hn[c]);
+                             return below(c, G::N0 + m, hn[c] & kSumMask, tab[m].z);
                            });
-          uint32_t most = 0;
+          int most = 0;
 #pragma unroll
           for (int c = 0; c < kCols; c++)
-            most = max(most, v[c]);
-          if (__any_sync(0xffffffffu, most >= G::Cap)) {
+            most = max(most, (int)v[c]);
+          if (__any_sync(0xffffffffu, most >= (int)G::Cap)) {
             // A saturated pixel's own test is left to the next pass.
 #pragma unroll
             for (int c = 0; c < kCols; c++)
-              out2 |= v[c] >= G::Cap ? 1u << c : 0u;
+              out2 |= (int)v[c] >= (int)G::Cap ? 1u << c : 0u;
           }
         }
         out2 &= ~masked12;
@@ -206,10 +204,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
       write_bits(r, out_row, bytes_left, out);
       out_row += r.bytes_per_row;
     }
-    s_in = after(s_in);
     s_cur = after(s_cur);
-    s_mid = after(s_mid);
-    s_old = after(s_old);
   }
   cp_async_wait<0>();
 }

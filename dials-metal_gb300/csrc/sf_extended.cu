@@ -65,6 +65,21 @@ __device__ __noinline__ bool ext_exact(uint32_t n, unsigned long long S, unsigne
   return stage0_u32(n, S, Q, P, P.root_lo, P.root_hi);
 }
 
+// Pixels of 32-bit frames are kept up to kLargePixel in the ring. A column's sum
+// of those of 2K + 1 rows stays below the count field, and n Q of a window below
+// 2^53: with gain 1 and a whole sigma the reference's own difference is exact.
+constexpr uint32_t kLargePixel = 1u << 20;
+static_assert(9u * kLargePixel < (1u << kCountShift) &&
+                  81ull * 81ull * kLargePixel * kLargePixel < (1ull << 53),
+              "the sums of large pixels fit");
+
+// A window's constants, of n valid pixels: the 2^-4 tests' {-nk,
+// clo, chi - clo} and n, and the 2^-8 tests' {nk, clo, chi}; for 16-bit frames
+// {n, rootf} as floats (rootf NaN, no test passes, below min_local).
+struct ExtRow {
+  uint4 a, b;
+};
+
 // The stage-0 bits (signal or masked; off the frame counts as set) of the 12
 // windows centred on row y, columns cx ..: from 64-bit sums of the frame's
 // pixels, for rows whose windows may hold a pixel too large for the strip's
@@ -120,12 +135,74 @@ __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image
   return bits;
 }
 
-// A window's constants by its masked count m (n = N0 - m): the 2^-4 tests' {nk,
-// clo, chi - clo} and n, and the 2^-8 tests' {nk, clo, chi}; for 16-bit frames
-// {n, rootf} as floats (rootf NaN, no test passes, below min_local).
-struct ExtRow {
-  uint4 a, b;
-};
+// The stage-0 bits of the 12 windows of a lane whose newest row is the ring's
+// slot s, for rows whose windows may hold a pixel of Cap or more: the columns'
+// sums again from the ring's rows, squares in 64 bits, and the 2^-8 tests in 64
+// bits; by ext_wide_row where one of the warp's pixels is kLargePixel or more. (Two dense frames of 353 x 944 at kernel 4,
+// every row of them so, take 80 us in all, 272 with every such row by
+// ext_wide_row; 16 of 2162 x 2068 at kernel 2 take 0.97 ms.)
+template <int K>
+__device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int lane,
+                                               const ExtRow *tab, const LaunchParams &P,
+                                               const uint32_t *image, int height, int width, int y,
+                                               int cx) {
+  using G = StripG<K>;
+  uint32_t n[kCols + 2 * K], top = 0;
+  unsigned long long q[kCols + 2 * K];
+#pragma unroll
+  for (int c = 0; c < kCols; c++)
+    n[K + c] = 0u, q[K + c] = 0ull;
+#pragma unroll 1
+  for (int d = 0; d < G::W0; d++) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(ring + s * kStripStride + kCols * lane);
+#pragma unroll
+    for (int i = 0; i < kCols / 4; i++) {
+      const uint4 x = src[i];
+      const uint32_t v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t u = (uint32_t)max((int)v[k], 0);
+        top = max(top, u);
+        n[K + 4 * i + k] += v[k];
+        q[K + 4 * i + k] += (unsigned long long)u * u;
+      }
+    }
+    s = s == 0 ? G::Slots - 1 : s - 1;
+  }
+  if (__any_sync(0xffffffffu, top >= kLargePixel))
+    return ext_wide_row<K>(image, height, width, y, cx, P);
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    n[k] = __shfl_up_sync(0xffffffffu, n[kCols + k], 1);
+    q[k] = __shfl_up_sync(0xffffffffu, q[kCols + k], 1);
+    n[K + kCols + k] = __shfl_down_sync(0xffffffffu, n[K + k], 1);
+    q[K + kCols + k] = __shfl_down_sync(0xffffffffu, q[K + k], 1);
+  }
+  // With another gain or sigma it rounds, by far less than the 2 units between the
+  // tests below this.
+  const unsigned long long limit = P.int_ok ? ~0ull : 1ull << 42;
+  uint32_t m = 0, S = 0, bits = 0;
+  unsigned long long Q = 0;
+#pragma unroll
+  for (int j = 0; j < kCols + 2 * K; j++) {
+    m -= masked_of(n[j]);
+    S += n[j] & kSumMask;
+    Q += q[j];
+    if (j >= 2 * K) {
+      const uint32_t masked = min(m, (uint32_t)G::N0);
+      const uint4 t = tab[-(int)masked].b;
+      const unsigned long long L = Q * t.x, S8 = (unsigned long long)S << 8;
+      bool sig = L >= S * (S8 + t.z) + (2ull << 8);
+      if (Q >= limit || (!sig && L > S * (S8 + t.y)))
+        sig = ext_exact(G::N0 - masked, S, Q, P);
+      bits |= sig ? 1u << (j - 2 * K) : 0u;
+      m += masked_of(n[j - 2 * K]);
+      S -= n[j - 2 * K] & kSumMask;
+      Q -= q[j - 2 * K];
+    }
+  }
+  return bits;
+}
 
 // The walk of sf_strips.cuh for stage 0, then the erosion (dext.cc:117-142):
 // the rows' 12 decision bits are kept for 2E + 1 rows and ANDed down the
@@ -133,9 +210,9 @@ struct ExtRow {
 // only as far as it must: the lower 2^-4 bound alone where no window of the
 // row may be signal; both 2^-4 bounds; both 2^-8 bounds where a window lies
 // between those or is too big for them; the reference's sequence between
-// those; and 64-bit sums where a window may hold a saturated pixel. Bound by
-// issue and, at 10 to 13 warps an SM (registers), its latency: 48 instructions a
-// pixel at 59% of the issue rate. 16 frames of 3262 x 3108 at kernel 4 take 372
+// those; and 64-bit squares where a window may hold a pixel of Cap or more. Bound by
+// issue and, at 10 to 13 warps an SM (registers), its latency: 51 instructions a
+// pixel at 61% of the issue rate. 16 frames of 3262 x 3108 at kernel 4 take 372
 // us, 425 with the decisions compared, selected and ORed (66 instructions), 556
 // as 240-column strips with the windows' row sums carried in shared memory, the
 // 64-bit rows and the ambiguous windows in passes of their own.
@@ -150,16 +227,16 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
   constexpr bool k16 = sizeof(Pix) == 2;
   constexpr int E = K - 1;
   extern __shared__ __align__(16) unsigned char ext_raw[];
-  __shared__ ExtRow tab[G::N0 + 1];
-  for (int m = threadIdx.x; m <= G::N0; m += blockDim.x) {
-    const int n = G::N0 - m;
+  __shared__ ExtRow rows_tab[G::N0 + 1];  // by n
+  ExtRow *tab = rows_tab + G::N0;  // by -m, m masked pixels of the window
+  for (int n = threadIdx.x; n <= G::N0; n += blockDim.x) {
     if constexpr (k16) {
       const float root = (uint32_t)n < P.min_local ? __uint_as_float(0x7FFFFFFFu) : P.rootf[n];
-      tab[m].a = make_uint4(__float_as_uint((float)n), __float_as_uint(root), 0u, 0u);
-      tab[m].b = make_uint4(0u, 0u, 0u, 0u);
+      rows_tab[n].a = make_uint4(__float_as_uint((float)n), __float_as_uint(root), 0u, 0u);
+      rows_tab[n].b = make_uint4(0u, 0u, 0u, 0u);
     } else {
-      tab[m].a = make_uint4(0u - (T.nk[n] >> 4), T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
-      tab[m].b = make_uint4(T.nk[n], T.clo[n], T.chi[n], 0u);
+      rows_tab[n].a = make_uint4(0u - (T.nk[n] >> 4), T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
+      rows_tab[n].b = make_uint4(T.nk[n], T.clo[n], T.chi[n], 0u);
     }
   }
   __syncthreads();
@@ -188,25 +265,35 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
   // The last 2E + 1 rows' decision bits and the last E + 1 rows' masked bits,
   // 12 bits a row in 16-bit halves, the newest lowest.
   uint32_t dec[4] = {0u, 0u, 0u, 0u}, msk[2] = {0u, 0u};
-  // Slots of the row in flight, the current, the centre and the leaving row.
-  int s_in = G::Ahead, s_cur = 0, s_mid = G::Slots - K, s_old = G::Slots - G::W0;
+  int large = 0;
+  int s_cur = 0;  // the current row's slot
   for (int i = 0; i < rows; i++) {
     __syncwarp();  // every lane is done with the slot that is filled next
+    const int s_in = s_cur + G::Ahead < G::Slots ? s_cur + G::Ahead : s_cur + G::Ahead - G::Slots;
     reader.fetch(ring + s_in * kStripStride);
     cp_async_commit();
     cp_async_wait<G::Ahead>();
     __syncwarp();
     {
       uint32_t v[kCols], o[kCols];
-      read_row<K, Pix, true>(ring + s_cur * kStripStride, lane, v);
+      read_row<Pix, kLargePixel, true>(ring + s_cur * kStripStride, lane, v);
       if (i >= G::W0) {  // warp-uniform
-        read_row<K, Pix, false>(ring + s_old * kStripStride, lane, o);
+        read_row<Pix, kLargePixel, false>(ring + after(s_in) * kStripStride, lane, o);
       } else {
 #pragma unroll
         for (int c = 0; c < kCols; c++)
           o[c] = 0u;
       }
       add_rows(Vn, Vq, v, o);
+      if constexpr (!k16) {
+        // Rows left whose windows may hold a pixel too large for these sums (they
+        // wrap, and are right again when it has left them).
+        int top = 0;
+#pragma unroll
+        for (int c = 0; c < kCols; c++)
+          top = max(top, (int)v[c]);
+        large = __any_sync(0xffffffffu, top >= (int)G::Cap) ? G::W0 : large - 1;
+      }
     }
     if (i >= 2 * K) {  // warp-uniform: the windows are whole
       uint32_t hn[kCols], hq[kCols];
@@ -218,14 +305,13 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
         any_masked |= hn[c];
       // Warp rows whose windows hold no masked pixel (most) take the whole
       // window's constants; the others look each window's count up.
-      const bool uniform = !__any_sync(0xffffffffu, any_masked >> kCountShift);
+      const bool uniform = !__any_sync(0xffffffffu, any_masked >> kCountShift) && large <= 0;
       uint32_t sig = 0, masked12 = 0;
       if (!uniform) {
         uint32_t v[kCols];
-        read_row<K, Pix, false>(ring + s_mid * kStripStride, lane, v);
-#pragma unroll
-        for (int c = 0; c < kCols; c++)
-          masked12 |= v[c] >> kCountShift << c;
+        const int s_mid = s_cur >= K ? s_cur - K : s_cur + G::Slots - K;
+        read_row<Pix, kLargePixel, false>(ring + s_mid * kStripStride, lane, v);
+        masked12 = sign_bits([&](int c) { return v[c]; });
       }
       if constexpr (k16) {
         if (uniform) {
@@ -237,13 +323,17 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
         } else {
 #pragma unroll
           for (int c = 0; c < kCols; c++) {
-            const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].a;
+            const uint4 t = tab[masked_of(hn[c])].a;
             sig |= stage0_float(__uint_as_float(t.x), __uint_as_float(t.y), hn[c] & kSumMask, hq[c],
                              gain, sigma_b)
                        ? 1u << c
                        : 0u;
           }
         }
+      } else if (large > 0) {  // warp-uniform
+        sig = ext_large_row<K>(reinterpret_cast<const uint32_t *>(ring), s_cur, lane, tab, P,
+                               reinterpret_cast<const uint32_t *>(image), r.height, r.width,
+                               r.ra - E + i - 2 * K, r.cx);
       } else {
         // A row with a window too big for the 2^-4 bounds takes the 2^-8 ones at
         // once; else the lower 2^-4 bound, and the upper where it leaves any.
@@ -259,7 +349,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           // The lower bound's difference (and what the upper adds to it).
           auto plain = [&](int c) { return hq[c] * t0.x + hn[c] * ((hn[c] << 4) + t0.y); };
           auto looked_up = [&](int c, bool upper) {
-            const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].a;
+            const uint4 t = tab[masked_of(hn[c])].a;
             const uint32_t s = hn[c] & kSumMask;
             return hq[c] * t.x + s * ((s << 4) + t.y) + (upper ? s * t.z + 31u : 0u);
           };
@@ -275,31 +365,24 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           }
         }
         if (finer) {
-          if (__any_sync(0xffffffffu, most >= G::Cap * G::Cap)) {
-            // A window may hold a saturated pixel: this row in 64 bits.
-            sig = ext_wide_row<K>(reinterpret_cast<const uint32_t *>(image), r.height, r.width,
-                                  r.ra - E + i - 2 * K, r.cx, P);
-          } else {
-            uint32_t between = 0;
-            sig = 0;
+          uint32_t between = 0;
+          sig = 0;
+#pragma unroll
+          for (int c = 0; c < kCols; c++) {
+            const uint4 t = tab[masked_of(hn[c])].b;
+            const uint32_t s = hn[c] & kSumMask;
+            const unsigned long long L = (unsigned long long)hq[c] * t.x;
+            const bool above = L > (unsigned long long)s * ((s << 8) + t.y);
+            const bool over = L >= (unsigned long long)s * ((s << 8) + t.z) + (2ull << 8);
+            sig |= over ? 1u << c : 0u;
+            between |= above & !over ? 1u << c : 0u;
+          }
+          if (__any_sync(0xffffffffu, between != 0u)) {
 #pragma unroll
             for (int c = 0; c < kCols; c++) {
-              const uint4 t = tab[min(hn[c] >> kCountShift, (uint32_t)G::N0)].b;
-              const uint32_t s = hn[c] & kSumMask;
-              const unsigned long long L = (unsigned long long)hq[c] * t.x;
-              const bool above = L > (unsigned long long)s * ((s << 8) + t.y);
-              const bool over = L >= (unsigned long long)s * ((s << 8) + t.z) + (2ull << 8);
-              sig |= over ? 1u << c : 0u;
-              between |= above & !over ? 1u << c : 0u;
-            }
-            if (__any_sync(0xffffffffu, between != 0u)) {
-#pragma unroll
-              for (int c = 0; c < kCols; c++) {
-                if ((between >> c) & 1u) {
-                  const uint32_t m = min(hn[c] >> kCountShift, (uint32_t)G::N0);
-                  if (ext_exact(G::N0 - m, hn[c] & kSumMask, hq[c], P))
-                    sig |= 1u << c;
-                }
+              if ((between >> c) & 1u) {
+                if (ext_exact(G::N0 + masked_of(hn[c]), hn[c] & kSumMask, hq[c], P))
+                  sig |= 1u << c;
               }
             }
           }
@@ -330,10 +413,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
         out_row += r.bytes_per_row;
       }
     }
-    s_in = after(s_in);
     s_cur = after(s_cur);
-    s_mid = after(s_mid);
-    s_old = after(s_old);
   }
   cp_async_wait<0>();
 }

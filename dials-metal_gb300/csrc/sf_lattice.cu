@@ -712,14 +712,15 @@ __device__ __forceinline__ uint32_t ver_group(const VerWarp<uint16_t> &sm, int d
 // sum of squares in 48 bits. (A launch of 4 dense frames of 4362 x 4148, whose
 // tiles nearly all hold an overload, takes less than half of what summing each
 // window's 49 pixels took: 2136 us.)
-constexpr uint32_t kWidePixel = 1u << 22;
+constexpr uint32_t kWidePixel = 1u << 20;
 constexpr int kWideCount = 28;
 static_assert((2 * kLatK + 1) * (kWidePixel - 1) < (1u << kWideCount) &&
                   (2ull * kLatK + 1) * (kWidePixel - 1) * (kWidePixel - 1) < (1ull << 48),
               "a column's sums fit their fields");
-// 2^8 n Q and S (2^8 S + c), c < 2^26, stay below 2^64.
-static_assert(49ull * 49ull * (kWidePixel >> 11) * (kWidePixel >> 11) < (1ull << 34),
-              "a window's products fit 64 bits");
+// n Q below 2^53: the reference's own difference is exact, as the tests' 2 units
+// between them need, and 2^8 n Q and S (2^8 S + c) stay below 2^64.
+static_assert(49ull * 49ull * (kWidePixel - 1) * (kWidePixel - 1) < (1ull << 53),
+              "a window's sums are exact in double");
 
 __device__ __noinline__ void ver_wide_columns(VerWarp<uint32_t> &sm, int off, int npass,
                                               int lane) {
@@ -752,8 +753,8 @@ __device__ __noinline__ void ver_wide_columns(VerWarp<uint32_t> &sm, int off, in
   }
 }
 
-// ver_group from those sums: the same two bounds in 64 bits (S < 2^28, Q <
-// 2^50), then the reference's sequence.
+// ver_group from those sums: the same two bounds in 64 bits, then the reference's
+// sequence.
 __device__ __noinline__ uint32_t ver_wide_group(const VerWarp<uint32_t> &sm, int d, int j,
                                                 uint32_t need, const uint4 *tab,
                                                 const LaunchParams &P) {

@@ -102,9 +102,13 @@ constexpr int kCols = 12;              // columns a lane owns
 constexpr int kStripOut = kCols * 30;  // output columns a warp
 constexpr int kStripStride = kCols * 32;  // pixels a staged row
 constexpr int kStripWarps = 2;         // warps a block
-// A window's masked count above its sum: 81 << 25 and 81 x 65533 both fit.
-constexpr uint32_t kCountShift = 25;
+// A sum of pixels of which m are masked: the valid ones' sum (81 x 65533 is below
+// 2^24) less m << 24. masked_of is -m, the place of a window's constants before
+// the end of their table; a masked pixel is negative and its square wraps to 0.
+constexpr uint32_t kCountShift = 24;
 constexpr uint32_t kSumMask = (1u << kCountShift) - 1u;
+constexpr uint32_t kMaskedPixel = 0u - (1u << kCountShift);
+__device__ __forceinline__ int masked_of(uint32_t sum) { return (int)sum >> kCountShift; }
 
 // Windows of 2K + 1 pixels square, with E rows of decisions either side of an
 // output row (0: none).
@@ -118,8 +122,8 @@ template <int K> struct StripG {
   static constexpr int Ahead = K == 4 ? 1 : 2;
   static constexpr int Slots = W0 + Ahead + 1;
   static constexpr int Occ = K == 2 ? 8 : K == 3 ? 7 : 6;
-  // Valid 32-bit pixels saturate at Cap, so that a window's sum of squares
-  // stays below 2^32. Below Big a window's sum S is below sqrt(N0 Big) = 2^13,
+  // Valid 32-bit pixels saturate at Cap, or rows whose windows hold a larger one
+  // are summed apart, so that a window's sum of squares stays below 2^32. Below Big a window's sum S is below sqrt(N0 Big) = 2^13,
   // and both sides of the 32-bit tests (16 n Q; S (16 S + c) + 32, c < kMaxC16)
   // below 2^31: their difference's sign bit is the decision.
   static constexpr uint32_t Cap = K == 2 ? 13107 : K == 3 ? 9362 : 7281;
@@ -155,26 +159,25 @@ template <int K, typename Pix> constexpr size_t strip_smem() {
   return (size_t)kStripWarps * StripG<K>::Slots * kStripStride * sizeof(Pix);
 }
 
-// A valid pixel's value, or a lone count bit for a masked one (whose square
-// wraps to 0).
-template <int K, typename Pix> __device__ __forceinline__ uint32_t pack_pixel(uint32_t v) {
+// A valid pixel's value, 32-bit ones saturated at kCap, or a masked one's.
+template <typename Pix, uint32_t kCap> __device__ __forceinline__ uint32_t pack_pixel(uint32_t v) {
   if (sizeof(Pix) == 2)
-    return v >= 0xFFFEu ? 1u << kCountShift : v;
-  return v >= 0xFFFFFFFEu ? 1u << kCountShift : min(v, StripG<K>::Cap);
+    return v >= 0xFFFEu ? kMaskedPixel : v;
+  return v >= 0xFFFFFFFEu ? kMaskedPixel : min(v, kCap);
 }
 
 // A lane's 12 staged pixels, packed. 32-bit rows are packed in place when
 // they arrive (kRaw reads them first), 16-bit rows whenever they are read.
-template <int K, typename Pix, bool kRaw>
+template <typename Pix, uint32_t kCap, bool kRaw>
 __device__ __forceinline__ void read_row(Pix *slot, int lane, uint32_t v[kCols]) {
   if constexpr (sizeof(Pix) == 2) {
     const uint2 *src = reinterpret_cast<const uint2 *>(slot + kCols * lane);
 #pragma unroll
     for (int i = 0; i < kCols / 4; i++) {
       const uint2 x = src[i];
-      v[4 * i] = pack_pixel<K, Pix>(x.x & 0xFFFFu), v[4 * i + 1] = pack_pixel<K, Pix>(x.x >> 16);
-      v[4 * i + 2] = pack_pixel<K, Pix>(x.y & 0xFFFFu);
-      v[4 * i + 3] = pack_pixel<K, Pix>(x.y >> 16);
+      v[4 * i] = pack_pixel<Pix, kCap>(x.x & 0xFFFFu), v[4 * i + 1] = pack_pixel<Pix, kCap>(x.x >> 16);
+      v[4 * i + 2] = pack_pixel<Pix, kCap>(x.y & 0xFFFFu);
+      v[4 * i + 3] = pack_pixel<Pix, kCap>(x.y >> 16);
     }
   } else {
     uint4 *src = reinterpret_cast<uint4 *>(slot + kCols * lane);
@@ -182,8 +185,8 @@ __device__ __forceinline__ void read_row(Pix *slot, int lane, uint32_t v[kCols])
     for (int i = 0; i < kCols / 4; i++) {
       uint4 x = src[i];
       if (kRaw) {
-        x.x = pack_pixel<K, Pix>(x.x), x.y = pack_pixel<K, Pix>(x.y);
-        x.z = pack_pixel<K, Pix>(x.z), x.w = pack_pixel<K, Pix>(x.w);
+        x.x = pack_pixel<Pix, kCap>(x.x), x.y = pack_pixel<Pix, kCap>(x.y);
+        x.z = pack_pixel<Pix, kCap>(x.z), x.w = pack_pixel<Pix, kCap>(x.w);
         src[i] = x;
       }
       v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
