@@ -60,7 +60,7 @@ __device__ __forceinline__ bool disp_float2(uint32_t p, uint32_t n, uint32_t S,
 // 64 bits from shared memory, the halo staged 2.6 times over), and take 0.39 ms
 // here: 282 us in this kernel (344 with both tests compared, selected and ORed,
 // 437 with branches around their halves), 70 and 30 in the two below.
-template <int K, typename Pix>
+template <int K, typename Pix, int C>
 __global__ void __launch_bounds__(kStripWarps * 32, StripG<K>::Occ)
 disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,
            int run_rows, const __grid_constant__ DispTables T,
@@ -76,21 +76,21 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   StripRun r;
-  if (!strip_run(F, nframes, S, run_rows, r))
+  if (!strip_run<C>(F, nframes, S, run_rows, r))
     return;  // whole warp
   const Pix *image = reinterpret_cast<const Pix *>(F.image[r.frame]);
   const int rows = r.rb - r.ra + 2 * K;
-  Pix *ring = reinterpret_cast<Pix *>(disp_raw) + (size_t)warp * G::Slots * kStripStride;
-  RowReader<Pix> reader(image, r, r.ra - K, rows);
+  Pix *ring = reinterpret_cast<Pix *>(disp_raw) + (size_t)warp * G::Slots * kStripStride<C>;
+  RowReader<Pix, C> reader(image, r, r.ra - K, rows);
   auto after = [&](int s) { return s + 1 == G::Slots ? 0 : s + 1; };
 #pragma unroll
   for (int i = 0; i < G::Ahead; i++) {
-    reader.fetch(ring + i * kStripStride);
+    reader.fetch(ring + i * kStripStride<C>);
     cp_async_commit();
   }
-  uint32_t Vn[kCols], Vq[kCols];
+  uint32_t Vn[C], Vq[C];
 #pragma unroll
-  for (int c = 0; c < kCols; c++)
+  for (int c = 0; c < C; c++)
     Vn[c] = Vq[c] = 0u;
   const uint4 whole = tab[0];
   uint8_t *out_row = mask_all + (size_t)r.frame * mask_bytes + (size_t)r.ra * r.bytes_per_row +
@@ -100,27 +100,27 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
   for (int i = 0; i < rows; i++) {
     __syncwarp();  // every lane is done with the slot that is filled next
     const int s_in = s_cur + G::Ahead < G::Slots ? s_cur + G::Ahead : s_cur + G::Ahead - G::Slots;
-    reader.fetch(ring + s_in * kStripStride);
+    reader.fetch(ring + s_in * kStripStride<C>);
     cp_async_commit();
     cp_async_wait<G::Ahead>();
     __syncwarp();
-    uint32_t v[kCols], o[kCols];
-    read_row<Pix, G::Cap, true>(ring + s_cur * kStripStride, lane, v);
+    uint32_t v[C], o[C];
+    read_row<Pix, C, G::Cap, true>(ring + s_cur * kStripStride<C>, lane, v);
     if (i >= G::W0) {  // warp-uniform
-      read_row<Pix, G::Cap, false>(ring + after(s_in) * kStripStride, lane, o);
+      read_row<Pix, C, G::Cap, false>(ring + after(s_in) * kStripStride<C>, lane, o);
     } else {
 #pragma unroll
-      for (int c = 0; c < kCols; c++)
+      for (int c = 0; c < C; c++)
         o[c] = 0u;
     }
-    add_rows(Vn, Vq, v, o);
+    add_rows<C>(Vn, Vq, v, o);
     if (i >= 2 * K) {  // warp-uniform: the windows are whole
-      uint32_t hn[kCols], hq[kCols];
-      window_sums<K>(Vn, hn);
-      window_sums<K>(Vq, hq);
+      uint32_t hn[C], hq[C];
+      window_sums<K, C>(Vn, hn);
+      window_sums<K, C>(Vq, hq);
       uint32_t any_masked = 0;
 #pragma unroll
-      for (int c = 0; c < kCols; c++)
+      for (int c = 0; c < C; c++)
         any_masked |= hn[c];
       // Warp rows whose windows hold no masked pixel (most) take the whole
       // window's constants; the others look each window's count up.
@@ -132,43 +132,43 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
         // (The reference's float test itself.)
         if (uniform) {
 #pragma unroll
-          for (int c = 0; c < kCols; c++)
+          for (int c = 0; c < C; c++)
             out |= stage0_u16(G::N0, hn[c], hq[c], P) ? 1u << c : 0u;
         } else {
 #pragma unroll
-          for (int c = 0; c < kCols; c++) {
+          for (int c = 0; c < C; c++) {
             out |= stage0_u16(G::N0 + masked_of(hn[c]), hn[c] & kSumMask, hq[c], P) ? 1u << c : 0u;
           }
         }
       } else {
-        out = uniform ? sign_bits([&](int c) {
+        out = uniform ? sign_bits<C>([&](int c) {
           return hq[c] * whole.x + hn[c] * ((hn[c] << 4) + whole.y);
         })
-                      : sign_bits([&](int c) {
+                      : sign_bits<C>([&](int c) {
                           const uint4 t = tab[masked_of(hn[c])];
                           const uint32_t s = hn[c] & kSumMask;
                           return hq[c] * t.x + s * ((s << 4) + t.y);
                         });
         uint32_t most = 0;
 #pragma unroll
-        for (int c = 0; c < kCols; c++)
+        for (int c = 0; c < C; c++)
           most = max(most, hq[c]);
         if (__any_sync(0xffffffffu, most >= G::Big)) {
 #pragma unroll
-          for (int c = 0; c < kCols; c++)
+          for (int c = 0; c < C; c++)
             out |= hq[c] >= G::Big ? 1u << c : 0u;
         }
       }
-      out &= r.inside12;
+      out &= r.inside;
       if (__any_sync(0xffffffffu, out != 0u)) {
         const int s_mid = s_cur >= K ? s_cur - K : s_cur + G::Slots - K;
-        read_row<Pix, G::Cap, false>(ring + s_mid * kStripStride, lane, v);
+        read_row<Pix, C, G::Cap, false>(ring + s_mid * kStripStride<C>, lane, v);
         uint32_t out2 = 0, masked12 = 0;
         if (!uniform)
-          masked12 = sign_bits([&](int c) { return v[c]; });
+          masked12 = sign_bits<C>([&](int c) { return v[c]; });
         if constexpr (sizeof(Pix) == 2) {
 #pragma unroll
-          for (int c = 0; c < kCols; c++) {
+          for (int c = 0; c < C; c++) {
             const uint32_t n = G::N0 + (uniform ? 0 : masked_of(hn[c]));
             out2 |= disp_float2(v[c], n, hn[c] & kSumMask, P) ? 1u << c : 0u;
           }
@@ -182,26 +182,26 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
             const uint32_t e = (uint32_t)max(min((int)(n * v[c]) - (int)s, kDispMaxD), 0);
             return s * kk - (e * e + e);
           };
-          out2 = uniform ? sign_bits([&](int c) { return below(c, G::N0, hn[c], whole.z); })
-                         : sign_bits([&](int c) {
+          out2 = uniform ? sign_bits<C>([&](int c) { return below(c, G::N0, hn[c], whole.z); })
+                         : sign_bits<C>([&](int c) {
                              const int m = masked_of(hn[c]);
                              return below(c, G::N0 + m, hn[c] & kSumMask, tab[m].z);
                            });
           int most = 0;
 #pragma unroll
-          for (int c = 0; c < kCols; c++)
+          for (int c = 0; c < C; c++)
             most = max(most, (int)v[c]);
           if (__any_sync(0xffffffffu, most >= (int)G::Cap)) {
             // A saturated pixel's own test is left to the next pass.
 #pragma unroll
-            for (int c = 0; c < kCols; c++)
+            for (int c = 0; c < C; c++)
               out2 |= (int)v[c] >= (int)G::Cap ? 1u << c : 0u;
           }
         }
         out2 &= ~masked12;
         out &= out2;
       }
-      write_bits(r, out_row, bytes_left, out);
+      write_bits<C>(r, out_row, bytes_left, out);
       out_row += r.bytes_per_row;
     }
     s_cur = after(s_cur);
@@ -403,35 +403,56 @@ DispTables make_disp_tables(const LaunchParams &P) {
   return T;
 }
 
-template <int K, typename Pix>
-cudaError_t launch_disp(const FramePtrs &F, int nframes, int h, int w, const LaunchParams &P,
-                        const StreamBuffers &b, int run_rows, cudaStream_t stream,
-                        const StreamMarks *marks) {
+template <int K, typename Pix, int C> cudaError_t disp_slots(int *slots_out) {
   using G = StripG<K>;
-  constexpr size_t smem = strip_smem<K, Pix>();
+  constexpr size_t smem = strip_smem<K, Pix, C>();
+  static_assert(sizeof(Pix) == 2 || (smem + sizeof(uint4) * (G::N0 + 1) + 1024) * G::Occ <=
+                                        228 * 1024,
+                "the blocks an SM that the kernel is built for");
   static std::once_flag configured;
   static cudaError_t config_error = cudaSuccess;
   static int slots = 0;
   std::call_once(configured, [] {
-    config_error = cudaFuncSetAttribute(disp_strip<K, Pix>,
+    config_error = cudaFuncSetAttribute(disp_strip<K, Pix, C>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per = 0;
     if (config_error == cudaSuccess)
-      config_error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, disp_strip<K, Pix>,
+      config_error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, disp_strip<K, Pix, C>,
                                                                    kStripWarps * 32, smem);
     slots = std::max(1, per) * kStripWarps * device_sms();
   });
-  if (config_error != cudaSuccess)
-    return config_error;
-  static_assert(sizeof(Pix) == 2 || (smem + sizeof(uint4) * (G::N0 + 1) + 1024) * G::Occ <=
-                                        228 * 1024,
-                "the blocks an SM that the kernel is built for");
+  *slots_out = slots;
+  return config_error;
+}
+
+template <int K, typename Pix, int C>
+cudaError_t launch_strips(const FramePtrs &F, int nframes, const LaunchParams &P,
+                          const StreamBuffers &b, int run_rows, cudaStream_t stream) {
+  int slots = 0;
+  const cudaError_t e = disp_slots<K, Pix, C>(&slots);
+  if (e != cudaSuccess)
+    return e;
   FrameSpans S;
-  run_rows = strip_spans(F, nframes, slots, run_rows, &S);
+  run_rows = strip_spans<C>(F, nframes, slots, run_rows, &S);
   const unsigned blocks = (unsigned)((S.start[nframes] + kStripWarps - 1) / kStripWarps);
-  disp_strip<K, Pix><<<blocks, kStripWarps * 32, smem, stream>>>(
+  disp_strip<K, Pix, C><<<blocks, kStripWarps * 32, strip_smem<K, Pix, C>(), stream>>>(
       F, nframes, S, run_rows, make_disp_tables(P), P, reinterpret_cast<uint8_t *>(b.bits),
       b.words * sizeof(uint32_t));
+  return cudaSuccess;
+}
+
+template <int K, typename Pix>
+cudaError_t launch_disp(const FramePtrs &F, int nframes, int h, int w, const LaunchParams &P,
+                        const StreamBuffers &b, int run_rows, cudaStream_t stream,
+                        const StreamMarks *marks) {
+  int slots = 0;
+  cudaError_t e = disp_slots<K, Pix, kWideCols>(&slots);
+  if (e == cudaSuccess)
+    e = narrow_strips(F, nframes, slots)
+            ? launch_strips<K, Pix, kNarrowCols>(F, nframes, P, b, run_rows, stream)
+            : launch_strips<K, Pix, kWideCols>(F, nframes, P, b, run_rows, stream);
+  if (e != cudaSuccess)
+    return e;
   if (marks)
     cudaEventRecord(marks->stage01, stream);
   const dim3 grid = band_grid(nframes, h, w);

@@ -85,18 +85,18 @@ struct ExtRow {
 // pixels, for rows whose windows may hold a pixel too large for the strip's
 // sums. A column's sums of 2K + 1 rows enter as the windows move right and
 // leave again; a window off the frame is clipped as the reference's is.
-template <int K>
+template <int K, int C>
 __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image, int height,
                                               int width, int y, int cx, const LaunchParams &P) {
   constexpr int W0 = 2 * K + 1;
   if (y < 0 || y >= height)
-    return 0xFFFu;  // off the frame: set
+    return (1u << C) - 1u;  // off the frame: set
   uint32_t cn[W0];
   unsigned long long cS[W0], cQ[W0];
   uint32_t n = 0, bits = 0;
   unsigned long long S = 0, Q = 0;
 #pragma unroll
-  for (int j = 0; j < kCols + 2 * K; j++) {
+  for (int j = 0; j < C + 2 * K; j++) {
     const int x = cx - K + j;
     uint32_t an = 0;
     unsigned long long aS = 0, aQ = 0;
@@ -141,22 +141,22 @@ __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image
 // bits; by ext_wide_row where one of the warp's pixels is kLargePixel or more. (Two dense frames of 353 x 944 at kernel 4,
 // every row of them so, take 80 us in all, 272 with every such row by
 // ext_wide_row; 16 of 2162 x 2068 at kernel 2 take 0.97 ms.)
-template <int K>
+template <int K, int C>
 __device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int lane,
                                                const ExtRow *tab, const LaunchParams &P,
                                                const uint32_t *image, int height, int width, int y,
                                                int cx) {
   using G = StripG<K>;
-  uint32_t n[kCols + 2 * K], top = 0;
-  unsigned long long q[kCols + 2 * K];
+  uint32_t n[C + 2 * K], top = 0;
+  unsigned long long q[C + 2 * K];
 #pragma unroll
-  for (int c = 0; c < kCols; c++)
+  for (int c = 0; c < C; c++)
     n[K + c] = 0u, q[K + c] = 0ull;
 #pragma unroll 1
   for (int d = 0; d < G::W0; d++) {
-    const uint4 *src = reinterpret_cast<const uint4 *>(ring + s * kStripStride + kCols * lane);
+    const uint4 *src = reinterpret_cast<const uint4 *>(ring + s * kStripStride<C> + C * lane);
 #pragma unroll
-    for (int i = 0; i < kCols / 4; i++) {
+    for (int i = 0; i < C / 4; i++) {
       const uint4 x = src[i];
       const uint32_t v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -170,13 +170,13 @@ __device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int 
     s = s == 0 ? G::Slots - 1 : s - 1;
   }
   if (__any_sync(0xffffffffu, top >= kLargePixel))
-    return ext_wide_row<K>(image, height, width, y, cx, P);
+    return ext_wide_row<K, C>(image, height, width, y, cx, P);
 #pragma unroll
   for (int k = 0; k < K; k++) {
-    n[k] = __shfl_up_sync(0xffffffffu, n[kCols + k], 1);
-    q[k] = __shfl_up_sync(0xffffffffu, q[kCols + k], 1);
-    n[K + kCols + k] = __shfl_down_sync(0xffffffffu, n[K + k], 1);
-    q[K + kCols + k] = __shfl_down_sync(0xffffffffu, q[K + k], 1);
+    n[k] = __shfl_up_sync(0xffffffffu, n[C + k], 1);
+    q[k] = __shfl_up_sync(0xffffffffu, q[C + k], 1);
+    n[K + C + k] = __shfl_down_sync(0xffffffffu, n[K + k], 1);
+    q[K + C + k] = __shfl_down_sync(0xffffffffu, q[K + k], 1);
   }
   // With another gain or sigma it rounds, by far less than the 2 units between the
   // tests below this.
@@ -184,7 +184,7 @@ __device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int 
   uint32_t m = 0, S = 0, bits = 0;
   unsigned long long Q = 0;
 #pragma unroll
-  for (int j = 0; j < kCols + 2 * K; j++) {
+  for (int j = 0; j < C + 2 * K; j++) {
     m -= masked_of(n[j]);
     S += n[j] & kSumMask;
     Q += q[j];
@@ -216,7 +216,7 @@ __device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int 
 // us, 425 with the decisions compared, selected and ORed (66 instructions), 556
 // as 240-column strips with the windows' row sums carried in shared memory, the
 // 64-bit rows and the ambiguous windows in passes of their own.
-template <int K, typename Pix>
+template <int K, typename Pix, int C>
 __global__ void __launch_bounds__(kStripWarps * 32, StripG<K>::Occ)
 ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,
           int run_rows, const __grid_constant__ ExtTables T,
@@ -242,21 +242,21 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   StripRun r;
-  if (!strip_run(F, nframes, S, run_rows, r))
+  if (!strip_run<C>(F, nframes, S, run_rows, r))
     return;  // whole warp
   const Pix *image = reinterpret_cast<const Pix *>(F.image[r.frame]);
   const int rows = r.rb - r.ra + 2 * (K + E);
-  Pix *ring = reinterpret_cast<Pix *>(ext_raw) + (size_t)warp * G::Slots * kStripStride;
-  RowReader<Pix> reader(image, r, r.ra - E - K, rows);
+  Pix *ring = reinterpret_cast<Pix *>(ext_raw) + (size_t)warp * G::Slots * kStripStride<C>;
+  RowReader<Pix, C> reader(image, r, r.ra - E - K, rows);
   auto after = [&](int s) { return s + 1 == G::Slots ? 0 : s + 1; };
 #pragma unroll
   for (int i = 0; i < G::Ahead; i++) {
-    reader.fetch(ring + i * kStripStride);
+    reader.fetch(ring + i * kStripStride<C>);
     cp_async_commit();
   }
-  uint32_t Vn[kCols], Vq[kCols];
+  uint32_t Vn[C], Vq[C];
 #pragma unroll
-  for (int c = 0; c < kCols; c++)
+  for (int c = 0; c < C; c++)
     Vn[c] = Vq[c] = 0u;
   const float gain = (float)P.gain, sigma_b = (float)P.sigma_b;
   uint8_t *out_row = cand_all + (size_t)r.frame * mask_bytes + (size_t)r.ra * r.bytes_per_row +
@@ -270,59 +270,59 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
   for (int i = 0; i < rows; i++) {
     __syncwarp();  // every lane is done with the slot that is filled next
     const int s_in = s_cur + G::Ahead < G::Slots ? s_cur + G::Ahead : s_cur + G::Ahead - G::Slots;
-    reader.fetch(ring + s_in * kStripStride);
+    reader.fetch(ring + s_in * kStripStride<C>);
     cp_async_commit();
     cp_async_wait<G::Ahead>();
     __syncwarp();
     {
-      uint32_t v[kCols], o[kCols];
-      read_row<Pix, kLargePixel, true>(ring + s_cur * kStripStride, lane, v);
+      uint32_t v[C], o[C];
+      read_row<Pix, C, kLargePixel, true>(ring + s_cur * kStripStride<C>, lane, v);
       if (i >= G::W0) {  // warp-uniform
-        read_row<Pix, kLargePixel, false>(ring + after(s_in) * kStripStride, lane, o);
+        read_row<Pix, C, kLargePixel, false>(ring + after(s_in) * kStripStride<C>, lane, o);
       } else {
 #pragma unroll
-        for (int c = 0; c < kCols; c++)
+        for (int c = 0; c < C; c++)
           o[c] = 0u;
       }
-      add_rows(Vn, Vq, v, o);
+      add_rows<C>(Vn, Vq, v, o);
       if constexpr (!k16) {
         // Rows left whose windows may hold a pixel too large for these sums (they
         // wrap, and are right again when it has left them).
         int top = 0;
 #pragma unroll
-        for (int c = 0; c < kCols; c++)
+        for (int c = 0; c < C; c++)
           top = max(top, (int)v[c]);
         large = __any_sync(0xffffffffu, top >= (int)G::Cap) ? G::W0 : large - 1;
       }
     }
     if (i >= 2 * K) {  // warp-uniform: the windows are whole
-      uint32_t hn[kCols], hq[kCols];
-      window_sums<K>(Vn, hn);
-      window_sums<K>(Vq, hq);
+      uint32_t hn[C], hq[C];
+      window_sums<K, C>(Vn, hn);
+      window_sums<K, C>(Vq, hq);
       uint32_t any_masked = 0;
 #pragma unroll
-      for (int c = 0; c < kCols; c++)
+      for (int c = 0; c < C; c++)
         any_masked |= hn[c];
       // Warp rows whose windows hold no masked pixel (most) take the whole
       // window's constants; the others look each window's count up.
       const bool uniform = !__any_sync(0xffffffffu, any_masked >> kCountShift) && large <= 0;
       uint32_t sig = 0, masked12 = 0;
       if (!uniform) {
-        uint32_t v[kCols];
+        uint32_t v[C];
         const int s_mid = s_cur >= K ? s_cur - K : s_cur + G::Slots - K;
-        read_row<Pix, kLargePixel, false>(ring + s_mid * kStripStride, lane, v);
-        masked12 = sign_bits([&](int c) { return v[c]; });
+        read_row<Pix, C, kLargePixel, false>(ring + s_mid * kStripStride<C>, lane, v);
+        masked12 = sign_bits<C>([&](int c) { return v[c]; });
       }
       if constexpr (k16) {
         if (uniform) {
           const uint4 t = tab[0].a;
           const float m = __uint_as_float(t.x), root = __uint_as_float(t.y);
 #pragma unroll
-          for (int c = 0; c < kCols; c++)
+          for (int c = 0; c < C; c++)
             sig |= stage0_float(m, root, hn[c], hq[c], gain, sigma_b) ? 1u << c : 0u;
         } else {
 #pragma unroll
-          for (int c = 0; c < kCols; c++) {
+          for (int c = 0; c < C; c++) {
             const uint4 t = tab[masked_of(hn[c])].a;
             sig |= stage0_float(__uint_as_float(t.x), __uint_as_float(t.y), hn[c] & kSumMask, hq[c],
                              gain, sigma_b)
@@ -331,7 +331,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           }
         }
       } else if (large > 0) {  // warp-uniform
-        sig = ext_large_row<K>(reinterpret_cast<const uint32_t *>(ring), s_cur, lane, tab, P,
+        sig = ext_large_row<K, C>(reinterpret_cast<const uint32_t *>(ring), s_cur, lane, tab, P,
                                reinterpret_cast<const uint32_t *>(image), r.height, r.width,
                                r.ra - E + i - 2 * K, r.cx);
       } else {
@@ -341,7 +341,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
         // seven compared, selected and ORed.)
         uint32_t most = 0;
 #pragma unroll
-        for (int c = 0; c < kCols; c++)
+        for (int c = 0; c < C; c++)
           most = max(most, hq[c]);
         bool finer = __any_sync(0xffffffffu, most >= T.big);
         if (!finer) {
@@ -354,12 +354,12 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
             return hq[c] * t.x + s * ((s << 4) + t.y) + (upper ? s * t.z + 31u : 0u);
           };
           const uint32_t maybe =
-              uniform ? sign_bits(plain) : sign_bits([&](int c) { return looked_up(c, false); });
+              uniform ? sign_bits<C>(plain) : sign_bits<C>([&](int c) { return looked_up(c, false); });
           sig = maybe;
           if (__any_sync(0xffffffffu, maybe != 0u)) {
             const uint32_t sure =
-                uniform ? sign_bits([&](int c) { return plain(c) + hn[c] * t0.z + 31u; })
-                        : sign_bits([&](int c) { return looked_up(c, true); });
+                uniform ? sign_bits<C>([&](int c) { return plain(c) + hn[c] * t0.z + 31u; })
+                        : sign_bits<C>([&](int c) { return looked_up(c, true); });
             sig = sure;
             finer = __any_sync(0xffffffffu, (maybe & ~sure) != 0u);
           }
@@ -368,7 +368,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           uint32_t between = 0;
           sig = 0;
 #pragma unroll
-          for (int c = 0; c < kCols; c++) {
+          for (int c = 0; c < C; c++) {
             const uint4 t = tab[masked_of(hn[c])].b;
             const uint32_t s = hn[c] & kSumMask;
             const unsigned long long L = (unsigned long long)hq[c] * t.x;
@@ -379,7 +379,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
           }
           if (__any_sync(0xffffffffu, between != 0u)) {
 #pragma unroll
-            for (int c = 0; c < kCols; c++) {
+            for (int c = 0; c < C; c++) {
               if ((between >> c) & 1u) {
                 if (ext_exact(G::N0 + masked_of(hn[c]), hn[c] & kSumMask, hq[c], P))
                   sig |= 1u << c;
@@ -400,16 +400,16 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
 #pragma unroll
         for (int k = 1; k <= 2 * E; k++)
           col &= k & 1 ? dec[k >> 1] >> 16 : dec[k >> 1];
-        col &= 0xFFFu;
+        col &= (1u << C) - 1u;
         const uint32_t left = __shfl_up_sync(0xffffffffu, col, 1);
         const uint32_t right = __shfl_down_sync(0xffffffffu, col, 1);
-        const uint32_t all = left >> (kCols - E) | col << E | right << (kCols + E);
+        const uint32_t all = left >> (C - E) | col << E | right << (C + E);
         uint32_t kept = all;
 #pragma unroll
         for (int k = 1; k <= 2 * E; k++)
           kept &= all >> k;
         const uint32_t mrow = E & 1 ? msk[E >> 1] >> 16 : msk[E >> 1];
-        write_bits(r, out_row, bytes_left, kept & ~mrow & r.inside12);
+        write_bits<C>(r, out_row, bytes_left, kept & ~mrow & r.inside);
         out_row += r.bytes_per_row;
       }
     }
@@ -744,16 +744,19 @@ ExtTables make_ext_tables(const LaunchParams &P) {
 // 32-bit frames at gain 1 with integral sigmas, or 16-bit ones where 4 | width
 // and they are 8-byte aligned. Spots cover a few percent of such frames, and
 // the lattice decides a ninth of the windows and the tiles that hold a
-// candidate: 32 frames of 4362 x 4148 take 0.95 ms so and 1.38 ms on strips. One
-// frame alone takes strips up to kStripAlone pixels, where the call is bound by
-// its launches (lattice and strips, called directly: 512 x 512 53 and 43 us, 1065
-// x 1030 52 and 43, 2162 x 2068 53-58 and 46-60, 3262 x 3108 60 and 66; in a
-// captured graph: 32 and 33, 37 and 38, 41 and 45, 59 and 66).
-constexpr long long kStripAlone = 3000000;
+// candidate: 32 frames of 4362 x 4148 take 0.95 ms so and 1.38 ms on strips.
+// Launches of up to kStripPixels take strips, narrow ones that size (sf_strips.cuh):
+// there the lattice's two more launches cost more than they save (both ways, called
+// directly: one frame of 1065 x 1030 55 and 43 us, 4 of 1024 x 1024 60 and 45, 2 of
+// 2162 x 2068 57 and 56; in a captured graph: 37 and 32, 41 and 42, 50 and 56).
+constexpr long long kStripPixels = 5000000;
 bool lattice_path(const FramePtrs &F, int nframes, int pixel_bytes, const LaunchParams &P) {
   if (P.half != 3 || P.algorithm != SF_DISPERSION_EXTENDED)
     return false;
-  if (nframes == 1 && (long long)F.h[0] * F.w[0] <= kStripAlone)
+  long long pixels = 0;
+  for (int f = 0; f < nframes; f++)
+    pixels += (long long)F.h[f] * F.w[f];
+  if (pixels <= kStripPixels)
     return false;
   if (pixel_bytes == 4)
     return P.int_ok != 0;
@@ -763,9 +766,9 @@ bool lattice_path(const FramePtrs &F, int nframes, int pixel_bytes, const Launch
   return true;
 }
 
-template <int K, typename Pix> cudaError_t ext_slots(int *slots_out) {
+template <int K, typename Pix, int C> cudaError_t ext_slots(int *slots_out) {
   using G = StripG<K>;
-  constexpr size_t smem = strip_smem<K, Pix>();
+  constexpr size_t smem = strip_smem<K, Pix, C>();
   static_assert(sizeof(Pix) == 2 ||
                     (smem + sizeof(ExtRow) * (G::N0 + 1) + 1024) * G::Occ <= 228 * 1024,
                 "the blocks an SM that the kernel is built for");
@@ -773,16 +776,32 @@ template <int K, typename Pix> cudaError_t ext_slots(int *slots_out) {
   static cudaError_t config_error = cudaSuccess;
   static int slots = 0;
   std::call_once(configured, [] {
-    config_error = cudaFuncSetAttribute(ext_strip<K, Pix>,
+    config_error = cudaFuncSetAttribute(ext_strip<K, Pix, C>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per = 0;
     if (config_error == cudaSuccess)
-      config_error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ext_strip<K, Pix>,
+      config_error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ext_strip<K, Pix, C>,
                                                                    kStripWarps * 32, smem);
     slots = std::max(1, per) * kStripWarps * device_sms();
   });
   *slots_out = slots;
   return config_error;
+}
+
+template <int K, typename Pix, int C>
+cudaError_t launch_strips(const FramePtrs &F, int nframes, const LaunchParams &P,
+                          const StreamBuffers &b, int run_rows, cudaStream_t stream) {
+  int slots = 0;
+  const cudaError_t e = ext_slots<K, Pix, C>(&slots);
+  if (e != cudaSuccess)
+    return e;
+  FrameSpans S;
+  run_rows = strip_spans<C>(F, nframes, slots, run_rows, &S);
+  const unsigned blocks = (unsigned)((S.start[nframes] + kStripWarps - 1) / kStripWarps);
+  ext_strip<K, Pix, C><<<blocks, kStripWarps * 32, strip_smem<K, Pix, C>(), stream>>>(
+      F, nframes, S, run_rows, make_ext_tables(P), P, reinterpret_cast<uint8_t *>(b.cand),
+      b.words * sizeof(uint32_t));
+  return cudaSuccess;
 }
 
 template <int K, typename Pix>
@@ -797,14 +816,13 @@ cudaError_t launch_ext(const FramePtrs &F, int nframes, int h, int w, const Laun
       return e;
   } else {
     int slots = 0;
-    if ((e = ext_slots<K, Pix>(&slots)) != cudaSuccess)
+    if ((e = ext_slots<K, Pix, kWideCols>(&slots)) != cudaSuccess)
       return e;
-    FrameSpans S;
-    run_rows = strip_spans(F, nframes, slots, run_rows, &S);
-    const unsigned blocks = (unsigned)((S.start[nframes] + kStripWarps - 1) / kStripWarps);
-    ext_strip<K, Pix><<<blocks, kStripWarps * 32, strip_smem<K, Pix>(), stream>>>(
-        F, nframes, S, run_rows, make_ext_tables(P), P, reinterpret_cast<uint8_t *>(b.cand),
-        b.words * sizeof(uint32_t));
+    e = narrow_strips(F, nframes, slots)
+            ? launch_strips<K, Pix, kNarrowCols>(F, nframes, P, b, run_rows, stream)
+            : launch_strips<K, Pix, kWideCols>(F, nframes, P, b, run_rows, stream);
+    if (e != cudaSuccess)
+      return e;
   }
   if (marks)
     cudaEventRecord(marks->stage01, stream);
@@ -873,16 +891,33 @@ cudaError_t launch_extended(const FramePtrs &F, int nframes, int h, int w, int p
   }
 }
 
-int stream_default_run_rows(const LaunchParams &P, int h, int w, int nframes) {
-  if (P.half == 3 && P.int_ok)
-    return lattice_geometry(h, w, nframes, 0).run_rows;
+template <int K> cudaError_t default_run_rows(const FramePtrs &F, int nframes, int *rows) {
   int slots = 0;
-  const cudaError_t e = P.half == 2   ? ext_slots<2, uint32_t>(&slots)
-                        : P.half == 3 ? ext_slots<3, uint32_t>(&slots)
-                                      : ext_slots<4, uint32_t>(&slots);
+  cudaError_t e = ext_slots<K, uint32_t, kWideCols>(&slots);
   if (e != cudaSuccess)
+    return e;
+  FrameSpans S;
+  if (!narrow_strips(F, nframes, slots)) {
+    *rows = strip_spans<kWideCols>(F, nframes, slots, 0, &S);
+  } else if ((e = ext_slots<K, uint32_t, kNarrowCols>(&slots)) == cudaSuccess) {
+    *rows = strip_spans<kNarrowCols>(F, nframes, slots, 0, &S);
+  }
+  return e;
+}
+
+int stream_default_run_rows(const LaunchParams &P, int h, int w, int nframes) {
+  FramePtrs F = {};
+  nframes = std::min(nframes, kMaxBatch);
+  for (int f = 0; f < nframes; f++)
+    F.h[f] = h, F.w[f] = w;
+  if (lattice_path(F, nframes, 4, P))
+    return lattice_geometry(h, w, nframes, 0).run_rows;
+  int rows = kMinRunRows;
+  if ((P.half == 2   ? default_run_rows<2>(F, nframes, &rows)
+       : P.half == 3 ? default_run_rows<3>(F, nframes, &rows)
+                     : default_run_rows<4>(F, nframes, &rows)) != cudaSuccess)
     cudaGetLastError();
-  return strip_run_rows(h, (long long)nframes * strips_of(w), slots, 0);
+  return rows;
 }
 
 } // namespace sf

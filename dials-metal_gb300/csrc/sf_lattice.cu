@@ -130,7 +130,7 @@ __device__ __forceinline__ void lat_row(const uint32_t v[kLatCols], int lane, ui
 constexpr int kRingSlots = 4;
 template <typename Pix>
 constexpr size_t ring_bytes() {
-  return (size_t)kLatWarps * kRingSlots * kStripStride * sizeof(Pix);
+  return (size_t)kLatWarps * kRingSlots * kStripStride<kLatCols> * sizeof(Pix);
 }
 
 template <int kOcc, typename Pix>
@@ -175,7 +175,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
   const int pair_byte = (kLatOut * sx + 24 * ((lane - 1) >> 1)) >> 3;
   const bool writer = lane >= 1 && lane <= kLatOutLanes;
   const bool first_of_pair = (lane & 1) != 0;
-  const uint32_t inside12 =
+  const uint32_t inside =
       (cx < 0 || cx >= width) ? 0u
                               : (cx + kLatCols <= width ? 0xFFFu : ((1u << (width - cx)) - 1u));
   const int ra = ry * run_rows;
@@ -193,15 +193,15 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
 
   // Pixel rows [pbeg, pend) of the run.
   const int pbeg = 3 * (ja - 2), pend = 3 * (ja + ntrip + 1);
-  Pix *ring = lat_ring + (size_t)warp * kRingSlots * kStripStride;
+  Pix *ring = lat_ring + (size_t)warp * kRingSlots * kStripStride<kLatCols>;
   StripRun r;
   r.X = kLatOut * sx;
   r.height = height;
   r.width = width;
-  RowReader<Pix> reader(image, r, pbeg, pend - pbeg);
+  RowReader<Pix, kLatCols> reader(image, r, pbeg, pend - pbeg);
 #pragma unroll
   for (int i = 0; i < kRingSlots - 1; i++) {
-    reader.fetch(ring + i * kStripStride);
+    reader.fetch(ring + i * kStripStride<kLatCols>);
     cp_async_commit();
   }
 
@@ -214,11 +214,11 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
     for (int k = 0; k < 3; k++) {
       // Row p0 + k + kRingSlots - 1 goes out; row p0 + k has landed.
       __syncwarp();
-      reader.fetch(ring + slot_in * kStripStride);
+      reader.fetch(ring + slot_in * kStripStride<kLatCols>);
       cp_async_commit();
       cp_async_wait<kRingSlots - 1>();
       __syncwarp();
-      const Pix *slot = ring + slot_now * kStripStride;
+      const Pix *slot = ring + slot_now * kStripStride<kLatCols>;
       slot_in = (slot_in + 1) % kRingSlots;
       slot_now = (slot_now + 1) % kRingSlots;
       if constexpr (k16) {
@@ -301,7 +301,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
         const int r = p0 - 3 + k;
         const uint32_t bd = k < 2 ? bd01 : bd2;
         const uint32_t mk = mprev[k];
-        const uint32_t c12 = bd & ~mk & inside12;
+        const uint32_t c12 = bd & ~mk & inside;
         // Lane pairs: the first lane (odd) writes the pair's first two bytes,
         // the second the third.
         const uint32_t odd = __shfl_down_sync(0xffffffffu, c12, 1);

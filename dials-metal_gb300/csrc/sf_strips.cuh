@@ -1,7 +1,7 @@
 // What the kernels that walk strips of a frame share (sf_extended.cu,
-// sf_dispersion.cu). A warp walks down a strip of 360 output columns for a run
-// of rows. Lane l owns 12 columns; lanes 1-30 write, and lanes 0 and 31 hold the
-// columns on either side of the strip that the others' windows reach into.
+// sf_dispersion.cu). A warp walks down a strip of 360 output columns (or 112) for
+// a run of rows. Lane l owns 12 columns (4); lanes 1-30 (2-29) write, and the others
+// hold the columns on either side of the strip that their windows reach into.
 // Each pixel row is staged in shared memory by cp.async a row or two ahead and
 // stays there until it leaves the window.
 #pragma once
@@ -98,9 +98,14 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 }
 
 
-constexpr int kCols = 12;              // columns a lane owns
-constexpr int kStripOut = kCols * 30;  // output columns a warp
-constexpr int kStripStride = kCols * 32;  // pixels a staged row
+// Columns a lane owns (C below): wide strips, and narrow ones for launches too
+// small to fill the device with wide ones.
+constexpr int kWideCols = 12, kNarrowCols = 4;
+// Lanes at either end that hold the columns which the others' windows, and the
+// erosion of their decisions, reach into: up to 7.
+template <int C> constexpr int kHalo = C == kNarrowCols ? 2 : 1;
+template <int C> constexpr int kStripOut = C * (32 - 2 * kHalo<C>);  // output columns a warp
+template <int C> constexpr int kStripStride = C * 32;  // pixels a staged row
 constexpr int kStripWarps = 2;         // warps a block
 // A sum of pixels of which m are masked: the valid ones' sum (81 x 65533 is below
 // 2^24) less m << 24. masked_of is -m, the place of a window's constants before
@@ -134,29 +139,30 @@ template <int K> struct StripG {
 constexpr uint32_t kMaxC16 = 1u << 17;
 
 // The sign bits of x(c) for the lane's columns c, two chains of shifts.
-template <class X> __device__ __forceinline__ uint32_t sign_bits(X x) {
+template <int C, class X> __device__ __forceinline__ uint32_t sign_bits(X x) {
   uint32_t lo = 0, hi = 0;
 #pragma unroll
-  for (int c = kCols / 2 - 1; c >= 0; c--) {
+  for (int c = C / 2 - 1; c >= 0; c--) {
     lo = __funnelshift_l(x(c), lo, 1);
-    hi = __funnelshift_l(x(c + kCols / 2), hi, 1);
+    hi = __funnelshift_l(x(c + C / 2), hi, 1);
   }
-  return hi << (kCols / 2) | lo;
+  return hi << (C / 2) | lo;
 }
 
 // A row into and another out of a lane's column sums and sums of squares.
-__device__ __forceinline__ void add_rows(uint32_t Vn[kCols], uint32_t Vq[kCols],
-                                         const uint32_t v[kCols], const uint32_t o[kCols]) {
+template <int C>
+__device__ __forceinline__ void add_rows(uint32_t Vn[C], uint32_t Vq[C],
+                                         const uint32_t v[C], const uint32_t o[C]) {
 #pragma unroll
-  for (int c = 0; c < kCols; c++) {
+  for (int c = 0; c < C; c++) {
     Vn[c] += v[c] - o[c];
     const uint32_t u = o[c] * o[c] - Vq[c];  // (two multiply-adds)
     Vq[c] = v[c] * v[c] - u;
   }
 }
 
-template <int K, typename Pix> constexpr size_t strip_smem() {
-  return (size_t)kStripWarps * StripG<K>::Slots * kStripStride * sizeof(Pix);
+template <int K, typename Pix, int C> constexpr size_t strip_smem() {
+  return (size_t)kStripWarps * StripG<K>::Slots * kStripStride<C> * sizeof(Pix);
 }
 
 // A valid pixel's value, 32-bit ones saturated at kCap, or a masked one's.
@@ -166,23 +172,23 @@ template <typename Pix, uint32_t kCap> __device__ __forceinline__ uint32_t pack_
   return v >= 0xFFFFFFFEu ? kMaskedPixel : min(v, kCap);
 }
 
-// A lane's 12 staged pixels, packed. 32-bit rows are packed in place when
+// A lane's staged pixels, packed. 32-bit rows are packed in place when
 // they arrive (kRaw reads them first), 16-bit rows whenever they are read.
-template <typename Pix, uint32_t kCap, bool kRaw>
-__device__ __forceinline__ void read_row(Pix *slot, int lane, uint32_t v[kCols]) {
+template <typename Pix, int C, uint32_t kCap, bool kRaw>
+__device__ __forceinline__ void read_row(Pix *slot, int lane, uint32_t v[C]) {
   if constexpr (sizeof(Pix) == 2) {
-    const uint2 *src = reinterpret_cast<const uint2 *>(slot + kCols * lane);
+    const uint2 *src = reinterpret_cast<const uint2 *>(slot + C * lane);
 #pragma unroll
-    for (int i = 0; i < kCols / 4; i++) {
+    for (int i = 0; i < C / 4; i++) {
       const uint2 x = src[i];
       v[4 * i] = pack_pixel<Pix, kCap>(x.x & 0xFFFFu), v[4 * i + 1] = pack_pixel<Pix, kCap>(x.x >> 16);
       v[4 * i + 2] = pack_pixel<Pix, kCap>(x.y & 0xFFFFu);
       v[4 * i + 3] = pack_pixel<Pix, kCap>(x.y >> 16);
     }
   } else {
-    uint4 *src = reinterpret_cast<uint4 *>(slot + kCols * lane);
+    uint4 *src = reinterpret_cast<uint4 *>(slot + C * lane);
 #pragma unroll
-    for (int i = 0; i < kCols / 4; i++) {
+    for (int i = 0; i < C / 4; i++) {
       uint4 x = src[i];
       if (kRaw) {
         x.x = pack_pixel<Pix, kCap>(x.x), x.y = pack_pixel<Pix, kCap>(x.y);
@@ -200,11 +206,12 @@ struct StripRun {
   int X, cx;      // the strip's and this lane's first column
   int ra, rb;     // output rows
   bool writer, first_of_pair;
-  int pair_byte;  // this lane's first mask byte (lane pairs share three)
-  uint32_t inside12;
+  int pair_byte;  // this lane's first mask byte (lane pairs share C / 4)
+  uint32_t inside;  // bit c: the lane's column c lies in the frame
 };
 
 // False (for the whole warp) past the last strip.
+template <int C>
 __device__ __forceinline__ bool strip_run(const FramePtrs &F, int nframes, const FrameSpans &S,
                                           int run_rows, StripRun &r) {
   const int lane = threadIdx.x & 31;
@@ -219,25 +226,24 @@ __device__ __forceinline__ bool strip_run(const FramePtrs &F, int nframes, const
   r.height = F.h[f];
   r.width = F.w[f];
   r.bytes_per_row = ((r.width + 31) >> 5) * 4;
-  r.X = kStripOut * sx;
-  r.cx = r.X + kCols * (lane - 1);
+  r.X = kStripOut<C> * sx;
+  r.cx = r.X + C * (lane - kHalo<C>);
   r.ra = ry * run_rows;
   r.rb = min(r.height, r.ra + run_rows);
-  r.writer = lane >= 1 && lane <= 30;
-  r.first_of_pair = (lane & 1) != 0;
-  r.pair_byte = (r.X + 24 * ((lane - 1) >> 1)) >> 3;
-  r.inside12 = (r.cx < 0 || r.cx >= r.width)
+  r.writer = lane >= kHalo<C> && lane < 32 - kHalo<C>;
+  r.first_of_pair = ((lane - kHalo<C>) & 1) == 0;
+  r.pair_byte = (r.X + 2 * C * ((lane - kHalo<C>) >> 1)) >> 3;
+  r.inside = (r.cx < 0 || r.cx >= r.width)
                    ? 0u
-                   : (r.cx + kCols <= r.width ? 0xFFFu : ((1u << (r.width - r.cx)) - 1u));
+                   : (r.cx + C <= r.width ? (1u << C) - 1u : ((1u << (r.width - r.cx)) - 1u));
   return true;
 }
 
 // The strip's pixel rows [pbeg, pend), fetched in turn into slots of the ring.
 // Where the frame's rows are whole aligned pieces of 4 pixels a lane copies
-// pieces l, l + 32, l + 64 (a warp's copy covers 128 pixels), else pixels a
-// lane apart. Bit u of `inside`: its u-th piece or pixel lies in the frame;
+// pieces l, l + 32 .. (a warp's copy covers 128 pixels), else pixels a lane apart. Bit u of `inside`: its u-th piece or pixel lies in the frame;
 // what lies off it is staged as masked.
-template <typename Pix> struct RowReader {
+template <typename Pix, int C> struct RowReader {
   const Pix *next_row;
   int next_p, pend, width, lane;
   uint32_t inside;
@@ -247,26 +253,26 @@ template <typename Pix> struct RowReader {
       : next_p(pbeg), pend(min(r.height, pbeg + rows)), width(r.width),
         lane(threadIdx.x & 31), inside(0) {
     aligned = width % 4 == 0 && reinterpret_cast<uintptr_t>(image) % (4 * sizeof(Pix)) == 0;
-    const int x0 = r.X - kCols;  // the staged row's first column
+    const int x0 = r.X - kHalo<C> * C;  // the staged row's first column
 #pragma unroll
-    for (int u = 0; u < kCols; u++) {
+    for (int u = 0; u < C; u++) {
       const int c = aligned ? x0 + 4 * lane + 128 * u : x0 + lane + 32 * u;
-      const bool in = aligned ? u < 3 && c >= 0 && c + 4 <= width : c >= 0 && c < width;
+      const bool in = aligned ? u < C / 4 && c >= 0 && c + 4 <= width : c >= 0 && c < width;
       inside |= in ? 1u << u : 0u;
     }
-    whole = __all_sync(0xffffffffu, aligned && inside == 7u);
+    whole = __all_sync(0xffffffffu, aligned && inside == (1u << C / 4) - 1u);
     next_row = image + (ptrdiff_t)pbeg * width + x0 + (aligned ? 4 * lane : lane);
   }
   __device__ __forceinline__ void fetch(Pix *slot) {
     const uint32_t in = next_p >= 0 && next_p < pend ? inside : 0u;
     if (whole && next_p >= 0 && next_p < pend) {
 #pragma unroll
-      for (int u = 0; u < 3; u++)
+      for (int u = 0; u < C / 4; u++)
         cp_async_piece<Pix>(slot + 4 * lane + 128 * u, next_row + 128 * u);
     } else if (aligned) {
       Pix *dst = slot + 4 * lane;
 #pragma unroll
-      for (int u = 0; u < 3; u++) {
+      for (int u = 0; u < C / 4; u++) {
         if ((in >> u) & 1u)
           cp_async_piece<Pix>(dst + 128 * u, next_row + 128 * u);
         else
@@ -275,7 +281,7 @@ template <typename Pix> struct RowReader {
     } else {
       Pix *dst = slot + lane;
 #pragma unroll
-      for (int u = 0; u < kCols; u++) {
+      for (int u = 0; u < C; u++) {
         if constexpr (sizeof(Pix) == 4) {
           if ((in >> u) & 1u)
             cp_async4(dst + 32 * u, next_row + 32 * u);
@@ -291,15 +297,21 @@ template <typename Pix> struct RowReader {
   }
 };
 
-// A lane's 12 mask bits of a row into the mask: lane pairs write three bytes,
-// the first lane (odd) two and the second the third. The whole warp calls it;
-// `row` is the row's pair_byte in a mask row that has `left` bytes from there.
+// A lane's C mask bits of a row into the mask: lane pairs write three bytes, the
+// first lane two and the second the third, or with C = 4 the first lane one.
+// The whole warp calls it; `row` is the row's pair_byte in a mask row that has
+// `left` bytes from there.
+template <int C>
 __device__ __forceinline__ void write_bits(const StripRun &r, uint8_t *row, int left,
                                            uint32_t bits) {
+  static_assert(C == kWideCols || C == kNarrowCols, "whole bytes a lane pair");
   const uint32_t next = __shfl_down_sync(0xffffffffu, bits, 1);
   if (!r.writer)
     return;
-  if (r.first_of_pair) {
+  if (C == kNarrowCols) {
+    if (r.first_of_pair && left > 0)
+      row[0] = (uint8_t)(bits | next << C);
+  } else if (r.first_of_pair) {
     if (left > 0)
       row[0] = (uint8_t)bits;
     if (left > 1)
@@ -310,24 +322,24 @@ __device__ __forceinline__ void write_bits(const StripRun &r, uint8_t *row, int 
 }
 
 // The column sums V of a lane and, by shuffles, of the K columns either side
-// of its own, summed over the 2K + 1 columns around each of the 12.
-template <int K>
-__device__ __forceinline__ void window_sums(const uint32_t V[kCols], uint32_t h[kCols]) {
-  uint32_t e[kCols + 2 * K];
+// of its own, summed over the 2K + 1 columns around each of its own.
+template <int K, int C>
+__device__ __forceinline__ void window_sums(const uint32_t V[C], uint32_t h[C]) {
+  uint32_t e[C + 2 * K];
 #pragma unroll
-  for (int c = 0; c < kCols; c++)
+  for (int c = 0; c < C; c++)
     e[K + c] = V[c];
 #pragma unroll
   for (int k = 0; k < K; k++) {
-    e[k] = __shfl_up_sync(0xffffffffu, V[kCols - K + k], 1);
-    e[K + kCols + k] = __shfl_down_sync(0xffffffffu, V[k], 1);
+    e[k] = __shfl_up_sync(0xffffffffu, V[C - K + k], 1);
+    e[K + C + k] = __shfl_down_sync(0xffffffffu, V[k], 1);
   }
   h[0] = 0u;
 #pragma unroll
   for (int k = 0; k <= 2 * K; k++)
     h[0] += e[k];
 #pragma unroll
-  for (int c = 1; c < kCols; c++)
+  for (int c = 1; c < C; c++)
     h[c] = h[c - 1] + e[c + 2 * K] - e[c - 1];
 }
 
@@ -344,7 +356,9 @@ constexpr int kMinRunRows = 2;
 constexpr int kLongRun = 64;
 constexpr int kStripWaves = 4;
 
-inline int strips_of(int w) { return ((w + 31) / 32 * 32 + kStripOut - 1) / kStripOut; }
+template <int C> inline int strips_of(int w) {
+  return ((w + 31) / 32 * 32 + kStripOut<C> - 1) / kStripOut<C>;
+}
 
 inline int strip_run_rows(int tallest, long long strips, int slots, int run_rows) {
   if (run_rows <= 0) {
@@ -355,18 +369,31 @@ inline int strip_run_rows(int tallest, long long strips, int slots, int run_rows
   return std::max(run_rows, kMinRunRows);
 }
 
+// Whether a launch takes narrow strips: where wide ones would fill `slots` resident
+// warps with runs of fewer than kNarrowRun rows, and a warp's walk sets its time.
+// (Wide and narrow, kernel 4 in a captured graph: one frame of 1065 x 1030, 2 rows,
+// 40 and 34 us; of 2162 x 2068, 7 rows, 45 and 44; two of those 56 and 60.)
+constexpr int kNarrowRun = 8;
+inline bool narrow_strips(const FramePtrs &F, int nframes, int slots) {
+  long long rows = 0;
+  for (int f = 0; f < nframes; f++)
+    rows += (long long)strips_of<kWideCols>(F.w[f]) * F.h[f];
+  return rows < (long long)kNarrowRun * slots;
+}
+
+template <int C>
 inline int strip_spans(const FramePtrs &F, int nframes, int slots, int run_rows, FrameSpans *S) {
   long long strips = 0;
   int tallest = 0;
   for (int f = 0; f < nframes; f++) {
-    strips += strips_of(F.w[f]);
+    strips += strips_of<C>(F.w[f]);
     tallest = std::max(tallest, F.h[f]);
   }
   run_rows = strip_run_rows(tallest, strips, slots, run_rows);
   S->start[0] = 0;
   for (int f = 0; f < nframes; f++) {
-    S->start[f + 1] = S->start[f] + strips_of(F.w[f]) * ((F.h[f] + run_rows - 1) / run_rows);
-    S->by_row[f] = make_fastdiv((uint32_t)strips_of(F.w[f]));
+    S->start[f + 1] = S->start[f] + strips_of<C>(F.w[f]) * ((F.h[f] + run_rows - 1) / run_rows);
+    S->by_row[f] = make_fastdiv((uint32_t)strips_of<C>(F.w[f]));
   }
   return run_rows;
 }

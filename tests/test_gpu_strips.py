@@ -70,12 +70,13 @@ def test_strips_against_oracle(h, w, kernel, bits, algorithm):
 
 
 @pytest.mark.parametrize("top", [7281, 9361, 9362, 13107, (1 << 20) - 1, 1 << 20, 1 << 22])
+@pytest.mark.parametrize("algorithm", [0, 1])
 @pytest.mark.parametrize("kernel", [2, 3, 4])
 @pytest.mark.parametrize("h,w", [(24, 84), (37, 361), (90, 412)])
-def test_large_counts_against_oracle(h, w, kernel, top):
+def test_large_counts_against_oracle(h, w, kernel, algorithm, top):
     """Frames whose largest pixel is just below or at the counts where a strip's
-    rows and a tile's check change their sums: spots and flat fields of that count, with and without
-    masked pixels beside them."""
+    rows and a tile's check change their sums: spots and flat fields of that
+    count, with and without masked pixels beside them."""
     import torch
     from sfgb import api
     rng = np.random.default_rng(h + top)
@@ -95,7 +96,7 @@ def test_large_counts_against_oracle(h, w, kernel, top):
         frames.append(g)
     for kw in (dict(), dict(sigma_b=2.0, sigma_s=1.0, min_local=5), dict(sigma_b=0.0, sigma_s=0.0),
                dict(gain=1.5, sigma_b=2.5)):
-        p = dict(algorithm=1, kernel_x=kernel, kernel_y=kernel, **kw)
+        p = dict(algorithm=algorithm, kernel_x=kernel, kernel_y=kernel, **kw)
         b = api.DeviceBatch(h, w, len(frames), capacity=h * w, params=api.Params(**p))
         b([torch.from_numpy(f.view(np.int32)).cuda() for f in frames])
         for j, f in enumerate(frames):
