@@ -1146,7 +1146,8 @@ size_t lattice_tiles(int h, int w) { return (size_t)ver_ntx(w) * (size_t)ver_nty
 // have `strips` strips in all, unless run_rows is given, in whole triples of
 // rows: the resident warps filled kLatWaves times over by runs of at least
 // kLatLongRun rows (each reads 9 rows more than it writes), so that warps of
-// unequal speed even out; else once, down to runs of kLatMinRunRows.
+// unequal speed even out (32 frames of 4362 x 4148: 424 us, 447 with three times
+// and 144 rows); else once, down to runs of kLatMinRunRows.
 static int lat_run_rows(int h, long long strips, int run_rows) {
   if (run_rows <= 0) {
     const long long nruns = std::max(1ll, (long long)lat_slots() / std::max(1ll, strips));

@@ -40,7 +40,7 @@ struct StreamTables {
 
 // The lattice pass for kernel 3,3 (sf_lattice.cu): strips of 360 output
 // columns (one warp each) by runs of run_rows rows, a multiple of 3.
-constexpr int kLatMinRunRows = 9, kLatLongRun = 144, kLatWaves = 3;
+constexpr int kLatMinRunRows = 9, kLatLongRun = 96, kLatWaves = 5;
 struct LatticeGeometry {
   int nstrips, nruns, run_rows;
 };
