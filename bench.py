@@ -52,19 +52,18 @@ H, W = 4362, 4148
 
 
 # DRAM bytes (read + write) that one 16M frame of the eiger_16m workload costs
-# across the threshold's kernels in a timed 64-frame launch, from an ncu
-# capture of this bench without cache flushes between kernels (11,235 MB for
-# the launch: lat_stage01 5,266 MB, lat_verify 2,098 MB, lat_stage2 2,621 MB,
-# the scans and the list 1,250 MB); the algorithmic bytes are 76.5 MB a frame.
-DRAM_BYTES_PER_FRAME = 162.0e6
+# across the threshold's kernels, from an ncu capture of a 32-frame launch
+# without cache flushes between kernels (4,826 MB for the launch: lat_stage01
+# 2,577 MB, lat_tiles 73 MB, lat_verify 1,015 MB, ext_decide 827 MB,
+# scatter_pixels 334 MB); the algorithmic bytes are 76.5 MB a frame.
+DRAM_BYTES_PER_FRAME = 150.8e6
 
 
 # Kernels a timed step launches: the threshold plan's graph (lat_stage01,
-# lat_tiles, lat_verify, mask_sums, mask_prefix, lat_stage2, pass_sums,
-# pass_scatter) and the labeller's (27 kernels and six three-kernel
-# exclusive scans; sf_label.cu, Labeller::enqueue).
-THRESHOLD_KERNELS = 8
-LABEL_KERNELS = 45
+# lat_tiles, lat_verify, ext_decide, scatter_pixels) and the labeller's
+# (sf_label.cu, Labeller::enqueue: 13 kernels and three two-kernel scans).
+THRESHOLD_KERNELS = 5
+LABEL_KERNELS = 19
 
 
 def dist_env():
@@ -1013,7 +1012,7 @@ def run_ours(args):
             traffic = DRAM_BYTES_PER_FRAME * B
             traffic_source = (
                 "ncu dram__bytes_read.sum + dram__bytes_write.sum of one timed 32-frame launch "
-                "of this workload (32 frames in HBM), one capture a kernel for its 8 kernels, no "
+                "of this workload (32 frames in HBM), one capture a kernel for its 5 kernels, no "
                 "cache flush between kernels "
                 f"({DRAM_BYTES_PER_FRAME / 1e6:.1f} MB a frame), times the {B} frames of a launch; "
                 "a frame's traffic grows a little with the batch")
@@ -1035,9 +1034,8 @@ def run_ours(args):
                          "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind,
                          "kernel": "threshold launch sequence of a batch (lat_stage01, "
-                                   "lat_tiles, lat_verify, mask_sums, mask_prefix, lat_stage2, "
-                                   "pass_sums, pass_scatter) replayed as one CUDA graph, "
-                                   "CUDA events around each batch",
+                                   "lat_tiles, lat_verify, ext_decide, scatter_pixels) replayed "
+                                   "as one CUDA graph, CUDA events around each batch",
                          "algorithmic_bytes_per_launch": algo_bytes,
                          "launch_ms": launch_ms, "traffic": traffic,
                          "traffic_source": traffic_source},

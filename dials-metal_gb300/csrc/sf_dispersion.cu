@@ -55,11 +55,11 @@ __device__ __forceinline__ bool disp_float2(uint32_t p, uint32_t n, uint32_t S,
 // The walk of sf_strips.cuh: a lane adds each row to its 12 column sums as it
 // enters the window, subtracts it as it leaves, and reads it once more as the
 // centre row; a window is 2K + 1 column sums.
-// Bound by issue: 40 instructions a pixel at 66% of the issue rate. 16 frames of
+// Bound by issue: 39 instructions a pixel at 66% of the issue rate. 16 frames of
 // 3262 x 3108 took 4.57 ms as 32 x 32 tiles (each pixel's window summed in
-// 64 bits from shared memory, the halo staged 2.6 times over), and take 0.39 ms
-// here: 282 us in this kernel (344 with both tests compared, selected and ORed,
-// 437 with branches around their halves), 70 and 30 in the two below.
+// 64 bits from shared memory, the halo staged 2.6 times over), and take 0.37 ms
+// here: 271 us in this kernel (344 with both tests compared, selected and ORed,
+// 437 with branches around their halves), 79 and 30 in the two below.
 template <int K, typename Pix, int C>
 __global__ void __launch_bounds__(kStripWarps * 32, StripG<K>::Occ)
 disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constant__ FrameSpans S,

@@ -138,8 +138,8 @@ __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image
 // The stage-0 bits of the 12 windows of a lane whose newest row is the ring's
 // slot s, for rows whose windows may hold a pixel of Cap or more: the columns'
 // sums again from the ring's rows, squares in 64 bits, and the 2^-8 tests in 64
-// bits; by ext_wide_row where one of the warp's pixels is kLargePixel or more. (Two dense frames of 353 x 944 at kernel 4,
-// every row of them so, take 80 us in all, 272 with every such row by
+// bits; by ext_wide_row where one of the warp's pixels is kLargePixel or more.
+// (Two dense frames of 353 x 944 at kernel 4, every row of them so, take 80 us in all, 272 with every such row by
 // ext_wide_row; 16 of 2162 x 2068 at kernel 2 take 0.97 ms.)
 template <int K, int C>
 __device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int lane,
@@ -235,7 +235,8 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
       rows_tab[n].a = make_uint4(__float_as_uint((float)n), __float_as_uint(root), 0u, 0u);
       rows_tab[n].b = make_uint4(0u, 0u, 0u, 0u);
     } else {
-      rows_tab[n].a = make_uint4(0u - (T.nk[n] >> 4), T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
+      rows_tab[n].a =
+          make_uint4(0u - (T.nk[n] >> 4), T.clo16[n], T.chi16[n] - T.clo16[n], (uint32_t)n);
       rows_tab[n].b = make_uint4(T.nk[n], T.clo[n], T.chi[n], 0u);
     }
   }
@@ -465,14 +466,14 @@ constexpr uint32_t kHeavyRun = 48;  // candidates of a run that is taken early
 // columns whose windows 32 columns cover, for all 8 rows (a spot's candidates
 // are about 7 x 7). The chunk's pixels are read once, a lane a column, added up
 // over the window's rows into shared memory; then its candidates are spread
-// over the lanes, each adding up its window's columns for the test. A
-// block first lists the runs of its bands that hold a candidate, four a warp on
+// over the lanes, each adding up its window's columns for the test. A block
+// first lists the runs of its bands that hold a candidate, four a warp on
 // their way at once; its warps then take them in turn, those with many candidates
 // first, so that they even out. Bound by issue: 32 frames of 4362 x 4148 (174
 // thousand candidates each) take 266 us, 290 with the runs taken in order, the
-// empty ones among them, each read when its turn came (one frame 19 and 22). A window a candidate, four lanes each,
-// took 568 us, chunks of one row 427, and tests row by row, only the row's
-// candidates' lanes busy, 553.
+// empty ones among them, each read when its turn came (one frame 19 and 22). A
+// window a candidate, four lanes each, took 568 us, chunks of one row 427, and
+// tests row by row, only the row's candidates' lanes busy, 553.
 template <int K, typename Pix>
 __global__ void __launch_bounds__(kScanT, 4)
 ext_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchParams P,

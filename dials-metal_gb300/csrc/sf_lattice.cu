@@ -795,7 +795,8 @@ __global__ void __launch_bounds__(kVerWarps * 32, kOcc)
 lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps M, int env_h,
            int env_w, const __grid_constant__ LaunchParams P,
            const __grid_constant__ StreamTables T, uint32_t *__restrict__ final_all, size_t words,
-           const uint32_t *list, uint32_t *__restrict__ counters, FastDiv by_ntiles, FastDiv by_ntx) {
+           const uint32_t *list, uint32_t *__restrict__ counters, FastDiv by_ntiles,
+           FastDiv by_ntx) {
   previous_done();
   extern __shared__ __align__(128) unsigned char ver_smem_raw[];
   // The launch gives 128 bytes more than the layout needs: the tile buffers

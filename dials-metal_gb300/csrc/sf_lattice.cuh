@@ -11,8 +11,8 @@
 //   2^8 n Q >= S (2^8 S + chi) + 2^9     =>  A >= X + 2 > RN(X): signal
 // both exact in 64-bit integers. The thin band between goes to the exact
 // decision of sf_common.cuh. The packed sums (the window's masked-pixel count above
-// a 26-bit sum) and the 32-bit sum of squares hold while every valid pixel is below narrow_max; a tile holding a
-// larger valid pixel is decided in 64 bits.
+// a 26-bit sum) and the 32-bit sum of squares hold while every valid pixel is below
+// narrow_max; a tile holding a larger valid pixel is decided in 64 bits.
 #pragma once
 
 #include <cuda_runtime.h>

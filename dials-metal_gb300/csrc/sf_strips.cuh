@@ -128,8 +128,8 @@ template <int K> struct StripG {
   static constexpr int Slots = W0 + Ahead + 1;
   static constexpr int Occ = K == 2 ? 8 : K == 3 ? 7 : 6;
   // Valid 32-bit pixels saturate at Cap, or rows whose windows hold a larger one
-  // are summed apart, so that a window's sum of squares stays below 2^32. Below Big a window's sum S is below sqrt(N0 Big) = 2^13,
-  // and both sides of the 32-bit tests (16 n Q; S (16 S + c) + 32, c < kMaxC16)
+  // are summed apart, so that a window's sum of squares stays below 2^32. Below Big
+  // a window's sum S is below sqrt(N0 Big) = 2^13, and both sides of the 32-bit tests (16 n Q; S (16 S + c) + 32, c < kMaxC16)
   // below 2^31: their difference's sign bit is the decision.
   static constexpr uint32_t Cap = K == 2 ? 13107 : K == 3 ? 9362 : 7281;
   static constexpr uint32_t Big = (1u << 26) / N0;
@@ -181,7 +181,8 @@ __device__ __forceinline__ void read_row(Pix *slot, int lane, uint32_t v[C]) {
 #pragma unroll
     for (int i = 0; i < C / 4; i++) {
       const uint2 x = src[i];
-      v[4 * i] = pack_pixel<Pix, kCap>(x.x & 0xFFFFu), v[4 * i + 1] = pack_pixel<Pix, kCap>(x.x >> 16);
+      v[4 * i] = pack_pixel<Pix, kCap>(x.x & 0xFFFFu);
+      v[4 * i + 1] = pack_pixel<Pix, kCap>(x.x >> 16);
       v[4 * i + 2] = pack_pixel<Pix, kCap>(x.y & 0xFFFFu);
       v[4 * i + 3] = pack_pixel<Pix, kCap>(x.y >> 16);
     }
