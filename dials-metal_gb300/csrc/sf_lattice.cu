@@ -347,7 +347,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
 // mask words, so the clearing is an atomic AND; each candidate belongs to one
 // tile, so the order does not matter. Bound by issue (64% of its rate, 820
 // instructions a tile): 32 frames of 4362 x 4148 take 297 us, 148 of 16 bits, 4
-// dense ones 783; with a lane a column for the windows too, each lane taking its
+// dense ones 621; with a lane a column for the windows too, each lane taking its
 // column's needed ones in turn (11 rounds a tile, 12 lanes in them), and the
 // erosion a row after another in every lane, 449, 250 and 967 us.
 // ---------------------------------------------------------------------------
@@ -710,8 +710,8 @@ __device__ __forceinline__ uint32_t ver_group(const VerWarp<uint16_t> &sm, int d
 // A tile that holds a valid pixel too large for the 32-bit sums but below
 // kWidePixel: its column sums again, the masked count above a 28-bit sum and the
 // sum of squares in 48 bits. (A launch of 4 dense frames of 4362 x 4148, whose
-// tiles nearly all hold an overload, takes less than half of what summing each
-// window's 49 pixels took: 2136 us.)
+// tiles nearly all hold an overload, takes 621 us: 783 with the 32-bit sums taken
+// first there too, 2136 summing each window's 49 pixels.)
 constexpr uint32_t kWidePixel = 1u << 20;
 constexpr int kWideCount = 28;
 static_assert((2 * kLatK + 1) * (kWidePixel - 1) < (1u << kWideCount) &&
@@ -722,35 +722,39 @@ static_assert((2 * kLatK + 1) * (kWidePixel - 1) < (1u << kWideCount) &&
 static_assert(49ull * 49ull * (kWidePixel - 1) * (kWidePixel - 1) < (1ull << 53),
               "a window's sums are exact in double");
 
-__device__ __noinline__ void ver_wide_columns(VerWarp<uint32_t> &sm, int off, int npass,
-                                              int lane) {
+// Returns the lane's largest valid pixel.
+__device__ __noinline__ uint32_t ver_wide_columns(VerWarp<uint32_t> &sm, int off, int npass,
+                                                  int lane) {
+  uint32_t top = 0;
   for (int pass = 0; pass < npass; pass++) {
     const int i = 32 * pass + lane;
     if (i >= kVerPC)
       break;
-    uint32_t cs = 0;  // count and sum
+    uint32_t u[kVerPR], masked = 0, cs = 0;  // (cs: count and sum)
     unsigned long long cq = 0;
-    uint32_t mk = 0;
 #pragma unroll
     for (int r = 0; r < kVerPR; r++) {
       const uint32_t v = sm.pix[0].px[r][off + i];
-      const uint32_t u = is_masked_px<uint32_t>(v) ? 0u : v;
-      cs += is_masked_px<uint32_t>(v) ? 1u << kWideCount : v;
-      cq += (unsigned long long)u * u;
-      if (r >= kLatK && r < kLatK + kVerDR)
-        mk |= is_masked_px<uint32_t>(v) ? 1u << (r - kLatK) : 0u;
+      const bool m = is_masked_px<uint32_t>(v);
+      masked |= m ? 1u << r : 0u;
+      u[r] = m ? 0u : v;
+      top = max(top, u[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < kVerPR; r++) {
+      cs += u[r] + ((masked >> r & 1u) << kWideCount);
+      cq += (unsigned long long)u[r] * u[r];
       if (r >= 2 * kLatK) {
         const int d = r - 2 * kLatK;
         sm.vs[d][i] = make_uint2(cs, (uint32_t)cq);
         sm.vh[d][i] = (uint16_t)(cq >> 32);
-        const uint32_t o = sm.pix[0].px[d][off + i];
-        const uint32_t w = is_masked_px<uint32_t>(o) ? 0u : o;
-        cs -= is_masked_px<uint32_t>(o) ? 1u << kWideCount : o;
-        cq -= (unsigned long long)w * w;
+        cs -= u[d] + ((masked >> d & 1u) << kWideCount);
+        cq -= (unsigned long long)u[d] * u[d];
       }
     }
-    sm.msk[i + 1] = mk;
+    sm.msk[i + 1] = masked >> kLatK;  // (rows past the centres' are not looked at)
   }
+  return top;
 }
 
 // ver_group from those sums: the same two bounds in 64 bits, then the reference's
@@ -886,23 +890,32 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     // masked centres, the largest valid pixel, and the column sums of 7
     // rows for the 12 stage-0 rows (exact in 32 bits unless the tile holds a
     // valid pixel at or above narrow_max, which the check below catches).
-    uint32_t mx = 0, masked = 0;
+    // (A tile with a larger one leaves this for the wide sums at once.)
+    uint32_t masked = 0;
+    bool wide = false;
 #pragma unroll
     for (int pass = 0; pass < 2; pass++) {
       if (pass == npass)
         break;  // warp-uniform
-      if (pass == 1 && lane >= kVerPC - 32)
-        break;
-      const int col = off + 32 * pass + lane;
-      uint32_t ns[kVerPR], q[kVerPR], mk = 0;
+      const bool on = pass == 0 || lane < kVerPC - 32;
+      const int col = off + 32 * pass + (on ? lane : 0);
+      uint32_t ns[kVerPR], q[kVerPR], mk = 0, mx = 0;
 #pragma unroll
       for (int r = 0; r < kVerPR; r++) {
         const uint32_t v = sm.pix[0].px[r][col];
         if (!k16)
           mx = max(mx, v + 2u);
         ns[r] = is_masked_px<Pix>(v) ? (1u << kLatPS) : v;
-        q[r] = ns[r] * ns[r];
       }
+      if (!k16 && __any_sync(0xffffffffu, mx >= narrow2)) {
+        wide = true;
+        break;  // warp-uniform
+      }
+      if (!on)
+        break;
+#pragma unroll
+      for (int r = 0; r < kVerPR; r++)
+        q[r] = ns[r] * ns[r];
       // A valid pixel below narrow_max (2^14) leaves nothing of itself when
       // its count bit is shifted down; a 16-bit one may.
 #pragma unroll
@@ -928,11 +941,11 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     }
     __syncwarp();
     // 16-bit frames sum in 32 bits as the reference does: never wide.
-    const bool wide = !k16 && __any_sync(0xffffffffu, mx >= narrow2);
-    const bool huge = !k16 && wide && __any_sync(0xffffffffu, mx >= kWidePixel + 2u);
+    bool huge = false;
     if constexpr (!k16) {
-      if (wide && !huge) {
-        ver_wide_columns(sm, off, npass, lane);
+      if (wide) {
+        const uint32_t top = ver_wide_columns(sm, off, npass, lane);
+        huge = __any_sync(0xffffffffu, top >= kWidePixel);
         __syncwarp();
       }
     }
