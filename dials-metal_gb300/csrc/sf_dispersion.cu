@@ -357,7 +357,7 @@ disp_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchP
                                       (uint32_t)__ldg(image + (size_t)y * width + x), n, S, Q, P);
                       const unsigned pass = __ballot_sync(0xffffffffu, ok);
                       const uint32_t at = passed + __popc(pass & ((1u << lane) - 1u));
-                      if (ok && at < min(32u, end - run0) * kept.keep)
+                      if (ok && at < group_places(kept, run0, end))
                         res[at] =
                             make_uint2(__float_as_uint(window_mean<Pix>(n, S, P.min_local)), n);
                       if (mine && !ok)

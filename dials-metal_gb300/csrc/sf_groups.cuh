@@ -83,6 +83,13 @@ inline Kept make_kept(const StreamBuffers &b, int h, int w) {
           (uint32_t)(b.res_stride / ((size_t)h * (size_t)runs_per_row(w)))};
 }
 
+// The places of a warp's group of runs [run0, min(run0 + 32, end)) whose results are
+// kept together: what lies beyond belongs to the next group. (The last group of a
+// block's bands is mostly a partial one: 8 of the 72 runs of a band 1030 wide.)
+__device__ __forceinline__ uint32_t group_places(const Kept &kept, uint32_t run0, uint32_t end) {
+  return min(32u, end - run0) * kept.keep;
+}
+
 // The window's mean as the records hold it: float(RN_double(S / n)) is
 // RN_float(S / n) for S below 2^24 (sf_common.cuh), and 16-bit frames divide in
 // float. A window short of valid pixels has the mean 0 (dext.cc:204).
@@ -280,7 +287,7 @@ scatter_pixels(const __grid_constant__ FramePtrs F, const uint32_t *bits_all, si
     visit_pixels<1>(r, incl, lane,
                     [&](bool live, uint32_t q, uint32_t rank, int owner, int, int, int y, int x) {
                       const uint32_t index = (uint32_t)y * (uint32_t)width + (uint32_t)x;
-                      const uint32_t held = kByRun ? kept.keep : 32u * kept.keep;
+                      const uint32_t held = kByRun ? kept.keep : group_places(kept, run0, end);
                       const uint32_t place = kByRun ? rank : q;
                       const size_t at =
                           (size_t)(run0 + (kByRun ? (uint32_t)owner : 0u)) * kept.keep + place;
