@@ -495,6 +495,7 @@ ext_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchPa
   uint2 *res = kept.res + (size_t)f * kept.stride;
   if (threadIdx.x < 2)
     s_count[threadIdx.x] = 0u;
+  __syncthreads();  // (a block without rows comes to no other barrier before the counts)
   int row_lo, row_hi;
   band_share(height, &row_lo, &row_hi);
   const uint32_t items = (uint32_t)((row_hi - row_lo + kBandRows - 1) / kBandRows) * rpr;
