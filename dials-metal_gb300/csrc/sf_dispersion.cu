@@ -318,8 +318,150 @@ __device__ __forceinline__ bool disp_strong(uint32_t p, uint32_t n, unsigned lon
   }
 }
 
+// The windows' sums of a lane's four columns from its own column sums and those of
+// the K columns either side: its neighbours', and at the run's ends the halo's (lane
+// j < K holds that of the run's j-th column before, lane K + j of its j-th after).
+template <int K>
+__device__ __forceinline__ void run_windows(const unsigned long long col[4],
+                                            unsigned long long halo, int lane,
+                                            unsigned long long win[4]) {
+  unsigned long long e[4 + 2 * K];
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+    e[K + c] = col[c];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const unsigned long long l = __shfl_up_sync(0xffffffffu, col[4 - K + k], 1),
+                             hl = __shfl_sync(0xffffffffu, halo, k),
+                             r = __shfl_down_sync(0xffffffffu, col[k], 1),
+                             hr = __shfl_sync(0xffffffffu, halo, K + k);
+    e[k] = lane == 0 ? hl : l;
+    e[K + 4 + k] = lane == 31 ? hr : r;
+  }
+  win[0] = 0ull;
+#pragma unroll
+  for (int k = 0; k <= 2 * K; k++)
+    win[0] += e[k];
+#pragma unroll
+  for (int c = 1; c < 4; c++)
+    win[c] = win[c - 1] + e[c + 2 * K] - e[c - 1];
+}
+
+// One run's candidates decided by the whole warp, four columns a lane (`cand` the
+// lane's four bits): every window's sums, from the columns' sums over its rows.
+// Returns the lane's passing bits and fills their results.
+constexpr int kPackedN = 48;  // a sum's valid pixels above it: 81 x 2^32 is below 2^39
 template <int K, typename Pix>
-__global__ void __launch_bounds__(kScanT)
+__device__ __forceinline__ uint32_t disp_dense_run(const Pix *__restrict__ image, int height,
+                                                   int width, int y, int x0, uint32_t cand,
+                                                   const LaunchParams &P, uint2 *mine) {
+  const int lane = threadIdx.x & 31, x = x0 + 4 * lane;
+  const int xh = lane < K ? x0 - K + lane : x0 + 128 + (lane - K);  // the halo column, lanes < 2K
+  const bool has_halo = lane < 2 * K && xh >= 0 && xh < width;
+  unsigned long long s[4] = {0, 0, 0, 0}, q[4] = {0, 0, 0, 0}, hs = 0, hq = 0;
+  uint32_t centre[4] = {0, 0, 0, 0};
+  auto add = [](uint32_t v, unsigned long long &sum, unsigned long long &sq) {
+    const bool ok = v < Traits<Pix>::kMasked;
+    sum += ok ? (1ull << kPackedN) + v : 0ull;
+    sq += ok ? (unsigned long long)v * v : 0ull;
+  };
+#pragma unroll 3
+  for (int d = -K; d <= K; d++) {
+    const bool in = y + d >= 0 && y + d < height;  // warp-uniform
+    const Pix *row = image + (ptrdiff_t)(y + d) * width;
+    uint32_t v[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      v[c] = in && x + c < width ? (uint32_t)__ldg(row + x + c) : Traits<Pix>::kMasked;
+    const uint32_t vh = in && has_halo ? (uint32_t)__ldg(row + xh) : Traits<Pix>::kMasked;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      add(v[c], s[c], q[c]);
+      centre[c] = d == 0 ? v[c] : centre[c];
+    }
+    add(vh, hs, hq);
+  }
+  unsigned long long ws[4], wq[4];
+  run_windows<K>(s, hs, lane, ws);
+  run_windows<K>(q, hq, lane, wq);
+  uint32_t pass = 0;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const uint32_t n = (uint32_t)(ws[c] >> kPackedN);
+    const unsigned long long S = ws[c] & ((1ull << kPackedN) - 1ull);
+    if ((cand >> c & 1u) && disp_strong<Pix>(centre[c], n, S, wq[c], P)) {
+      pass |= 1u << c;
+      mine[c] = make_uint2(__float_as_uint(window_mean<Pix>(n, S, P.min_local)), n);
+    }
+  }
+  return pass;
+}
+
+// Whether a group of runs that holds `all` candidates is taken run by run, all
+// windows of a run at once, instead of candidate by candidate. (Frames whose
+// background reaches the strips' saturation are candidates everywhere: 4 of 3262 x
+// 3108 with 15,000 counts a pixel take 0.63 ms so at kernel 3 and 4.03 the other
+// way; with a third of the pixels strong 0.87 and 1.30; with a fifth 1.13 and 0.90,
+// where the line of 40 leaves them.) Those groups come after the warp's others: the
+// call in their midst cost frames without any 1%.
+constexpr uint32_t kDenseRun = 40;  // candidates a run of 128 pixels
+__device__ __forceinline__ bool dense_group(uint32_t all, uint32_t run0, uint32_t end) {
+  return all >= kDenseRun * min(32u, end - run0);
+}
+
+// The dense groups of a warp (its groups start at first, first + kScanT, ..): as
+// disp_decide's own loop. Returns the number of passing pixels.
+template <int K, typename Pix>
+__device__ __noinline__ uint32_t disp_dense_groups(const Pix *__restrict__ image, int height,
+                                                   int width, uint32_t first, uint32_t end,
+                                                   const LaunchParams &P, uint32_t *bits,
+                                                   const Kept &kept, uint2 *res_all) {
+  const int lane = threadIdx.x & 31, shift = (lane & 7) * 4;
+  const uint32_t wpr = ((uint32_t)width + 31u) >> 5, rpr = (uint32_t)runs_per_row(width);
+  uint32_t count = 0;
+  for (uint32_t run0 = first; run0 < end; run0 += kScanT) {
+    const LaneRun r = load_run(bits, run0 + lane, end, rpr, wpr);
+    if (!dense_group(__reduce_add_sync(0xffffffffu, run_pixels(r)), run0, end))
+      continue;  // whole warp
+    uint2 *res = res_all + (size_t)run0 * kept.keep;
+    const uint32_t places = group_places(kept, run0, end);
+    uint32_t passed = 0;
+    for (uint32_t run = run0; run < min(end, run0 + 32u); run++) {
+      // The run's word of this lane's columns.
+      const uint32_t y = run / rpr, word = (run - y * rpr) * kRunWords + (uint32_t)(lane >> 3);
+      uint32_t *at_word = bits + (size_t)y * wpr + word;
+      const uint32_t w = word < wpr ? *at_word : 0u;
+      if (!__any_sync(0xffffffffu, w != 0u))
+        continue;  // whole warp
+      uint2 mine[4];
+      const uint32_t pass = disp_dense_run<K, Pix>(
+          image, height, width, (int)y, (int)((run - y * rpr) * kRunWords * 32u),
+          w >> shift & 15u, P, mine);
+      const uint32_t upto = warp_inclusive((uint32_t)__popc(pass), lane);
+      uint32_t at = passed + upto - (uint32_t)__popc(pass);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        if (pass >> c & 1u) {
+          if (at < places)
+            res[at] = mine[c];
+          at++;
+        }
+      }
+      passed += __shfl_sync(0xffffffffu, upto, 31);
+      uint32_t left = pass << shift;
+      left |= __shfl_xor_sync(0xffffffffu, left, 1);
+      left |= __shfl_xor_sync(0xffffffffu, left, 2);
+      left |= __shfl_xor_sync(0xffffffffu, left, 4);
+      if ((lane & 7) == 0 && left != w)
+        *at_word = left;
+    }
+    count += passed;
+  }
+  return count;
+}
+
+template <int K, typename Pix>
+__global__ void __launch_bounds__(kScanT, 4)
 disp_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchParams P,
             uint32_t *__restrict__ bits_all, size_t words, Kept kept,
             uint32_t *__restrict__ block_sums) {
@@ -332,13 +474,19 @@ disp_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchP
   uint32_t *bits = bits_all + (size_t)f * words;
   int row_lo, row_hi;
   band_share(height, &row_lo, &row_hi);
+  const uint32_t first = (uint32_t)row_lo * rpr + (uint32_t)warp * 32u;
   const uint32_t end = (uint32_t)row_hi * rpr;
   uint32_t count = 0;
-  for (uint32_t run0 = (uint32_t)row_lo * rpr + (uint32_t)warp * 32u; run0 < end;
-       run0 += kScanT) {
+  bool dense = false;  // a group is left for disp_dense_groups
+  for (uint32_t run0 = first; run0 < end; run0 += kScanT) {
     const LaneRun r = load_run(bits, run0 + lane, end, rpr, wpr);
     const uint32_t incl = warp_inclusive(run_pixels(r), lane);
-    if (__shfl_sync(0xffffffffu, incl, 31) == 0)
+    const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+    if (dense_group(all, run0, end)) {
+      dense = true;
+      continue;  // whole warp
+    }
+    if (all == 0)
       continue;  // whole warp
 #pragma unroll
     for (int k = 0; k < kRunWords; k++)
@@ -372,6 +520,12 @@ disp_decide(const __grid_constant__ FramePtrs F, const __grid_constant__ LaunchP
         bits[(size_t)r.y * wpr + r.word + k] = r.w[k] & ~clear;
     }
     __syncwarp();
+    count += lane == 0 ? passed : 0u;
+  }
+  if (dense) {  // whole warp
+    const uint32_t passed =
+        disp_dense_groups<K, Pix>(image, height, width, first, end, P, bits, kept,
+                                  kept.res + (size_t)f * kept.stride);
     count += lane == 0 ? passed : 0u;
   }
   uint32_t total;
