@@ -80,58 +80,78 @@ struct ExtRow {
   uint4 a, b;
 };
 
-// The stage-0 bits (signal or masked; off the frame counts as set) of the 12
-// windows centred on row y, columns cx ..: from 64-bit sums of the frame's
-// pixels, for rows whose windows may hold a pixel too large for the strip's
-// sums. A column's sums of 2K + 1 rows enter as the windows move right and
-// leave again; a window off the frame is clipped as the reference's is.
+// A lane's 64-bit column sums, and by shuffles those of the K columns either side of
+// its own, summed over the 2K + 1 columns around each of its own, in place.
+template <int K, int C> __device__ __forceinline__ void wide_sums(unsigned long long v[C]) {
+  unsigned long long e[C + 2 * K], h = 0;
+#pragma unroll
+  for (int c = 0; c < C; c++)
+    e[K + c] = v[c];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    e[k] = __shfl_up_sync(0xffffffffu, v[C - K + k], 1);
+    e[K + C + k] = __shfl_down_sync(0xffffffffu, v[k], 1);
+  }
+#pragma unroll
+  for (int k = 0; k < 2 * K; k++)
+    h += e[k];
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    h += e[c + 2 * K];
+    v[c] = h;
+    h -= e[c];
+  }
+}
+
+// The stage-0 bits of the windows centred on row y, columns cx ..: from 64-bit sums
+// of the frame's pixels, for rows whose windows may hold a pixel too large for the
+// strip's sums; a window off the frame is clipped as the reference's is. Masked
+// centres, and those off the frame, are the caller's to set. (4 frames of 3262 x 3108
+// with 2 million counts a pixel: 1.26 ms at kernel 2 and 2.37 at 4; 1.66 and 3.99
+// where each lane read its neighbours' columns too, a pixel a load.)
 template <int K, int C>
 __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image, int height,
                                               int width, int y, int cx, const LaunchParams &P) {
-  constexpr int W0 = 2 * K + 1;
-  if (y < 0 || y >= height)
-    return (1u << C) - 1u;  // off the frame: set
-  uint32_t cn[W0];
-  unsigned long long cS[W0], cQ[W0];
-  uint32_t n = 0, bits = 0;
-  unsigned long long S = 0, Q = 0;
+  constexpr int kPacked = 48;  // valid pixels above their sum: 81 x 2^32 is below 2^39
+  unsigned long long s[C], q[C];
 #pragma unroll
-  for (int j = 0; j < C + 2 * K; j++) {
-    const int x = cx - K + j;
-    uint32_t an = 0;
-    unsigned long long aS = 0, aQ = 0;
-    if (x >= 0 && x < width) {
+  for (int c = 0; c < C; c++)
+    s[c] = q[c] = 0ull;
+  const bool pieces = cx >= 0 && cx + C <= width && width % 4 == 0 &&
+                      reinterpret_cast<uintptr_t>(image) % 16 == 0;
+  constexpr int kInFlight = C == kNarrowCols ? 2 * K + 1 : 1;  // rows (12 columns a lane spill)
+#pragma unroll kInFlight
+  for (int yy = max(0, y - K); yy <= min(height - 1, y + K); yy++) {
+    const uint32_t *row = image + ((ptrdiff_t)yy * width + cx);
 #pragma unroll
-      for (int d = -K; d <= K; d++) {
-        const uint32_t v = y + d >= 0 && y + d < height
-                               ? __ldg(image + (size_t)(y + d) * width + x)
-                               : 0xFFFFFFFFu;
-        const bool ok = v < 0xFFFFFFFEu;
-        const uint32_t u = ok ? v : 0u;
-        an += ok ? 1u : 0u;
-        aS += u;
-        aQ += (unsigned long long)u * u;
+    for (int i = 0; i < C; i += 4) {
+      uint4 x;
+      if (pieces) {
+        x = __ldg(reinterpret_cast<const uint4 *>(row + i));
+      } else {
+        auto at = [&](int c) {
+          return cx + c >= 0 && cx + c < width ? __ldg(row + c) : 0xFFFFFFFFu;
+        };
+        x = make_uint4(at(i), at(i + 1), at(i + 2), at(i + 3));
+      }
+      const uint32_t v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const bool ok = v[c] < 0xFFFFFFFEu;
+        s[i + c] += ok ? (1ull << kPacked) + v[c] : 0ull;
+        q[i + c] += ok ? (unsigned long long)v[c] * v[c] : 0ull;
       }
     }
-    if (j >= W0) {
-      n -= cn[j % W0];
-      S -= cS[j % W0];
-      Q -= cQ[j % W0];
-    }
-    cn[j % W0] = an;
-    cS[j % W0] = aS;
-    cQ[j % W0] = aQ;
-    n += an;
-    S += aS;
-    Q += aQ;
-    if (j >= 2 * K) {
-      const int xc = x - K;  // the window's centre
-      bool set = true;
-      if (xc >= 0 && xc < width && __ldg(image + (size_t)y * width + xc) < 0xFFFFFFFEu)
-        set = ext_exact(n, S, Q, P);
-      bits |= set ? 1u << (j - 2 * K) : 0u;
-    }
   }
+  __syncwarp();
+  wide_sums<K, C>(s);
+  wide_sums<K, C>(q);
+  uint32_t bits = 0;
+#pragma unroll
+  for (int c = 0; c < C; c++)
+    bits |= ext_exact((uint32_t)(s[c] >> kPacked), s[c] & ((1ull << kPacked) - 1ull), q[c], P)
+                ? 1u << c
+                : 0u;
   return bits;
 }
 
