@@ -1156,7 +1156,6 @@ extern "C" int sf_threshold_u32_device_noalloc(
 namespace sf {
 
 constexpr size_t kPlanMaxGraphs = 16;
-constexpr int kTuneMinRows = 16;  // shortest run length the tuner tries
 
 struct Plan {
   size_t h = 0, w = 0, max_frames = 0, capacity = 0, words = 0;
@@ -1323,7 +1322,7 @@ int sf_plan_tune(sf_plan *plan, const uint32_t *const *d_images, size_t n_frames
   if (rc != SF_OK)
     return rc;
   if (P.algorithm != SF_DISPERSION_EXTENDED || !P.int_ok)
-    return SF_OK;  // the tile path has nothing to tune
+    return SF_OK;  // (the other settings keep the default geometry)
   // Two knobs, timed together on the given frames (median of 3 runs each):
   // the frames a launch sequence takes (all of them, 32 or 16: fewer frames
   // a launch keep more of a batch's tiles in L2 between the passes, more
@@ -1346,7 +1345,7 @@ int sf_plan_tune(sf_plan *plan, const uint32_t *const *d_images, size_t n_frames
     cands.erase(std::unique(cands.begin(), cands.end()), cands.end());
     p.per_launch = q == n_frames ? 0 : q;
     for (int rr : cands) {
-      if (rr < kTuneMinRows || rr > (int)p.h)
+      if (rr < kShortRun || rr > (int)p.h)
         continue;
       p.run_rows = rr;
       float ms[3];

@@ -1157,17 +1157,18 @@ bool encode_frame_map(CUtensorMap *map, const void *base, int h, int w, int byte
 size_t lattice_tiles(int h, int w) { return (size_t)ver_ntx(w) * (size_t)ver_nty(h); }
 
 // The run length for a launch whose tallest frame has h rows and whose frames
-// have `strips` strips in all, unless run_rows is given, in whole triples of
+// have `strips` strips in all, unless run_rows is given (but see kShortRun), in whole triples of
 // rows: the resident warps filled kLatWaves times over by runs of at least
 // kLatLongRun rows (each reads 9 rows more than it writes), so that warps of
 // unequal speed even out (32 frames of 4362 x 4148: 424 us, 447 with three times
 // and 144 rows); else once, down to runs of kLatMinRunRows.
 static int lat_run_rows(int h, long long strips, int run_rows) {
-  if (run_rows <= 0) {
-    const long long nruns = std::max(1ll, (long long)lat_slots() / std::max(1ll, strips));
-    const int once = (int)((h + nruns - 1) / nruns);
+  const long long nruns = std::max(1ll, (long long)lat_slots() / std::max(1ll, strips));
+  const int once = (int)((h + nruns - 1) / nruns);
+  if (run_rows <= 0)
     run_rows = std::min(once, std::max(kLatLongRun, (once + kLatWaves - 1) / kLatWaves));
-  }
+  else if (once < kShortRun)
+    run_rows = std::min(run_rows, once);
   run_rows = std::max(run_rows, kLatMinRunRows);
   return (run_rows + 2) / 3 * 3;
 }

@@ -74,6 +74,12 @@ struct StreamMarks {
 // a bounded size. The tile path (sf_threshold.cu) has the others.
 bool streaming_path(const LaunchParams &P, int pixel_bytes);
 
+// A launch that fills the device once with runs of fewer rows takes those whatever
+// run length it is given: longer ones only leave warps without work. (One frame of
+// 1065 x 1030 in a captured graph, L2 cold: 35 us so, 60 with the 64 rows that a
+// tuned plan gave it.) Run lengths from here on are the tuner's to choose.
+constexpr int kShortRun = 16;
+
 // run_rows 0: the default geometry. marks may be null. h and w are the batch's
 // envelope.
 cudaError_t launch_extended(const FramePtrs &frames, int nframes, int h, int w, int pixel_bytes,

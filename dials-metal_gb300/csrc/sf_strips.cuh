@@ -362,11 +362,12 @@ template <int C> inline int strips_of(int w) {
 }
 
 inline int strip_run_rows(int tallest, long long strips, int slots, int run_rows) {
-  if (run_rows <= 0) {
-    const long long runs = std::max(1ll, slots / std::max(1ll, strips));
-    const int once = (int)((tallest + runs - 1) / runs);
+  const long long runs = std::max(1ll, slots / std::max(1ll, strips));
+  const int once = (int)((tallest + runs - 1) / runs);
+  if (run_rows <= 0)
     run_rows = std::min(once, std::max(kLongRun, (once + kStripWaves - 1) / kStripWaves));
-  }
+  else if (once < kShortRun)
+    run_rows = std::min(run_rows, once);
   return std::max(run_rows, kMinRunRows);
 }
 

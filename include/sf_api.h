@@ -274,10 +274,11 @@ int sf_threshold_u32_mixed_batch_device(const uint32_t *const *d_images, const s
  * sets are kept). sf_plan_tune times, on the given frames, the frames a
  * launch sequence takes (all, 32 or 16; sf_plan_frames_per_launch, 0 for
  * all) and the strip run lengths (sf_plan_run_rows), and keeps the fastest
- * pair; the results are the same for any of them. Outputs (device pointers, valid until sf_plan_destroy): frame j's
- * list at sf_plan_lists(p) + j * capacity, its count at sf_plan_counts(p)[j],
- * its mask at sf_plan_masks(p) + j * ceil(width/32) * height. NULL on failure
- * (the reason in sf_last_error()).
+ * pair; the results are the same for any of them, and a launch that fills the
+ * device with runs of fewer than 16 rows takes those. Outputs (device pointers,
+ * valid until sf_plan_destroy): frame j's list at sf_plan_lists(p) + j *
+ * capacity, its count at sf_plan_counts(p)[j], its mask at sf_plan_masks(p) +
+ * j * ceil(width/32) * height. NULL on failure (the reason in sf_last_error()).
  */
 typedef struct sf_plan sf_plan;
 sf_plan *sf_plan_create(size_t height, size_t width, size_t max_frames, size_t capacity,

@@ -236,3 +236,33 @@ def test_tiles(params, kernel, algorithm):
     b = api.MixedBatch([f.shape for f in frames], capacity=200 * 333, params=api.Params(**p))
     b([_device(f) for f in frames])
     _check(b, frames, p)
+
+
+@pytest.mark.parametrize("h,w,kernel", [(1065, 1030, 3), (1065, 1030, 4), (2400, 2400, 3)])
+def test_a_run_length_never_starves_a_small_launch(h, w, kernel):
+    # A plan whose run length would leave most of the device without work takes
+    # the default geometry: the same kernels in the same time (half again and the
+    # best of many runs, against twice as long where the length was taken as given).
+    import torch
+    from sfgb import api
+    frame = _device(_spots(h, w, 5))
+    took = {}
+    for rows in (0, 512):
+        plan = api.Plan(h, w, 1, params=api.Params(kernel_x=kernel, kernel_y=kernel))
+        plan.configure(rows)
+        for _ in range(3):
+            plan([frame])
+        torch.cuda.synchronize()
+        begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        times = []
+        for _ in range(20):
+            begin.record()
+            for _ in range(20):
+                plan([frame])
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        took[rows] = min(times)
+        _check(plan, [frame.cpu().numpy().view(np.uint32)], dict(kernel_x=kernel, kernel_y=kernel))
+        plan.close()
+    assert took[512] < 1.5 * took[0], took
