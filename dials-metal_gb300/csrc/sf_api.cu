@@ -227,13 +227,15 @@ static int threshold_frames(const T *const *d_images, size_t n, size_t h, size_t
                                    d_counts, d_word_prefix, d_ws, ws_bytes, run_rows, stream);
 }
 
-// The streaming path's launches for frames whose buffers L lays out in d_ws.
+// The streaming path's launches for frames whose buffers L lays out in d_ws. marks:
+// where their times are taken, or null.
 template <typename T>
 static int threshold_streamed(const T *const *d_images, size_t n, const size_t *heights,
                               const size_t *widths, size_t h, size_t w, const LaunchParams &P,
                               const WorkspaceLayout &L, sf_signal_pixel *d_out, size_t capacity,
                               uint32_t *d_bits, uint32_t *d_counts, uint32_t *d_word_prefix,
-                              void *d_ws, bool limited, int run_rows, cudaStream_t stream) {
+                              void *d_ws, bool limited, int run_rows, cudaStream_t stream,
+                              const StreamMarks *marks) {
   unsigned char *ws = static_cast<unsigned char *>(d_ws);
   FramePtrs F;
   for (size_t j = 0; j < n; j++) {
@@ -257,8 +259,6 @@ static int threshold_streamed(const T *const *d_images, size_t n, const size_t *
   b.out = d_out;
   b.out_stride = capacity;
   b.count_out = d_counts;
-  const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
-  t_marks.staged = true;
   const cudaError_t e =
       P.algorithm == SF_DISPERSION
           ? launch_dispersion(F, (int)n, (int)h, (int)w, (int)sizeof(T), P, b, run_rows, stream,
@@ -298,29 +298,33 @@ static int threshold_frames_mixed(const T *const *d_images, size_t n, const size
   const WorkspaceLayout L = all ? Ln : layout(h, w, capacity);
   if (batch ? !all : ws_bytes < L.total)
     return SF_EBADARG;
-  if (streamed && !all && n > 1) {
-    // A workspace for one frame: the frames one after another, each into its
-    // slots of the envelope's layout.
+  const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
+  const bool one_sequence = streamed && (all || n == 1);
+  t_marks.staged = one_sequence;
+  if (one_sequence)
+    return threshold_streamed<T>(d_images, n, heights, widths, h, w, P, L, d_out, capacity, d_bits,
+                                 d_counts, d_word_prefix, d_ws, batch, run_rows, stream, marks);
+  // The frames one after another on the stream, timed as a whole.
+  if (marks)
+    cudaEventRecord(marks->start, stream);
+  if (streamed) {
+    // A workspace for one frame: each frame into its slots of the envelope's
+    // layout.
     for (size_t j = 0; j < n; j++) {
       const T *one[1] = {d_images[j]};
       rc = threshold_streamed<T>(one, 1, heights + j, widths + j, h, w, P, L, d_out + j * capacity,
                                  capacity, d_bits + j * L.words, d_counts + j,
                                  d_word_prefix ? d_word_prefix + j * L.words : nullptr, d_ws,
-                                 batch, run_rows, stream);
+                                 batch, run_rows, stream, nullptr);
       if (rc != SF_OK)
         return rc;
     }
+    if (marks)
+      cudaEventRecord(marks->order, stream);
     return SF_OK;
   }
-  if (streamed)
-    return threshold_streamed<T>(d_images, n, heights, widths, h, w, P, L, d_out, capacity, d_bits,
-                                 d_counts, d_word_prefix, d_ws, batch, run_rows, stream);
   unsigned char *ws = static_cast<unsigned char *>(d_ws);
-  const StreamMarks *marks = g_profiling && !t_capturing ? t_marks.arm() : nullptr;
-  t_marks.staged = false;
-  if (marks)
-    cudaEventRecord(marks->start, stream);
-  // The tile path, one frame after another on the stream.
+  // The tile path.
   for (size_t j = 0; j < n; j++) {
     FrameBuffers fb;
     fb.bits = d_bits + j * L.words;

@@ -169,10 +169,12 @@ int sf_scan_compressed(const uint8_t *data, size_t nbytes, const char *algorithm
  * (src/spots/dext_gpu.hh:89-127). Times in milliseconds for the calling
  * thread's last profiled call (host frame, device frame or batch, all its
  * frames): upload (host-frame calls), `fused` (the whole threshold), copy
- * (list read-back). On the 32-bit dispersion_extended path also stage0
- * (stage 0 and the erosion, one kernel: the reference's stage0 + stage1),
- * stage2 and sort (ordering the list); stage1 stays 0. A device call's
- * times are read when sf_last_stage_times is called, which waits for it. */
+ * (list read-back). Where the frames go in one launch sequence (not with a
+ * negative gain or sigma, nor a batch given a workspace for one frame) also
+ * stage0 (stage 0 and the erosion, the reference's stage0 + stage1; the plain
+ * dispersion's filter), stage2 (the decision) and sort (writing the list);
+ * stage1 stays 0. A device call's times are read when sf_last_stage_times is
+ * called, which waits for it. */
 typedef struct {
   double upload, stage0, stage1, stage2, fused, copy, sort;
 } sf_stage_times;

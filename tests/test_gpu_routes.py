@@ -266,3 +266,40 @@ def test_a_run_length_never_starves_a_small_launch(h, w, kernel):
         _check(plan, [frame.cpu().numpy().view(np.uint32)], dict(kernel_x=kernel, kernel_y=kernel))
         plan.close()
     assert took[512] < 1.5 * took[0], took
+
+
+def test_profile_covers_frames_one_after_another():
+    # A batch of the plain dispersion in a workspace for one frame runs frame by
+    # frame; its profiled time is all frames' (eight here, against one's).
+    import ctypes
+
+    import torch
+    from sfgb import api
+    h, w, capacity = 1024, 1024, 1 << 16
+    frame = _device(_spots(h, w, 9))
+    p = api.Params(algorithm=1)
+    L = api.lib()
+    b = api.DeviceBatch(h, w, 8, capacity=capacity, params=p)
+    small = L.sf_workspace_bytes(h, w, capacity)
+    ptrs = (ctypes.c_void_p * 8)(*[frame.data_ptr()] * 8)
+
+    def fused(n):
+        best = 1e9
+        for _ in range(10):
+            rc = L.sf_threshold_u32_batch_device(
+                ctypes.cast(ptrs, ctypes.c_void_p), n, h, w, ctypes.byref(b.params),
+                b.out.data_ptr(), capacity, b.bits.data_ptr(), b.counts.data_ptr(), None,
+                b.workspace.data_ptr(), small, torch.cuda.current_stream().cuda_stream)
+            assert rc == 0, api.last_error()
+            best = min(best, api.last_stage_times()["fused"])
+        return best
+
+    api.profile_stages(True)
+    try:
+        one, eight = fused(1), fused(8)
+    finally:
+        api.profile_stages(False)
+    assert 0.0 < 1.8 * one < eight, (one, eight)
+    want = O.dext(frame.cpu().numpy().view(np.uint32), O.Params(algorithm=1))
+    for j in range(8):
+        assert b.result(j).tobytes() == want.tobytes()
