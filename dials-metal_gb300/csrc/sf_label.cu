@@ -1597,19 +1597,18 @@ static cudaError_t load_label_kernels() {
   return cudaSuccess;
 }
 
-struct Labeller {
-  size_t height = 0, width = 0, capacity = 0, spots_cap = 0;
-  sf_label_options opt;
-  cudaStream_t own_stream = nullptr;
-  void *arena = nullptr, *host_block = nullptr;
-  bool started = false;
-  int64_t last_frame = 0;
-  bool finished = false;
+// At most one accepted spot (and one candidate) per min_spot_size pixels closed in
+// a batch.
+static size_t spots_capacity(size_t capacity, size_t min_spot_size) {
+  return capacity / std::max<size_t>(min_spot_size, 1) + 1;
+}
+
+// A labeller's device buffers for n open pixels.
+struct LabelBuffers {
   // Live pool, ping-pong.
   int32_t *frame[2] = {nullptr, nullptr};
   uint32_t *index[2] = {nullptr, nullptr}, *value[2] = {nullptr, nullptr};
   uint32_t *parent[2] = {nullptr, nullptr};
-  int cur = 0;
   // Scratch sized by capacity.
   uint32_t *root = nullptr, *csize = nullptr, *candid = nullptr, *flag = nullptr,
            *newpos = nullptr, *clist = nullptr, *cbucket = nullptr, *order = nullptr,
@@ -1626,64 +1625,23 @@ struct Labeller {
   double *terms = nullptr;
   uint2 *edges = nullptr;  // the unions k_link lists, capacity of them
   LabelStatus *st = nullptr;
-  LabelStatus *host_st = nullptr;
-  BatchArgs *d_args = nullptr, *h_args = nullptr;
-  // Captured launch sequences by (live pool, frames in the batch).
-  cudaGraphExec_t graphs[2][kLabelMaxBatch + 1] = {};
-  bool seen[2][kLabelMaxBatch + 1] = {};
-  bool use_graphs = true;
-  // Batch outputs, copied to the host vectors after every batch.
+  BatchArgs *d_args = nullptr;
+  // Batch outputs, appended to the stores after every batch.
   sf_spot *d_spots = nullptr;
   sf_pixel *d_pixels = nullptr;
-  // Host-list upload staging.
-  sf_signal_pixel *d_list = nullptr;
-  size_t d_list_cap = 0;
   uint32_t *d_counts = nullptr;
-  DeviceStore<sf_spot> spots;
-  DeviceStore<sf_pixel> pixels;
-  // Recorded after each call's appends: the next call (on whatever stream)
-  // and the readers wait for it before touching the batch outputs or the
-  // stores.
-  cudaEvent_t appended = nullptr;
-  // With blocking waits (label_set_blocking_wait), a call's end is waited
-  // for on this event, created with cudaEventBlockingSync: the calling thread
-  // sleeps instead of spinning (the served form runs a thread per sweep).
-  cudaEvent_t call_done = nullptr;
-  sf_counts counts{};
-  uint32_t live = 0;
-  std::string error;
-
-  ~Labeller() {
-    if (own_stream) {
-      cudaStreamSynchronize(own_stream);
-      cudaStreamDestroy(own_stream);
-    }
-    for (auto &row : graphs)
-      for (cudaGraphExec_t g : row)
-        if (g)
-          cudaGraphExecDestroy(g);
-    cudaFree(arena);
-    cudaFree(d_list);
-    if (host_block)
-      cudaFreeHost(host_block);
-    if (appended)
-      cudaEventDestroy(appended);
-    if (call_done)
-      cudaEventDestroy(call_done);
-  }
 
   // Every device buffer of a call, carved out of one allocation at `base`;
   // returns its size. (An allocation each cost 45 calls, 1.1 ms of a labeller's
   // opening and 1.6 ms of its closing.) Buffers whose uses do not overlap
   // within a call share their place.
-  size_t carve(unsigned char *base) {
+  size_t carve(size_t height, size_t n, size_t spots_cap, unsigned char *base) {
     size_t off = 0;
     auto take = [&](auto *&p, size_t cnt) {
       using T = std::remove_reference_t<decltype(*p)>;
       p = reinterpret_cast<T *>(base + off);
       off += ((cnt ? cnt : 1) * sizeof(T) + 255) / 256 * 256;
     };
-    const size_t n = capacity;
     for (int i = 0; i < 2; i++) {
       take(frame[i], n);
       take(index[i], n);
@@ -1729,15 +1687,65 @@ struct Labeller {
     take(d_args, 1);
     return off;
   }
+};
+
+struct Labeller : LabelBuffers {
+  size_t height = 0, width = 0, capacity = 0, spots_cap = 0;
+  sf_label_options opt;
+  cudaStream_t own_stream = nullptr;
+  void *arena = nullptr, *host_block = nullptr;
+  bool started = false;
+  int64_t last_frame = 0;
+  bool finished = false;
+  int cur = 0;
+  LabelStatus *host_st = nullptr;
+  BatchArgs *h_args = nullptr;
+  // Captured launch sequences by (live pool, frames in the batch).
+  cudaGraphExec_t graphs[2][kLabelMaxBatch + 1] = {};
+  bool seen[2][kLabelMaxBatch + 1] = {};
+  bool use_graphs = true;
+  // Host-list upload staging.
+  sf_signal_pixel *d_list = nullptr;
+  size_t d_list_cap = 0;
+  DeviceStore<sf_spot> spots;
+  DeviceStore<sf_pixel> pixels;
+  // Recorded after each call's appends: the next call (on whatever stream)
+  // and the readers wait for it before touching the batch outputs or the
+  // stores.
+  cudaEvent_t appended = nullptr;
+  // With blocking waits (label_set_blocking_wait), a call's end is waited
+  // for on this event, created with cudaEventBlockingSync: the calling thread
+  // sleeps instead of spinning (the served form runs a thread per sweep).
+  cudaEvent_t call_done = nullptr;
+  sf_counts counts{};
+  uint32_t live = 0;
+  std::string error;
+
+  ~Labeller() {
+    if (own_stream) {
+      cudaStreamSynchronize(own_stream);
+      cudaStreamDestroy(own_stream);
+    }
+    for (auto &row : graphs)
+      for (cudaGraphExec_t g : row)
+        if (g)
+          cudaGraphExecDestroy(g);
+    cudaFree(arena);
+    cudaFree(d_list);
+    if (host_block)
+      cudaFreeHost(host_block);
+    if (appended)
+      cudaEventDestroy(appended);
+    if (call_done)
+      cudaEventDestroy(call_done);
+  }
 
   int init() {
     cudaError_t e;
-    // At most one accepted spot (and one candidate) per min_spot_size pixels
-    // closed in a batch.
-    spots_cap = capacity / (opt.min_spot_size ? opt.min_spot_size : 1) + 1;
-    if ((e = cudaMalloc(&arena, carve(nullptr))) != cudaSuccess)
+    spots_cap = spots_capacity(capacity, opt.min_spot_size);
+    if ((e = cudaMalloc(&arena, carve(height, capacity, spots_cap, nullptr))) != cudaSuccess)
       return fail(e, "cudaMalloc for the labeller");
-    carve(static_cast<unsigned char *>(arena));
+    carve(height, capacity, spots_cap, static_cast<unsigned char *>(arena));
     // The status read back and the arguments, page-locked.
     constexpr size_t args_at = (sizeof(LabelStatus) + 255) / 256 * 256;
     if ((e = cudaMallocHost(&host_block, args_at + sizeof(BatchArgs))) != cudaSuccess)
@@ -1990,19 +1998,8 @@ namespace sf {
 size_t label_width(const sf_labeller *l) { return l ? l->impl.width : 0; }
 
 size_t label_device_bytes(size_t height, size_t capacity, size_t min_spot_size) {
-  // The pools (two of frame, index, value, parent), 22 scratch words, the
-  // batch's kept pixels, the member records and tags, three variance terms
-  // and an edge a slot; a spot record, a candidate record and a size-order
-  // entry per possible spot.
-  const size_t per =
-      2 * 4 * 4 + 22 * 4 + sizeof(sf_pixel) + 4 + sizeof(sf_pixel) + 3 * 8 + 8 + 1;
-  const size_t spots = capacity / std::max<size_t>(min_spot_size, 1) + 1;
-  const size_t rows =
-      height <= kRowTableMaxRows ? (size_t)(kLabelMaxBatch + 1) * (height + 1) * 4 : 0;
-  return capacity * per + spots * (sizeof(sf_spot) + sizeof(CandSpot) + 4) + rows +
-         2 * kSizeBins * 4 +
-         (size_t)kGrid * kBuckets * 4 + (size_t)kScanBlocks * 4 + kLabelMaxBatch * 4 +
-         2 * sizeof(LabelStatus) + 2 * sizeof(BatchArgs);
+  LabelBuffers b;
+  return b.carve(height, capacity, spots_capacity(capacity, min_spot_size), nullptr);
 }
 
 void label_set_growth(sf_labeller *l, LabelGrowth growth) {

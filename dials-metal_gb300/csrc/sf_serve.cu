@@ -138,7 +138,8 @@ struct SrvSweep {
   size_t bytes = 0, ring = 0;
   size_t result_bytes = 0;              // its labeller's spot and pixel stores, granted
   sf_server *server = nullptr;
-  std::vector<uint32_t *> slots;        // frames
+  uint32_t *frames = nullptr;           // the slots' frames, one allocation
+  std::vector<uint32_t *> slots;        // each slot's
   sf_signal_pixel *lists = nullptr;     // ring * capacity records
   uint32_t *counts = nullptr;           // ring
   uint32_t *host_counts = nullptr;      // pinned, ring
@@ -175,8 +176,7 @@ struct SrvSweep {
       thread.join();
     if (lab)
       sf_label_close(lab);
-    for (uint32_t *p : slots)
-      cudaFree(p);
+    cudaFree(frames);
     for (sf::DecodeBlock *p : tables)
       cudaFree(p);
     for (void *p : host_tables)
@@ -207,6 +207,9 @@ size_t labeller_capacity(const sf_server_options &o, size_t h, size_t w) {
 size_t labeller_bytes(size_t height, size_t capacity, size_t min_spot_size) {
   return sf::label_device_bytes(height, capacity, min_spot_size) + ((size_t)16 << 20);
 }
+
+// A slot's frame, whole 256 bytes.
+size_t slot_bytes(size_t h, size_t w) { return (h * w * sizeof(uint32_t) + 255) / 256 * 256; }
 
 size_t group_bytes(size_t h, size_t w, size_t capacity, size_t max_batch) {
   const size_t words = (w + 31) / 32 * h;
@@ -334,7 +337,7 @@ void sf_server::label_loop(SrvSweep *s) {
         return stop || !s->tasks.empty() || (s->finishing && s->in_flight == 0);
       });
       // A short wait for more of the sweep's frames when the call would be
-      // small: a label call has a fixed cost of some forty launches.
+      // small: a label call has a fixed cost of some twenty launches.
       auto queued = [&] {
         size_t n = 0;
         for (const LabelTask &u : s->tasks)
@@ -626,7 +629,7 @@ size_t sf_server_sweep_bytes(const sf_server *sv, size_t height, size_t width,
     return 0;
   const size_t min_size = label ? label->min_spot_size : 3;
   const size_t capacity = std::max<size_t>(1, height * width / sv->opt.capacity_divisor);
-  return sv->opt.ring * (height * width * sizeof(uint32_t) + capacity * sizeof(sf_signal_pixel) +
+  return sv->opt.ring * (slot_bytes(height, width) + capacity * sizeof(sf_signal_pixel) +
                          sizeof(uint32_t)) +
          labeller_bytes(height, labeller_capacity(sv->opt, height, width), min_size);
 }
@@ -699,12 +702,11 @@ int sf_server_open_sweep(sf_server *sv, size_t height, size_t width,
     lrc = sf::label_prepare(s->lab, (int)sv->opt.max_batch);
   if (lrc != SF_OK)
     return lrc;
-  for (size_t i = 0; i < s->ring; i++) {
-    uint32_t *slot = nullptr;
-    if ((e = cudaMalloc(&slot, height * width * sizeof(uint32_t))) != cudaSuccess)
-      return SF_ECUDA;
-    s->slots.push_back(slot);
-  }
+  // (Slots of their own would each be rounded up to the allocator's 2 MiB.)
+  if ((e = cudaMalloc(&s->frames, s->ring * slot_bytes(height, width))) != cudaSuccess)
+    return SF_ECUDA;
+  for (size_t i = 0; i < s->ring; i++)
+    s->slots.push_back(s->frames + i * (slot_bytes(height, width) / sizeof(uint32_t)));
   s->tables.assign(s->ring, nullptr);
   s->host_tables.assign(s->ring, nullptr);
   s->table_bytes.assign(s->ring, 0);
