@@ -323,22 +323,23 @@ static int threshold_frames_mixed(const T *const *d_images, size_t n, const size
       cudaEventRecord(marks->order, stream);
     return SF_OK;
   }
-  unsigned char *ws = static_cast<unsigned char *>(d_ws);
-  // The tile path.
-  for (size_t j = 0; j < n; j++) {
-    FrameBuffers fb;
-    fb.bits = d_bits + j * L.words;
-    fb.staging = reinterpret_cast<sf_signal_pixel *>(ws + L.staging);
-    fb.out = d_out + j * capacity;
-    fb.word_prefix = d_word_prefix ? d_word_prefix + j * L.words : nullptr;
-    fb.tile_base = reinterpret_cast<uint32_t *>(ws + L.tile_base);
-    fb.row_total = reinterpret_cast<uint32_t *>(ws + L.row_total);
-    fb.total = d_counts + j;
-    fb.capacity = (uint32_t)capacity;
-    cudaError_t e =
-        launch_threshold<T>(d_images[j], (int)heights[j], (int)widths[j], P, fb, stream);
-    if (e != cudaSuccess)
-      return fail(e, "launching the threshold");
+  if constexpr (sizeof(T) == 4) {  // The tile path (16-bit frames are all streamed).
+    unsigned char *ws = static_cast<unsigned char *>(d_ws);
+    for (size_t j = 0; j < n; j++) {
+      FrameBuffers fb;
+      fb.bits = d_bits + j * L.words;
+      fb.staging = reinterpret_cast<sf_signal_pixel *>(ws + L.staging);
+      fb.out = d_out + j * capacity;
+      fb.word_prefix = d_word_prefix ? d_word_prefix + j * L.words : nullptr;
+      fb.tile_base = reinterpret_cast<uint32_t *>(ws + L.tile_base);
+      fb.row_total = reinterpret_cast<uint32_t *>(ws + L.row_total);
+      fb.total = d_counts + j;
+      fb.capacity = (uint32_t)capacity;
+      const cudaError_t e =
+          launch_threshold(d_images[j], (int)heights[j], (int)widths[j], P, fb, stream);
+      if (e != cudaSuccess)
+        return fail(e, "launching the threshold");
+    }
   }
   if (marks)
     cudaEventRecord(marks->order, stream);

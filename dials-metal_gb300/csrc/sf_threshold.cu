@@ -1,9 +1,11 @@
-// The fused threshold for sm_103a: every stage of src/spots/dext.cc (the
-// dispersion test, the erosion, the background-only Poisson test) for one
-// output tile per block, from one read of the tile and its halo, with the
-// masks kept in shared memory. Then an ordering pass that writes the signal
-// list ascending by index, which the reference's device path had to sort on
-// the host (src/spots/dext_cuda.cu:855-861).
+// The fused threshold of 32-bit frames under settings that the streaming
+// kernels do not take (a negative gain or sigma, constants beyond the integer
+// tests): every stage of src/spots/dext.cc (the dispersion test, the erosion,
+// the background-only Poisson test) for one output tile per block, from one
+// read of the tile and its halo, with the masks kept in shared memory. Then an
+// ordering pass that writes the signal list ascending by index, which the
+// reference's device path had to sort on the host
+// (src/spots/dext_cuda.cu:855-861).
 //
 // Per frame, kernel 1 (threshold_tile) writes
 //   - the strong-pixel bitmask, one bit per pixel, row-major, ceil(W/32)
@@ -39,9 +41,9 @@ template <int K, int TW, int TH> struct Geom {
   static_assert(S1W == TW + 2 * K2, "erosion region spans the stage-2 window");
 };
 
-template <typename T, int K, int TW, int TH> struct Smem {
+template <int K, int TW, int TH> struct Smem {
   using G = Geom<K, TW, TH>;
-  using W = typename Traits<T>::W;
+  using W = Traits<uint32_t>::W;
   uint32_t pix[G::IH][G::IW];
   W hS[G::IH][G::S0W];          // stage-0 row sums of I; later stage-2 rows
   W hQ[G::IH][G::S0W];          // stage-0 row sums of I^2
@@ -57,22 +59,21 @@ template <typename T, int K, int TW, int TH> struct Smem {
   uint32_t tile_base;
 };
 
-template <typename T>
 __device__ __forceinline__ bool is_masked(uint32_t v) {
-  return v >= Traits<T>::kMasked;
+  return v >= Traits<uint32_t>::kMasked;
 }
 
-template <typename T, int K, int TW, int TH>
+template <int K, int TW, int TH>
 __global__ void __launch_bounds__(256)
-threshold_tile(const T *__restrict__ image, int height, int width,
+threshold_tile(const uint32_t *__restrict__ image, int height, int width,
                const __grid_constant__ LaunchParams P, uint32_t *__restrict__ bits,
                sf_signal_pixel *__restrict__ staging, uint32_t capacity,
                uint32_t *__restrict__ total, uint32_t *__restrict__ tile_base,
                uint32_t *__restrict__ row_total) {
   using G = Geom<K, TW, TH>;
-  using W = typename Traits<T>::W;
+  using W = Traits<uint32_t>::W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem<T, K, TW, TH> &s = *reinterpret_cast<Smem<T, K, TW, TH> *>(smem_raw);
+  Smem<K, TW, TH> &s = *reinterpret_cast<Smem<K, TW, TH> *>(smem_raw);
 
   const int tid = threadIdx.x;
   const int nthreads = blockDim.x;
@@ -90,7 +91,7 @@ threshold_tile(const T *__restrict__ image, int height, int width,
   for (int idx = tid; idx < G::IH * G::IW; idx += nthreads) {
     const int r = idx / G::IW, c = idx - r * G::IW;
     const int gy = y_base + r, gx = x_base + c;
-    uint32_t v = Traits<T>::kOutside;
+    uint32_t v = Traits<uint32_t>::kOutside;
     if (gy >= 0 && gy < height && gx >= 0 && gx < width)
       v = (uint32_t)image[(size_t)gy * width + gx];
     s.pix[r][c] = v;
@@ -105,7 +106,7 @@ threshold_tile(const T *__restrict__ image, int height, int width,
 #pragma unroll
     for (int d = 0; d <= 2 * K; d++) {
       const uint32_t v = s.pix[r][c + d];
-      if (!is_masked<T>(v)) {
+      if (!is_masked(v)) {
         n++;
         sum += (W)v;
         sq += (W)v * (W)v;
@@ -130,34 +131,21 @@ threshold_tile(const T *__restrict__ image, int height, int width,
       sum += s.hS[r + d][c];
       sq += s.hQ[r + d][c];
     }
-    bool sig;
-    if constexpr (sizeof(T) == 4)
-      sig = stage0_u32(n, sum, sq, P, s.root_lo, s.root_hi);
-    else
-      sig = stage0_u16(n, (uint32_t)sum, (uint32_t)sq, P);
+    const bool sig = stage0_u32(n, sum, sq, P, s.root_lo, s.root_hi);
     const uint32_t v = s.pix[r + K][c + K];
-    s.scr0[r][c] = (sig || is_masked<T>(v)) ? 1 : 0;
+    s.scr0[r][c] = (sig || is_masked(v)) ? 1 : 0;
 
     if (P.algorithm == SF_DISPERSION) {
       const int orow = r + K - G::R, ocol = c + K - G::R;
       if (orow >= 0 && orow < TH && ocol >= 0 && ocol < TW) {
         bool strong = false;
         float bg = 0.0f;
-        if (sig && !is_masked<T>(v) && v >= P.p_min) {
-          // (m p - s) > sigma_s sqrt(g s m), in the pixel type's real type.
-          if constexpr (sizeof(T) == 4) {
-            const double m = (double)n, sd = __ull2double_rn(sum), pv = (double)v;
-            strong = __dsub_rn(__dmul_rn(m, pv), sd) >
-                     __dmul_rn(P.sigma_s, __dsqrt_rn(__dmul_rn(__dmul_rn(P.gain, sd), m)));
-            bg = __double2float_rn(__ddiv_rn(sd, m));
-          } else {
-            const float m = __uint2float_rn(n), sd = __uint2float_rn((uint32_t)sum),
-                        pv = __uint2float_rn(v);
-            strong = __fsub_rn(__fmul_rn(m, pv), sd) >
-                     __fmul_rn((float)P.sigma_s,
-                               __fsqrt_rn(__fmul_rn(__fmul_rn((float)P.gain, sd), m)));
-            bg = __fdiv_rn(sd, m);
-          }
+        if (sig && !is_masked(v) && v >= P.p_min) {
+          // (m p - s) > sigma_s sqrt(g s m)
+          const double m = (double)n, sd = __ull2double_rn(sum), pv = (double)v;
+          strong = __dsub_rn(__dmul_rn(m, pv), sd) >
+                   __dmul_rn(P.sigma_s, __dsqrt_rn(__dmul_rn(__dmul_rn(P.gain, sd), m)));
+          bg = __double2float_rn(__ddiv_rn(sd, m));
         }
         s.bg[orow][ocol] = strong ? bg : -1.0f;
         s.pop[orow][ocol] = (uint16_t)n;
@@ -172,7 +160,7 @@ threshold_tile(const T *__restrict__ image, int height, int width,
       const int r = idx / G::S1W, c = idx - r * G::S1W;
       const uint32_t v = s.pix[r + G::O1][c + G::O1];
       uint8_t m = 1;
-      if (!is_masked<T>(v)) {
+      if (!is_masked(v)) {
         m = s.scr0[r + G::E][c + G::E];
         for (int dr = 0; dr <= 2 * G::E && m; dr++)
           for (int dc = 0; dc <= 2 * G::E; dc++)
@@ -208,7 +196,7 @@ threshold_tile(const T *__restrict__ image, int height, int width,
     for (int idx = tid; idx < TH * TW; idx += nthreads) {
       const int r = idx / TW, c = idx - r * TW;
       const uint32_t v = s.pix[r + G::R][c + G::R];
-      const bool cand = !is_masked<T>(v) && v >= P.p_min && s.scr1[r + G::K2][c + G::K2];
+      const bool cand = !is_masked(v) && v >= P.p_min && s.scr1[r + G::K2][c + G::K2];
       float bg = -1.0f;
       uint32_t n = 0;
       if (cand) {
@@ -218,12 +206,7 @@ threshold_tile(const T *__restrict__ image, int height, int width,
           sum += h2S[r + d][c];
         }
         float b;
-        bool sig;
-        if constexpr (sizeof(T) == 4)
-          sig = stage2_u32(v, n, sum, P, &b);
-        else
-          sig = stage2_u16(v, n, (uint32_t)sum, P, &b);
-        if (sig)
+        if (stage2_u32(v, n, sum, P, &b))
           bg = b;
       }
       s.bg[r][c] = bg;
@@ -425,23 +408,23 @@ order_signal(int height, int width, const uint32_t *__restrict__ bits,
 // Host-side launch.
 // ---------------------------------------------------------------------------
 
-template <typename T, int K>
-static cudaError_t launch_k(const T *image, int h, int w, const LaunchParams &P,
+template <int K>
+static cudaError_t launch_k(const uint32_t *image, int h, int w, const LaunchParams &P,
                             const FrameBuffers &fb, cudaStream_t stream) {
   constexpr int TW = kTileW, TH = kTileH;
-  using S = Smem<T, K, TW, TH>;
+  using S = Smem<K, TW, TH>;
   const size_t smem = sizeof(S);
   static bool configured = false; // per instantiation; attribute is per device
   cudaError_t e = cudaSuccess;
   if (!configured) {
-    e = cudaFuncSetAttribute(threshold_tile<T, K, TW, TH>,
+    e = cudaFuncSetAttribute(threshold_tile<K, TW, TH>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
       return e;
     configured = true;
   }
   const dim3 grid((w + TW - 1) / TW, (h + TH - 1) / TH);
-  threshold_tile<T, K, TW, TH><<<grid, 256, smem, stream>>>(
+  threshold_tile<K, TW, TH><<<grid, 256, smem, stream>>>(
       image, h, w, P, fb.bits, fb.staging, fb.capacity, fb.total, fb.tile_base,
       fb.row_total);
   e = cudaGetLastError();
@@ -464,8 +447,7 @@ size_t order_smem_bytes(int width) {
   return 2 * sizeof(uint32_t) * (size_t)kTileH * ((width + 31) / 32);
 }
 
-template <typename T>
-cudaError_t launch_threshold(const T *image, int h, int w, const LaunchParams &P,
+cudaError_t launch_threshold(const uint32_t *image, int h, int w, const LaunchParams &P,
                              const FrameBuffers &fb, cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(fb.total, 0, sizeof(uint32_t), stream);
   if (e == cudaSuccess)
@@ -474,21 +456,14 @@ cudaError_t launch_threshold(const T *image, int h, int w, const LaunchParams &P
     return e;
   switch (P.half) {
   case 2:
-    return launch_k<T, 2>(image, h, w, P, fb, stream);
+    return launch_k<2>(image, h, w, P, fb, stream);
   case 3:
-    return launch_k<T, 3>(image, h, w, P, fb, stream);
+    return launch_k<3>(image, h, w, P, fb, stream);
   case 4:
-    return launch_k<T, 4>(image, h, w, P, fb, stream);
+    return launch_k<4>(image, h, w, P, fb, stream);
   default:
     return cudaErrorInvalidValue;
   }
 }
-
-template cudaError_t launch_threshold<uint32_t>(const uint32_t *, int, int,
-                                                const LaunchParams &,
-                                                const FrameBuffers &, cudaStream_t);
-template cudaError_t launch_threshold<uint16_t>(const uint16_t *, int, int,
-                                                const LaunchParams &,
-                                                const FrameBuffers &, cudaStream_t);
 
 } // namespace sf

@@ -30,8 +30,7 @@ inline size_t words_per_row(int w) { return (size_t)((w + 31) / 32); }
 
 size_t order_smem_bytes(int width);
 
-template <typename T>
-cudaError_t launch_threshold(const T *image, int h, int w, const LaunchParams &P,
+cudaError_t launch_threshold(const uint32_t *image, int h, int w, const LaunchParams &P,
                              const FrameBuffers &fb, cudaStream_t stream);
 
 } // namespace sf
