@@ -3,8 +3,8 @@
 // (2K + 1)-square window passes the dispersion test of stage 0 and
 // (n p - S) > sigma_s sqrt(gain S n).
 //
-//   disp_strip    every pixel's window, one warp per 360-column strip and run
-//                 of rows: a mask that holds every strong pixel and few others
+//   disp_strip    every pixel's window, one warp per strip and run of rows: a
+//                 mask that holds every strong pixel and few others
 //   disp_decide   each set pixel decided from its window's full sums by the
 //                 reference's sequence; the failures leave the mask, which is
 //                 then the strong-pixel mask, and the blocks count theirs
@@ -52,7 +52,7 @@ __device__ __forceinline__ bool disp_float2(uint32_t p, uint32_t n, uint32_t S,
          __fmul_rn((float)P.sigma_s, __fsqrt_rn(__fmul_rn(__fmul_rn((float)P.gain, s), m)));
 }
 
-// The walk of sf_strips.cuh: a lane adds each row to its 12 column sums as it
+// The walk of sf_strips.cuh: a lane adds each row to its column sums as it
 // enters the window, subtracts it as it leaves, and reads it once more as the
 // centre row; a window is 2K + 1 column sums.
 // Bound by issue: 39 instructions a pixel at 66% of the issue rate. 16 frames of
@@ -163,9 +163,9 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
       if (__any_sync(0xffffffffu, out != 0u)) {
         const int s_mid = s_cur >= K ? s_cur - K : s_cur + G::Slots - K;
         read_row<Pix, C, G::Cap, false>(ring + s_mid * kStripStride<C>, lane, v);
-        uint32_t out2 = 0, masked12 = 0;
+        uint32_t out2 = 0, masked_at = 0;
         if (!uniform)
-          masked12 = sign_bits<C>([&](int c) { return v[c]; });
+          masked_at = sign_bits<C>([&](int c) { return v[c]; });
         if constexpr (sizeof(Pix) == 2) {
 #pragma unroll
           for (int c = 0; c < C; c++) {
@@ -198,7 +198,7 @@ disp_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_consta
               out2 |= (int)v[c] >= (int)G::Cap ? 1u << c : 0u;
           }
         }
-        out2 &= ~masked12;
+        out2 &= ~masked_at;
         out &= out2;
       }
       write_bits<C>(r, out_row, bytes_left, out);

@@ -155,8 +155,7 @@ __device__ __noinline__ uint32_t ext_wide_row(const uint32_t *__restrict__ image
   return bits;
 }
 
-// The stage-0 bits of the 12 windows of a lane whose newest row is the ring's
-// slot s, for rows whose windows may hold a pixel of Cap or more: the columns'
+// The stage-0 bits of a lane's windows whose newest row is the ring's slot s, for rows whose windows may hold a pixel of Cap or more: the columns'
 // sums again from the ring's rows, squares in 64 bits, and the 2^-8 tests in 64
 // bits; by ext_wide_row where one of the warp's pixels is kLargePixel or more.
 // (Two dense frames of 353 x 944 at kernel 4, every row of them so, take 80 us in all, 272 with every such row by
@@ -225,7 +224,7 @@ __device__ __noinline__ uint32_t ext_large_row(const uint32_t *ring, int s, int 
 }
 
 // The walk of sf_strips.cuh for stage 0, then the erosion (dext.cc:117-142):
-// the rows' 12 decision bits are kept for 2E + 1 rows and ANDed down the
+// the rows' decision bits are kept for 2E + 1 rows and ANDed down the
 // column, then across the lane's and its neighbours' columns. A warp row goes
 // only as far as it must: the lower 2^-4 bound alone where no window of the
 // row may be signal; both 2^-4 bounds; both 2^-8 bounds where a window lies
@@ -284,7 +283,7 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
                      r.pair_byte;
   const int bytes_left = r.bytes_per_row - r.pair_byte;
   // The last 2E + 1 rows' decision bits and the last E + 1 rows' masked bits,
-  // 12 bits a row in 16-bit halves, the newest lowest.
+  // a bit a column in 16-bit halves, the newest lowest.
   uint32_t dec[4] = {0u, 0u, 0u, 0u}, msk[2] = {0u, 0u};
   int large = 0;
   int s_cur = 0;  // the current row's slot
@@ -327,12 +326,12 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
       // Warp rows whose windows hold no masked pixel (most) take the whole
       // window's constants; the others look each window's count up.
       const bool uniform = !__any_sync(0xffffffffu, any_masked >> kCountShift) && large <= 0;
-      uint32_t sig = 0, masked12 = 0;
+      uint32_t sig = 0, masked_at = 0;
       if (!uniform) {
         uint32_t v[C];
         const int s_mid = s_cur >= K ? s_cur - K : s_cur + G::Slots - K;
         read_row<Pix, C, kLargePixel, false>(ring + s_mid * kStripStride<C>, lane, v);
-        masked12 = sign_bits<C>([&](int c) { return v[c]; });
+        masked_at = sign_bits<C>([&](int c) { return v[c]; });
       }
       if constexpr (k16) {
         if (uniform) {
@@ -413,9 +412,9 @@ ext_strip(const __grid_constant__ FramePtrs F, int nframes, const __grid_constan
 #pragma unroll
       for (int k = 3; k > 0; k--)
         dec[k] = __funnelshift_l(dec[k - 1], dec[k], 16);
-      dec[0] = dec[0] << 16 | sig | masked12;
+      dec[0] = dec[0] << 16 | sig | masked_at;
       msk[1] = __funnelshift_l(msk[0], msk[1], 16);
-      msk[0] = msk[0] << 16 | masked12;
+      msk[0] = msk[0] << 16 | masked_at;
       if (i >= 2 * K + 2 * E) {  // warp-uniform
         uint32_t col = dec[0];
 #pragma unroll
@@ -768,9 +767,14 @@ ExtTables make_ext_tables(const LaunchParams &P) {
 // the lattice decides a ninth of the windows and the tiles that hold a
 // candidate: 32 frames of 4362 x 4148 take 0.95 ms so and 1.38 ms on strips.
 // Launches of up to kStripPixels take strips, narrow ones that size (sf_strips.cuh):
-// there the lattice's two more launches cost more than they save (both ways, called
-// directly: one frame of 1065 x 1030 55 and 43 us, 4 of 1024 x 1024 60 and 45, 2 of
-// 2162 x 2068 57 and 56; in a captured graph: 37 and 32, 41 and 42, 50 and 56).
+// there the lattice's two more launches cost more than they save. In a captured graph,
+// us on the lattice and on strips: one frame of 1065 x 1030 35 and 29, 2 of 1024 x 1024
+// 37 and 35, 3 and 4 of them 37 and 37, 39 and 41, one of 2162 x 2068 39 and 39, of 2400
+// x 2400 43 and 46; the last two with a tenth of the pixels masked 45 and 39, 51 and 49,
+// with a fiftieth overloaded 109 and 103, 133 and 135, 16-bit 36 and 37, 39 and 41. Frames
+// with few large pixels (1 in 2000) would be better off on the lattice from 2 million
+// pixels on (39 and 49, at one of 2162 x 2068 47 and 61): a strip's whole row is summed
+// again for one.
 constexpr long long kStripPixels = 5000000;
 bool lattice_path(const FramePtrs &F, int nframes, int pixel_bytes, const LaunchParams &P) {
   if (P.half != 3 || P.algorithm != SF_DISPERSION_EXTENDED)

@@ -346,7 +346,7 @@ lat_stage01(const __grid_constant__ FramePtrs F, int nframes,
 // The candidates, the decisions and the erosion are a row a lane. Tiles share
 // mask words, so the clearing is an atomic AND; each candidate belongs to one
 // tile, so the order does not matter. Bound by issue (64% of its rate, 820
-// instructions a tile): 32 frames of 4362 x 4148 take 297 us, 148 of 16 bits, 4
+// instructions a tile): 32 frames of 4362 x 4148 take 297 us, 16 of 16 bits 148, 4
 // dense ones 621; with a lane a column for the windows too, each lane taking its
 // column's needed ones in turn (11 rounds a tile, 12 lanes in them), and the
 // erosion a row after another in every lane, 449, 250 and 967 us.
@@ -382,9 +382,9 @@ template <typename Pix> struct alignas(128) TileBuf {
 };
 
 template <typename Pix> struct alignas(128) VerWarp {
-  TileBuf<Pix> pix[1];                   // staged pixels (the next tile's load goes out
+  TileBuf<Pix> pix;                      // staged pixels (the next tile's load goes out
                                          // once the current one's are read)
-  uint64_t bar[1];                       // its TMA mbarrier
+  uint64_t bar;                          // its TMA mbarrier
   uint32_t cw[2][kVerRows][2];           // the tile's candidate words, two tiles (s)
   alignas(16) uint2 vs[kVerDR][kVerPC + 2];  // column sums of 7 rows
   // Masked centres, a word a column (column i's at i + 1, so that a lane's four
@@ -394,8 +394,8 @@ template <typename Pix> struct alignas(128) VerWarp {
   alignas(8) uint16_t vh[sizeof(Pix) == 4 ? kVerDR : 1][kVerPC + 2];
 };
 
-// The frames' 2-D tensor maps, boxes of one tile (kPW x 18 pixels), for the
-// TMA staging of the exact check and stage 2.
+// The frames' 2-D tensor maps, boxes of one tile (kPW x 18 pixels), for the TMA
+// staging of the exact check.
 struct TileMaps {
   CUtensorMap map[kMaxBatch];
   unsigned long long mapped;  // bit f: frame f has a map (else its tiles are staged per lane)
@@ -514,11 +514,10 @@ lat_tiles(const __grid_constant__ FramePtrs F, int nframes, int env_h, int env_w
   }
 }
 
-// Copies listed tile e's pixels and candidate words into buffer s (pieces
-// off the frame are written as masked pixels / zero words).
 // Copies a tile's pixel rows (r0 - 5 .. r0 + 12, the staged columns from xs)
-// into pix (pieces off the frame are written as masked pixels). 16-bit frames
-// come here only when 4 | width and they are 8-byte aligned.
+// into pix (pieces off the frame are written as masked pixels), for frames
+// without a tensor map. 16-bit frames come here only when 4 | width and they are
+// 8-byte aligned.
 template <typename Pix>
 __device__ __forceinline__ void stage_pixels(Pix (*pix)[VerPix<Pix>::kPW], const Pix *image,
                                              int height, int width, int r0, int xs,
@@ -615,9 +614,9 @@ __device__ __forceinline__ void ver_stage(VerWarp<Pix> &sm, int s, uint32_t e, c
   const int xs = tile_xs<Pix>(c0);
   __syncwarp();  // every lane is done with the pixel buffer
   if (M.has(f))
-    tma_stage<Pix>(sm.pix[0], &sm.bar[0], M, f, r0, xs, lane);
+    tma_stage<Pix>(sm.pix, &sm.bar, M, f, r0, xs, lane);
   else
-    stage_pixels<Pix>(sm.pix[0].px, reinterpret_cast<const Pix *>(F.image[f]), height, width, r0,
+    stage_pixels<Pix>(sm.pix.px, reinterpret_cast<const Pix *>(F.image[f]), height, width, r0,
                       xs, lane);
   if (lane < 2 * kVerRows) {
     const int o = lane >> 1, wdx = (c0 >> 5) + (lane & 1);
@@ -734,7 +733,7 @@ __device__ __noinline__ uint32_t ver_wide_columns(VerWarp<uint32_t> &sm, int off
     unsigned long long cq = 0;
 #pragma unroll
     for (int r = 0; r < kVerPR; r++) {
-      const uint32_t v = sm.pix[0].px[r][off + i];
+      const uint32_t v = sm.pix.px[r][off + i];
       const bool m = is_masked_px<uint32_t>(v);
       masked |= m ? 1u << r : 0u;
       u[r] = m ? 0u : v;
@@ -821,11 +820,11 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   VerWarp<Pix> &sm = warps[warp];
   if (lane == 0) {
-    mbar_init(&sm.bar[0], 1);
+    mbar_init(&sm.bar, 1);
     mbar_init_fence();
   }
   __syncthreads();
-  uint32_t parity = 0;  // bit b: the phase the next wait on bar[b] waits for
+  uint32_t parity = 0;  // the phase the next wait on bar waits for
   // Tile numbers are laid out over the batch's largest frame.
   const int ntx = ver_ntx(env_w);
   const uint32_t ntiles = (uint32_t)ntx * (uint32_t)ver_nty(env_h);
@@ -857,7 +856,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
     const int height = F.h[f], width = F.w[f], wpr = (width + 31) >> 5;
     if (inflight) {
       inflight = false;
-      if (!tma_landed<Pix>(sm.pix[0], &sm.bar[0], parity & 1u, height, width, r0,
+      if (!tma_landed<Pix>(sm.pix, &sm.bar, parity, height, width, r0,
                            tile_xs<Pix>(c0), lane)) {
         if (lane == 0)
           atomicOr(counters + kCtrFault, 1u);
@@ -902,7 +901,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
       uint32_t ns[kVerPR], q[kVerPR], mk = 0, mx = 0;
 #pragma unroll
       for (int r = 0; r < kVerPR; r++) {
-        const uint32_t v = sm.pix[0].px[r][col];
+        const uint32_t v = sm.pix.px[r][col];
         if (!k16)
           mx = max(mx, v + 2u);
         ns[r] = is_masked_px<Pix>(v) ? (1u << kLatPS) : v;
@@ -975,7 +974,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
         if constexpr (!k16)
           for (int c = 0; c < kVerGroup; c++)
             if (nd >> c & 1u)
-              sig |= lat_wide(sm.pix[0].px, d, off + kVerGroup * j + c, P) ? 1u << c : 0u;
+              sig |= lat_wide(sm.pix.px, d, off + kVerGroup * j + c, P) ? 1u << c : 0u;
       } else if (clean) {
         sig = ver_group<true>(sm, d, j, nd, tab, P);
       } else {
@@ -1017,7 +1016,7 @@ lat_verify(const __grid_constant__ FramePtrs F, const __grid_constant__ TileMaps
   }
   // After a fault: the load still in flight (bounded) before the buffer goes.
   if (inflight)
-    (void)mbar_wait(&sm.bar[0], parity & 1u);
+    (void)mbar_wait(&sm.bar, parity);
   cp_async_wait<0>();
 }
 

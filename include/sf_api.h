@@ -250,10 +250,9 @@ int sf_threshold_u16_batch_device(const uint16_t *const *d_images, size_t n_fram
  * the largest width): frame j's list at d_out + j * capacity, its count at
  * d_counts[j], its mask at d_bits + j * sf_mixed_batch_mask_words(...) (=
  * ceil(W/32) * H words) in its own rows of ceil(widths[j]/32) words, the
- * optional word positions likewise. For 32-bit frames with the reference's
- * window (kernel 3,3, dispersion_extended, gain 1, integral sigmas) the
- * whole batch is one launch sequence; other settings run frames of another
- * shape one launch sequence each. The workspace is
+ * optional word positions likewise. The whole batch is one launch sequence
+ * (but for negative gains and sigmas, and constants beyond the integer tests,
+ * which take the frames one by one). The workspace is
  * sf_mixed_batch_workspace_bytes (the batch workspace of the envelope).
  */
 size_t sf_mixed_batch_workspace_bytes(size_t n_frames, const size_t *heights,
