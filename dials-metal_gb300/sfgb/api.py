@@ -437,9 +437,9 @@ MAX_BATCH = 64
 class MixedBatch:
     """Batched device threshold of frames of different shapes
     (sf_threshold_u32_mixed_batch_device): up to MAX_BATCH 32-bit frames in
-    HBM per call, each with its own shape, one launch sequence on the
-    reference's window; each frame's list, mask and count as a single-frame
-    call gives. Outputs are laid out for the batch's envelope."""
+    HBM per call, each with its own shape, in one launch sequence; each
+    frame's list, mask and count as a single-frame call gives. Outputs are
+    laid out for the batch's envelope."""
 
     def __init__(self, shapes, capacity: int | None = None, params: Params | None = None,
                  word_prefix: bool = False):
